@@ -449,8 +449,8 @@ int ogr_route_pass(const ogr_graph* g, const ogr_state* st, const ogr_net_table*
  * 8219-8262, into find_path_roi :2451-2548 with roi_nodes = all nodes).  Same
  * result, statistics and status codes as ogr_find_path with
  * net->full_graph = 1, computed by one cooperative launch on all SMs.  The
- * workspace (about 108 bytes per node + 4 per arc) is initialised once with
- * ogr_full_workspace_init; a search rewrites the 8-byte key word of every
+ * workspace (about 110 bytes per node + 4 per arc) is initialised once with
+ * ogr_full_workspace_init; a search rewrites the 16-byte record of every
  * node and otherwise touches only the nodes it reaches.
  * OGR_ERR_TIMEOUT: a grid barrier gave up (not expected; the launch is
  * sized so every CTA is resident).  Synchronises. */
@@ -483,25 +483,24 @@ int ogr_find_path_full_multi(const ogr_graph* g, const ogr_state* st, const ogr_
                              int32_t* path_len_out, int64_t* stats, void* stream);
 
 /* Grid of the whole-lattice search on the current device (a tuning knob;
- * results do not depend on it): ctas > 0 sets the number of cooperative CTAs
- * (at most *limit = SMs x resident CTAs per SM), 0 only reads.  *current and
- * *limit (host, may be NULL) receive the grid in use and the maximum.  The
- * setting is per device and per host thread.  Chosen by the autotuner
- * (orthoroute_gb300/autotune.py); no reference counterpart. */
+ * results do not depend on it): ctas > 0 sets the number of cooperative CTAs,
+ * 0 only reads.  *limit (host, may be NULL) receives the maximum, one per SM
+ * (a CTA's shared memory holds its part of the frontier); up to twice that
+ * may be asked for and runs as the maximum.  *current (may be NULL) receives
+ * the grid in use.  The setting is per device and per host thread.  Chosen by
+ * the autotuner (orthoroute_gb300/autotune.py); no reference counterpart. */
 int ogr_full_grid(int32_t ctas, int32_t* current, int32_t* limit);
 
 /* Lanes per examined frontier node of the whole-lattice search (4, 8 or 16;
- * default 16) for searches launched afterwards; 0 only reads.  A tuning
- * knob (results do not depend on it), per host thread (each job of a
- * server routes in its own thread), chosen by the
- * autotuner; no reference counterpart. */
+ * default 16); 0 only reads.  Kept per host thread for callers that set it;
+ * the search fits its lanes to the lattice's rows itself.  Results do not
+ * depend on it; no reference counterpart. */
 int ogr_full_lanes(int32_t lanes, int32_t* current);
 
-/* Whether the whole-lattice search keeps the last pull of a carried frontier
- * node none of whose in-neighbours settled since (mode 1) or pulls every
- * frontier node every phase (0, default); -1 only reads.  A tuning knob
- * (results do not depend on it), per host thread, chosen by the autotuner; no
- * reference counterpart. */
+/* Whether the whole-lattice search may keep the last pull of a carried
+ * frontier node (mode 1) or not (0, default); -1 only reads.  Kept per host
+ * thread for callers that set it; results do not depend on it; no reference
+ * counterpart. */
 int ogr_full_reuse(int32_t mode, int32_t* current);
 
 /* Engine of the whole-lattice search for searches launched afterwards:

@@ -1,0 +1,102 @@
+"""The phase-settled search (csrc/phases.cuh) at the edges of its forms, against the oracle's heap search, paths and
+heap statistics alike (whole numbers: equal or wrong).
+
+* rows of up to 4, 8, 16 and 32 arcs have forms of their own, longer rows the general one;
+* costs, penalties and seed costs that 2^-30 ticks cannot hold (below 2^-7, 2^22 and more, labels above 2^22) are
+  searched in doubles;
+* one CTA (every entry local), three CTAs and every SM (surplus entries dealt out).
+"""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from oracle.dijkstra import find_path_multisource, find_path_roi_c
+
+from test_gpu_kernels import make
+
+ROWS = {                      # longest row: lattice
+    4: ((40, 33, 4), {}), 6: ((31, 30, 6), {}), 8: ((33, 27, 8), {}), 10: ((23, 19, 8), {"wrong_way_cost_multiplier": 3.0}),
+    16: ((17, 13, 16), {}), 22: ((13, 11, 22), {"allow_any_layer_via": True}),
+    40: ((9, 8, 40), {"allow_any_layer_via": True}),
+}
+
+
+def values(kind, E, rng):
+    if kind == "ticks":
+        return (0.12 + rng.random(E) * 0.05).astype(np.float32)
+    if kind == "ties":        # many equal float32 keys, some arcs blocked
+        c = (0.125 + rng.integers(0, 3, size=E) * 0.125).astype(np.float32)
+        c[rng.random(E) < 0.05] = np.float32("inf")
+        return c
+    if kind == "small":       # below 2^-7: off the tick grid
+        return (0.001 + rng.random(E) * 0.004).astype(np.float32)
+    if kind == "some small":  # a few off-grid costs, met on the way
+        c = (0.12 + rng.random(E) * 0.05).astype(np.float32)
+        c[rng.random(E) < 0.002] = np.float32(0.0031)
+        return c
+    c = (3.0e5 + rng.random(E) * 3.0e5).astype(np.float32)      # "large": labels pass 2^22
+    c[rng.random(E) < 0.01] = np.float32(5.0e6)
+    return c
+
+
+def check(g, s, ops, ref, costs, rng, pen_scale, n=3):
+    s.total_cost.copy_(torch.from_numpy(costs))
+    ident = np.arange(g.N, dtype=np.int32)
+    pen = None
+    if pen_scale:
+        hist = np.where(rng.random(g.N) < 0.1, rng.random(g.N) * pen_scale, 0.0).astype(np.float32)
+        s.node_history.copy_(torch.from_numpy(hist))
+        pen = (hist * np.float32(5.0)).astype(np.float32)
+    for _ in range(n):
+        src, dst = (int(v) for v in rng.integers(0, ref.plane, size=2))
+        st = {}
+        want = find_path_roi_c(ref.indptr, ref.indices, src, dst, costs, ident, ident, node_penalty=pen, stats=st)
+        ops.stats.zero_()
+        got = ops.find_path(ops.net_args(7, src, dst, full_graph=True, penalty=pen is not None), engine="grid")
+        assert got == want, (src, dst)
+        if src != dst:
+            assert ops.stats.cpu().tolist()[:2] == [st["scanned"], st["settled"]], (src, dst)
+
+
+@pytest.mark.parametrize("row", sorted(ROWS))
+@pytest.mark.parametrize("kind", ["ticks", "ties", "small", "some small", "large"])
+def test_forms_match_oracle(row, kind):
+    dims, kw = ROWS[row]
+    g, s, ops, ref = make(*dims, **kw)
+    assert int(np.diff(ref.indptr).max()) <= row
+    rng = np.random.default_rng(row * 10 + len(kind))
+    # penalties on the tick grid, then (off the grid) around 2^-7
+    for pen_scale in (0.0, 2.0, 0.002):
+        check(g, s, ops, ref, values(kind, g.E, rng), rng, pen_scale)
+
+
+@pytest.mark.parametrize("ctas", [1, 2, 3, 0])
+@pytest.mark.parametrize("kind", ["ties", "some small"])
+def test_team_sizes_match_oracle(ctas, kind):
+    """A frontier larger than its CTA's places and uneven shares; 0 = every SM."""
+    from orthoroute_gb300.autotune import full_grid
+    g, s, ops, ref = make(260, 210, 4)
+    rng = np.random.default_rng(17)
+    before, limit = full_grid(0)
+    try:
+        full_grid(ctas or limit)
+        check(g, s, ops, ref, values(kind, g.E, rng), rng, 1.0, n=2)
+    finally:
+        full_grid(before)
+
+
+@pytest.mark.parametrize("seed_costs", [(0.0, 0.25, 1.5), (0.1, 0.30000001, 1e-9), (0.0, 5.0e6, 0.5)])
+def test_seed_costs_match_oracle(seed_costs):
+    g, s, ops, ref = make(30, 26, 6)
+    rng = np.random.default_rng(5)
+    costs = values("ties", g.E, rng)
+    s.total_cost.copy_(torch.from_numpy(costs))
+    ident = np.arange(g.N, dtype=np.int32)
+    net = ops.net_args(0, 0, 1, full_graph=True, penalty=False)
+    for _ in range(4):
+        seeds = [(int(n), c) for n, c in zip(rng.choice(g.N, size=3, replace=False), seed_costs)]
+        targets = [(int(n), float(c)) for n, c in zip(rng.choice(g.N, size=4, replace=False), rng.random(4))]
+        want = find_path_multisource(ref.indptr, ref.indices, seeds, targets, costs, ident, ident, plane=ref.plane)
+        assert ops.find_path_full_multi(seeds, targets, net) == (tuple(want) if want else None)
