@@ -257,7 +257,7 @@ typedef struct {
   int32_t penalty_enabled;     /* 0: no node penalty at all                   */
 } ogr_net_args;
 
-/* Per-search scratch (one "slot"): about 70 bytes per lattice node.  It must
+/* Per-search scratch (one "slot"): about 68 bytes per lattice node.  It must
  * be initialised once with ogr_route_workspace_init; every search leaves it
  * initialised again.  Two searches must not share a slot concurrently. */
 size_t ogr_route_workspace_bytes(int32_t num_nodes);
@@ -401,7 +401,7 @@ typedef struct {
 
 /* Batched disjoint-ROI windows for the ROI nets of a pass.  Consecutive ROI
  * nets whose footprints (the ROI's box and the box of the net's old path) are
- * pairwise disjoint are ripped up and searched together, one CTA each, in one
+ * pairwise disjoint are ripped up and searched together, a team of CTAs each, in one
  * cooperative launch; they then commit in order.  A net whose ROI search
  * fails ends its window: the later nets' rip-ups are undone and it takes its
  * fallback in order.  The results are those of the sequential pass.
@@ -436,8 +436,8 @@ int ogr_bfs_workspace_init(void* workspace, int32_t num_nodes, int64_t qcap, int
  * order_full (HOST uint8[count], may be NULL) marks the entries of `order`
  * that are full-graph nets; each of those is searched by the whole-lattice
  * search (ogr_find_path_full) in full_workspace, the ROI nets between them by
- * single-CTA launches, in the same order.  With order_full NULL every net,
- * long or not, is searched by the single-CTA pass. */
+ * launches of their own, in the same order.  With order_full NULL every net,
+ * long or not, is searched in the pass of the ROI nets. */
 int ogr_route_pass(const ogr_graph* g, const ogr_state* st, const ogr_net_table* t,
                    const ogr_pass_args* pa, const ogr_roi_batch* rb, void* workspace,
                    size_t workspace_bytes, const uint8_t* order_full, void* full_workspace,
@@ -527,10 +527,10 @@ int ogr_full_tile(int32_t enable, double delta, int32_t tx, int32_t ty, int32_t*
  * evaluations; ns of first sweeps.  Synchronous. */
 int ogr_tile_profile(int64_t* out24, int32_t reset);
 
-/* Lanes per node of the single-CTA ROI search (2, 4, 8 or 16; default 4) for
- * every search launched afterwards; 0 only reads.  *current (host, may be
- * NULL) receives the setting.  A tuning knob (results do not depend on it),
- * per host thread, chosen by the autotuner; no reference counterpart. */
+/* Lanes per node of the ROI search (2, 4, 8 or 16; default 4); 0 only reads.
+ * Kept per host thread for callers that set it; the search fits its lanes to
+ * the lattice's rows itself.  Results do not depend on it; no reference
+ * counterpart. */
 int ogr_search_lanes(int32_t lanes, int32_t* current);
 
 /* How many clashing nets a disjoint-ROI window of ogr_route_pass may skip
@@ -561,20 +561,21 @@ int ogr_debug_limits(int32_t barrier_spin, int32_t max_phases, int32_t* cur_spin
  * backtrace ns of CTA 0.  Synchronous. */
 int ogr_full_profile(int64_t* out8, int32_t reset);
 
-/* Tracing: cumulative per-stage cycle counters of all searches on the
- * current device since the last reset (host int64[16]: BFS, compaction,
- * search init, queueing, recompute, frontier min, settle, statistics and
- * backtrace, cleanup; then searches, settle phases, BFS waves, ROI nodes,
- * recomputed nodes).  Synchronous. */
+/* Tracing: cumulative per-stage cycle counters of all ROI searches on the
+ * current device since the last reset, taken by each team's first thread (host
+ * int64[16]: BFS, compaction, search init, phases, of these waiting for the
+ * team, 0, 0, statistics and backtrace, cleanup; then searches, settle
+ * phases, BFS waves, ROI nodes, entries examined, ROIs taken from the batched
+ * extraction).  Synchronous. */
 int ogr_search_profile(int64_t* out16, int32_t reset);
 
 /* Allocation-free variant of ogr_find_path.  It has no counterpart in the
  * reference: it exists for callers that cannot allocate device memory for a
  * workspace (a plugin inside an application that owns the device allocator,
  * or a serving process whose memory budget is fixed at start-up).  Its
- * scratch is a fixed array inside the library (36 MB: about 76 bytes per
- * node for OGR_NOALLOC_MAX_NODES nodes plus a 16 MB local adjacency, resident on each GPU that loads the library
- * until exit), so lattices above OGR_NOALLOC_MAX_NODES nodes are refused with
+ * scratch is a fixed array inside the library (18 MB: about 68 bytes per
+ * node for OGR_NOALLOC_MAX_NODES nodes, resident on each GPU that loads the
+ * library until exit), so lattices above OGR_NOALLOC_MAX_NODES nodes are refused with
  * OGR_ERR_CAPACITY.  The first call on a device looks up that array's device
  * address and keeps it for the process; make it before any stream capture,
  * and do not call this entry point again after resetting that device

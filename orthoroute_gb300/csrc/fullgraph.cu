@@ -55,8 +55,7 @@ struct FWs {
   int32_t* par;              // winning in-neighbour of a settled node
   int32_t* claim;
   float* rcost;              // reverse-arc cost gather when the state carries none
-  int4* ov;                  // three surplus lists
-  int64_t ov_stride;
+  int4* ov[2];               // surplus lists
   unsigned bar_spin;         // barrier spin bound
   int32_t max_phases;        // > 0: cap on settle phases (else 2N + 4)
   FCtl* ctl;
@@ -81,8 +80,7 @@ size_t fws_layout(int32_t N, int64_t E, char* base, FWs* w) {
   t.par = (int32_t*)take(4 * n);
   t.claim = (int32_t*)take(4 * n);
   t.rcost = (float*)take(4 * (size_t)E);
-  t.ov_stride = (int64_t)(r256(16 * n) / 16);
-  t.ov = (int4*)take(3 * r256(16 * n));
+  for (int i = 0; i < 2; ++i) t.ov[i] = (int4*)take(16 * n);
   t.tile = take(ogr_tile::workspace_bytes(N));
   t.mseed = (double*)take(8 * n);
   t.mtgt = (double*)take(8 * n);
@@ -162,8 +160,8 @@ full_sssp_kernel(ogr_graph g, ogr_state st, ogr_full::Job job, FWs w) {
   pr.rec = w.rec;
   pr.par = w.par;
   pr.claim = w.claim;
-  pr.ov = w.ov;
-  pr.ov_stride = w.ov_stride;
+  pr.ov[0] = w.ov[0];
+  pr.ov[1] = w.ov[1];
   pr.mseed = w.mseed;
   pr.mtgt = w.mtgt;
   pr.none = kNoTerm;
@@ -205,10 +203,11 @@ full_sssp_kernel(ogr_graph g, ogr_state st, ogr_full::Job job, FWs w) {
       arrive(pr, sm, k0, kArrive, ~(unsigned long long)md);
       await(pr, sm, k0);
       sm.res[2] = (int)sm.t;
+      const bool in_ticks = fix && (int)sm.t <= kMaxRow;
       if (leader && attempt) clear_slot(pr, k0 + 3);
       if (leader && !kMulti) {
         w.claim[src] = pr.sid;
-        w.ov[0] = make_int4(src, indptr[src], indptr[src + 1] - indptr[src], __float_as_int(0.0f));
+        w.ov[0][0] = make_int4(src, indptr[src], indptr[src + 1] - indptr[src], __float_as_int(0.0f));
         nf0 = 1;
         t0 = 0ull;
       } else if (leader) {
@@ -233,9 +232,9 @@ full_sssp_kernel(ogr_graph g, ogr_state st, ogr_full::Job job, FWs w) {
           const float pen = ogr_node_penalty(st, a, s0);
           w.claim[s0] = pr.sid;
           w.rec[s0].sp = 1;
-          w.ov[nf0++] = make_int4(s0, indptr[s0], indptr[s0 + 1] - indptr[s0], __float_as_int(pen));
+          w.ov[0][nf0++] = make_int4(s0, indptr[s0], indptr[s0 + 1] - indptr[s0], __float_as_int(pen));
           unsigned long long lb = ogr_dbits(sc + (double)pen);
-          if (fix) {
+          if (in_ticks) {
             lb = 0ull;
             if (seed_ticks(sc, &lb) && tick_finite(pen)) lb += ticks(pen);
           }
@@ -261,13 +260,14 @@ full_sssp_kernel(ogr_graph g, ogr_state st, ogr_full::Job job, FWs w) {
     const int ok = sm.ok, max_deg = sm.res[2];
     __syncthreads();
     ++k0;
+    if (max_deg > kMaxRow) fix = false;
     if (ok != 1) {
       o.status = ok == 0 ? OGR_ERR_TIMEOUT : OGR_ERR_ARG;
       o.phases = 0;
       k0 += 1;
       break;
     }
-    o = run_search<L, K, kMulti, false>(pr, smem_raw, k0, max_deg, !fix);
+    o = run_search<L, K, kMulti, false>(pr, smem_raw, k0, max_deg, fix);
     k0 += o.phases;
     if (o.status != kStInexact) break;
     fix = false;
@@ -419,17 +419,6 @@ const void* kernel_for(int row, bool multi) {
                      : (const void*)full_sssp_kernel<16, 2, false>;
 }
 
-// As many arcs as a row of the lattice's inner layers has.  The outermost
-// layer has few arcs or none, so the average over the others comes near the
-// longest row (600x400x12, spans up to 4: 8.0, longest 10; 300x200x8: 7.7,
-// longest 8; 1000x800x32: 3.9, longest 4).  A lattice whose rows are longer
-// all the same is still searched right (run_search).
-int row_for(const ogr_graph& g) {
-  const double n = (double)(g.num_nodes > 0 ? g.num_nodes : 1), z = (double)(g.nz > 1 ? g.nz : 2);
-  const double inner = (double)g.num_edges / n * z / (z - 1.0);
-  return inner <= 3.95 ? 4 : inner <= 7.75 ? 8 : inner <= 16.0 ? 16 : 32;
-}
-
 int size_grid(int dev) {
   if (g_grid_limit[dev] == 0) {
     int sms = 0, coop = 0;
@@ -452,6 +441,23 @@ int size_grid(int dev) {
 }  // namespace
 
 namespace ogr_full {
+
+// As many arcs as a row of the lattice's inner layers has.  The outermost
+// layer has few arcs or none, so the average over the others comes near the
+// longest row (600x400x12, spans up to 4: 8.0, longest 10; 300x200x8: 7.7,
+// longest 8; 1000x800x32: 3.9, longest 4).  A lattice whose rows are longer
+// all the same is still searched right (run_search).
+int row_for(const ogr_graph& g) {
+  const double n = (double)(g.num_nodes > 0 ? g.num_nodes : 1), z = (double)(g.nz > 1 ? g.nz : 2);
+  const double inner = (double)g.num_edges / n * z / (z - 1.0);
+  return inner <= 3.95 ? 4 : inner <= 7.75 ? 8 : inner <= 16.0 ? 16 : 32;
+}
+
+int grid_blocks() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+  return size_grid(dev) == OGR_OK ? g_grid_blocks[dev] : 0;
+}
 
 size_t workspace_bytes(int32_t num_nodes, int64_t num_edges) {
   return fws_layout(num_nodes, num_edges, nullptr, nullptr);
@@ -487,7 +493,7 @@ int launch(const ogr_graph& g, const ogr_state& st, const Job& job, void* ws, cu
   ogr_graph gv = g;
   ogr_state sv = st;
   void* args[] = {&gv, &sv, &jv, &w};
-  const void* fn = kernel_for(row_for(g), job.multi != 0);
+  const void* fn = kernel_for(ogr_full::row_for(g), job.multi != 0);
   OGR_CUDA_TRY(cudaLaunchCooperativeKernel(fn, dim3(g_grid_blocks[dev]), dim3(kThreads), args, kSmemBytes, s));
   return OGR_OK;
 }

@@ -34,6 +34,13 @@ struct Job {
 
 size_t workspace_bytes(int32_t num_nodes, int64_t num_edges);
 
+// The row length (4, 8, 16 or 32 arcs) whose form of the search fits lattice g.
+int row_for(const ogr_graph& g);
+
+// CTAs that this host thread's cooperative searches take on the current device
+// (ogr_full_grid), 0 on an error.
+int grid_blocks();
+
 // Device int32[4] the search writes: status, path length, phases, 0.
 int32_t* result_words(void* ws, int32_t num_nodes, int64_t num_edges);
 

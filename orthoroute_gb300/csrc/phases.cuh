@@ -158,8 +158,7 @@ struct Problem {
   int32_t* par;
   int32_t* claim;                  // == sid: the node has its entry
   int32_t sid;
-  int4* ov;                        // three surplus lists of {node, row start, row length, penalty},
-  int64_t ov_stride;               // ov_stride entries apart
+  int4* ov[2];                     // surplus lists of {node, row start, row length, penalty}, by phase
   const double* mseed;             // multi-source: seed cost / target cost per node, `none` bits elsewhere
   const double* mtgt;
   unsigned long long none;
@@ -382,7 +381,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
         slot = idx < ncarr ? bd.carr[q][idx] : bd.fresh[q][idx - ncarr];
         en = bd.ent[slot];
       } else if (valid) {
-        en = __ldcg(&pr.ov[b3 * pr.ov_stride + pr.rank + (int64_t)(idx - nloc) * pr.nranks]);
+        en = __ldcg((q ? pr.ov[1] : pr.ov[0]) + pr.rank + (int64_t)(idx - nloc) * pr.nranks);
       }
       const int32_t v = en.x, f0 = en.y, deg = en.z & 0x7fffffff;
       const bool unclaimed = en.z < 0;
@@ -589,7 +588,9 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
             }
           }
           bool push = false;
-          if (expand && (unsigned)r[j].sp < 2u) {      // settled nodes cannot improve
+          // open: not settled before this phase (whether it settles in this
+          // one must not matter: T is the same whatever the timing)
+          if (expand && r[j].sp >= 0 && (unsigned)(r[j].sp - 2) >= (unsigned)phase) {
             u64 ly = kNone;
             if (!kGen) {
               // (whoever reached u first checked its penalty)
@@ -637,7 +638,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
                 atomicAdd(&sm.nov_out, __popc(ms));
               }
               b = __shfl_sync(kAll, b, 0);
-              if (surplus) __stcg(&pr.ov[bn * pr.ov_stride + b + __popc(ms & below)], ne);
+              if (surplus) __stcg((q ? pr.ov[0] : pr.ov[1]) + b + __popc(ms & below), ne);
             }
           }
           f += L;
@@ -728,18 +729,22 @@ __device__ __noinline__ void run_rare(const Problem* ppr, char* smem, int k0, Ou
   *out = run_phases<L, K, kGen, kMulti, kRoi>(pr, sm, bd, k0);
 }
 
+// The longest row that is searched in ticks.
+constexpr int kMaxRow = 32;
+
 // The search with L lanes of K arcs per entry if the rows (of at most max_deg
-// arcs) allow it, else in the form that takes them (general: the general form).
+// arcs) allow it, else in the form that takes them; labels in ticks, or (only
+// and always in the general form) in doubles.
 template <int L, int K, bool kMulti, bool kRoi>
-__device__ __forceinline__ Outcome run_search(const Problem& pr, char* smem, int k0, int max_deg, bool general) {
-  if (!general && max_deg <= L * K) {
+__device__ __forceinline__ Outcome run_search(const Problem& pr, char* smem, int k0, int max_deg, bool in_ticks) {
+  if (in_ticks && max_deg <= L * K) {
     Head& sm = *reinterpret_cast<Head*>(smem);
     Body<L * K>& bd = *reinterpret_cast<Body<L * K>*>(smem + kHeadBytes);
     return run_phases<L, K, false, kMulti, kRoi>(pr, sm, bd, k0);
   }
   Outcome o;
   const Problem p = pr;
-  if (general || max_deg > 32)
+  if (!in_ticks)
     run_rare<16, 1, true, kMulti, kRoi>(&p, smem, k0, &o);
   else
     run_rare<32, 1, false, kMulti, kRoi>(&p, smem, k0, &o);

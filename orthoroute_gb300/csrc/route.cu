@@ -11,25 +11,11 @@
 // costs, so a routing pass extracts the ROIs of all its nets in parallel on
 // many SMs before the sequential part starts (roi_batch_kernel).
 //
-// Search (SimpleDijkstra.find_path_roi, :2451-2548): the reference pops
-// (label, roi_idx) from a heap of FP64 labels, and accepts a relaxation iff
-// float32(alt) < dist32[v] (numpy 2 compares a Python float with a float32
-// in float32).  Hence every node ends with the FIRST candidate, in pop order
-// of its relaxer, that reaches the minimal float32 value; its label is that
-// candidate's FP64 alt.  Equivalently, each node takes the lexicographic
-// minimum of (float32(alt), L(u), roi_idx(u)) over its relaxers u.
-// We settle nodes in phases (IN-criterion): with T = the smallest tentative
-// label, a node whose float32 key is below float32((T + cin) + pen) — cin
-// being its cheapest in-arc from an unsettled node — can no longer change,
-// and nodes whose label equals T are final as in Dijkstra.  Tentative states
-// are recomputed by pulling from all settled in-neighbours, which makes the
-// result independent of thread scheduling and bit-identical to the heap.
-//
-// Latency: before the phases, each search gathers an ROI-local adjacency
-// (neighbour's ROI index and the in-arc cost, 32 slots per node, one 128-byte
-// row) so a phase touches two dependent loads per arc instead of six; a
-// 16-lane group handles one node's arcs in parallel; node state is packed in
-// one 32-byte sector; the per-group key reduction uses shuffles.
+// Search (SimpleDijkstra.find_path_roi, :2451-2548): phases.cuh on the ROI's
+// nodes, by a team of CTAs.  One SM searched an ROI in phases of 11 to 22 us
+// (a few hundred to two thousand entries to examine in each); a team shares
+// them out, so a phase costs little more than its chain of round trips and
+// the team's barrier.
 //
 // ogr_route_pass runs the reference's per-net sequence (_route_all,
 // :7949-8449: rip-up, ROI search, one larger-ROI retry while the pass has
@@ -39,66 +25,51 @@
 
 #include "common.cuh"
 #include "fullgraph.cuh"
+#include "phases.cuh"
 
 namespace {
 
-constexpr int kThreads = 1024;
-constexpr int kWarps = kThreads / 32;
+using ogr_phase::kThreads;
+using ogr_phase::kWarps;
 constexpr int kSub = 16;                       // lanes per node (ROI BFS)
 constexpr int kGroups = kThreads / kSub;       // nodes in flight per CTA (ROI BFS)
-#ifndef OGR_SEARCH_LANES
-#define OGR_SEARCH_LANES 4
-#endif
-constexpr int kSearchLanes = OGR_SEARCH_LANES;  // default lanes per node of the ROI search
 
-// Lanes per node of the ROI search for the launches that follow (set by
-// ogr_search_lanes; the autotuner picks it per lattice).  Every searching
-// kernel exists for 2, 4, 8 and 16 lanes; results do not depend on the choice.
-thread_local int g_search_lanes = kSearchLanes;
+// Accepted and kept for callers (ogr_search_lanes); the search fits its lanes
+// to the lattice's rows, and results never depended on it.
+thread_local int g_search_lanes = 4;
 
 // Nets a disjoint-ROI window may skip over to take later disjoint ones
 // (ogr_window_lookahead; 0 = consecutive nets only).
 thread_local int g_window_look = 8;
 
-#define OGR_WITH_LANES(LV, ...)                                \
-  do {                                                         \
-    switch (g_search_lanes) {                                  \
-      case 2: { constexpr int LV = 2; __VA_ARGS__; } break;    \
-      case 8: { constexpr int LV = 8; __VA_ARGS__; } break;    \
-      case 16: { constexpr int LV = 16; __VA_ARGS__; } break;  \
-      default: { constexpr int LV = 4; __VA_ARGS__; } break;   \
-    }                                                          \
-  } while (0)
-constexpr int32_t ST_NONE = 0, ST_FRONT = 1, ST_DONE = 2, ST_SINK = 3;  // SINK: a settled target (multi-seed)
 constexpr int kMaxViaNodes = 4096;
-constexpr int kDMax = 32;                      // arcs per node the local adjacency holds
-constexpr int kAdjCap = 65536;                 // ROI nodes the local adjacency holds
 constexpr int kMaxSkip = 16;                   // nets a window may skip over (look-ahead)
+// CTAs of one ROI search.  More of them share a phase's entries but make its
+// barrier dearer.
+constexpr int kTeam = 16;
 
-struct __align__(32) NodeSt {
-  double lab;      // FP64 label (tentative until settled)
-  float m32;       // float32 key of the label
-  float pen;       // node penalty (fixed once reached)
-  float cin;       // cheapest in-arc cost from an unsettled ROI neighbour
-  int32_t par;     // ROI index of the winning relaxer
-  int32_t st;      // ST_NONE / ST_FRONT / ST_DONE
-  int32_t stamp;   // phase in which the node was last queued for recompute
+// Control words of one search slot, kept between searches (sid) or zero at
+// the start of each (team).
+struct SlotCtl {
+  ogr_phase::Ctl team;
+  int32_t sid;               // searches so far: the claim stamp
+  int32_t merr;              // multi-source: a bad or repeated seed / target
 };
-static_assert(sizeof(NodeSt) == 32, "NodeSt must fill one 32-byte sector");
 
+// A search slot: the ROI's node arrays, the global->ROI map, and (route
+// workspace only) the BFS.
 struct Ws {
   int32_t* seen;
   int32_t* g2r;
-  int32_t* q[4];
+  int32_t* q[4];             // BFS queues; the search's first surplus list lies over them
   int32_t* roi;
-  NodeSt* node;
-  int32_t* fr[2];
-  int32_t* dl;
-  int32_t* blist;
-  int32_t* adj;      // [kAdjCap][kDMax] neighbour ROI index or -1
-  float* acost;      // [kAdjCap][kDMax] cost of the arc neighbour -> node
-  int32_t* deg;      // [kAdjCap] arcs of the node
-  int64_t* result;   // [0] status, [1] path len
+  ogr_phase::Rec* rec;
+  int32_t* par;
+  int32_t* claim;
+  int4* ov[2];
+  SlotCtl* ctl;
+  char* win1;                // control block of a pass without windows
+  int64_t* result;           // [0] status, [1] path length, [2] fallbacks used, [3] ROI size
   int64_t qcap;
 };
 
@@ -112,17 +83,19 @@ struct MultiSeeds {
   const int32_t* targets;
   const double* target_cost;
   int32_t ntargets;
-  double* init;    // [R] seed cost before the node penalty, +inf for other nodes
-  double* tcost;   // [R] target cost, NaN for other nodes
+  double* init;    // [R] seed cost before the node penalty, kNoTerm bits for other nodes
+  double* tcost;   // [R] target cost, kNoTerm bits for other nodes
 };
+constexpr unsigned long long kNoTerm = 0x7ff8deadbeef0001ull;
 
 __host__ __device__ constexpr size_t round256(size_t v) { return (v + 255) & ~(size_t)255; }
-__host__ __device__ constexpr size_t min_sz(size_t a, size_t b) { return a < b ? a : b; }
 
-// Bytes of one search slot for n nodes.
+constexpr size_t kWin1Bytes = 4096;
+
+// Bytes of a route workspace for n nodes.
 __host__ __device__ constexpr size_t ws_bytes_for(size_t n) {
-  return 10 * round256(4 * n) + round256(32 * n) + 2 * round256(4 * min_sz(n, kAdjCap) * kDMax) +
-         round256(4 * min_sz(n, kAdjCap)) + round256(64);
+  return 5 * round256(4 * n) + 3 * round256(16 * n) + round256(sizeof(SlotCtl)) +
+         kWin1Bytes + round256(64);
 }
 
 __host__ inline size_t ws_layout(int32_t N, char* base, Ws* w) {
@@ -133,20 +106,18 @@ __host__ inline size_t ws_layout(int32_t N, char* base, Ws* w) {
     return p;
   };
   const size_t n = (size_t)N;
-  const size_t a = min_sz(n, kAdjCap);
   Ws t{};
   t.seen = (int32_t*)take(4 * n);
   t.g2r = (int32_t*)take(4 * n);
-  for (int i = 0; i < 4; ++i) t.q[i] = (int32_t*)take(4 * n);
   t.roi = (int32_t*)take(4 * n);
-  t.fr[0] = (int32_t*)take(4 * n);
-  t.fr[1] = (int32_t*)take(4 * n);
-  t.dl = (int32_t*)take(4 * n);
-  t.node = (NodeSt*)take(32 * n);
-  t.adj = (int32_t*)take(4 * a * kDMax);
-  t.acost = (float*)take(4 * a * kDMax);
-  t.deg = (int32_t*)take(4 * a);
-  t.blist = t.q[0];  // the BFS queues are free while the search runs
+  t.par = (int32_t*)take(4 * n);
+  t.claim = (int32_t*)take(4 * n);
+  t.rec = (ogr_phase::Rec*)take(16 * n);
+  t.ov[0] = (int4*)take(16 * n);
+  t.ov[1] = (int4*)take(16 * n);
+  for (int i = 0; i < 4; ++i) t.q[i] = (int32_t*)t.ov[0] + i * n;   // the queues are free while the search runs
+  t.ctl = (SlotCtl*)take(sizeof(SlotCtl));
+  t.win1 = take(kWin1Bytes);
   t.result = (int64_t*)take(64);
   t.qcap = (int64_t)n;
   if (w) *w = t;
@@ -156,27 +127,23 @@ __host__ inline size_t ws_layout(int32_t N, char* base, Ws* w) {
 // A search-only slot for the window pass: the global->ROI map and ROI-sized
 // arrays (the ROI comes from the batched extraction, so no BFS state).
 __host__ __device__ inline size_t ws_slot_layout(int32_t N, int32_t Rmax, char* base, Ws* w) {
+  const size_t n = (size_t)N, r = (size_t)Rmax;
+  const size_t sz[7] = {4 * n, 16 * r, 4 * r, 4 * r, 16 * r, 16 * r, sizeof(SlotCtl)};
+  char* p[7];
   size_t off = 0;
-  char* p[11];
-  const size_t n = (size_t)N, r = (size_t)Rmax, ad = min_sz(r, kAdjCap);
-  const size_t sz[11] = {4 * n, 32 * r, 4 * r, 4 * r, 4 * r, 4 * r, 4 * ad * kDMax, 4 * ad * kDMax, 4 * ad, 64, 0};
-  for (int i = 0; i < 10; ++i) {
+  for (int i = 0; i < 7; ++i) {
     p[i] = base ? base + off : nullptr;
     off += round256(sz[i]);
   }
   if (w) {
     Ws t{};
     t.g2r = (int32_t*)p[0];
-    t.node = (NodeSt*)p[1];
-    t.fr[0] = (int32_t*)p[2];
-    t.fr[1] = (int32_t*)p[3];
-    t.dl = (int32_t*)p[4];
-    t.blist = (int32_t*)p[5];
-    t.adj = (int32_t*)p[6];
-    t.acost = (float*)p[7];
-    t.deg = (int32_t*)p[8];
-    t.result = (int64_t*)p[9];
-    t.qcap = 0;
+    t.rec = (ogr_phase::Rec*)p[1];
+    t.par = (int32_t*)p[2];
+    t.claim = (int32_t*)p[3];
+    t.ov[0] = (int4*)p[4];
+    t.ov[1] = (int4*)p[5];
+    t.ctl = (SlotCtl*)p[6];
     *w = t;
   }
   return off;
@@ -206,41 +173,15 @@ __host__ __device__ inline BfsSlot bfs_slot_at(char* base, int32_t N, int64_t qc
   return s;
 }
 
-// ---- block primitives ------------------------------------------------------
-__device__ __forceinline__ unsigned long long block_min_u64(unsigned long long v, unsigned long long* s) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    unsigned long long y = __shfl_down_sync(0xffffffffu, v, o);
-    v = y < v ? y : v;
-  }
-  if (lane == 0) s[wid] = v;
-  __syncthreads();
-  if (wid == 0) {
-    unsigned long long w = (lane < kWarps) ? s[lane] : ~0ull;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      unsigned long long y = __shfl_down_sync(0xffffffffu, w, o);
-      w = y < w ? y : w;
-    }
-    if (lane == 0) s[0] = w;
-  }
-  __syncthreads();
-  unsigned long long r = s[0];
-  __syncthreads();
-  return r;
-}
-
-// Per-stage cycle counters of the search (a tracing aid, read with
-// ogr_search_profile): [0] BFS waves, [1] ROI compaction, [2] SSSP init and
-// local adjacency, [3] phase queueing, [4] recompute, [5] frontier min,
-// [6] settle, [7] statistics + backtrace, [8] cleanup, [9] searches,
-// [10] phases, [11] BFS waves run, [12] ROI nodes, [13] recomputed nodes,
-// [14] ROIs taken from the batched extraction.
+// Per-stage cycle counters of the ROI searches (a tracing aid, read with
+// ogr_search_profile; thread 0 of a team's first CTA): [0] BFS waves, [1] ROI
+// compaction, [2] search init, [3] phases, [4] of these waiting for the team,
+// [7] statistics + backtrace, [8] cleanup, [9] searches, [10] phases, [11] BFS
+// waves run, [12] ROI nodes, [13] entries examined, [14] ROIs taken from the
+// batched extraction.
 __device__ unsigned long long g_stage[16];
 
 struct Shared {
-  unsigned long long s_min[kWarps];
   int s_cnt[kWarps];
   int s_off[kWarps];
   int nq[4];
@@ -250,11 +191,8 @@ struct Shared {
   int bx0, bx1, by0, by1;
   int pos_src, pos_dst;
   int R;
-  int nfront, nnext, ndirty, nb;
   int status;
-  int found;
   int len;
-  int local;
 };
 
 struct StageClock {
@@ -366,7 +304,7 @@ __device__ void roi_build(Shared& sh, const ogr_graph& g, const ogr_net_args& a,
   __syncthreads();
   clk.mark(0);
   // Ordered compaction over the bounding box (ascending global id): each warp
-  // owns a contiguous segment; count, scan the 32 counts, then write.  Only
+  // owns a contiguous segment; count, scan the counts, then write.  Only
   // positions below out_cap are stored; those of src and dst are recorded.
   const int W = sh.bx1 - sh.bx0 + 1, H = sh.by1 - sh.by0 + 1;
   const int32_t area = W * H;
@@ -390,14 +328,14 @@ __device__ void roi_build(Shared& sh, const ogr_graph& g, const ogr_net_args& a,
   if (lane == 0) sh.s_cnt[warp] = cnt;
   __syncthreads();
   if (warp == 0) {
-    const int c = sh.s_cnt[lane];
+    const int c = lane < kWarps ? sh.s_cnt[lane] : 0;
     int x = c;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int y = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o) x += y;
     }
-    sh.s_off[lane] = x - c;
+    if (lane < kWarps) sh.s_off[lane] = x - c;
     if (lane == 31) sh.R = x;
   }
   __syncthreads();
@@ -451,523 +389,341 @@ __device__ void roi_build(Shared& sh, const ogr_graph& g, const ogr_net_args& a,
 }
 
 // ---- the search on a given ROI ---------------------------------------------------
-// roi[0..R) in ROI order (ignored when full).  Writes the path (global ids,
-// src first) to path_out and its length to sh.len, or a status to sh.status.
+// What a team searches: roi[0..R) in ROI order (= tie order); with full the
+// ROI is the whole lattice in id order.  The path (global ids, src first) goes
+// to path_out.
 //
-// With kMulti the search is the reference's multi-source multi-sink form: every
+// With ms the search is the reference's multi-source multi-sink form: every
 // seed starts with label seed_cost + penalty and no parent (a first relaxation
 // that later ones must beat in float32), targets are settled but never
 // expanded, the search runs until nothing is left, and the result is the
 // settled target with the least (label + target cost), first in pop order
 // (label, ROI index) among equals.
-//
-// kLanes lanes serve one node (its arcs, then a shuffle reduction), so a CTA
-// keeps 1024 / kLanes nodes in flight per round of a phase.
-// Arcs per lane that the local-adjacency stages of the ROI search load in one
-// batch: the first 12 arcs of a row (a lattice node has at most 10; at most 4
-// per lane, to stay in registers) are read at once, then the records they
-// name at once, so a row costs two dependent round trips instead of two per
-// kLanes arcs.  Slots past the degree lie in the row's 32-slot allocation and
-// are loaded but never used.
-constexpr int kBatchArcs = 12;
-static_assert(kBatchArcs <= kDMax, "a batch stays inside a local-adjacency row");
+struct RoiJob {
+  const ogr_graph* g;
+  const ogr_state* st;
+  const ogr_net_args* a;
+  const Ws* w;
+  const int32_t* roi;
+  int32_t R;
+  const float* roi_pen;      // ROI-local penalty, or NULL: the state's
+  const MultiSeeds* ms;
+  int32_t* path_out;
+  int32_t path_cap;
+  unsigned long long* stats;
+  int rank, nranks;
+};
 
-template <bool kMulti = false, int kLanes = kSearchLanes>
-__device__ void sssp_roi(Shared& sh, const ogr_graph& g, const ogr_state& st, const ogr_net_args& a, const Ws& w,
-                         const int32_t* roi, int32_t R, int32_t* path_out, int32_t path_cap,
-                         unsigned long long* stats_acc, StageClock& clk, const float* roi_pen = nullptr,
-                         const MultiSeeds* ms = nullptr) {
-  static_assert(kLanes == 2 || kLanes == 4 || kLanes == 8 || kLanes == 16 || kLanes == 32,
-                "lanes per node: a power of two from 2 to 32");
-  constexpr int kSub = kLanes;                  // shadows the BFS's lane count inside the search
-  constexpr int kGroups = kThreads / kLanes;
-  constexpr int kPerWarp = 32 / kLanes;
+// One team's search.  Every CTA of the team calls it with the slot's team
+// words zero; *status_out / *len_out are the result in the team's first CTA
+// (in the others the status lacks what the backtrace finds).
+template <int L, int K, bool kMulti>
+__device__ __noinline__ void roi_search(const RoiJob* jp, char* smem, int* status_out, int* len_out) {
+  using namespace ogr_phase;
+  const RoiJob job = *jp;
+  const ogr_graph& g = *job.g;
+  const ogr_state& st = *job.st;
+  const ogr_net_args& a = *job.a;
+  const Ws& w = *job.w;
+  Head& sm = *reinterpret_cast<Head*>(smem);
   const int tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5;
-  const int sl = tid & (kSub - 1), grp = tid / kSub;
-  const int32_t src = a.src, dst = a.dst;
-  const bool full = a.full_graph != 0;
-  const int32_t* __restrict__ indptr = g.indptr;
-  const int32_t* __restrict__ indices = g.indices;
-  NodeSt* __restrict__ node = w.node;
-  const float kInf = __int_as_float(0x7f800000);
-
-  if (!full)
-    for (int r = tid; r < R; r += kThreads) w.g2r[roi[r]] = r;
-  if (tid == 0) {
-    sh.local = (!full && R <= kAdjCap) ? 1 : 0;
-    sh.nfront = 0;
-    sh.nb = 0;
-    sh.found = 0;
-    sh.len = 0;
-  }
-  for (int r = tid; r < R; r += kThreads) {
-    node[r].st = ST_NONE;
-    node[r].stamp = -1;
-    if constexpr (kMulti) {
-      node[r].par = -1;
-      ms->init[r] = __longlong_as_double(0x7ff0000000000000ll);
-      ms->tcost[r] = __longlong_as_double(0x7ff8000000000000ll);
+  const bool full = a.full_graph != 0, leader = job.rank == 0 && tid == 0;
+  const int32_t R = job.R;
+  const int step = job.nranks * kThreads, first = job.rank * kThreads + tid;
+  long long t0 = clock64();
+  auto mark = [&](int k) {
+    if (leader) {
+      const long long now = clock64();
+      atomicAdd(&g_stage[k], (unsigned long long)(now - t0));
+      t0 = now;
     }
-  }
-  __syncthreads();
-  if constexpr (kMulti) {
-    // Seeds and targets outside the ROI are dropped (as the reference does);
-    // a repeated seed or target id is an argument error.
-    for (int i = tid; i < ms->nseeds; i += kThreads) {
-      const int32_t gid = ms->seeds[i];
-      if (gid < 0 || gid >= g.num_nodes) { sh.status = OGR_ERR_ARG; continue; }
-      const int32_t r = full ? gid : w.g2r[gid];
-      if (r < 0) continue;
-      if (atomicCAS(&node[r].stamp, -1, -2) != -1) { sh.status = OGR_ERR_ARG; continue; }
-      ms->init[r] = ms->seed_cost[i];
+  };
+  int32_t* roi_w = w.roi;
+  const int32_t* roi = full ? roi_w : job.roi;
+  int32_t sid = __ldcg(&w.ctl->sid) + 1;
+  const bool wrap = sid < 1 || sid == 0x7fffffff;
+  if (wrap) sid = 1;
+  Problem pr{};
+  pr.R = R;
+  pr.indptr = g.indptr;
+  pr.indices = g.indices;
+  pr.rev = g.rev;
+  pr.cost = st.total_cost;
+  pr.rcost = st.rcost;
+  pr.roi = roi;
+  pr.g2r = w.g2r;
+  pr.rec = w.rec;
+  pr.par = w.par;
+  pr.claim = w.claim;
+  pr.ov[0] = w.ov[0];
+  pr.ov[1] = w.ov[1];
+  pr.mseed = kMulti ? job.ms->init : nullptr;
+  pr.mtgt = kMulti ? job.ms->tcost : nullptr;
+  pr.none = kNoTerm;
+  pr.ctl = &w.ctl->team;
+  pr.rank = job.rank;
+  pr.nranks = job.nranks;
+  pr.spin = 1u << 22;
+  pr.max_phase = 2 * R + 4;
+  // With statistics requested the search goes on after dst is settled until
+  // every node with a label <= L(dst) is settled (T > L(dst)): the IN bound
+  // can settle dst before cheaper nodes, which the heap pops earlier.
+  pr.want_stats = job.stats != nullptr;
+  Outcome o{};
+  bool fix = true;
+  int k0 = 0;
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    pr.sid = sid + attempt;
+    int md = 0;
+    for (int r = first; r < R; r += step) {
+      const int32_t gid = full ? r : roi[r];
+      if (full) roi_w[r] = r;
+      w.g2r[gid] = r;
+      if (wrap && attempt == 0) w.claim[r] = 0;
+      const int32_t f0 = g.indptr[gid], f1 = g.indptr[gid + 1];
+      md = max(md, f1 - f0);
+      const float pen = job.roi_pen ? job.roi_pen[r] : ogr_node_penalty(st, a, gid);
+      __stcg(reinterpret_cast<int4*>(&w.rec[r]), make_int4(f0, f1 - f0, 0, __float_as_int(pen)));
+      if (kMulti) {
+        job.ms->init[r] = __longlong_as_double((long long)kNoTerm);
+        job.ms->tcost[r] = __longlong_as_double((long long)kNoTerm);
+      }
     }
-    for (int i = tid; i < ms->ntargets; i += kThreads) {
-      const int32_t gid = ms->targets[i];
-      if (gid < 0 || gid >= g.num_nodes) { sh.status = OGR_ERR_ARG; continue; }
-      const int32_t r = full ? gid : w.g2r[gid];
-      if (r < 0) continue;
-      if (atomicCAS(&node[r].par, -1, -3) != -1) { sh.status = OGR_ERR_ARG; continue; }
-      ms->tcost[r] = ms->target_cost[i];
+    md = __reduce_max_sync(0xffffffffu, md);
+    if ((tid & 31) == 0) sm.wmin[tid >> 5] = (unsigned long long)md;
+    __syncthreads();
+    if (tid == 0) {
+      sm.ok = 1;
+      for (int i = 1; i < kWarps; ++i) md = max(md, (int)sm.wmin[i]);
+      if (leader && attempt) clear_slot(pr, k0 + 2);   // the last two barriers' words are used ones
+      arrive(pr, sm, k0, kArrive, ~(unsigned long long)md);
+      await(pr, sm, k0);
+      sm.res[2] = (int)sm.t;
+      if (leader && attempt) clear_slot(pr, k0 + 3);
+      sm.res[0] = 0;               // first entries
+      sm.res[1] = 0;               // bad seeds or targets
+      sm.wmin[0] = kNone;          // their least label
     }
     __syncthreads();
-    for (int r = tid; r < R; r += kThreads) {
-      node[r].stamp = -1;
-      node[r].par = -1;
+    const int max_deg = sm.res[2];
+    const int ready = sm.ok;
+    if (max_deg > kMaxRow) fix = false;
+    int32_t rs = -1, rd = -1;
+    if (!kMulti && ready) {
+      rs = __ldcg(&w.g2r[a.src]);
+      rd = __ldcg(&w.g2r[a.dst]);
     }
-  }
-  __syncthreads();
-  // ROI-local adjacency: neighbour ROI index and in-arc cost per slot.
-  if (sh.local) {
-    int too_wide = 0;
-    for (int r = grp; r < R; r += kGroups) {
-      const int32_t rg = roi[r];
-      const int32_t e0 = indptr[rg], e1 = indptr[rg + 1];
-      if (e1 - e0 > kDMax) too_wide = 1;
-      // only the node's own arcs: slots past its degree are never read
-      const int dr = min(e1 - e0, kDMax);
-      for (int k = sl; k < dr; k += kSub) {
-        const int32_t e = e0 + k;
-        w.adj[(int64_t)r * kDMax + k] = w.g2r[indices[e]];
-        w.acost[(int64_t)r * kDMax + k] = st.rcost ? st.rcost[e] : st.total_cost[g.rev[e]];
+    const bool none = !kMulti && (rs < 0 || rd < 0 || rs == rd);
+    pr.src = rs;
+    pr.dst = rd;
+    auto enter = [&](int32_t r, int at) {
+      const int32_t gid = roi[r], f0 = g.indptr[gid];
+      w.claim[r] = pr.sid;
+      w.ov[0][at] = make_int4(r, f0, g.indptr[gid + 1] - f0, __float_as_int(__ldcg(&w.rec[r].pen)));
+    };
+    if (ready && job.rank == 0) {
+      if constexpr (kMulti) {
+        // Seeds and targets outside the ROI are dropped (as the reference
+        // does); a repeated seed or target id is an argument error.
+        const MultiSeeds& ms = *job.ms;
+        for (int i = tid; i < ms.ntargets; i += kThreads) {
+          const int32_t gid = ms.targets[i];
+          const int32_t r = gid < 0 || gid >= g.num_nodes ? -2 : w.g2r[gid];
+          if (r < 0) {
+            if (r == -2) sm.res[1] = 1;
+            continue;
+          }
+          const double c = ms.target_cost[i];
+          const unsigned long long was = atomicExch(reinterpret_cast<unsigned long long*>(&ms.tcost[r]),
+                                                    (unsigned long long)__double_as_longlong(c));
+          if (was != kNoTerm) sm.res[1] = 1;
+        }
+        for (int i = tid; i < ms.nseeds; i += kThreads) {
+          const int32_t gid = ms.seeds[i];
+          const int32_t r = gid < 0 || gid >= g.num_nodes ? -2 : w.g2r[gid];
+          if (r < 0) {
+            if (r == -2) sm.res[1] = 1;
+            continue;
+          }
+          const double c = ms.seed_cost[i];
+          const unsigned long long was = atomicExch(reinterpret_cast<unsigned long long*>(&ms.init[r]),
+                                                    (unsigned long long)__double_as_longlong(c));
+          if (was != kNoTerm) {
+            sm.res[1] = 1;
+            continue;
+          }
+          if (!(c < __longlong_as_double(0x7ff0000000000000ll))) {      // not a start
+            atomicExch(reinterpret_cast<unsigned long long*>(&ms.init[r]), kNoTerm);
+            continue;
+          }
+          const float pen = __ldcg(&w.rec[r].pen);
+          unsigned long long lb = ogr_dbits(c + (double)pen);
+          if (fix) {
+            lb = 0ull;
+            if (seed_ticks(c, &lb) && tick_finite(pen)) lb += ticks(pen);
+          }
+          enter(r, atomicAdd(&sm.res[0], 1));
+          w.rec[r].sp = 1;
+          atomicMin(&sm.wmin[0], lb);
+        }
+        __syncthreads();
+        // a target cost that is not a number marks no target
+        for (int i = tid; i < ms.ntargets; i += kThreads) {
+          const int32_t gid = ms.targets[i];
+          const int32_t r = gid < 0 || gid >= g.num_nodes ? -1 : w.g2r[gid];
+          if (r >= 0 && ms.target_cost[i] != ms.target_cost[i]) ms.tcost[r] = __longlong_as_double((long long)kNoTerm);
+        }
+      } else if (tid == 0 && !none) {
+        enter(rs, 0);
+        w.ov[0][0].w = 0;          // src's penalty does not count
+        sm.res[0] = 1;
+        sm.wmin[0] = 0ull;
       }
-      if (sl == 0) w.deg[r] = min(e1 - e0, kDMax);
-    }
-    too_wide = __reduce_or_sync(0xffffffffu, too_wide);
-    if (lane == 0 && too_wide) sh.local = 0;
-  }
-  const int32_t rs = kMulti ? -1 : (full ? src : w.g2r[src]);
-  int32_t rd = kMulti ? -1 : (full ? dst : w.g2r[dst]);
-  if (!kMulti && tid == 0 && (rs < 0 || rd < 0 || rs == rd)) sh.status = OGR_NO_PATH;
-  __syncthreads();
-  const bool local = sh.local != 0;
-  clk.mark(2);
-  int phase = 0;
-  bool exhausted = false;   // the frontier ran out before dst settled
-  if (sh.status == OGR_OK) {
-    if constexpr (kMulti) {
-      // the first recompute pass takes every seed (ROI order) from its initial
-      // candidate; nothing is settled yet
-      if (tid == 0) sh.ndirty = 0;
-      __syncthreads();
-      for (int r = tid; r < R; r += kThreads)
-        if (ms->init[r] < __longlong_as_double(0x7ff0000000000000ll)) w.dl[atomicAdd(&sh.ndirty, 1)] = r;
-    } else if (tid == 0) {
-      node[rs].st = ST_DONE;
-      node[rs].lab = 0.0;
-      node[rs].m32 = 0.0f;
-      node[rs].par = -1;
-      w.blist[0] = rs;
-      sh.nb = 1;
     }
     __syncthreads();
-    int cur = 0;
-    const int max_phase = 2 * R + 4;
-    // With statistics requested the search goes on after dst is settled until
-    // every node with a label <= L(dst) is settled (T > L(dst)): the IN bound
-    // can settle dst before cheaper nodes, which the heap pops earlier.
-    bool dst_done = false;
-    double ld_stop = 0.0;
-    while (true) {
-      // 1. queue the unsettled ROI neighbours of the newly settled nodes
-      if (!(kMulti && phase == 0)) {
-      if (tid == 0) sh.ndirty = 0;
-      __syncthreads();
-      const int nb = sh.nb;
-      for (int i = grp; i < nb; i += kGroups) {
-        const int32_t x = w.blist[i];
-        if (local) {
-          constexpr int kB = (kBatchArcs + kSub - 1) / kSub < 4 ? (kBatchArcs + kSub - 1) / kSub : 4;
-          const int dx = w.deg[x];
-          const int32_t* arow = w.adj + (int64_t)x * kDMax;
-          int32_t yb[kB];
-#pragma unroll
-          for (int j = 0; j < kB; ++j) yb[j] = arow[sl + j * kSub];
-          int32_t sb[kB];
-#pragma unroll
-          for (int j = 0; j < kB; ++j) {
-            const bool ok = sl + j * kSub < dx && yb[j] >= 0;
-            sb[j] = ok ? node[yb[j]].st : ST_DONE;
-          }
-#pragma unroll
-          for (int j = 0; j < kB; ++j) {
-            if (sb[j] >= ST_DONE) continue;
-            if (atomicExch(&node[yb[j]].stamp, phase) != phase) w.dl[atomicAdd(&sh.ndirty, 1)] = yb[j];
-          }
-          for (int k = sl + kB * kSub; k < dx; k += kSub) {   // rows wider than a batch
-            const int32_t y = arow[k];
-            if (y < 0 || node[y].st >= ST_DONE) continue;
-            if (atomicExch(&node[y].stamp, phase) != phase) w.dl[atomicAdd(&sh.ndirty, 1)] = y;
-          }
-        } else {
-          const int32_t xg = full ? x : roi[x];
-          const int32_t e1 = indptr[xg + 1];
-          for (int32_t e = indptr[xg] + sl; e < e1; e += kSub) {
-            const int32_t yg = indices[e];
-            const int32_t y = full ? yg : w.g2r[yg];
-            if (y < 0 || node[y].st >= ST_DONE) continue;
-            if (atomicExch(&node[y].stamp, phase) != phase) w.dl[atomicAdd(&sh.ndirty, 1)] = y;
-          }
-        }
+    if (tid == 0 && ready) {
+      unsigned long long nf0 = 0, tl = kNone;
+      if (job.rank == 0) {
+        nf0 = sm.res[1] ? 0 : (unsigned)sm.res[0];
+        tl = sm.wmin[0];
+        w.ctl->merr = sm.res[1];
+        w.ctl->team.nov[0] = (int)nf0;
+        w.ctl->team.nov[1] = 0;
+        w.ctl->team.nov[2] = 0;
       }
-      }
-      __syncthreads();
-      clk.mark(3);
-      // 2. recompute each queued node from all settled in-neighbours: a
-      //    kLanes-lane group per node, lanes over its arcs, shuffle reduction.
-      const int nd = sh.ndirty;
-      const int half = lane / kLanes;
-      for (int base = warp * kPerWarp; base < nd; base += kWarps * kPerWarp) {
-        const int idx = base + half;
-        const bool valid = idx < nd;
-        const int32_t y = valid ? w.dl[idx] : 0;
-        bool fresh = false;
-        float p = 0.0f;
-        if (valid) {
-          fresh = node[y].st == ST_NONE;
-          if (sl == 0)
-            p = !fresh ? node[y].pen : (roi_pen ? roi_pen[y] : ogr_node_penalty(st, a, full ? y : roi[y]));
-        }
-        p = __shfl_sync(0xffffffffu, p, lane & ~(kLanes - 1));
-        const double pd = (double)p;
-        float ba = kInf, bc = kInf;
-        double bl = 0.0;
-        int32_t bu = 0x7fffffff;
-        float cin = kInf;
-        if constexpr (kMulti) {
-          // the seed's own start: relaxed before any pop, so it wins float32 ties
-          if (valid && sl == 0) {
-            const double s0 = ms->init[y];
-            if (s0 < __longlong_as_double(0x7ff0000000000000ll)) {
-              ba = __double2float_rn(s0 + pd);
-              bl = -__longlong_as_double(0x7ff0000000000000ll);
-              bu = -1;
-            }
-          }
-        }
-        if (valid) {
-          if (local) {
-            constexpr int kB = (kBatchArcs + kSub - 1) / kSub < 4 ? (kBatchArcs + kSub - 1) / kSub : 4;
-            const int dy = w.deg[y];
-            const int32_t* arow = w.adj + (int64_t)y * kDMax;
-            const float* crow = w.acost + (int64_t)y * kDMax;
-            int32_t ub[kB];
-            float cb[kB];
-#pragma unroll
-            for (int j = 0; j < kB; ++j) {
-              ub[j] = arow[sl + j * kSub];
-              cb[j] = crow[sl + j * kSub];
-            }
-            int32_t sb[kB];
-            double lb[kB];
-#pragma unroll
-            for (int j = 0; j < kB; ++j) {
-              const bool ok = sl + j * kSub < dy && ub[j] >= 0;
-              sb[j] = ok ? node[ub[j]].st : -1;
-              lb[j] = ok ? node[ub[j]].lab : 0.0;
-            }
-            auto relax = [&](int32_t u, float c, int32_t su, double lu) {
-              if (kMulti && su == ST_SINK) return;   // targets relax nothing
-              if (su != ST_DONE) {
-                cin = fminf(cin, c);
-                return;
-              }
-              const float a32 = __double2float_rn((lu + (double)c) + pd);
-              if (!(a32 < kInf)) return;
-              if (ogr_key_lt(a32, lu, u, ba, bl, bu)) { ba = a32; bl = lu; bu = u; bc = c; }
-            };
-#pragma unroll
-            for (int j = 0; j < kB; ++j)
-              if (sb[j] >= 0) relax(ub[j], cb[j], sb[j], lb[j]);
-            for (int k = sl + kB * kSub; k < dy; k += kSub) {   // rows wider than a batch
-              const int32_t u = arow[k];
-              if (u < 0) continue;
-              relax(u, crow[k], node[u].st, node[u].lab);
-            }
-          } else {
-            const int32_t yg = full ? y : roi[y];
-            const int32_t e1 = indptr[yg + 1];
-            for (int32_t e = indptr[yg] + sl; e < e1; e += kSub) {
-              const int32_t ug = indices[e];
-              const int32_t u = full ? ug : w.g2r[ug];
-              if (u < 0) continue;
-              const float c = st.rcost ? st.rcost[e] : st.total_cost[g.rev[e]];
-              if (kMulti && node[u].st == ST_SINK) continue;   // targets relax nothing
-              if (node[u].st != ST_DONE) {
-                cin = fminf(cin, c);
-                continue;
-              }
-              const double lu = node[u].lab;
-              const float a32 = __double2float_rn((lu + (double)c) + pd);
-              if (!(a32 < kInf)) continue;
-              if (ogr_key_lt(a32, lu, u, ba, bl, bu)) { ba = a32; bl = lu; bu = u; bc = c; }
-            }
-          }
-        }
-#pragma unroll
-        for (int o = kLanes / 2; o > 0; o >>= 1) {
-          const float oa = __shfl_xor_sync(0xffffffffu, ba, o);
-          const double ol = __shfl_xor_sync(0xffffffffu, bl, o);
-          const int32_t ou = __shfl_xor_sync(0xffffffffu, bu, o);
-          const float oc = __shfl_xor_sync(0xffffffffu, bc, o);
-          if (ogr_key_lt(oa, ol, ou, ba, bl, bu)) { ba = oa; bl = ol; bu = ou; bc = oc; }
-          cin = fminf(cin, __shfl_xor_sync(0xffffffffu, cin, o));
-        }
-        if (valid && sl == 0) {
-          NodeSt& ns = node[y];
-          if (fresh) ns.pen = p;
-          ns.cin = cin;
-          if (ba < kInf) {
-            ns.m32 = ba;
-            ns.lab = (kMulti && bu == -1) ? ms->init[y] + pd : (bl + (double)bc) + pd;
-            ns.par = bu;
-            if (fresh) {
-              ns.st = ST_FRONT;
-              w.fr[cur][atomicAdd(&sh.nfront, 1)] = y;
-            }
-          }
-        }
-      }
-      __syncthreads();
-      clk.mark(4);
-      if (tid == 0) atomicAdd(&g_stage[13], (unsigned long long)nd);
-      const int nf = sh.nfront;
-      if (nf == 0) {
-        if (!kMulti && !dst_done) exhausted = true;
-        if (tid == 0 && !kMulti) {
-          if (dst_done)
-            sh.found = 1;
-          else
-            sh.status = OGR_NO_PATH;
-        }
-        break;
-      }
-      // 3. T = smallest tentative label in the frontier.
-      unsigned long long mn = ~0ull;
-      for (int i = tid; i < nf; i += kThreads) {
-        const unsigned long long b = ogr_dbits(node[w.fr[cur][i]].lab);
-        mn = b < mn ? b : mn;
-      }
-      mn = block_min_u64(mn, sh.s_min);
-      const double T = __longlong_as_double((long long)mn);
-      clk.mark(5);
-      if (dst_done && T > ld_stop) {
-        if (tid == 0) sh.found = 1;
-        break;
-      }
-      // 4. settle every node whose state can no longer change.
-      if (tid == 0) { sh.nb = 0; sh.nnext = 0; }
-      __syncthreads();
-      for (int i = tid; i < nf; i += kThreads) {
-        const int32_t x = w.fr[cur][i];
-        NodeSt& ns = node[x];
-        bool settle = (ns.lab == T);
-        if (!settle) settle = ns.m32 < __double2float_rn((T + (double)ns.cin) + (double)ns.pen);
-        if (settle) {
-          if (kMulti && ms->tcost[x] == ms->tcost[x]) {
-            ns.st = ST_SINK;   // settled, never expanded
-          } else {
-            ns.st = ST_DONE;
-            w.blist[atomicAdd(&sh.nb, 1)] = x;
-          }
-        } else {
-          w.fr[cur ^ 1][atomicAdd(&sh.nnext, 1)] = x;
-        }
-      }
-      __syncthreads();
-      if (tid == 0) sh.nfront = sh.nnext;
-      cur ^= 1;
-      clk.mark(6);
-      if (tid == 0) atomicAdd(&g_stage[10], 1ull);
-      const bool done = !kMulti && !dst_done && node[rd].st == ST_DONE;
-      const bool capped = phase + 1 > max_phase;
-      if (done) ld_stop = node[rd].lab;
-      __syncthreads();
-      if (done) {
-        dst_done = true;
-        if (stats_acc == nullptr) {
-          if (tid == 0) sh.found = 1;
-          break;
-        }
-      }
-      if (capped) {
-        if (tid == 0) sh.status = OGR_ERR_ITER_CAP;
-        break;
-      }
-      ++phase;
+      arrive(pr, sm, k0 + 1, kArrive + kOut * (nf0 < kMostOut ? nf0 : kMostOut) + kCount * nf0, tl);
+      await(pr, sm, k0 + 1);
+      if (kMulti && sm.ok && __ldcg(&w.ctl->merr)) sm.ok = 2;
     }
+    __syncthreads();
+    const int ok = sm.ok;
+    __syncthreads();
+    if (attempt == 0) mark(2);
+    ++k0;
+    if (ok != 1 || none) {
+      o.status = ok == 0 ? OGR_ERR_TIMEOUT : ok == 2 ? OGR_ERR_ARG : OGR_NO_PATH;
+      ++k0;
+      break;
+    }
+    o = run_search<L, K, kMulti, true>(pr, smem, k0, max_deg, fix);
+    k0 += o.phases;
+    if (o.status != kStInexact) break;
+    fix = false;
+    __syncthreads();
   }
-  __syncthreads();
-  if constexpr (kMulti) {
+  mark(3);
+  if (leader) {
+    atomicAdd(&g_stage[4], (unsigned long long)o.wait);
+    atomicAdd(&g_stage[9], 1ull);
+    atomicAdd(&g_stage[10], (unsigned long long)o.phases);
+  }
+  if (tid == 0) atomicAdd(&g_stage[13], o.examined);
+  int status = o.status;
+  int32_t tgt = pr.dst;
+  if (kMulti && status == OGR_OK) {
     // The reference keeps the first popped target whose label + target cost is
     // strictly below the best so far: the least (total, label, ROI index).
-    if (sh.status == OGR_OK) {
-      unsigned long long k1 = ~0ull;
-      for (int r = tid; r < R; r += kThreads) {
-        if (node[r].st != ST_SINK) continue;
-        const double tot = node[r].lab + ms->tcost[r];
-        if (!(tot < __longlong_as_double(0x7ff0000000000000ll))) continue;
-        k1 = min(k1, ogr_order_bits(tot));
+    // Every CTA of the team makes the choice (the statistics depend on it).
+    const MultiSeeds& ms = *job.ms;
+    const double dinf = __longlong_as_double(0x7ff0000000000000ll);
+    unsigned long long best[3] = {kNone, kNone, kNone};
+    for (int pass = 0; pass < 3; ++pass) {
+      unsigned long long k = kNone;
+      for (int i = tid & 31; i < ms.ntargets; i += 32) {
+        const int32_t r = w.g2r[ms.targets[i]];
+        if (r < 0) continue;
+        const Rec x = ld_rec(&w.rec[r]);
+        if (x.sp < 2) continue;
+        const double lr = fix ? label_value<true>(x.lab) : label_value<false>(x.lab);
+        const double tot = lr + ms.target_cost[i];
+        if (!(tot < dinf)) continue;
+        const unsigned long long kt = ogr_order_bits(tot), kl = ogr_order_bits(lr);
+        const unsigned long long y = pass == 0   ? kt
+                                     : pass == 1 ? (kt == best[0] ? kl : kNone)
+                                                 : (kt == best[0] && kl == best[1] ? (unsigned long long)r : kNone);
+        k = y < k ? y : k;
       }
-      k1 = block_min_u64(k1, sh.s_min);
-      unsigned long long k2 = ~0ull;
-      if (k1 != ~0ull)
-        for (int r = tid; r < R; r += kThreads)
-          if (node[r].st == ST_SINK && ogr_order_bits(node[r].lab + ms->tcost[r]) == k1)
-            k2 = min(k2, ogr_order_bits(node[r].lab));
-      k2 = block_min_u64(k2, sh.s_min);
-      unsigned long long k3 = ~0ull;
-      if (k1 != ~0ull)
-        for (int r = tid; r < R; r += kThreads)
-          if (node[r].st == ST_SINK && ogr_order_bits(node[r].lab + ms->tcost[r]) == k1 &&
-              ogr_order_bits(node[r].lab) == k2)
-            k3 = min(k3, (unsigned long long)r);
-      k3 = block_min_u64(k3, sh.s_min);
+      best[pass] = warp_min_u64(k);
+    }
+    tgt = best[0] == kNone ? -1 : (int32_t)best[2];
+    if (tgt < 0) status = OGR_NO_PATH;
+  }
+  // Statistics of the sequential heap search: the rows of the nodes popped
+  // before dst; of a search that cannot reach dst, every node it reaches; of a
+  // multi-source search, every settled node, the expanded ones' rows.
+  const bool found = status == OGR_OK;
+  if (job.stats != nullptr && (found || (!kMulti && o.exhausted))) {
+    count_work<kMulti, true>(pr, o, first, step, job.stats);
+    if (leader) {
+      if (found && !kMulti) atomicAdd(&job.stats[1], 1ull);   // dst's own pop
+      atomicAdd(&job.stats[2], (unsigned long long)R);
+      atomicAdd(&job.stats[3], (unsigned long long)o.phases);
+    }
+  }
+  // Backtrace dst -> src (reversed into path_out), by the first CTA.
+  int len = 0;
+  if (job.rank == 0 && found) {
+    if (tid < 32) {
+      const int limit = min(job.path_cap, R);
+      int32_t c = -1;
+      len = walk_parents(w.par, tgt, R, limit, job.path_out, &c);
+      // (a parent chain longer than the ROI is a cycle)
+      if (c != -1) status = len >= R ? OGR_ERR_ITER_CAP : OGR_ERR_CAPACITY;
+      else if (len < 2) status = OGR_NO_PATH;
       if (tid == 0) {
-        if (k1 == ~0ull) {
-          sh.status = OGR_NO_PATH;
-        } else {
-          sh.found = 1;
-          sh.nb = (int)k3;   // the chosen target
-        }
+        sm.res[0] = status;
+        sm.res[1] = len;
       }
     }
     __syncthreads();
-    if (sh.found) rd = sh.nb;
-    // every settled node was popped once; expanded ones scanned their row
-    if (sh.status == OGR_OK && stats_acc != nullptr) {
-      unsigned arcs = 0, pops = 0;
-      for (int r = tid; r < R; r += kThreads) {
-        const int32_t sr = node[r].st;
-        if (sr < ST_DONE) continue;
-        ++pops;
-        if (sr == ST_DONE) {
-          const int32_t rg = full ? r : roi[r];
-          arcs += (unsigned)(indptr[rg + 1] - indptr[rg]);
-        }
-      }
-      arcs = __reduce_add_sync(0xffffffffu, arcs);
-      pops = __reduce_add_sync(0xffffffffu, pops);
-      if (lane == 0) {
-        atomicAdd(&stats_acc[0], (unsigned long long)arcs);
-        atomicAdd(&stats_acc[1], (unsigned long long)pops);
-      }
-      if (tid == 0) {
-        atomicAdd(&stats_acc[2], (unsigned long long)R);
-        atomicAdd(&stats_acc[3], (unsigned long long)(phase + 1));
-      }
+    status = sm.res[0];
+    len = status == OGR_OK ? sm.res[1] : 0;
+    for (int i = tid; i < len / 2; i += kThreads) {
+      const int32_t x = job.path_out[i], y = job.path_out[len - 1 - i];
+      job.path_out[i] = roi[y];
+      job.path_out[len - 1 - i] = roi[x];
     }
+    if ((len & 1) && tid == 0) job.path_out[len / 2] = roi[job.path_out[len / 2]];
   }
-  // A search that cannot reach dst pops every node it reaches and scans each
-  // one's row, as the heap does before it runs empty.
-  if (!kMulti && exhausted && stats_acc != nullptr) {
-    unsigned arcs = 0, pops = 0;
-    for (int r = tid; r < R; r += kThreads) {
-      if (node[r].st != ST_DONE) continue;
-      const int32_t rg = full ? r : roi[r];
-      arcs += (unsigned)(indptr[rg + 1] - indptr[rg]);
-      ++pops;
-    }
-    arcs = __reduce_add_sync(0xffffffffu, arcs);
-    pops = __reduce_add_sync(0xffffffffu, pops);
-    if (lane == 0) {
-      atomicAdd(&stats_acc[0], (unsigned long long)arcs);
-      atomicAdd(&stats_acc[1], (unsigned long long)pops);
-    }
+  mark(7);
+  if (kMulti && job.nranks > 1) {
+    // the choice of the target reads the map in every CTA
     if (tid == 0) {
-      atomicAdd(&stats_acc[2], (unsigned long long)R);
-      atomicAdd(&stats_acc[3], (unsigned long long)(phase + 1));
+      arrive(pr, sm, k0, kArrive, kNone);
+      await(pr, sm, k0);
     }
+    __syncthreads();
   }
-  // Arcs the sequential search scans before popping dst: the rows of all
-  // nodes popped before it, i.e. settled with (L, idx) < (L(dst), dst).
-  if (!kMulti && sh.found && stats_acc != nullptr) {
-    const double ld = node[rd].lab;
-    unsigned arcs = 0, pops = 0;
-    for (int r = tid; r < R; r += kThreads) {
-      if (node[r].st != ST_DONE) continue;
-      const double lr = node[r].lab;
-      if (lr < ld || (lr == ld && r < rd)) {
-        const int32_t rg = full ? r : roi[r];
-        arcs += (unsigned)(indptr[rg + 1] - indptr[rg]);
-        ++pops;
-      }
-    }
-    arcs = __reduce_add_sync(0xffffffffu, arcs);
-    pops = __reduce_add_sync(0xffffffffu, pops);
-    if (lane == 0) {
-      atomicAdd(&stats_acc[0], (unsigned long long)arcs);
-      atomicAdd(&stats_acc[1], (unsigned long long)pops);
-    }
-    if (tid == 0) {
-      atomicAdd(&stats_acc[1], 1ull);
-      atomicAdd(&stats_acc[2], (unsigned long long)R);
-      atomicAdd(&stats_acc[3], (unsigned long long)(phase + 1));
-    }
-  }
-  // Backtrace dst -> src.
-  if (tid == 0 && sh.found && sh.status == OGR_OK) {
-    int len = 0;
-    for (int32_t c = rd; c != -1 && len <= R; c = node[c].par) ++len;
-    if (len > R) {
-      sh.status = OGR_ERR_ITER_CAP;  // a parent chain longer than the ROI is a cycle
-    } else if (len > path_cap) {
-      sh.status = OGR_ERR_CAPACITY;
-    } else {
-      int i = len - 1;
-      for (int32_t c = rd; c != -1; c = node[c].par) path_out[i--] = full ? c : roi[c];
-      sh.len = len;
-      if (len < 2) sh.status = OGR_NO_PATH;
-    }
-  }
+  for (int r = first; r < R; r += step) w.g2r[roi[r]] = -1;
+  if (leader) w.ctl->sid = pr.sid;
   __syncthreads();
-  clk.mark(7);
-  if (!full)
-    for (int r = tid; r < R; r += kThreads) w.g2r[roi[r]] = -1;
-  __syncthreads();
-  clk.mark(8);
-  if (tid == 0) atomicAdd(&g_stage[9], 1ull);
+  mark(8);
+  *status_out = status;
+  *len_out = len;
 }
 
-// Whole search for one net on one CTA (ROI extraction inline).
-template <int L>
-__device__ void search_net(Shared& sh, const ogr_graph& g, const ogr_state& st, const ogr_net_args& a, const Ws& w,
-                           int32_t* path_out, int32_t path_cap, unsigned long long* stats_acc) {
+// The search in the form for rows of ROW arcs.
+template <int ROW, bool kMulti>
+__device__ __forceinline__ void roi_search_row(const RoiJob& job, char* smem, int* status, int* len) {
+  if constexpr (ROW == 4) roi_search<4, 1, kMulti>(&job, smem, status, len);
+  else if constexpr (ROW == 8) roi_search<8, 1, kMulti>(&job, smem, status, len);
+  else if constexpr (ROW == 16) roi_search<8, 2, kMulti>(&job, smem, status, len);
+  else roi_search<16, 2, kMulti>(&job, smem, status, len);
+}
+
+// The ROI of one net into w.roi (nothing for a full-graph net), by one CTA:
+// sh.status and sh.R tell.
+__device__ void build_roi(Shared& sh, const ogr_graph& g, const ogr_net_args& a, const Ws& w) {
   StageClock clk;
   clk.start();
-  if (threadIdx.x == 0) {
-    sh.status = OGR_OK;
-    sh.len = 0;
-    sh.found = 0;
-  }
+  if (threadIdx.x == 0) sh.status = OGR_OK;
   __syncthreads();
-  int32_t R = g.num_nodes;
-  if (!a.full_graph) {
-    roi_build(sh, g, a, w.seen, w.q, w.qcap, w.roi, a.max_roi_nodes, clk);
-    R = sh.R;
+  if (a.full_graph) {
+    if (threadIdx.x == 0) sh.R = g.num_nodes;
+    __syncthreads();
+    return;
   }
-  if (sh.status != OGR_OK) return;
-  sssp_roi<false, L>(sh, g, st, a, w, w.roi, R, path_out, path_cap, stats_acc, clk);
+  roi_build(sh, g, a, w.seen, w.q, w.qcap, w.roi, a.max_roi_nodes, clk);
 }
 
 // ---- commit / rip-up ---------------------------------------------------------
@@ -1045,60 +801,37 @@ __device__ int apply_path_dev(const ogr_graph& g, const ogr_state& st, const int
 }
 
 // ---- kernels -------------------------------------------------------------------
-template <int L>
+// The ROI of a net into w.roi: result[0] = status, result[3] = its size.
 __global__ void __launch_bounds__(kThreads, 1)
-find_path_kernel(ogr_graph g, ogr_state st, ogr_net_args a, Ws w, int32_t* path_out, int32_t path_cap,
-                 int64_t* stats) {
+build_roi_kernel(ogr_graph g, ogr_net_args a, Ws w) {
   __shared__ Shared sh;
-  search_net<L>(sh, g, st, a, w, path_out, path_cap, reinterpret_cast<unsigned long long*>(stats));
+  build_roi(sh, g, a, w);
   if (threadIdx.x == 0) {
     w.result[0] = sh.status;
-    w.result[1] = sh.len;
+    w.result[1] = 0;
+    w.result[3] = sh.R;
   }
 }
 
-// The reference's solver seam: search a given ROI (ROI order = tie order)
-// with a given ROI-local penalty array (or none).
-template <int L>
+// One team's search of a net (or, kMulti, of seeds and targets): a caller's
+// ROI, or (roi NULL) the one build_roi_kernel left, or the whole lattice.
+template <int ROW, bool kMulti>
 __global__ void __launch_bounds__(kThreads, 1)
-find_path_given_roi_kernel(ogr_graph g, ogr_state st, ogr_net_args a, Ws w, const int32_t* roi, int32_t R,
-                           const float* roi_pen, int32_t* path_out, int32_t path_cap, int64_t* stats) {
-  __shared__ Shared sh;
-  StageClock clk;
-  clk.start();
-  if (threadIdx.x == 0) {
-    sh.status = OGR_OK;
-    sh.len = 0;
-    sh.found = 0;
+find_team_kernel(ogr_graph g, ogr_state st, ogr_net_args a, Ws w, const int32_t* roi, int32_t R, const float* roi_pen,
+                 MultiSeeds ms, int32_t* path_out, int32_t path_cap, int64_t* stats) {
+  extern __shared__ __align__(16) char smem[];
+  if (roi == nullptr && !a.full_graph) {
+    if (w.result[0] != OGR_OK) return;             // uniform: written by an earlier launch
+    roi = w.roi;
+    R = (int32_t)w.result[3];
   }
-  __syncthreads();
-  sssp_roi<false, L>(sh, g, st, a, w, roi, R, path_out, path_cap, reinterpret_cast<unsigned long long*>(stats), clk,
-                     roi_pen);
-  if (threadIdx.x == 0) {
-    w.result[0] = sh.status;
-    w.result[1] = sh.len;
-  }
-}
-
-// The multi-source multi-sink seam on a given ROI.
-template <int L>
-__global__ void __launch_bounds__(kThreads, 1)
-find_path_multi_kernel(ogr_graph g, ogr_state st, ogr_net_args a, Ws w, const int32_t* roi, int32_t R,
-                       const float* roi_pen, MultiSeeds ms, int32_t* path_out, int32_t path_cap, int64_t* stats) {
-  __shared__ Shared sh;
-  StageClock clk;
-  clk.start();
-  if (threadIdx.x == 0) {
-    sh.status = OGR_OK;
-    sh.len = 0;
-    sh.found = 0;
-  }
-  __syncthreads();
-  sssp_roi<true, L>(sh, g, st, a, w, roi, R, path_out, path_cap, reinterpret_cast<unsigned long long*>(stats), clk,
-                 roi_pen, &ms);
-  if (threadIdx.x == 0) {
-    w.result[0] = sh.status;
-    w.result[1] = sh.len;
+  const RoiJob job{&g,       &st,      &a,    &w, roi, R, roi_pen, &ms, path_out, path_cap,
+                   reinterpret_cast<unsigned long long*>(stats), (int)blockIdx.x, (int)gridDim.x};
+  int status, len;
+  roi_search_row<ROW, kMulti>(job, smem, &status, &len);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    w.result[0] = status;
+    w.result[1] = len;
   }
 }
 
@@ -1130,7 +863,10 @@ __global__ void ws_init_kernel(Ws w, int64_t N) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
     w.seen[i] = 0;
     w.g2r[i] = -1;
+    w.claim[i] = 0;
   }
+  if (blockIdx.x == 0)
+    for (int i = threadIdx.x; i < (int)(sizeof(SlotCtl) / 4); i += blockDim.x) reinterpret_cast<int32_t*>(w.ctl)[i] = 0;
 }
 
 __global__ void bfs_init_kernel(char* base, int32_t slots, size_t slot_bytes, int32_t N, int64_t qcap) {
@@ -1266,90 +1002,6 @@ roi_batch_kernel(ogr_graph g, ogr_net_table t, ogr_pass_args pa, ogr_roi_batch r
   }
 }
 
-// One launch routes an ordered list of nets the way _route_all does.
-template <int L>
-__global__ void __launch_bounds__(kThreads, 1)
-route_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa, ogr_roi_batch rb, int use_batch,
-                  Ws w) {
-  __shared__ Shared sh;
-  __shared__ int32_t s_via[kMaxViaNodes];
-  __shared__ int s_flags[2];
-  __shared__ int s_fallbacks;
-  __shared__ int s_error;
-  unsigned long long* stats = reinterpret_cast<unsigned long long*>(pa.stats);
-  if (w.result[0] < 0) return;  // an earlier step of this pass failed
-  if (threadIdx.x == 0) { s_fallbacks = (int)w.result[2]; s_error = OGR_OK; }
-  __syncthreads();
-  for (int k = 0; k < pa.count; ++k) {
-    const int32_t n = pa.order[k];
-    int32_t* slot = t.store_path + (int64_t)n * t.slot_cap;
-    int32_t* arcs = t.store_arcs + (int64_t)n * 2 * t.slot_cap;
-    const int32_t old_len = t.store_len[n];
-    if (old_len >= 2) {
-      const int rc = apply_path_dev(g, st, slot, old_len, t.net_id[n], -1, pa.pres_fac, pa.live, nullptr, s_via,
-                                    s_flags);
-      if (rc != OGR_OK) {
-        if (threadIdx.x == 0) s_error = rc;
-        break;
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) t.store_len[n] = 0;
-    ogr_net_args a = ogr_pass_net_args(t, pa, n, 0);
-    const int pre = (use_batch && !a.full_graph) ? rb.roi_len[n] : -1;
-    if (pre > 0) {
-      StageClock clk;
-      clk.start();
-      if (threadIdx.x == 0) {
-        sh.status = OGR_OK;
-        atomicAdd(&g_stage[14], 1ull);
-      }
-      __syncthreads();
-      sssp_roi<false, L>(sh, g, st, a, w, rb.roi_pool + (int64_t)n * rb.roi_cap, pre, slot, t.slot_cap, stats, clk);
-    } else {
-      search_net<L>(sh, g, st, a, w, slot, t.slot_cap, stats);
-    }
-    int flags = 0;
-    const int st1 = sh.status;
-    if (st1 < 0) {
-      if (threadIdx.x == 0) s_error = st1;
-      break;
-    }
-    if (st1 != OGR_OK && s_fallbacks < pa.fallback_quota) {
-      a = ogr_pass_net_args(t, pa, n, 1);
-      __syncthreads();
-      if (threadIdx.x == 0) ++s_fallbacks;
-      search_net<L>(sh, g, st, a, w, slot, t.slot_cap, stats);
-      const int st2 = sh.status;
-      if (st2 < 0) {
-        if (threadIdx.x == 0) s_error = st2;
-        break;
-      }
-      flags |= 2;
-    }
-    const int fin = sh.status;
-    const int len = sh.len;
-    __syncthreads();
-    if (fin == OGR_OK) {
-      const int rc = apply_path_dev(g, st, slot, len, t.net_id[n], +1, pa.pres_fac, pa.live, arcs, s_via, s_flags);
-      if (rc != OGR_OK) {
-        if (threadIdx.x == 0) s_error = rc;
-        break;
-      }
-      if (threadIdx.x == 0) t.store_len[n] = len;
-    } else {
-      flags |= 1;
-    }
-    if (threadIdx.x == 0) pa.net_status[k] = flags;
-    __syncthreads();
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    w.result[2] = s_fallbacks;
-    if (s_error != OGR_OK) w.result[0] = s_error;
-  }
-}
-
 // ---- batched disjoint-ROI windows ---------------------------------------------
 // Control block of the window pass (device scratch, cleared per launch).
 struct WinCtl {
@@ -1358,6 +1010,9 @@ struct WinCtl {
   int32_t cursor;
   int32_t wsize;
   int32_t error;
+  int32_t solo_R;            // size of the ROI built inline (solo member or fallback)
+  int32_t fb;                // 1 + position of the net whose fallback is to be searched
+  int32_t fb_st, fb_len;
 };
 
 struct WinSlots {
@@ -1436,34 +1091,52 @@ __device__ int commit_from(const ogr_graph& g, const ogr_state& st, const ogr_ne
   return rc;
 }
 
+// Clears a search slot's team words (between searches).
+__device__ __forceinline__ void clear_team(SlotCtl* c) {
+  for (int i = threadIdx.x; i < (int)(sizeof(ogr_phase::Ctl) / 4); i += blockDim.x)
+    reinterpret_cast<int32_t*>(&c->team)[i] = 0;
+}
+
 // The ROI nets of a pass (pa.order[0..count)) in windows of mutually disjoint
-// footprints.  CTA 0 forms each window; CTA b rips up and searches its net
-// into scratch; then either every net commits (no failure) or CTA 0 commits in
-// order up to the first failed net, undoes the later nets' rip-ups and runs
-// the failed net's fallback.
-template <int L>
+// footprints.  CTA 0 forms each window; the CTAs split into one team per
+// member, which rips up and searches its net into scratch; then either every
+// net commits (no failure) or CTA 0 commits in order up to the first failed
+// net and undoes the later nets' rip-ups, and a team runs the failed net's
+// fallback.  Without windows (nslots = 0) every window is one net, searched in
+// the route workspace w.
+template <int ROW>
 __global__ void __launch_bounds__(kThreads, 1)
-window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa, ogr_roi_batch rb, char* slot_base,
-                   size_t slot_bytes, int32_t rmax, int32_t* scratch, char* ctl_base, Ws w, int32_t look,
-                   unsigned long long* discarded) {
+window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa, ogr_roi_batch rb, int use_batch,
+                   char* slot_base, size_t slot_bytes, int32_t rmax, int32_t nslots, int32_t* scratch,
+                   char* ctl_base, Ws w, int32_t look, unsigned long long* discarded) {
+  extern __shared__ __align__(16) char smem[];
   __shared__ Shared sh;
-  __shared__ int32_t s_via[kMaxViaNodes];
   __shared__ int s_flags[2];
   __shared__ int s_bar;
   __shared__ int s_box[4];
   __shared__ int s_skip[4 * kMaxSkip];
   __shared__ int s_win[4];
-  WinCtl* c;
-  WinSlots ws;
-  win_ctl_layout(gridDim.x, ctl_base, &c, &ws);
+  int32_t* s_via = reinterpret_cast<int32_t*>(smem);     // (no search is on while paths are applied)
   const int b = blockIdx.x, tid = threadIdx.x, G = gridDim.x;
   if (w.result[0] < 0) return;  // uniform: an earlier step of this pass failed
-  Ws mine;
-  ws_slot_layout(g.num_nodes, rmax, slot_base + (size_t)b * slot_bytes, &mine);
-  int32_t* my_path = scratch + (int64_t)b * t.slot_cap;
+  const int wmax = nslots > 0 ? nslots : 1;
+  WinCtl* c;
+  WinSlots ws;
+  win_ctl_layout(wmax, ctl_base, &c, &ws);
   unsigned long long* stats = reinterpret_cast<unsigned long long*>(pa.stats);
   const int32_t plane = g.nx * g.ny;
   unsigned long long target = 0;
+  // member m's search slot and path buffer
+  auto slot_of = [&](int m, bool solo) {
+    Ws x = w;
+    if (nslots > 0 && !solo) ws_slot_layout(g.num_nodes, rmax, slot_base + (size_t)m * slot_bytes, &x);
+    return x;
+  };
+  auto path_of = [&](int m, int32_t n) {
+    return nslots > 0 ? scratch + (int64_t)m * t.slot_cap : t.store_path + (int64_t)n * t.slot_cap;
+  };
+  if (b < wmax) clear_team(slot_of(b, false).ctl);
+  if (b == 0) clear_team(w.ctl);
   while (true) {
     // 1. window formation (CTA 0).  Nets are taken in order from the first
     // pending one while their footprints (ROI box and old-path box) are
@@ -1478,20 +1151,26 @@ window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa,
         int cur = c->cursor;
         while (cur < pa.count && pa.net_status[cur] != -1) ++cur;
         c->cursor = cur;
+        c->fb = 0;
         s_win[0] = cur;
       }
       __syncthreads();
       const int k0 = s_win[0];
       int W = 0, nskip = 0;
-      for (int k = k0; k < pa.count && W < G && k - k0 < 4 * G; ++k) {
+      for (int k = k0; k < pa.count && W < wmax && k - k0 < 4 * wmax; ++k) {
         if (*(volatile int32_t*)&pa.net_status[k] != -1) continue;   // done out of order earlier
         const int32_t n = pa.order[k];
-        const int32_t R = rb.roi_len[n];
+        const int32_t R = use_batch ? rb.roi_len[n] : -1;
         if (R <= 0) {
           if (W == 0 && nskip == 0) {
             if (tid == 0) { ws.k[0] = k; ws.solo[0] = 1; ws.inorder[0] = 1; }
             W = 1;
           }
+          break;
+        }
+        if (nslots == 0) {                   // one net at a time: no footprints to compare
+          if (tid == 0) { ws.k[0] = k; ws.solo[0] = 0; ws.inorder[0] = 1; }
+          W = 1;
           break;
         }
         if (tid == 0) {
@@ -1540,42 +1219,51 @@ window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa,
     if (!win_barrier(c, target, &s_bar)) break;
     const int W = *(volatile int32_t*)&c->wsize;
     if (W == 0 || *(volatile int32_t*)&c->error) break;
-    // 2. rip-up and search, one net per CTA, paths into scratch
+    // 2. rip-up, one member per CTA (and the ROI of a member without one)
+    const bool solo = *(volatile int32_t*)&ws.solo[0] != 0;
     if (b < W) {
-      const int32_t k = ws.k[b];
-      const int32_t n = pa.order[k];
+      const int32_t n = pa.order[ws.k[b]];
       const int32_t ol = t.store_len[n];
       int rc = OGR_OK;
       if (ol >= 2)
         rc = apply_path_dev(g, st, t.store_path + (int64_t)n * t.slot_cap, ol, t.net_id[n], -1, pa.pres_fac,
                             pa.live, nullptr, s_via, s_flags);
       if (tid < 4) ws.stats[4 * b + tid] = 0ull;
-      __syncthreads();
-      if (rc == OGR_OK) {
+      if (nslots == 0 && tid == 0) t.store_len[n] = 0;   // (a window's rip-ups may yet be undone)
+      if (solo && rc == OGR_OK) {
         const ogr_net_args a = ogr_pass_net_args(t, pa, n, 0);
-        if (ws.solo[b]) {
-          search_net<L>(sh, g, st, a, w, my_path, t.slot_cap, ws.stats + 4 * b);
-        } else {
-          StageClock clk;
-          clk.start();
-          if (tid == 0) sh.status = OGR_OK;
-          __syncthreads();
-          sssp_roi<false, L>(sh, g, st, a, mine, rb.roi_pool + (int64_t)n * rb.roi_cap, rb.roi_len[n], my_path,
-                             t.slot_cap,
-                   ws.stats + 4 * b, clk);
-        }
-        if (tid == 0) {
-          ws.st[b] = sh.status;
-          ws.len[b] = sh.len;
-          if (sh.status < 0) atomicExch(&c->error, sh.status);
-        }
-      } else if (tid == 0) {
-        atomicExch(&c->error, rc);
+        build_roi(sh, g, a, w);
+        rc = sh.status;
+        if (tid == 0) c->solo_R = sh.R;
+      } else if (use_batch && tid == 0) {
+        atomicAdd(&g_stage[14], 1ull);
+      }
+      if (tid == 0 && rc != OGR_OK) atomicExch(&c->error, rc);
+    }
+    if (!win_barrier(c, target, &s_bar)) break;
+    if (*(volatile int32_t*)&c->error) break;
+    // 3. search, one team of CTAs per member, paths into scratch
+    const int T = min(kTeam, G / W), mem = b / T, rank = b - mem * T;
+    if (mem < W) {
+      const int32_t n = pa.order[ws.k[mem]];
+      const ogr_net_args a = ogr_pass_net_args(t, pa, n, 0);
+      const Ws mine = slot_of(mem, solo);
+      const RoiJob job{&g, &st, &a, &mine,
+                       solo ? w.roi : rb.roi_pool + (int64_t)n * rb.roi_cap,
+                       solo ? *(volatile int32_t*)&c->solo_R : rb.roi_len[n],
+                       nullptr, nullptr, path_of(mem, n), t.slot_cap, ws.stats + 4 * mem, rank, T};
+      int status, len;
+      roi_search_row<ROW, false>(job, smem, &status, &len);
+      if (tid == 0 && rank == 0) {
+        ws.st[mem] = status;
+        ws.len[mem] = len;
+        if (status < 0) atomicExch(&c->error, status);
       }
     }
     if (!win_barrier(c, target, &s_bar)) break;
     if (*(volatile int32_t*)&c->error) break;
-    // 3. commit
+    // 4. commit
+    if (b < W) clear_team(slot_of(b, solo).ctl);
     int ff = W;
     for (int m = 0; m < W; ++m)
       if (ws.st[m] != OGR_OK) { ff = m; break; }
@@ -1590,7 +1278,7 @@ window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa,
         const int32_t k = ws.k[b], n = pa.order[k];
         if (tid < 4) atomicAdd(&stats[tid], ws.stats[4 * b + tid]);
         if (ws.st[b] == OGR_OK) {
-          const int rc = commit_from(g, st, t, pa, n, my_path, ws.len[b], s_via, s_flags);
+          const int rc = commit_from(g, st, t, pa, n, path_of(b, n), ws.len[b], s_via, s_flags);
           if (tid == 0) {
             pa.net_status[k] = 0;
             if (rc != OGR_OK) atomicExch(&c->error, rc);
@@ -1604,7 +1292,7 @@ window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa,
       int rc = OGR_OK;
       for (int m = 0; m < ff && rc == OGR_OK; ++m) {
         const int32_t k = ws.k[m], n = pa.order[k];
-        rc = commit_from(g, st, t, pa, n, scratch + (int64_t)m * t.slot_cap, ws.len[m], s_via, s_flags);
+        rc = commit_from(g, st, t, pa, n, path_of(m, n), ws.len[m], s_via, s_flags);
         if (tid < 4) atomicAdd(&stats[tid], ws.stats[4 * m + tid]);
         if (tid == 0) pa.net_status[k] = 0;
         __syncthreads();
@@ -1625,40 +1313,66 @@ window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa,
           rc = apply_path_dev(g, st, t.store_path + (int64_t)n * t.slot_cap, ol, t.net_id[n], +1, pa.pres_fac,
                               pa.live, nullptr, s_via, s_flags);
       }
-      const int32_t kf = ws.k[ff], nf = pa.order[kf];
-      if (defer) {
-        if (tid == 0 && rc != OGR_OK) atomicExch(&c->error, rc);
-      } else {
-      if (tid < 4) atomicAdd(&stats[tid], ws.stats[4 * ff + tid]);
-      if (tid == 0) t.store_len[nf] = 0;
-      __syncthreads();
-      int flags = 0, fin = ws.st[ff], len = 0;
-      const int used = (int)w.result[2];
-      if (rc == OGR_OK && fin != OGR_OK && used < pa.fallback_quota) {
-        const ogr_net_args a = ogr_pass_net_args(t, pa, nf, 1);
-        search_net<L>(sh, g, st, a, w, t.store_path + (int64_t)nf * t.slot_cap, t.slot_cap, stats);
-        fin = sh.status;
-        len = sh.len;
-        flags |= 2;
-        if (tid == 0) w.result[2] = used + 1;
-        if (fin < 0) rc = fin;
+      if (!defer) {
+        // its fallback's ROI; a team searches it below
+        const int32_t kf = ws.k[ff], nf = pa.order[kf];
+        if (tid < 4) atomicAdd(&stats[tid], ws.stats[4 * ff + tid]);
+        if (tid == 0) t.store_len[nf] = 0;
+        __syncthreads();
+        if (rc == OGR_OK) {
+          const ogr_net_args a = ogr_pass_net_args(t, pa, nf, 1);
+          build_roi(sh, g, a, w);
+          rc = sh.status;
+          if (tid == 0) {
+            c->solo_R = sh.R;
+            c->fb = 1 + kf;
+          }
+        }
       }
-      __syncthreads();
-      if (rc == OGR_OK && fin == OGR_OK) {
-        rc = apply_path_dev(g, st, t.store_path + (int64_t)nf * t.slot_cap, len, t.net_id[nf], +1, pa.pres_fac,
-                            pa.live, t.store_arcs + (int64_t)nf * 2 * t.slot_cap, s_via, s_flags);
-        if (tid == 0 && rc == OGR_OK) t.store_len[nf] = len;
-      } else {
-        flags |= 1;
-      }
-      if (tid == 0) {
-        pa.net_status[kf] = flags;
-        if (rc != OGR_OK) atomicExch(&c->error, rc);
-      }
+      if (tid == 0 && rc != OGR_OK) atomicExch(&c->error, rc);
+    }
+    if (!win_barrier(c, target, &s_bar)) break;
+    if (*(volatile int32_t*)&c->error) break;
+    const int fb = *(volatile int32_t*)&c->fb;
+    if (fb == 0) continue;
+    // 5. the fallback of the failed net
+    const int32_t kf = fb - 1, nf = pa.order[kf];
+    const int Tf = min(kTeam, G);
+    if (b < Tf) {
+      const ogr_net_args a = ogr_pass_net_args(t, pa, nf, 1);
+      const RoiJob job{&g, &st, &a, &w, w.roi, *(volatile int32_t*)&c->solo_R, nullptr, nullptr,
+                       t.store_path + (int64_t)nf * t.slot_cap, t.slot_cap, stats, b, Tf};
+      int status, len;
+      roi_search_row<ROW, false>(job, smem, &status, &len);
+      if (tid == 0 && b == 0) {
+        c->fb_st = status;
+        c->fb_len = len;
+        w.result[2] = w.result[2] + 1;
+        if (status < 0) atomicExch(&c->error, status);
       }
     }
     if (!win_barrier(c, target, &s_bar)) break;
     if (*(volatile int32_t*)&c->error) break;
+    if (b == 0) {
+      const int fin = *(volatile int32_t*)&c->fb_st, len = *(volatile int32_t*)&c->fb_len;
+      int flags = 2;
+      if (fin == OGR_OK) {
+        const int rc = apply_path_dev(g, st, t.store_path + (int64_t)nf * t.slot_cap, len, t.net_id[nf], +1,
+                                      pa.pres_fac, pa.live, t.store_arcs + (int64_t)nf * 2 * t.slot_cap, s_via,
+                                      s_flags);
+        if (tid == 0) {
+          if (rc == OGR_OK) t.store_len[nf] = len;
+          else atomicExch(&c->error, rc);
+        }
+      } else {
+        flags |= 1;
+      }
+      if (tid == 0) pa.net_status[kf] = flags;
+      clear_team(w.ctl);
+    }
+    // (the next window's first barrier orders this before anyone reads it;
+    // c->fb is cleared by CTA 0 only then, after every CTA has read it)
+    if (!win_barrier(c, target, &s_bar)) break;
   }
   if (b == 0 && tid == 0) {
     if (*(volatile int32_t*)&c->bar_err) w.result[0] = OGR_ERR_TIMEOUT;
@@ -1670,8 +1384,10 @@ __global__ void window_ws_init_kernel(char* base, int32_t slots, size_t slot_byt
   for (int32_t sidx = 0; sidx < slots; ++sidx) {
     Ws t;
     ws_slot_layout(N, rmax, base + (size_t)sidx * slot_bytes, &t);
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x)
-      t.g2r[i] = -1;
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = i0; i < N; i += step) t.g2r[i] = -1;
+    for (int64_t i = i0; i < rmax; i += step) t.claim[i] = 0;
+    for (int64_t i = i0; i < (int64_t)(sizeof(SlotCtl) / 4); i += step) reinterpret_cast<int32_t*>(t.ctl)[i] = 0;
   }
 }
 
@@ -1696,14 +1412,16 @@ pass_ripup_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa, 
 }
 
 // After the whole-lattice search of net order[k]: the fallback ROI search if
-// it failed and the pass has fallbacks left, then the commit.
-template <int L>
+// it failed and the pass has fallbacks left (at most five of a pass, by this
+// one CTA), then the commit.
+template <int ROW>
 __global__ void __launch_bounds__(kThreads, 1)
 pass_full_tail_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa, int32_t k, Ws w,
                       const int32_t* full_res) {
+  extern __shared__ __align__(16) char smem[];
   __shared__ Shared sh;
-  __shared__ int32_t s_via[kMaxViaNodes];
   __shared__ int s_flags[2];
+  int32_t* s_via = reinterpret_cast<int32_t*>(smem);
   if (w.result[0] < 0) return;
   const int32_t n = pa.order[k];
   int32_t* slot = t.store_path + (int64_t)n * t.slot_cap;
@@ -1718,14 +1436,21 @@ pass_full_tail_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args 
   const int used = (int)w.result[2];
   if (fin != OGR_OK && used < pa.fallback_quota) {
     const ogr_net_args a = ogr_pass_net_args(t, pa, n, 1);
-    search_net<L>(sh, g, st, a, w, slot, t.slot_cap, reinterpret_cast<unsigned long long*>(pa.stats));
+    build_roi(sh, g, a, w);
     fin = sh.status;
-    len = sh.len;
+    if (fin == OGR_OK) {
+      clear_team(w.ctl);
+      __syncthreads();
+      const RoiJob job{&g, &st, &a, &w, w.roi, sh.R, nullptr, nullptr, slot, t.slot_cap,
+                       reinterpret_cast<unsigned long long*>(pa.stats), 0, 1};
+      roi_search_row<ROW, false>(job, smem, &fin, &len);
+    }
     if (fin < 0) {
       if (threadIdx.x == 0) w.result[0] = fin;
       return;
     }
     flags |= 2;
+    __syncthreads();
     if (threadIdx.x == 0) w.result[2] = used + 1;
   }
   __syncthreads();
@@ -1740,6 +1465,45 @@ pass_full_tail_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args 
     flags |= 1;
   }
   if (threadIdx.x == 0) pa.net_status[k] = flags;
+}
+
+// Variants by the arcs of a row (phases.cuh).
+#define OGR_WITH_ROW(ROWV, g, ...)                             \
+  do {                                                         \
+    switch (ogr_full::row_for(g)) {                            \
+      case 4: { constexpr int ROWV = 4; __VA_ARGS__; } break;  \
+      case 8: { constexpr int ROWV = 8; __VA_ARGS__; } break;  \
+      case 16: { constexpr int ROWV = 16; __VA_ARGS__; } break;\
+      default: { constexpr int ROWV = 32; __VA_ARGS__; } break;\
+    }                                                          \
+  } while (0)
+
+// A cooperative launch of `grid` CTAs, all of them resident.
+int launch_team(const void* f, int grid, void** args, cudaStream_t s) {
+  OGR_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ogr_phase::kSmemBytes));
+  OGR_CUDA_TRY(cudaLaunchCooperativeKernel(f, dim3(grid), dim3(kThreads), args, ogr_phase::kSmemBytes, s));
+  return OGR_OK;
+}
+
+// The search of a net in workspace w (ROI built here if roi is NULL) on s.
+int launch_find(const ogr_graph& g, const ogr_state& st, const ogr_net_args& a, const Ws& w, const int32_t* roi,
+                int32_t R, const float* roi_pen, const MultiSeeds* ms, int32_t* path_out, int32_t path_cap,
+                int64_t* stats, cudaStream_t s) {
+  OGR_CUDA_TRY(cudaMemsetAsync(&w.ctl->team, 0, sizeof(ogr_phase::Ctl), s));
+  if (roi == nullptr && !a.full_graph) {
+    build_roi_kernel<<<1, kThreads, 0, s>>>(g, a, w);
+    OGR_LAUNCH_CHECK();
+  }
+  if (a.full_graph) R = g.num_nodes;
+  ogr_graph gv = g;
+  ogr_state sv = st;
+  ogr_net_args av = a;
+  Ws wv = w;
+  MultiSeeds mv = ms ? *ms : MultiSeeds{};
+  void* args[] = {&gv, &sv, &av, &wv, &roi, &R, &roi_pen, &mv, &path_out, &path_cap, &stats};
+  const void* f = nullptr;
+  OGR_WITH_ROW(ROW, g, f = ms ? (const void*)find_team_kernel<ROW, true> : (const void*)find_team_kernel<ROW, false>);
+  return launch_team(f, kTeam, args, s);
 }
 
 }  // namespace
@@ -1772,6 +1536,8 @@ extern "C" int ogr_window_workspace_init(void* ws, int32_t num_nodes, int32_t ma
   OGR_LAUNCH_CHECK();
   return OGR_OK;
 }
+
+static_assert(sizeof(SlotCtl) % 4 == 0, "cleared as words");
 
 extern "C" size_t ogr_window_ctl_bytes(int32_t slots) { return win_ctl_layout(slots, nullptr, nullptr, nullptr); }
 
@@ -1817,8 +1583,8 @@ extern "C" int ogr_find_path(const ogr_graph* g, const ogr_state* st, const ogr_
   Ws w;
   ws_layout(g->num_nodes, (char*)ws, &w);
   cudaStream_t s = ogr_stream(stream);
-  OGR_WITH_LANES(L, find_path_kernel<L><<<1, kThreads, 0, s>>>(*g, *st, *net, w, path_out, path_cap, stats));
-  OGR_LAUNCH_CHECK();
+  const int rc = launch_find(*g, *st, *net, w, nullptr, 0, nullptr, nullptr, path_out, path_cap, stats, s);
+  if (rc != OGR_OK) return rc;
   int64_t res[2];
   OGR_CUDA_TRY(cudaMemcpyAsync(res, w.result, sizeof(res), cudaMemcpyDeviceToHost, s));
   OGR_CUDA_TRY(cudaStreamSynchronize(s));
@@ -1847,9 +1613,8 @@ extern "C" int ogr_find_path_roi(const ogr_graph* g, const float* costs, const i
   a.full_graph = 0;
   a.penalty_enabled = 0;
   cudaStream_t s = ogr_stream(stream);
-  OGR_WITH_LANES(L, find_path_given_roi_kernel<L><<<1, kThreads, 0, s>>>(*g, st, a, w, roi_nodes, n_roi, roi_penalty,
-                                                                          path_out, path_cap, stats));
-  OGR_LAUNCH_CHECK();
+  const int rc = launch_find(*g, st, a, w, roi_nodes, n_roi, roi_penalty, nullptr, path_out, path_cap, stats, s);
+  if (rc != OGR_OK) return rc;
   int64_t res[2];
   OGR_CUDA_TRY(cudaMemcpyAsync(res, w.result, sizeof(res), cudaMemcpyDeviceToHost, s));
   OGR_CUDA_TRY(cudaStreamSynchronize(s));
@@ -1893,9 +1658,8 @@ extern "C" int ogr_find_path_multi(const ogr_graph* g, const float* costs, const
   a.full_graph = 0;
   a.penalty_enabled = 0;
   cudaStream_t s = ogr_stream(stream);
-  OGR_WITH_LANES(L, find_path_multi_kernel<L><<<1, kThreads, 0, s>>>(*g, st, a, w, roi_nodes, n_roi, roi_penalty, ms,
-                                                                      path_out, path_cap, stats));
-  OGR_LAUNCH_CHECK();
+  const int rc = launch_find(*g, st, a, w, roi_nodes, n_roi, roi_penalty, &ms, path_out, path_cap, stats, s);
+  if (rc != OGR_OK) return rc;
   int64_t res[2];
   OGR_CUDA_TRY(cudaMemcpyAsync(res, w.result, sizeof(res), cudaMemcpyDeviceToHost, s));
   OGR_CUDA_TRY(cudaStreamSynchronize(s));
@@ -1949,29 +1713,6 @@ extern "C" int ogr_path_apply(const ogr_graph* g, const ogr_state* st, const int
   return OGR_OK;
 }
 
-// Window-pass grid size: one 1024-thread CTA per SM, at most `slots`.
-template <int L>
-static int window_grid_for(int slots) {
-  static int per_dev[64] = {};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
-  if (per_dev[dev] == 0) {
-    int sms = 0, per_sm = 0, coop = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, window_pass_kernel<L>, kThreads, 0) != cudaSuccess)
-      return 0;
-    per_dev[dev] = sms * per_sm;
-  }
-  return slots < per_dev[dev] ? slots : per_dev[dev];
-}
-
-static int window_grid(int slots) {
-  int grid = 0;
-  OGR_WITH_LANES(L, grid = window_grid_for<L>(slots));
-  return grid;
-}
-
 extern "C" int ogr_route_pass(const ogr_graph* g, const ogr_state* st, const ogr_net_table* t,
                               const ogr_pass_args* pa, const ogr_roi_batch* rb, void* ws, size_t bytes,
                               const uint8_t* order_full, void* full_ws, size_t full_bytes,
@@ -2006,22 +1747,23 @@ extern "C" int ogr_route_pass(const ogr_graph* g, const ogr_state* st, const ogr
     OGR_LAUNCH_CHECK();
   }
   const bool windows = win != nullptr && win->slots > 0 && batch && rbv.roi_box != nullptr;
-  int grid = 0;
+  // CTAs: one team per window member, within this host thread's share of the
+  // SMs (ogr_full_grid)
+  const int share = ogr_full::grid_blocks();
+  if (share < 1) return OGR_ERR_CUDA;
+  int nslots = 0;
   if (windows) {
     if (!win->ws || !win->scratch || !win->ctl ||
         win->slot_bytes < ogr_window_workspace_bytes(g->num_nodes, pa->max_roi_nodes, 1))
       return OGR_ERR_ARG;
-    grid = window_grid(win->slots);
-    if (grid < 1) return OGR_ERR_CUDA;
+    nslots = win->slots < share ? win->slots : share;
   }
+  const int64_t want = (int64_t)(nslots > 0 ? nslots : 1) * kTeam;
+  const int grid = want < share ? (int)want : share;
   // one run of ROI nets: batched windows, or the single-CTA sequential pass
   auto roi_segment = [&](const ogr_pass_args& seg) -> int {
-    if (!windows) {
-      OGR_WITH_LANES(L, route_pass_kernel<L><<<1, kThreads, 0, s>>>(*g, *st, *t, seg, rbv, batch ? 1 : 0, w));
-      OGR_LAUNCH_CHECK();
-      return OGR_OK;
-    }
-    OGR_CUDA_TRY(cudaMemsetAsync(win->ctl, 0, ogr_window_ctl_bytes(grid), s));
+    char* ctl = windows ? (char*)win->ctl : w.win1;
+    OGR_CUDA_TRY(cudaMemsetAsync(ctl, 0, ogr_window_ctl_bytes(nslots > 0 ? nslots : 1), s));
     // every net of the segment starts pending (-1); the window pass sets its status when done
     OGR_CUDA_TRY(cudaMemsetAsync(seg.net_status, 0xff, sizeof(int32_t) * (size_t)seg.count, s));
     int32_t lookv = g_window_look < 0 ? 0 : (g_window_look > kMaxSkip ? kMaxSkip : g_window_look);
@@ -2029,20 +1771,18 @@ extern "C" int ogr_route_pass(const ogr_graph* g, const ogr_state* st, const ogr
     ogr_state sv = *st;
     ogr_net_table tv = *t;
     ogr_pass_args pv = seg;
-    char* slot_base = (char*)win->ws;
-    size_t slot_bytes = win->slot_bytes;
-    int32_t rmax = pa->max_roi_nodes < g->num_nodes ? pa->max_roi_nodes : g->num_nodes;
-    int32_t* scratch = win->scratch;
-    char* ctl = (char*)win->ctl;
+    int use_batch = batch ? 1 : 0;
+    char* slot_base = windows ? (char*)win->ws : nullptr;
+    size_t slot_bytes = windows ? win->slot_bytes : 0;
+    int32_t rmax = need_cap;
+    int32_t* scratch = windows ? win->scratch : nullptr;
     Ws wv = w;
-    unsigned long long* discarded = reinterpret_cast<unsigned long long*>(win->discarded);
-    void* args[] = {&gv, &sv, &tv, &pv, &rbv, &slot_base, &slot_bytes, &rmax, &scratch, &ctl, &wv, &lookv,
-                    &discarded};
+    unsigned long long* discarded = windows ? reinterpret_cast<unsigned long long*>(win->discarded) : nullptr;
+    void* args[] = {&gv, &sv, &tv, &pv, &rbv, &use_batch, &slot_base, &slot_bytes, &rmax, &nslots, &scratch, &ctl,
+                    &wv, &lookv, &discarded};
     const void* wk = nullptr;
-    OGR_WITH_LANES(L, wk = (const void*)window_pass_kernel<L>);
-    OGR_CUDA_TRY(cudaLaunchCooperativeKernel(wk, dim3(grid), dim3(kThreads), args, 0,
-                                             s));
-    return OGR_OK;
+    OGR_WITH_ROW(ROW, *g, wk = (const void*)window_pass_kernel<ROW>);
+    return launch_team(wk, grid, args, s);
   };
   if (!any_full) {
     const int rc = roi_segment(*pa);
@@ -2065,7 +1805,11 @@ extern "C" int ogr_route_pass(const ogr_graph* g, const ogr_state* st, const ogr
         job.stats = reinterpret_cast<unsigned long long*>(pa->stats);
         const int rc = ogr_full::launch(*g, *st, job, full_ws, s);
         if (rc != OGR_OK) return rc;
-        OGR_WITH_LANES(L, pass_full_tail_kernel<L><<<1, kThreads, 0, s>>>(*g, *st, *t, *pa, k, w, full_res));
+        OGR_WITH_ROW(ROW, *g, {
+          OGR_CUDA_TRY(cudaFuncSetAttribute(pass_full_tail_kernel<ROW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)ogr_phase::kSmemBytes));
+          pass_full_tail_kernel<ROW><<<1, kThreads, ogr_phase::kSmemBytes, s>>>(*g, *st, *t, *pa, k, w, full_res);
+        });
         OGR_LAUNCH_CHECK();
         ++k;
       } else {
@@ -2138,10 +1882,10 @@ extern "C" int ogr_find_path_noalloc(const ogr_graph* g, const ogr_state* st, co
   Ws w;
   ws_layout(g->num_nodes, (char*)base, &w);
   cudaStream_t s = ogr_stream(stream);
-  // The array keeps whatever the previous call left: clear seen[] / g2r[].
+  // The array keeps whatever the previous call left: clear seen[] / g2r[] / claims.
   ws_init_kernel<<<ogr_blocks(g->num_nodes, 256), 256, 0, s>>>(w, g->num_nodes);
-  OGR_WITH_LANES(L, find_path_kernel<L><<<1, kThreads, 0, s>>>(*g, *st, *net, w, path_out, path_cap, stats));
-  OGR_LAUNCH_CHECK();
+  const int rc = launch_find(*g, *st, *net, w, nullptr, 0, nullptr, nullptr, path_out, path_cap, stats, s);
+  if (rc != OGR_OK) return rc;
   int64_t res[2];
   OGR_CUDA_TRY(cudaMemcpyAsync(res, w.result, sizeof(res), cudaMemcpyDeviceToHost, s));
   OGR_CUDA_TRY(cudaStreamSynchronize(s));

@@ -88,8 +88,10 @@ def test_team_sizes_match_oracle(ctas, kind):
 
 
 @pytest.mark.parametrize("seed_costs", [(0.0, 0.25, 1.5), (0.1, 0.30000001, 1e-9), (0.0, 5.0e6, 0.5)])
-def test_seed_costs_match_oracle(seed_costs):
-    g, s, ops, ref = make(30, 26, 6)
+@pytest.mark.parametrize("row", [6, 22, 40])
+def test_seed_costs_match_oracle(seed_costs, row):
+    dims, kw = ROWS[row]
+    g, s, ops, ref = make(*dims, **kw)
     rng = np.random.default_rng(5)
     costs = values("ties", g.E, rng)
     s.total_cost.copy_(torch.from_numpy(costs))
@@ -100,3 +102,58 @@ def test_seed_costs_match_oracle(seed_costs):
         targets = [(int(n), float(c)) for n, c in zip(rng.choice(g.N, size=4, replace=False), rng.random(4))]
         want = find_path_multisource(ref.indptr, ref.indices, seeds, targets, costs, ident, ident, plane=ref.plane)
         assert ops.find_path_full_multi(seeds, targets, net) == (tuple(want) if want else None)
+
+
+@pytest.mark.parametrize("row", sorted(ROWS))
+@pytest.mark.parametrize("kind", ["ties", "some small", "large"])
+def test_roi_forms_match_oracle(row, kind):
+    """The ROI search (a team of CTAs) in every form, on shuffled partial ROIs whose order is the tie order."""
+    dims, kw = ROWS[row]
+    g, s, ops, ref = make(*dims, **kw)
+    rng = np.random.default_rng(row + 100)
+    costs = values(kind, g.E, rng)
+    dev = torch.from_numpy(costs).to(g.device)
+    for case in range(4):
+        roi = np.flatnonzero(rng.random(g.N) < 0.85).astype(np.int32)
+        if case % 2:
+            rng.shuffle(roi)
+        g2r = np.full(g.N, -1, dtype=np.int32)
+        g2r[roi] = np.arange(roi.size, dtype=np.int32)
+        pen = (rng.integers(0, 3, size=roi.size) * 0.5).astype(np.float32) if case >= 2 else None
+        src, dst = (int(v) for v in rng.choice(roi, size=2, replace=False))
+        st = {}
+        want = find_path_roi_c(ref.indptr, ref.indices, src, dst, costs, roi, g2r, node_penalty=pen, stats=st)
+        ops.stats.zero_()
+        assert ops.find_path_given_roi(src, dst, dev, roi, pen) == want
+        assert ops.stats.cpu().tolist()[:3] == [st["scanned"], st["settled"], roi.size]
+        seeds = [(int(n), float(c)) for n, c in zip(rng.choice(g.N, size=3, replace=False), rng.random(3))]
+        targets = [(int(n), float(c)) for n, c in zip(rng.choice(g.N, size=5, replace=False), rng.random(5))]
+        want = find_path_multisource(ref.indptr, ref.indices, seeds, targets, costs, roi, g2r, node_penalty=pen,
+                                     plane=ref.plane)
+        got = ops.find_path_multi(seeds, targets, dev, roi, pen)
+        assert got == (tuple(want) if want else None)
+
+
+@pytest.mark.parametrize("dims,max_nodes,depth,blocked", [
+    ((150, 140, 8), 50_000, 80, False),      # the box fits and the search stays in it
+    ((33, 200, 6), 50_000, 80, True),        # one axis cut off by the lattice's edge, blocked arcs
+    ((260, 250, 16), 400_000, 80, False),    # the box is cut to fit and the search leaves it
+    ((64, 64, 4), 900, 80, False),           # truncated, terminals swapped in
+    ((90, 70, 6), 50_000, 3, False),         # the waves do not meet
+])
+def test_roi_extraction_matches_oracle(dims, max_nodes, depth, blocked):
+    from oracle.roi import extract_roi_bfs
+    g, s, ops, ref = make(*dims)
+    rng = np.random.default_rng(dims[0])
+    mask = None
+    if blocked:
+        mask = rng.random(g.E) < 0.2
+        g.blocked = torch.from_numpy(mask.astype(np.uint8)).to(g.device)
+    for k in range(3):
+        src, dst = (int(v) for v in rng.integers(0, ref.plane, size=2))
+        if k == 2:
+            dst = src
+        want, _ = extract_roi_bfs(ref.indptr, ref.indices, g.N, src, dst, initial_radius=depth, blocked=mask,
+                                  max_nodes=max_nodes)
+        net = ops.net_args(0, src, dst, max_depth=depth, halo=2, max_roi_nodes=max_nodes)
+        np.testing.assert_array_equal(ops.extract_roi(net), want)
