@@ -187,6 +187,7 @@ struct Shared {
   int nq[4];
   int seen_count;
   int met;
+  int left;        // the BFS left its box
   int overflow;
   int bx0, bx1, by0, by1;
   int pos_src, pos_dst;
@@ -208,11 +209,259 @@ struct StageClock {
 };
 
 // ---- ROI extraction ---------------------------------------------------------
-// Bidirectional BFS from src/dst on seen[] (all zero on entry, restored to
-// zero on exit) with queues of qcap entries; writes the ROI (ascending id,
+// Cuts the ROI of sh.R nodes in out[0..out_cap) to max_roi_nodes; sh.pos_src /
+// sh.pos_dst are the terminals' positions.  Thread 0; sh.status =
+// OGR_ERR_CAPACITY when a queue overflowed or out is too small.
+__device__ void roi_finish(Shared& sh, const ogr_net_args& a, int32_t* out, int32_t out_cap) {
+  if (threadIdx.x != 0) return;
+  const int32_t src = a.src, dst = a.dst;
+  int R = sh.R;
+  if (R > a.max_roi_nodes) {
+    // Must-keep swap (extract_roi_bfs :2359-2379): the positions of src/dst
+    // in ascending order; each one beyond the cut swaps with slot 0 / 1.
+    int kp[2];
+    int32_t kn[2];
+    int nk = 0;
+    if (src == dst) {
+      kp[0] = sh.pos_src; kn[0] = src; nk = 1;
+    } else {
+      const bool s_first = sh.pos_src < sh.pos_dst;
+      kp[0] = s_first ? sh.pos_src : sh.pos_dst; kn[0] = s_first ? src : dst;
+      kp[1] = s_first ? sh.pos_dst : sh.pos_src; kn[1] = s_first ? dst : src;
+      nk = 2;
+    }
+    for (int k = 0; k < nk; ++k)
+      if (kp[k] >= a.max_roi_nodes) out[k] = kn[k];
+    R = a.max_roi_nodes;
+  }
+  sh.R = R;
+  if (sh.overflow || R > out_cap) sh.status = OGR_ERR_CAPACITY;
+  atomicAdd(&g_stage[12], (unsigned long long)R);
+}
+
+// Division by a fixed d > 0 of any v < 2^32: the high product with
+// floor(2^32 / d) is the quotient or one less.
+struct Div {
+  unsigned d, m;
+  __device__ explicit Div(unsigned dd) : d(dd), m(dd > 1 ? (unsigned)((1ull << 32) / dd) : 0xffffffffu) {}
+  __device__ unsigned operator()(unsigned v) const {
+    const unsigned q = __umulhi(v, m);
+    return v - q * d >= d ? q + 1 : q;
+  }
+};
+
+// Shared memory of a BFS: the four queues' first kBfsQ entries, then two
+// bitmaps of the box around both terminals.
+constexpr int kBfsQ = 4096;
+constexpr int kBfsArcs = 6;                    // arcs of a row that one of a node's two lanes loads at once
+constexpr size_t kBfsQBytes = 4 * kBfsQ * sizeof(int32_t);
+constexpr int kBfsWords = (int)((ogr_phase::kSmemBytes - kBfsQBytes) / 8);     // words per bitmap
+
+// Bidirectional BFS from src/dst on two bitmaps (bit set: seen by that wave;
+// both: where the waves met) of a box in shared memory; writes the ROI
+// (ascending id, truncated with the must-keep swap) into out[0..out_cap) and
+// its size into sh.R.  False: the search left the box (the caller takes
+// roi_build_large).
+//
+// A wave step is two dependent round trips (row bounds, row) for up to 256
+// nodes at once; marks, queues and the compaction never leave the SM.  With
+// the marks as compare-and-swaps in global memory (a third round trip and an
+// atomic per arc) an ROI of 50,000 nodes on 600x400x12 took 1,352 us and its
+// compaction 250; now 600 and 60.
+__device__ bool roi_build_box(Shared& sh, const ogr_graph& g, const ogr_net_args& a, int32_t* const* q, int64_t qcap,
+                              int32_t* out, int32_t out_cap, char* smem, StageClock& clk) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nx = g.nx, ny = g.ny, nz = g.nz;
+  const int32_t src = a.src, dst = a.dst;
+  const int32_t* __restrict__ indptr = g.indptr;
+  const int32_t* __restrict__ indices = g.indices;
+  const Div by_plane((unsigned)(nx * ny)), by_nx((unsigned)nx);
+  int32_t* sq = reinterpret_cast<int32_t*>(smem);
+  unsigned* bits[2] = {reinterpret_cast<unsigned*>(smem + kBfsQBytes),
+                       reinterpret_cast<unsigned*>(smem + kBfsQBytes) + kBfsWords};
+  auto coord = [&](int32_t v, int& x, int& y, int& z) {
+    z = (int)by_plane((unsigned)v);
+    const unsigned r = (unsigned)v - (unsigned)z * by_plane.d;
+    y = (int)by_nx(r);
+    x = (int)(r - (unsigned)y * by_nx.d);
+  };
+  int sx, sy, sz, dx, dy, dz;
+  coord(src, sx, sy, sz);
+  coord(dst, dx, dy, dz);
+  // the deepest search whose box fits (an arc leads at most one cell aside)
+  int reach = a.bfs_max_depth, X0, Y0, BW, BH, RW;
+  for (;; --reach) {
+    X0 = max(0, min(sx, dx) - reach);
+    Y0 = max(0, min(sy, dy) - reach);
+    BW = min(nx - 1, max(sx, dx) + reach) - X0 + 1;
+    BH = min(ny - 1, max(sy, dy) + reach) - Y0 + 1;
+    RW = (BW + 31) >> 5;
+    if ((int64_t)RW * BH * nz <= kBfsWords) break;
+    if (reach <= 0) return false;
+  }
+  const int NW = RW * BH * nz;
+  for (int i = tid; i < NW; i += kThreads) bits[0][i] = bits[1][i] = 0u;
+  if (tid == 0) {
+    sh.nq[0] = sh.nq[2] = 1;
+    sq[0] = src;
+    sq[2 * kBfsQ] = dst;
+    sh.overflow = 0;
+    sh.met = 0;
+    sh.pos_src = -1;
+    sh.pos_dst = -1;
+    sh.bx0 = min(sx, dx); sh.bx1 = max(sx, dx);
+    sh.by0 = min(sy, dy); sh.by1 = max(sy, dy);
+    sh.left = 0;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    if (src != dst) bits[0][(sz * BH + (sy - Y0)) * RW + ((sx - X0) >> 5)] |= 1u << ((sx - X0) & 31);
+    bits[1][(dz * BH + (dy - Y0)) * RW + ((dx - X0) >> 5)] |= 1u << ((dx - X0) & 31);
+  }
+  int depth = 0, meet = -1;
+  int64_t seen = src != dst ? 2 : 1;
+  int cur_s = 0, cur_d = 2;
+  int lx0 = 1 << 30, lx1 = -1, ly0 = 1 << 30, ly1 = -1;
+  __syncthreads();
+  while (depth < a.bfs_max_depth && (sh.nq[cur_s] > 0 || sh.nq[cur_d] > 0)) {
+    for (int wave = 0; wave < 2; ++wave) {
+      const int cur = wave == 0 ? cur_s : cur_d, nxt = cur ^ 1;
+      unsigned* mine = bits[wave];
+      const unsigned* other = bits[wave ^ 1];
+      const int n = (int)min((int64_t)sh.nq[cur], qcap);
+      if (tid == 0) sh.nq[nxt] = 0;
+      __syncthreads();
+      int met = 0;
+      for (int base = warp * 16; base < n; base += kWarps * 16) {
+        const int i = base + (lane >> 1);
+        int32_t f = 0, f1 = 0;
+        if (i < n) {
+          const int32_t u = i < kBfsQ ? sq[cur * kBfsQ + i] : q[cur][i];
+          f = indptr[u] + (lane & 1);
+          f1 = indptr[u + 1];
+        }
+        while (__any_sync(0xffffffffu, f < f1)) {
+          int32_t v[kBfsArcs];
+#pragma unroll
+          for (int j = 0; j < kBfsArcs; ++j) {
+            const int32_t e = f + 2 * j;
+            v[j] = e < f1 && !(g.blocked != nullptr && g.blocked[e]) ? indices[e] : -1;
+          }
+#pragma unroll
+          for (int j = 0; j < kBfsArcs; ++j) {
+            bool fresh = false;
+            if (v[j] >= 0) {
+              int x, y, z;
+              coord(v[j], x, y, z);
+              const int bx = x - X0, by = y - Y0;
+              if ((unsigned)bx >= (unsigned)BW || (unsigned)by >= (unsigned)BH) {
+                sh.left = 1;
+              } else {
+                const int wd = (z * BH + by) * RW + (bx >> 5);
+                const unsigned bit = 1u << (bx & 31);
+                if (!(mine[wd] & bit) && !(atomicOr(&mine[wd], bit) & bit)) {
+                  if (other[wd] & bit) {
+                    met = 1;
+                  } else {
+                    fresh = true;
+                    lx0 = min(lx0, x); lx1 = max(lx1, x);
+                    ly0 = min(ly0, y); ly1 = max(ly1, y);
+                  }
+                }
+              }
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, fresh);
+            if (m) {
+              int p = 0;
+              if (lane == 0) p = atomicAdd(&sh.nq[nxt], __popc(m));
+              p = __shfl_sync(0xffffffffu, p, 0) + __popc(m & ((1u << lane) - 1u));
+              if (fresh) {
+                if (p < kBfsQ) sq[nxt * kBfsQ + p] = v[j];
+                else if (p < qcap) q[nxt][p] = v[j];
+                else sh.overflow = 1;
+              }
+            }
+          }
+          f += 2 * kBfsArcs;
+        }
+      }
+      if (met) sh.met = 1;
+      __syncthreads();
+      seen += sh.nq[nxt];
+      if (wave == 0) cur_s = nxt; else cur_d = nxt;
+    }
+    ++depth;
+    if (tid == 0) atomicAdd(&g_stage[11], 2ull);
+    if (sh.left) return false;     // uniform: read after the wave's barrier, written before it
+    if (sh.met && meet < 0) meet = depth;
+    if (meet >= 0 && depth >= meet + a.bfs_halo) break;
+    if ((double)seen > a.bfs_stop_count) break;
+    if (sh.overflow) break;
+    __syncthreads();               // (the next wave resets what was read here)
+  }
+  lx0 = __reduce_min_sync(0xffffffffu, lx0);
+  lx1 = __reduce_max_sync(0xffffffffu, lx1);
+  ly0 = __reduce_min_sync(0xffffffffu, ly0);
+  ly1 = __reduce_max_sync(0xffffffffu, ly1);
+  if (lane == 0) {
+    atomicMin(&sh.bx0, lx0); atomicMax(&sh.bx1, lx1);
+    atomicMin(&sh.by0, ly0); atomicMax(&sh.by1, ly1);
+  }
+  __syncthreads();
+  clk.mark(0);
+  // Ordered compaction (ascending global id): each warp owns a contiguous run
+  // of words; count, scan the counts, then write.  Only positions below
+  // out_cap are stored; those of src and dst are recorded.
+  const int per = ((NW + kWarps - 1) / kWarps + 31) & ~31;
+  const int w0 = warp * per, w1 = min(NW, w0 + per);
+  int cnt = 0;
+  for (int i = w0 + lane; i < w1; i += 32) cnt += __popc(bits[0][i] | bits[1][i]);
+  cnt = __reduce_add_sync(0xffffffffu, cnt);
+  if (lane == 0) sh.s_cnt[warp] = cnt;
+  __syncthreads();
+  if (tid == 0) {
+    int t = 0;
+    for (int i = 0; i < kWarps; ++i) {
+      sh.s_off[i] = t;
+      t += sh.s_cnt[i];
+    }
+    sh.R = t;
+  }
+  __syncthreads();
+  int off = sh.s_off[warp];
+  const Div by_rw((unsigned)RW), by_bh((unsigned)BH);
+  for (int i0 = w0; i0 < w1; i0 += 32) {
+    const unsigned word = i0 + lane < w1 ? bits[0][i0 + lane] | bits[1][i0 + lane] : 0u;
+    unsigned some = __ballot_sync(0xffffffffu, word != 0u);
+    while (some) {
+      const int k = __ffs(some) - 1;
+      some &= some - 1;
+      const unsigned b = __shfl_sync(0xffffffffu, word, k);
+      const unsigned row = by_rw((unsigned)(i0 + k)), z = by_bh(row);
+      const int32_t first = (int32_t)(z * by_plane.d + (unsigned)(Y0 + (int)(row - z * by_bh.d)) * by_nx.d) + X0 +
+                            32 * (int)(i0 + k - row * by_rw.d);
+      if ((b >> lane) & 1u) {
+        const int pos = off + __popc(b & ((1u << lane) - 1u));
+        const int32_t gid = first + lane;
+        if (pos < out_cap) out[pos] = gid;
+        if (gid == src) sh.pos_src = pos;
+        if (gid == dst) sh.pos_dst = pos;
+      }
+      off += __popc(b);
+    }
+  }
+  __syncthreads();
+  roi_finish(sh, a, out, out_cap);
+  __syncthreads();
+  clk.mark(1);
+  return true;
+}
+
+// The same BFS for boxes that shared memory cannot hold, on seen[] (all zero on
+// entry, restored to zero on exit) with queues of qcap entries; writes the ROI (ascending id,
 // truncated with the must-keep swap) into out[0..out_cap) and its size into
 // sh.R.  sh.status = OGR_ERR_CAPACITY when a queue overflowed.
-__device__ void roi_build(Shared& sh, const ogr_graph& g, const ogr_net_args& a, int32_t* seen, int32_t* const* q,
+__device__ __noinline__ void roi_build_large(Shared& sh, const ogr_graph& g, const ogr_net_args& a, int32_t* seen, int32_t* const* q,
                           int64_t qcap, int32_t* out, int32_t out_cap, StageClock& clk) {
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
@@ -358,34 +607,18 @@ __device__ void roi_build(Shared& sh, const ogr_graph& g, const ogr_net_args& a,
     off += __popc(m);
   }
   __syncthreads();
-  if (tid == 0) {
-    int R = sh.R;
-    if (R > a.max_roi_nodes) {
-      // Must-keep swap (extract_roi_bfs :2359-2379): the positions of src/dst
-      // in ascending order; each one beyond the cut swaps with slot 0 / 1.
-      int kp[2];
-      int32_t kn[2];
-      int nk = 0;
-      if (src == dst) {
-        kp[0] = sh.pos_src; kn[0] = src; nk = 1;
-      } else {
-        const bool s_first = sh.pos_src < sh.pos_dst;
-        kp[0] = s_first ? sh.pos_src : sh.pos_dst; kn[0] = s_first ? src : dst;
-        kp[1] = s_first ? sh.pos_dst : sh.pos_src; kn[1] = s_first ? dst : src;
-        nk = 2;
-      }
-      for (int k = 0; k < nk; ++k)
-        if (kp[k] >= a.max_roi_nodes) out[k] = kn[k];
-      R = a.max_roi_nodes;
-    }
-    sh.R = R;
-    if (sh.overflow || R > out_cap) sh.status = OGR_ERR_CAPACITY;
-    atomicAdd(&g_stage[12], (unsigned long long)R);
-  }
+  roi_finish(sh, a, out, out_cap);
   // restore seen[] to zero over the bounding box
   for (int32_t i = tid; i < V; i += kThreads) seen[gid_of(i)] = 0;
   __syncthreads();
   clk.mark(1);
+}
+
+__device__ void roi_build(Shared& sh, const ogr_graph& g, const ogr_net_args& a, int32_t* seen, int32_t* const* q,
+                          int64_t qcap, int32_t* out, int32_t out_cap, char* smem, StageClock& clk) {
+  if (roi_build_box(sh, g, a, q, qcap, out, out_cap, smem, clk)) return;
+  __syncthreads();
+  roi_build_large(sh, g, a, seen, q, qcap, out, out_cap, clk);
 }
 
 // ---- the search on a given ROI ---------------------------------------------------
@@ -713,7 +946,7 @@ __device__ __forceinline__ void roi_search_row(const RoiJob& job, char* smem, in
 
 // The ROI of one net into w.roi (nothing for a full-graph net), by one CTA:
 // sh.status and sh.R tell.
-__device__ void build_roi(Shared& sh, const ogr_graph& g, const ogr_net_args& a, const Ws& w) {
+__device__ void build_roi(Shared& sh, const ogr_graph& g, const ogr_net_args& a, const Ws& w, char* smem) {
   StageClock clk;
   clk.start();
   if (threadIdx.x == 0) sh.status = OGR_OK;
@@ -723,7 +956,7 @@ __device__ void build_roi(Shared& sh, const ogr_graph& g, const ogr_net_args& a,
     __syncthreads();
     return;
   }
-  roi_build(sh, g, a, w.seen, w.q, w.qcap, w.roi, a.max_roi_nodes, clk);
+  roi_build(sh, g, a, w.seen, w.q, w.qcap, w.roi, a.max_roi_nodes, smem, clk);
 }
 
 // ---- commit / rip-up ---------------------------------------------------------
@@ -804,8 +1037,9 @@ __device__ int apply_path_dev(const ogr_graph& g, const ogr_state& st, const int
 // The ROI of a net into w.roi: result[0] = status, result[3] = its size.
 __global__ void __launch_bounds__(kThreads, 1)
 build_roi_kernel(ogr_graph g, ogr_net_args a, Ws w) {
+  extern __shared__ __align__(16) char smem[];
   __shared__ Shared sh;
-  build_roi(sh, g, a, w);
+  build_roi(sh, g, a, w, smem);
   if (threadIdx.x == 0) {
     w.result[0] = sh.status;
     w.result[1] = 0;
@@ -837,6 +1071,7 @@ find_team_kernel(ogr_graph g, ogr_state st, ogr_net_args a, Ws w, const int32_t*
 
 __global__ void __launch_bounds__(kThreads, 1)
 roi_kernel(ogr_graph g, ogr_net_args a, Ws w, int32_t* roi_out, int32_t roi_cap) {
+  extern __shared__ __align__(16) char smem[];
   __shared__ Shared sh;
   StageClock clk;
   clk.start();
@@ -850,7 +1085,7 @@ roi_kernel(ogr_graph g, ogr_net_args a, Ws w, int32_t* roi_out, int32_t roi_cap)
     if (sh.status == OGR_OK)
       for (int r = threadIdx.x; r < R; r += kThreads) roi_out[r] = r;
   } else {
-    roi_build(sh, g, a, w.seen, w.q, w.qcap, roi_out, roi_cap, clk);
+    roi_build(sh, g, a, w.seen, w.q, w.qcap, roi_out, roi_cap, smem, clk);
     R = sh.R;
   }
   if (threadIdx.x == 0) {
@@ -969,6 +1204,7 @@ paths_commit_kernel(ogr_graph g, ogr_state st, const int32_t* nodes, const int32
 // queue overflowed (the pass then extracts that ROI inline).
 __global__ void __launch_bounds__(kThreads, 1)
 roi_batch_kernel(ogr_graph g, ogr_net_table t, ogr_pass_args pa, ogr_roi_batch rb) {
+  extern __shared__ __align__(16) char smem[];
   __shared__ Shared sh;
   __shared__ int s_k;
   BfsSlot slot = bfs_slot_at((char*)rb.bfs_ws + (size_t)blockIdx.x * rb.slot_bytes, g.num_nodes, rb.qcap);
@@ -988,7 +1224,7 @@ roi_batch_kernel(ogr_graph g, ogr_net_table t, ogr_pass_args pa, ogr_roi_batch r
     clk.start();
     if (threadIdx.x == 0) sh.status = OGR_OK;
     __syncthreads();
-    roi_build(sh, g, a, slot.seen, slot.q, slot.qcap, rb.roi_pool + (int64_t)n * rb.roi_cap, rb.roi_cap, clk);
+    roi_build(sh, g, a, slot.seen, slot.q, slot.qcap, rb.roi_pool + (int64_t)n * rb.roi_cap, rb.roi_cap, smem, clk);
     if (threadIdx.x == 0) {
       rb.roi_len[n] = (sh.status == OGR_OK) ? sh.R : -1;
       if (rb.roi_box) {
@@ -1232,7 +1468,7 @@ window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa,
       if (nslots == 0 && tid == 0) t.store_len[n] = 0;   // (a window's rip-ups may yet be undone)
       if (solo && rc == OGR_OK) {
         const ogr_net_args a = ogr_pass_net_args(t, pa, n, 0);
-        build_roi(sh, g, a, w);
+        build_roi(sh, g, a, w, smem);
         rc = sh.status;
         if (tid == 0) c->solo_R = sh.R;
       } else if (use_batch && tid == 0) {
@@ -1321,7 +1557,7 @@ window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa,
         __syncthreads();
         if (rc == OGR_OK) {
           const ogr_net_args a = ogr_pass_net_args(t, pa, nf, 1);
-          build_roi(sh, g, a, w);
+          build_roi(sh, g, a, w, smem);
           rc = sh.status;
           if (tid == 0) {
             c->solo_R = sh.R;
@@ -1436,7 +1672,7 @@ pass_full_tail_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args 
   const int used = (int)w.result[2];
   if (fin != OGR_OK && used < pa.fallback_quota) {
     const ogr_net_args a = ogr_pass_net_args(t, pa, n, 1);
-    build_roi(sh, g, a, w);
+    build_roi(sh, g, a, w, smem);
     fin = sh.status;
     if (fin == OGR_OK) {
       clear_team(w.ctl);
@@ -1478,9 +1714,13 @@ pass_full_tail_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args 
     }                                                          \
   } while (0)
 
+cudaError_t wide_smem(const void* f) {
+  return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ogr_phase::kSmemBytes);
+}
+
 // A cooperative launch of `grid` CTAs, all of them resident.
 int launch_team(const void* f, int grid, void** args, cudaStream_t s) {
-  OGR_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ogr_phase::kSmemBytes));
+  OGR_CUDA_TRY(wide_smem(f));
   OGR_CUDA_TRY(cudaLaunchCooperativeKernel(f, dim3(grid), dim3(kThreads), args, ogr_phase::kSmemBytes, s));
   return OGR_OK;
 }
@@ -1491,7 +1731,8 @@ int launch_find(const ogr_graph& g, const ogr_state& st, const ogr_net_args& a, 
                 int64_t* stats, cudaStream_t s) {
   OGR_CUDA_TRY(cudaMemsetAsync(&w.ctl->team, 0, sizeof(ogr_phase::Ctl), s));
   if (roi == nullptr && !a.full_graph) {
-    build_roi_kernel<<<1, kThreads, 0, s>>>(g, a, w);
+    OGR_CUDA_TRY(wide_smem((const void*)build_roi_kernel));
+    build_roi_kernel<<<1, kThreads, ogr_phase::kSmemBytes, s>>>(g, a, w);
     OGR_LAUNCH_CHECK();
   }
   if (a.full_graph) R = g.num_nodes;
@@ -1676,7 +1917,8 @@ extern "C" int ogr_extract_roi(const ogr_graph* g, const ogr_net_args* net, void
   Ws w;
   ws_layout(g->num_nodes, (char*)ws, &w);
   cudaStream_t s = ogr_stream(stream);
-  roi_kernel<<<1, kThreads, 0, s>>>(*g, *net, w, roi_out, roi_cap);
+  OGR_CUDA_TRY(wide_smem((const void*)roi_kernel));
+  roi_kernel<<<1, kThreads, ogr_phase::kSmemBytes, s>>>(*g, *net, w, roi_out, roi_cap);
   OGR_LAUNCH_CHECK();
   int64_t res[2];
   OGR_CUDA_TRY(cudaMemcpyAsync(res, w.result, sizeof(res), cudaMemcpyDeviceToHost, s));
@@ -1743,7 +1985,8 @@ extern "C" int ogr_route_pass(const ogr_graph* g, const ogr_state* st, const ogr
   if (batch) {
     rbv = *rb;
     OGR_CUDA_TRY(cudaMemsetAsync(rbv.next, 0, sizeof(int32_t), s));
-    roi_batch_kernel<<<rbv.slots, kThreads, 0, s>>>(*g, *t, *pa, rbv);
+    OGR_CUDA_TRY(wide_smem((const void*)roi_batch_kernel));
+    roi_batch_kernel<<<rbv.slots, kThreads, ogr_phase::kSmemBytes, s>>>(*g, *t, *pa, rbv);
     OGR_LAUNCH_CHECK();
   }
   const bool windows = win != nullptr && win->slots > 0 && batch && rbv.roi_box != nullptr;
@@ -1806,8 +2049,7 @@ extern "C" int ogr_route_pass(const ogr_graph* g, const ogr_state* st, const ogr
         const int rc = ogr_full::launch(*g, *st, job, full_ws, s);
         if (rc != OGR_OK) return rc;
         OGR_WITH_ROW(ROW, *g, {
-          OGR_CUDA_TRY(cudaFuncSetAttribute(pass_full_tail_kernel<ROW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)ogr_phase::kSmemBytes));
+          OGR_CUDA_TRY(wide_smem((const void*)pass_full_tail_kernel<ROW>));
           pass_full_tail_kernel<ROW><<<1, kThreads, ogr_phase::kSmemBytes, s>>>(*g, *st, *t, *pa, k, w, full_res);
         });
         OGR_LAUNCH_CHECK();
