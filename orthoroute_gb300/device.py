@@ -131,8 +131,9 @@ class Ops:
         # {searches, arcs, pops} of window searches whose results were undone
         self.discarded = torch.zeros(3, dtype=torch.int64, device=graph.device)
         self.status = torch.zeros(1, dtype=torch.int32, device=graph.device)
-        self.tally_out = torch.zeros(5, dtype=torch.int64, device=graph.device)
-        self.layer_units = torch.zeros(graph.lattice.nz, dtype=torch.int64, device=graph.device)
+        # totals and per-layer units of a tally, side by side so that one copy reads both
+        self._tally = torch.zeros(5 + graph.lattice.nz, dtype=torch.int64, device=graph.device)
+        self.tally_out, self.layer_units = self._tally[:5], self._tally[5:]
         self.counters = dict(launches=0, h2d_bytes=0, d2h_bytes=0, search_launches=0, search_ms=0.0)
         self._full_ws = None
         self.full_ws_bytes = 0
@@ -198,12 +199,13 @@ class Ops:
                                       _p(g.edge_src), _p(g.indices), _p(g.edge_layer), _p(s.path_node_use),
                                       int(canonical_only), _p(self.tally_out), _p(self.layer_units), self._sp()),
                    "ogr_tally")
-        out = self.tally_out.cpu().numpy()
+        both = self._tally.cpu().numpy()
+        out, units = both[:5], both[5:]
         self.counters["launches"] += 1
         self.counters["d2h_bytes"] += 8 * (5 + g.lattice.nz)
         if out[4]:
             raise RuntimeError("present EMA off the 2^-23 grid: per-layer sums would not be exact")
-        return int(out[0]), int(out[1]), int(out[2]), int(out[3]), self.layer_units.cpu().numpy()
+        return int(out[0]), int(out[1]), int(out[2]), int(out[3]), units
 
     # -- A6–A8 ----------------------------------------------------------------
     def net_args(self, net_id, src, dst, *, full_graph=False, max_depth=80, halo=2, max_roi_nodes=50_000,
