@@ -6,6 +6,10 @@
 // Lateral arcs exist only on lateral layers and only along the layer's axis
 // (plus the other axis when wrong-way arcs are enabled).  A via partner is
 // present when (x, y) is a legal site of that layer pair.
+#include <string.h>
+
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace {
@@ -36,117 +40,132 @@ __device__ __forceinline__ bool site_ok(int mode, int x, int y) {
   return (x % mode) == 0 && (y % mode) == 0;
 }
 
-// Number of arcs and (optionally) the row itself.
-template <bool kWrite>
-__device__ __forceinline__ int node_row(const LatDev& L, int64_t n, int32_t* idx, float* cost, unsigned char* lay,
-                                        unsigned char* kind) {
-  const int nx = L.h.nx, ny = L.h.ny;
-  const int64_t plane = (int64_t)nx * ny;
-  const int z = (int)(n / plane);
-  const int64_t r = n - (int64_t)z * plane;
-  const int y = (int)(r / nx);
-  const int x = (int)(r - (int64_t)y * nx);
+// Division by a fixed d > 0 of any v < 2^32 (the high product with
+// floor(2^32 / d) is the quotient or one less).
+struct Div {
+  unsigned d, m;
+  __device__ explicit Div(unsigned dd) : d(dd), m(dd > 1 ? (unsigned)((1ull << 32) / dd) : 0xffffffffu) {}
+  __device__ unsigned operator()(unsigned v) const {
+    const unsigned q = __umulhi(v, m);
+    return v - q * d >= d ? q + 1 : q;
+  }
+};
+
+// Whether layer z has arcs along x / along y, and their costs.
+struct Axes {
+  bool h, v;
+  float ch, cv;
+  __device__ Axes(const LatticeConst& l, int z) {
+    const int ax = l.axis[z];
+    const bool ww = ax != 0 && l.wrong_way_cost > 0.f;
+    h = ax == 1 || ww;
+    v = ax == 2 || ww;
+    ch = ax == 1 ? l.lateral_cost : l.wrong_way_cost;
+    cv = ax == 2 ? l.lateral_cost : l.wrong_way_cost;
+  }
+};
+
+// Via partners of (x, y, z) below layer `upto`, in row order.
+__device__ __forceinline__ int partners_below(const LatDev& L, int x, int y, int z, int upto) {
   int k = 0;
-  const int p0 = L.h.pptr[z], p1 = L.h.pptr[z + 1];
-  for (int p = p0; p < p1; ++p) {
-    const int zz = L.pz[p];
-    if (zz >= z) break;
-    if (!site_ok(L.psite[p], x, y)) continue;
-    if (kWrite) {
-      idx[k] = (int32_t)((int64_t)zz * plane + r);
-      cost[k] = L.pcost[p];
-      lay[k] = (unsigned char)z;
-      kind[k] = 1;
-    }
-    ++k;
-  }
-  const int ax = L.h.axis[z];
-  if (ax != 0) {
-    const bool ww = L.h.wrong_way_cost > 0.f;
-    const bool h = (ax == 1) || ww;
-    const bool v = (ax == 2) || ww;
-    const float ch = (ax == 1) ? L.h.lateral_cost : L.h.wrong_way_cost;
-    const float cv = (ax == 2) ? L.h.lateral_cost : L.h.wrong_way_cost;
-    if (v && y > 0) {
-      if (kWrite) { idx[k] = (int32_t)(n - nx); cost[k] = cv; lay[k] = (unsigned char)z; kind[k] = 0; }
-      ++k;
-    }
-    if (h && x > 0) {
-      if (kWrite) { idx[k] = (int32_t)(n - 1); cost[k] = ch; lay[k] = (unsigned char)z; kind[k] = 0; }
-      ++k;
-    }
-    if (h && x + 1 < nx) {
-      if (kWrite) { idx[k] = (int32_t)(n + 1); cost[k] = ch; lay[k] = (unsigned char)z; kind[k] = 0; }
-      ++k;
-    }
-    if (v && y + 1 < ny) {
-      if (kWrite) { idx[k] = (int32_t)(n + nx); cost[k] = cv; lay[k] = (unsigned char)z; kind[k] = 0; }
-      ++k;
-    }
-  }
-  for (int p = p0; p < p1; ++p) {
-    const int zz = L.pz[p];
-    if (zz <= z) continue;
-    if (!site_ok(L.psite[p], x, y)) continue;
-    if (kWrite) {
-      idx[k] = (int32_t)((int64_t)zz * plane + r);
-      cost[k] = L.pcost[p];
-      lay[k] = (unsigned char)z;
-      kind[k] = 1;
-    }
-    ++k;
-  }
+  for (int p = L.h.pptr[z]; p < L.h.pptr[z + 1] && L.pz[p] < upto; ++p) k += site_ok(L.psite[p], x, y) ? 1 : 0;
   return k;
 }
 
-__global__ void degree_kernel(LatDev L, int64_t N, int32_t* deg) {
-  for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < N;
-       n += (int64_t)gridDim.x * blockDim.x)
-    deg[n] = node_row<false>(L, n, nullptr, nullptr, nullptr, nullptr);
-}
-
-// Exclusive scan, 3 phases: per-tile sums, scan of tile sums (1 block), add.
-constexpr int kScanTile = 1024;
-
-__global__ void scan_tiles(const int32_t* in, int64_t N, int32_t* out, int32_t* tile_sums) {
-  __shared__ int32_t s[kScanTile];
-  const int64_t base = (int64_t)blockIdx.x * kScanTile;
-  const int t = threadIdx.x;
-  const int64_t i = base + t;
-  int32_t v = (i < N) ? in[i] : 0;
-  s[t] = v;
-  __syncthreads();
-  for (int off = 1; off < kScanTile; off <<= 1) {
-    int32_t a = (t >= off) ? s[t - off] : 0;
-    __syncthreads();
-    s[t] += a;
-    __syncthreads();
+// Place of partner `want` among the via partners of (x, y, z) below or at it;
+// -1 if (x, y, z) has no arc to that layer.
+__device__ __forceinline__ int partner_place(const LatDev& L, int x, int y, int z, int want) {
+  int k = 0;
+  for (int p = L.h.pptr[z]; p < L.h.pptr[z + 1] && L.pz[p] <= want; ++p) {
+    const bool ok = site_ok(L.psite[p], x, y);
+    if (L.pz[p] == want) return ok ? k : -1;
+    k += ok ? 1 : 0;
   }
-  if (i < N) out[i] = s[t] - v;  // exclusive within tile
-  if (t == kScanTile - 1) tile_sums[blockIdx.x] = s[t];
+  return -1;
 }
 
-__global__ void scan_tile_sums(int32_t* tile_sums, int64_t ntiles, int32_t* total) {
-  // Single block, sequential over chunks of kScanTile.
-  __shared__ int32_t s[kScanTile];
-  __shared__ int32_t carry;
-  if (threadIdx.x == 0) carry = 0;
+// Lateral arcs of (x, y) on a layer with axes ax: all of them, or those that
+// come before the one to side (0: y-1, 1: x-1, 2: x+1, 3: y+1).
+__device__ __forceinline__ int laterals_before(const LatDev& L, const Axes& ax, int x, int y, int side) {
+  int k = 0;
+  if (side > 0 && ax.v && y > 0) ++k;
+  if (side > 1 && ax.h && x > 0) ++k;
+  if (side > 2 && ax.h && x + 1 < L.h.nx) ++k;
+  if (side > 3 && ax.v && y + 1 < L.h.ny) ++k;
+  return k;
+}
+
+__device__ __forceinline__ int degree(const LatDev& L, int x, int y, int z) {
+  const Axes ax(L.h, z);
+  return partners_below(L, x, y, z, kMaxLayers) + laterals_before(L, ax, x, y, 4);
+}
+
+// Row starts: degrees and their sums within tiles of kScanTile nodes, the sum
+// of the tiles before each (one block), and the sum of both.
+constexpr int kScanTile = 4096;
+constexpr int kScanThreads = 1024;
+constexpr int kScanPer = kScanTile / kScanThreads;
+
+// Exclusive sum over a block of 1024 threads; *total is the block's sum.
+__device__ __forceinline__ int block_scan(int v, int* s_warp, int* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) s_warp[warp] = x;
   __syncthreads();
-  for (int64_t base = 0; base < ntiles; base += kScanTile) {
-    const int t = threadIdx.x;
-    const int64_t i = base + t;
-    int32_t v = (i < ntiles) ? tile_sums[i] : 0;
-    s[t] = v;
-    __syncthreads();
-    for (int off = 1; off < kScanTile; off <<= 1) {
-      int32_t a = (t >= off) ? s[t - off] : 0;
-      __syncthreads();
-      s[t] += a;
-      __syncthreads();
+  if (warp == 0) {
+    int t = s_warp[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= o) t += y;
     }
-    if (i < ntiles) tile_sums[i] = carry + s[t] - v;
-    __syncthreads();
-    if (t == kScanTile - 1) carry += s[t];
+    s_warp[lane] = t;
+  }
+  __syncthreads();
+  *total = s_warp[31];
+  const int before = warp > 0 ? s_warp[warp - 1] : 0;
+  return before + x - v;
+}
+
+__global__ void __launch_bounds__(kScanThreads) scan_tiles(LatDev L, int64_t N, int32_t* out, int32_t* tile_sums) {
+  __shared__ int s_warp[32];
+  const Div by_plane((unsigned)(L.h.nx * L.h.ny)), by_nx((unsigned)L.h.nx);
+  const int64_t i0 = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanPer;
+  int d[kScanPer], sum = 0;
+#pragma unroll
+  for (int j = 0; j < kScanPer; ++j) {
+    d[j] = 0;
+    if (i0 + j < N) {
+      const unsigned n = (unsigned)(i0 + j), z = by_plane(n), r = n - z * by_plane.d, y = by_nx(r);
+      d[j] = degree(L, (int)(r - y * by_nx.d), (int)y, (int)z);
+    }
+    sum += d[j];
+  }
+  int total;
+  int at = block_scan(sum, s_warp, &total);
+#pragma unroll
+  for (int j = 0; j < kScanPer; ++j) {
+    if (i0 + j < N) out[i0 + j] = at;
+    at += d[j];
+  }
+  if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(kScanThreads) scan_tile_sums(int32_t* tile_sums, int64_t ntiles, int32_t* total) {
+  __shared__ int s_warp[32];
+  int carry = 0;
+  for (int64_t base = 0; base < ntiles; base += kScanThreads) {
+    const int64_t i = base + threadIdx.x;
+    const int v = i < ntiles ? tile_sums[i] : 0;
+    int sum;
+    const int x = block_scan(v, s_warp, &sum);
+    if (i < ntiles) tile_sums[i] = carry + x;
+    carry += sum;
     __syncthreads();
   }
   if (threadIdx.x == 0) *total = carry;
@@ -160,26 +179,83 @@ __global__ void scan_add(int32_t* out, int64_t N, const int32_t* tile_sums, cons
   }
 }
 
-__global__ void fill_kernel(LatDev L, int64_t N, const int32_t* indptr, int32_t* indices, float* cost,
-                            unsigned char* lay, unsigned char* kind, int32_t* edge_src) {
-  for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < N;
-       n += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t b = indptr[n];
-    const int k = node_row<true>(L, n, indices + b, cost + b, lay + b, kind + b);
-    for (int j = 0; j < k; ++j) edge_src[b + j] = (int32_t)n;
-  }
-}
-
-__global__ void rev_kernel(int64_t N, const int32_t* indptr, const int32_t* indices, int32_t* rev) {
-  for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < N;
-       u += (int64_t)gridDim.x * blockDim.x) {
-    for (int32_t e = indptr[u]; e < indptr[u + 1]; ++e) {
-      const int32_t v = indices[e];
-      int32_t found = -1;
-      for (int32_t f = indptr[v]; f < indptr[v + 1]; ++f)
-        if (indices[f] == (int32_t)u) { found = f; break; }
-      rev[e] = found;
+// The rows of a tile of nodes of one layer (blockIdx.y), staged in shared
+// memory and copied out in arc order.  A row written by its thread straight to
+// memory scattered 18 bytes per arc over six arrays (280 us for 21 M arcs),
+// and the reverse arc was found by walking the neighbour's row (132 us): it is
+// the neighbour's row start plus a count here, its place in that row.
+constexpr int kFillThreads = 128;
+__global__ void __launch_bounds__(kFillThreads) fill_kernel(LatDev L, int tile_nodes, const int32_t* __restrict__ indptr, int32_t* indices,
+                            float* cost, unsigned char* lay, unsigned char* kind, int32_t* edge_src, int32_t* rev,
+                            int cap) {
+  extern __shared__ __align__(16) int32_t s_buf[];
+  int32_t* s_idx = s_buf;
+  float* s_cost = reinterpret_cast<float*>(s_buf + cap);
+  int32_t* s_src = s_buf + 2 * cap;
+  int32_t* s_rev = s_buf + 3 * cap;
+  unsigned char* s_kind = reinterpret_cast<unsigned char*>(s_buf + 4 * cap);
+  const int nx = L.h.nx, ny = L.h.ny, z = blockIdx.y;
+  const int32_t plane = nx * ny;
+  const Axes ax(L.h, z);
+  const Div by_nx((unsigned)nx);
+  const int p0 = L.h.pptr[z], p1 = L.h.pptr[z + 1];
+  for (int32_t r0 = blockIdx.x * tile_nodes; r0 < plane; r0 += gridDim.x * tile_nodes) {
+    const int32_t r1 = min(plane, r0 + tile_nodes);
+    const int32_t e0 = indptr[z * plane + r0], e1 = indptr[z * plane + r1];
+    for (int32_t r = r0 + threadIdx.x; r < r1; r += kFillThreads) {
+      const int y = (int)by_nx((unsigned)r), x = r - y * nx;
+      const int32_t n = z * plane + r;
+      int k = indptr[n] - e0;
+      auto put = [&](int32_t v, float c, int via, int32_t back) {
+        s_idx[k] = v;
+        s_cost[k] = c;
+        s_src[k] = n;
+        s_rev[k] = back;
+        s_kind[k] = (unsigned char)via;
+        ++k;
+      };
+      // the arc back from a via partner zz: after its partners below z, and
+      // its laterals if zz < z (they come between)
+      auto via = [&](int p, int zz) {
+        const int32_t v = zz * plane + r;
+        int32_t back = -1;
+        if (rev) {
+          back = partner_place(L, x, y, zz, z);
+          if (back >= 0) back += indptr[v] + (zz < z ? laterals_before(L, Axes(L.h, zz), x, y, 4) : 0);
+        }
+        put(v, L.pcost[p], 1, back);
+      };
+      int p = p0;
+      for (; p < p1; ++p) {
+        const int zz = L.pz[p];
+        if (zz >= z) break;
+        if (site_ok(L.psite[p], x, y)) via(p, zz);
+      }
+      // laterals: the arc back stands on the neighbour's other side
+      auto lateral = [&](int dx, int dy, int32_t v, float c, int side) {
+        put(v, c, 0, rev ? indptr[v] + partners_below(L, x + dx, y + dy, z, z) +
+                               laterals_before(L, ax, x + dx, y + dy, side)
+                         : -1);
+      };
+      if (ax.v && y > 0) lateral(0, -1, n - nx, ax.cv, 3);
+      if (ax.h && x > 0) lateral(-1, 0, n - 1, ax.ch, 2);
+      if (ax.h && x + 1 < nx) lateral(1, 0, n + 1, ax.ch, 1);
+      if (ax.v && y + 1 < ny) lateral(0, 1, n + nx, ax.cv, 0);
+      for (; p < p1; ++p) {
+        const int zz = L.pz[p];
+        if (zz > z && site_ok(L.psite[p], x, y)) via(p, zz);
+      }
     }
+    __syncthreads();
+    for (int32_t i = threadIdx.x; i < e1 - e0; i += kFillThreads) {
+      indices[e0 + i] = s_idx[i];
+      cost[e0 + i] = s_cost[i];
+      edge_src[e0 + i] = s_src[i];
+      if (rev) rev[e0 + i] = s_rev[i];
+      lay[e0 + i] = (unsigned char)z;
+      kind[e0 + i] = s_kind[i];
+    }
+    __syncthreads();
   }
 }
 
@@ -197,14 +273,17 @@ int load_desc(const ogr_lattice_desc* d, int* dev_tab, cudaStream_t s, LatDev* o
   const int np = d->partner_ptr[d->nz];
   if (np > kMaxPartners || np < 0) return OGR_ERR_ARG;
   L.pz = dev_tab;
-  L.pcost = reinterpret_cast<const float*>(dev_tab + kMaxPartners);
-  L.psite = dev_tab + 2 * kMaxPartners;
+  L.pcost = nullptr;
+  L.psite = nullptr;
   if (np > 0) {
-    OGR_CUDA_TRY(cudaMemcpyAsync(dev_tab, d->partner_z, np * sizeof(int), cudaMemcpyHostToDevice, s));
-    OGR_CUDA_TRY(cudaMemcpyAsync(dev_tab + kMaxPartners, d->partner_cost, np * sizeof(float),
-                                 cudaMemcpyHostToDevice, s));
-    OGR_CUDA_TRY(cudaMemcpyAsync(dev_tab + 2 * kMaxPartners, d->partner_site, np * sizeof(int),
-                                 cudaMemcpyHostToDevice, s));
+    // one copy of the three tables (the source is pageable, so each copy waits)
+    int tab[3 * kMaxPartners];
+    memcpy(tab, d->partner_z, np * sizeof(int));
+    memcpy(tab + np, d->partner_cost, np * sizeof(float));
+    memcpy(tab + 2 * np, d->partner_site, np * sizeof(int));
+    L.pcost = reinterpret_cast<const float*>(dev_tab + np);
+    L.psite = dev_tab + 2 * np;
+    OGR_CUDA_TRY(cudaMemcpyAsync(dev_tab, tab, 3 * np * sizeof(int), cudaMemcpyHostToDevice, s));
   }
   *out = L;
   return OGR_OK;
@@ -247,7 +326,7 @@ extern "C" int ogr_csr_num_edges(const ogr_lattice_desc* d, int64_t* num_edges) 
 extern "C" size_t ogr_csr_workspace_bytes(const ogr_lattice_desc* d) {
   const int64_t N = (int64_t)d->nx * d->ny * d->nz;
   const int64_t tiles = (N + kScanTile - 1) / kScanTile;
-  return (size_t)(N * 4 + tiles * 4 + 64) + 3 * sizeof(int) * kMaxPartners + 256;
+  return (size_t)(tiles * 4 + 64) + 3 * sizeof(int) * kMaxPartners + 512;
 }
 
 extern "C" int ogr_csr_build(const ogr_lattice_desc* d, int32_t* indptr, int32_t* indices,
@@ -261,21 +340,30 @@ extern "C" int ogr_csr_build(const ogr_lattice_desc* d, int32_t* indptr, int32_t
   if (E >= (int64_t)1 << 31) return OGR_ERR_ARG;
   if (workspace_bytes < ogr_csr_workspace_bytes(d) || !workspace) return OGR_ERR_CAPACITY;
   cudaStream_t s = ogr_stream(stream);
-  int32_t* deg = reinterpret_cast<int32_t*>(workspace);
   const int64_t tiles = (N + kScanTile - 1) / kScanTile;
-  int32_t* tile_sums = deg + N;
+  int32_t* tile_sums = reinterpret_cast<int32_t*>(workspace);
   int32_t* total = tile_sums + tiles;
-  const size_t tab_off = ((size_t)(N * 4 + tiles * 4 + 64) + 255) & ~(size_t)255;
+  const size_t tab_off = ((size_t)(tiles * 4 + 64) + 255) & ~(size_t)255;
   LatDev L;
   const int rc = load_desc(d, reinterpret_cast<int*>((char*)workspace + tab_off), s, &L);
   if (rc != OGR_OK) return rc;
-  degree_kernel<<<ogr_blocks(N, 256), 256, 0, s>>>(L, N, deg);
-  scan_tiles<<<(unsigned)tiles, kScanTile, 0, s>>>(deg, N, indptr, tile_sums);
-  scan_tile_sums<<<1, kScanTile, 0, s>>>(tile_sums, tiles, total);
+  scan_tiles<<<(unsigned)tiles, kScanThreads, 0, s>>>(L, N, indptr, tile_sums);
+  OGR_LAUNCH_CHECK();
+  scan_tile_sums<<<1, kScanThreads, 0, s>>>(tile_sums, tiles, total);
+  OGR_LAUNCH_CHECK();
   scan_add<<<ogr_blocks(N + 1, 256), 256, 0, s>>>(indptr, N, tile_sums, total);
-  fill_kernel<<<ogr_blocks(N, 256), 256, 0, s>>>(L, N, indptr, indices, base_costs, edge_layer, edge_kind,
-                                                  edge_src);
-  if (rev) rev_kernel<<<ogr_blocks(N, 256), 256, 0, s>>>(N, indptr, indices, rev);
+  OGR_LAUNCH_CHECK();
+  // A tile's rows have to fit in shared memory: 17 bytes per arc, the layers'
+  // longest row times the tile's nodes (a multiple of 32), at most 48 KB.
+  int row = 1;
+  for (int z = 0; z < d->nz; ++z) row = std::max(row, d->partner_ptr[z + 1] - d->partner_ptr[z] + 4);
+  int tile_nodes = kFillThreads;
+  while (tile_nodes > 32 && tile_nodes * row * 17 > 48 * 1024) tile_nodes -= 32;
+  const int cap = tile_nodes * row;          // rows of up to 67 arcs: 36,448 bytes at 32 nodes
+  const int plane = d->nx * d->ny;
+  const dim3 grid((unsigned)std::min((plane + tile_nodes - 1) / tile_nodes, 65535), (unsigned)d->nz);
+  fill_kernel<<<grid, kFillThreads, (size_t)cap * 17, s>>>(L, tile_nodes, indptr, indices, base_costs, edge_layer,
+                                                          edge_kind, edge_src, rev, cap);
   OGR_LAUNCH_CHECK();
   return OGR_OK;
 }
