@@ -564,7 +564,8 @@ int ogr_full_profile(int64_t* out8, int32_t reset);
 /* Tracing: cumulative per-stage cycle counters of all ROI searches on the
  * current device since the last reset, taken by each team's first thread (host
  * int64[16]: BFS, compaction, search init, phases, of these waiting for the
- * team, 0, 0, statistics and backtrace, cleanup; then searches, settle
+ * team, rip-up and commit, window formation (both of a pass's first CTA),
+ * statistics and backtrace, cleanup; then searches, settle
  * phases, BFS waves, ROI nodes, entries examined, ROIs taken from the batched
  * extraction).  Synchronous. */
 int ogr_search_profile(int64_t* out16, int32_t reset);

@@ -163,8 +163,6 @@ full_sssp_kernel(ogr_graph g, ogr_state st, ogr_full::Job job, FWs w) {
   pr.ov[0] = w.ov[0];
   pr.ov[1] = w.ov[1];
   pr.mseed = w.mseed;
-  pr.mtgt = w.mtgt;
-  pr.none = kNoTerm;
   pr.ctl = &ctl->team;
   pr.rank = blockIdx.x;
   pr.nranks = gridDim.x;
@@ -181,7 +179,7 @@ full_sssp_kernel(ogr_graph g, ogr_state st, ogr_full::Job job, FWs w) {
     pr.sid = sid + attempt;
     // every node's record
     int md = 0;
-#pragma unroll 2
+#pragma unroll 4
     for (int64_t i = gtid; i < N; i += gthreads) {
       const int32_t f0 = indptr[i], f1 = indptr[i + 1];
       md = max(md, f1 - f0);
@@ -221,6 +219,7 @@ full_sssp_kernel(ogr_graph g, ogr_state st, ogr_full::Job job, FWs w) {
           unsigned long long* p = reinterpret_cast<unsigned long long*>(&w.mtgt[t]);
           if (attempt == 0 && *p != kNoTerm) { bad = 1; break; }   // repeated target
           *p = (unsigned long long)__double_as_longlong(tc);
+          w.rec[t].sp = kTgt;
         }
         for (int i = 0; i < job.n_seeds && !bad; ++i) {
           const int32_t s0 = job.seeds[i];
@@ -231,8 +230,9 @@ full_sssp_kernel(ogr_graph g, ogr_state st, ogr_full::Job job, FWs w) {
           *p = (unsigned long long)__double_as_longlong(sc);
           const float pen = ogr_node_penalty(st, a, s0);
           w.claim[s0] = pr.sid;
-          w.rec[s0].sp = 1;
-          w.ov[0][nf0++] = make_int4(s0, indptr[s0], indptr[s0 + 1] - indptr[s0], __float_as_int(pen));
+          const int32_t flags = kSeed | (w.rec[s0].sp & kTgt);
+          w.rec[s0].sp = 1 | flags;
+          w.ov[0][nf0++] = make_int4(s0, indptr[s0], (indptr[s0 + 1] - indptr[s0]) | flags, __float_as_int(pen));
           unsigned long long lb = ogr_dbits(sc + (double)pen);
           if (in_ticks) {
             lb = 0ull;
@@ -288,7 +288,7 @@ full_sssp_kernel(ogr_graph g, ogr_state st, ogr_full::Job job, FWs w) {
       for (int i = tid; i < job.n_targets; i += 32) {
         const int32_t r = job.targets[i];
         const Rec x = ld_rec(&w.rec[r]);
-        if (x.sp < 2) continue;
+        if ((x.sp & kSpMask) < 2) continue;
         const double lr = fix ? label_value<true>(x.lab) : label_value<false>(x.lab);
         const double tot = lr + job.target_cost[i];
         if (!(tot < dinf)) continue;
@@ -315,7 +315,7 @@ full_sssp_kernel(ogr_graph g, ogr_state st, ogr_full::Job job, FWs w) {
       for (int i = tid; i < job.n_targets; i += kThreads) {
         const Rec x = ld_rec(&w.rec[job.targets[i]]);
         const double lr = fix ? label_value<true>(x.lab) : label_value<false>(x.lab);
-        any |= x.sp >= 2 && lr + job.target_cost[i] < __longlong_as_double(0x7ff0000000000000ll);
+        any |= (x.sp & kSpMask) >= 2 && lr + job.target_cost[i] < __longlong_as_double(0x7ff0000000000000ll);
       }
       count = __syncthreads_or(any) != 0;
     }
@@ -409,11 +409,11 @@ std::atomic<int> g_grid_limit[kMaxDevices] = {};    // SMs x resident CTAs per S
 // Variants by the arcs of a row that an entry's lanes hold.
 const void* kernel_for(int row, bool multi) {
   if (multi)
-    return row == 4    ? (const void*)full_sssp_kernel<4, 1, true>
+    return row == 4    ? (const void*)full_sssp_kernel<2, 2, true>
            : row == 8  ? (const void*)full_sssp_kernel<8, 1, true>
            : row == 16 ? (const void*)full_sssp_kernel<8, 2, true>
                        : (const void*)full_sssp_kernel<16, 2, true>;
-  return row == 4    ? (const void*)full_sssp_kernel<4, 1, false>
+  return row == 4    ? (const void*)full_sssp_kernel<2, 2, false>
          : row == 8  ? (const void*)full_sssp_kernel<8, 1, false>
          : row == 16 ? (const void*)full_sssp_kernel<8, 2, false>
                      : (const void*)full_sssp_kernel<16, 2, false>;

@@ -30,7 +30,9 @@
 // * T, the frontier size and the flags of a phase travel in the barrier's own
 //   16-byte word, which one thread per CTA polls.
 // * One lane serves one arc of an entry (two in rows of 9 to 16 arcs: 64
-//   entries at a time instead of 32, 10.0 -> 9.5 us a phase at 600x400x12).
+//   entries at a time instead of 32, 10.0 -> 9.5 us a phase at 600x400x12; two
+//   lanes of two arcs in rows of up to 4: 18.8 -> 16.3 at 1000x800x32, where a
+//   thousand entries per SM make it a matter of instructions).
 //   512 threads with 128 registers, not 1024 with 64: idle warps cost issue
 //   slots and 64 registers spill (307x199x8: 6.5 -> 4.6 us a phase).  Rows
 //   longer than 32 arcs, and values that ticks cannot hold, are searched by
@@ -42,10 +44,8 @@
 //   are exact wherever the doubles are: costs and penalties of 2^-7 or more
 //   (or 0) are multiples of 2^-30, and below 2^22 their double sums do not
 //   round.  A search that meets any other value is redone in doubles.
-// * A CTA with half as many entries again as the team's average sends a
-//   phase's new entries to a list in global memory that the next phase deals
-//   over the team (1000x800x32: 26.6 -> 18.8 us a phase against sending only
-//   what was above twice the average).
+// * A CTA with more entries than its share sends a phase's new entries to a
+//   list in global memory that the next phase deals over the team (see plan()).
 #pragma once
 #include "common.cuh"
 
@@ -58,7 +58,8 @@ constexpr unsigned long long kNone = ~0ull;
 struct __align__(16) Rec {
   unsigned long long lab;   // label once settled (ticks, or a double's bits); before that
                             // {row start, row length}
-  int32_t sp;      // 0 unreached, 1 reached, 2 + the phase in which it settled
+  int32_t sp;      // 0 unreached, 1 reached, 2 + the phase in which it settled; multi-source:
+                   // | kTgt, | kSeed
   float pen;       // node penalty of this search
 };
 
@@ -83,6 +84,8 @@ struct Ctl {
   alignas(128) int32_t err;        // a CTA gave up waiting
   alignas(128) int32_t nov[3];     // surplus entries by phase mod 3
 };
+
+constexpr int32_t kTgt = 1 << 30, kSeed = 1 << 29, kSpMask = kSeed - 1;
 
 __device__ __forceinline__ Rec ld_rec(const Rec* p) {
   const int4 q = __ldcg(reinterpret_cast<const int4*>(p));
@@ -159,9 +162,7 @@ struct Problem {
   int32_t* claim;                  // == sid: the node has its entry
   int32_t sid;
   int4* ov[2];                     // surplus lists of {node, row start, row length, penalty}, by phase
-  const double* mseed;             // multi-source: seed cost / target cost per node, `none` bits elsewhere
-  const double* mtgt;
-  unsigned long long none;
+  const double* mseed;             // multi-source: cost of each node marked kSeed
   Ctl* ctl;
   int rank, nranks;                // this CTA and the CTAs of the team
   unsigned spin;                   // bound of a wait
@@ -202,7 +203,7 @@ struct Head {
 template <int A>
 struct Body {
   static constexpr int kS = A == 4 ? 3072 : A == 8 ? 1792 : A == 16 ? 1024 : 512;
-  int4 ent[kS];                    // {node, row start, row length | unclaimed << 31, penalty}
+  int4 ent[kS];                    // {node, row start, row length | kTgt | kSeed | unclaimed << 31, penalty}
   int32_t rid[kS * A];             // neighbour, in-cost and out-cost of each arc
   float rin[kS * A];
   float rout[kS * A];
@@ -279,8 +280,8 @@ __device__ __forceinline__ void await(const Problem& pr, Head& sm, int k) {
 }
 
 // The phases of one search.  Before the call: rec of every node holds
-// {row start, row length}, sp 0 and its penalty; the leader's first entries
-// (src, or the seeds: claimed) lie in surplus list 0 with their count in
+// {row start, row length}, sp 0 (targets kTgt, seeds 1 | kSeed) and its
+// penalty; the leader's first entries (src, or the seeds: claimed) lie in surplus list 0 with their count in
 // nov[0], all of it ordered before this call in every CTA of the team by the
 // caller's barrier k0, whose word (count, T) the caller left in sm.a / sm.t.
 // Uses barriers k0 + 1, k0 + 2, ..., of which the first two have clear words
@@ -334,11 +335,16 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
       if (nov >= kMostOut) nov = (unsigned)__ldcg(&pr.ctl->nov[b3]);
       if (nov > (unsigned)pr.rank) n += (int)((nov - pr.rank + pr.nranks - 1) / (unsigned)pr.nranks);
     }
-    // A CTA with more than half as many entries again as the team's average
-    // (and more than half a round) sends all of a phase's new ones away:
-    // seldom and many, since a phase with surplus is longer for everyone.
+    // A CTA with more entries than its share sends all of a phase's new ones
+    // away.  A phase that takes surplus in is longer for everyone, so only
+    // every other one deals the small excesses (a quarter above the average);
+    // in between it takes twice the average (and more than one round).
+    // us a phase at 600x400x12 / 307x199x8 / 1000x800x32: 8.7 / 4.4 / 16.8;
+    // dealing every phase 9.5 / 4.8 / 17.4, every fourth 8.9 / 4.6 / 16.5,
+    // every eighth 9.4 / 5.5 / 20.
     const float avg = __fdividef((float)total, (float)pr.nranks);
-    const bool over = pr.nranks > 1 && n > max(kGroups / 2, (int)fminf(1.5f * avg, 1e6f));
+    const bool deal = (phase & 1) != 0;
+    const bool over = pr.nranks > 1 && n > max(deal ? kGroups / 4 : kGroups, (int)fminf((deal ? 1.25f : 2.0f) * avg, 1e6f));
     head += nf;
     sm.plan.T = T;
     sm.plan.verdict = verdict;
@@ -383,23 +389,20 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
       } else if (valid) {
         en = __ldcg((q ? pr.ov[1] : pr.ov[0]) + pr.rank + (int64_t)(idx - nloc) * pr.nranks);
       }
-      const int32_t v = en.x, f0 = en.y, deg = en.z & 0x7fffffff;
+      const int32_t v = en.x, f0 = en.y, deg = en.z & (kMulti ? kSpMask : 0x7fffffff);
       const bool unclaimed = en.z < 0;
       const float pv = __int_as_float(en.w);
       int old = 0;
       if (unclaimed && sl == 0) old = atomicExch(&pr.claim[v], pr.sid);
+      const bool vt = kMulti && valid && (en.z & kTgt), vs = kMulti && valid && (en.z & kSeed);
       double msd = 0.0;
-      bool vt = false;             // multi-source: v is a target
-      if (kMulti && valid) {
-        msd = __ldcg(&pr.mseed[v]);
-        vt = (u64)__double_as_longlong(__ldcg(&pr.mtgt[v])) != pr.none;
-      }
+      if (vs) msd = __ldcg(&pr.mseed[v]);
       // this lane's arcs (the general form takes them one by one), and the
       // records they name
       int32_t u[K];
       float ci[K], co[K];
       Rec r[K];
-      bool ut[K];                  // multi-source: u is a target, which relaxes nothing
+      int32_t uf[K];               // multi-source: u's kTgt (it relaxes nothing) and kSeed
       auto fetch = [&](int j, int f) {       // in global memory
         const int32_t e = f0 + f;
         u[j] = pr.indices[e];
@@ -409,14 +412,19 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
         if (!kGen && !(tick_exact(ci[j]) && tick_exact(co[j]))) sm.inexact = 1;
       };
       auto load = [&](int j) {
-        if (!kRoi || u[j] >= 0) r[j] = ld_rec(&rec[u[j]]);
-        if (kMulti && r[j].sp >= 0) ut[j] = (u64)__double_as_longlong(__ldcg(&pr.mtgt[u[j]])) != pr.none;
+        if (!kRoi || u[j] >= 0) {
+          r[j] = ld_rec(&rec[u[j]]);
+          if (kMulti) {
+            uf[j] = r[j].sp & ~kSpMask;
+            r[j].sp &= kSpMask;
+          }
+        }
       };
 #pragma unroll
       for (int j = 0; j < K; ++j) {
         const int f = sl + j * L;
         r[j].sp = -1;              // no neighbour
-        ut[j] = false;
+        uf[j] = 0;
         if (!kGen && f < deg) {
           if (loc) {
             const int at = slot * kA + f;
@@ -441,8 +449,8 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
         for (int j = 0; j < K; ++j) {
           alt[j] = kNone;
           if ((unsigned)(r[j].sp - 2) < (unsigned)phase) {      // settled before this phase
-            if (!ut[j] && ci[j] < kInf) alt[j] = r[j].lab + (ticks(ci[j]) + pt);
-          } else if (r[j].sp >= 0 && !ut[j]) {
+            if (!(kMulti && (uf[j] & kTgt)) && ci[j] < kInf) alt[j] = r[j].lab + (ticks(ci[j]) + pt);
+          } else if (r[j].sp >= 0 && !(kMulti && (uf[j] & kTgt))) {
             cin = fminf(cin, ci[j]);
           }
           mx = alt[j] < mx ? alt[j] : mx;
@@ -452,7 +460,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
           r[0].sp = -1;
           fetch(0, f);
           load(0);
-          if (r[0].sp < 0 || ut[0]) continue;
+          if (r[0].sp < 0 || (kMulti && (uf[0] & kTgt))) continue;
           if ((unsigned)(r[0].sp - 2) >= (unsigned)phase) {
             cin = fminf(cin, ci[0]);
             continue;
@@ -517,7 +525,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
         hi = 0ull;
         bu = -1;
       }
-      if (kMulti && valid && (u64)__double_as_longlong(msd) != pr.none) {
+      if (vs) {
         // a seed's own start comes before every relaxation: it loses only to
         // a strictly smaller float32 value
         if (!kGen) {
@@ -552,7 +560,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
       const bool carry = mine && !settle;
       if (sl == 0) {
         if (settle) {
-          st_rec(&rec[v], lv, phase + 2, pv);
+          st_rec(&rec[v], lv, (phase + 2) | (kMulti ? en.z & (kTgt | kSeed) : 0), pv);
           pr.par[v] = bu;
           if (v == pr.dst) {
             sm.dst_hit = 1;
@@ -560,7 +568,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
           }
         } else if (carry) {
           tmin = lv < tmin ? lv : tmin;
-          if (loc && unclaimed) bd.ent[slot].z = deg;
+          if (loc && unclaimed) bd.ent[slot].z = en.z & 0x7fffffff;
         }
       }
       // entries that leave free their place
@@ -574,7 +582,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
       // Offer the labels of the open neighbours, mark and push the unreached
       // ones.  Carried entries keep their place; new ones (and carried surplus
       // entries) take a free one, or go to the surplus list.
-      const bool expand = settle && !(kMulti && vt);
+      const bool expand = settle && !vt;
       bool self = carry && sl == 0;
       int f = sl;
 #pragma unroll
@@ -616,8 +624,10 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
             int4 ne = en;
             if (take) {
               if (push) {
-                __stcg(&rec[u[j]].sp, 1);
-                ne = make_int4(u[j], (int)(unsigned)r[j].lab, (int)(unsigned)(r[j].lab >> 32), __float_as_int(r[j].pen));
+                const int32_t flags = kMulti ? uf[j] : 0;
+                __stcg(&rec[u[j]].sp, 1 | flags);
+                ne = make_int4(u[j], (int)(unsigned)r[j].lab, (int)(unsigned)(r[j].lab >> 32) | flags,
+                               __float_as_int(r[j].pen));
               }
               if (at < av) {
                 const int s = bd.freel[(unsigned)(hd + at) % (unsigned)kS];
@@ -666,7 +676,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
     if (!kGen && warp >= solo) {
       for (int i = (tid - 32 * solo) / L; i < nf; i += (kThreads - 32 * solo) / L) {
         const int s = bd.fresh[q ^ 1][i];
-        const int f0 = bd.ent[s].y, deg = bd.ent[s].z & 0x7fffffff;
+        const int f0 = bd.ent[s].y, deg = bd.ent[s].z & (kMulti ? kSpMask : 0x7fffffff);
         int32_t u[K];
         float ci[K], co[K];
 #pragma unroll
@@ -760,10 +770,10 @@ __device__ __forceinline__ void count_work(const Problem& pr, const Outcome& o, 
   for (int64_t i = first; i < pr.R; i += step) {
     const int32_t r = (int32_t)i;
     const Rec x = ld_rec(&pr.rec[r]);
-    if (x.sp < 2) continue;
+    if ((kMulti ? x.sp & kSpMask : x.sp) < 2) continue;
     if (kMulti) {
       ++pops;
-      if ((unsigned long long)__double_as_longlong(__ldcg(&pr.mtgt[r])) != pr.none) continue;
+      if (x.sp & kTgt) continue;
     } else {
       if (!(o.exhausted || x.lab < o.ld || (x.lab == o.ld && r < pr.dst))) continue;
       ++pops;

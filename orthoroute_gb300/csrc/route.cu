@@ -44,9 +44,11 @@ thread_local int g_window_look = 8;
 
 constexpr int kMaxViaNodes = 4096;
 constexpr int kMaxSkip = 16;                   // nets a window may skip over (look-ahead)
-// CTAs of one ROI search.  More of them share a phase's entries but make its
-// barrier dearer.
-constexpr int kTeam = 16;
+// CTAs of one ROI search (fewer where a window's members share the SMs): half
+// the SMs, so that two jobs' searches fit side by side.  A team's phase of an
+// ROI of 50,000 nodes on 600x400x12: 8.7 us with 8 CTAs, 6.5 with 16, 5.3
+// with 32, 4.5 with 76 and with 152; ROIs of 14,000 nodes: 4.4, 3.9, 3.8, 3.7.
+constexpr int kTeam = 76;
 
 // Control words of one search slot, kept between searches (sid) or zero at
 // the start of each (team).
@@ -176,7 +178,8 @@ __host__ __device__ inline BfsSlot bfs_slot_at(char* base, int32_t N, int64_t qc
 // Per-stage cycle counters of the ROI searches (a tracing aid, read with
 // ogr_search_profile; thread 0 of a team's first CTA): [0] BFS waves, [1] ROI
 // compaction, [2] search init, [3] phases, [4] of these waiting for the team,
-// [7] statistics + backtrace, [8] cleanup, [9] searches, [10] phases, [11] BFS
+// [5] rip-up and commit, [6] window formation (CTA 0 of a pass), [7] statistics
+// + backtrace, [8] cleanup, [9] searches, [10] phases, [11] BFS
 // waves run, [12] ROI nodes, [13] entries examined, [14] ROIs taken from the
 // batched extraction.
 __device__ unsigned long long g_stage[16];
@@ -691,8 +694,6 @@ __device__ __noinline__ void roi_search(const RoiJob* jp, char* smem, int* statu
   pr.ov[0] = w.ov[0];
   pr.ov[1] = w.ov[1];
   pr.mseed = kMulti ? job.ms->init : nullptr;
-  pr.mtgt = kMulti ? job.ms->tcost : nullptr;
-  pr.none = kNoTerm;
   pr.ctl = &w.ctl->team;
   pr.rank = job.rank;
   pr.nranks = job.nranks;
@@ -749,10 +750,10 @@ __device__ __noinline__ void roi_search(const RoiJob* jp, char* smem, int* statu
     const bool none = !kMulti && (rs < 0 || rd < 0 || rs == rd);
     pr.src = rs;
     pr.dst = rd;
-    auto enter = [&](int32_t r, int at) {
+    auto enter = [&](int32_t r, int at, int32_t flags) {
       const int32_t gid = roi[r], f0 = g.indptr[gid];
       w.claim[r] = pr.sid;
-      w.ov[0][at] = make_int4(r, f0, g.indptr[gid + 1] - f0, __float_as_int(__ldcg(&w.rec[r].pen)));
+      w.ov[0][at] = make_int4(r, f0, (g.indptr[gid + 1] - f0) | flags, __float_as_int(__ldcg(&w.rec[r].pen)));
     };
     if (ready && job.rank == 0) {
       if constexpr (kMulti) {
@@ -770,7 +771,10 @@ __device__ __noinline__ void roi_search(const RoiJob* jp, char* smem, int* statu
           const unsigned long long was = atomicExch(reinterpret_cast<unsigned long long*>(&ms.tcost[r]),
                                                     (unsigned long long)__double_as_longlong(c));
           if (was != kNoTerm) sm.res[1] = 1;
+          // (a target cost that is not a number marks no target)
+          if (c == c) w.rec[r].sp = kTgt;
         }
+        __syncthreads();
         for (int i = tid; i < ms.nseeds; i += kThreads) {
           const int32_t gid = ms.seeds[i];
           const int32_t r = gid < 0 || gid >= g.num_nodes ? -2 : w.g2r[gid];
@@ -785,29 +789,20 @@ __device__ __noinline__ void roi_search(const RoiJob* jp, char* smem, int* statu
             sm.res[1] = 1;
             continue;
           }
-          if (!(c < __longlong_as_double(0x7ff0000000000000ll))) {      // not a start
-            atomicExch(reinterpret_cast<unsigned long long*>(&ms.init[r]), kNoTerm);
-            continue;
-          }
+          if (!(c < __longlong_as_double(0x7ff0000000000000ll))) continue;      // not a start
           const float pen = __ldcg(&w.rec[r].pen);
           unsigned long long lb = ogr_dbits(c + (double)pen);
           if (fix) {
             lb = 0ull;
             if (seed_ticks(c, &lb) && tick_finite(pen)) lb += ticks(pen);
           }
-          enter(r, atomicAdd(&sm.res[0], 1));
-          w.rec[r].sp = 1;
+          const int32_t flags = kSeed | (__ldcg(&w.rec[r].sp) & kTgt);
+          enter(r, atomicAdd(&sm.res[0], 1), flags);
+          w.rec[r].sp = 1 | flags;
           atomicMin(&sm.wmin[0], lb);
         }
-        __syncthreads();
-        // a target cost that is not a number marks no target
-        for (int i = tid; i < ms.ntargets; i += kThreads) {
-          const int32_t gid = ms.targets[i];
-          const int32_t r = gid < 0 || gid >= g.num_nodes ? -1 : w.g2r[gid];
-          if (r >= 0 && ms.target_cost[i] != ms.target_cost[i]) ms.tcost[r] = __longlong_as_double((long long)kNoTerm);
-        }
       } else if (tid == 0 && !none) {
-        enter(rs, 0);
+        enter(rs, 0, 0);
         w.ov[0][0].w = 0;          // src's penalty does not count
         sm.res[0] = 1;
         sm.wmin[0] = 0ull;
@@ -866,7 +861,7 @@ __device__ __noinline__ void roi_search(const RoiJob* jp, char* smem, int* statu
         const int32_t r = w.g2r[ms.targets[i]];
         if (r < 0) continue;
         const Rec x = ld_rec(&w.rec[r]);
-        if (x.sp < 2) continue;
+        if ((x.sp & kSpMask) < 2) continue;
         const double lr = fix ? label_value<true>(x.lab) : label_value<false>(x.lab);
         const double tot = lr + ms.target_cost[i];
         if (!(tot < dinf)) continue;
@@ -938,7 +933,7 @@ __device__ __noinline__ void roi_search(const RoiJob* jp, char* smem, int* statu
 // The search in the form for rows of ROW arcs.
 template <int ROW, bool kMulti>
 __device__ __forceinline__ void roi_search_row(const RoiJob& job, char* smem, int* status, int* len) {
-  if constexpr (ROW == 4) roi_search<4, 1, kMulti>(&job, smem, status, len);
+  if constexpr (ROW == 4) roi_search<2, 2, kMulti>(&job, smem, status, len);
   else if constexpr (ROW == 8) roi_search<8, 1, kMulti>(&job, smem, status, len);
   else if constexpr (ROW == 16) roi_search<8, 2, kMulti>(&job, smem, status, len);
   else roi_search<16, 2, kMulti>(&job, smem, status, len);
@@ -1382,6 +1377,8 @@ window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa,
     // fallback ROI (terminals +- fallback BFS depth + halo), so it commutes
     // with the skipped nets whatever they do when their turn comes.
     // Pending = net_status still -1 (set before the launch).
+    StageClock clk;
+    clk.start();
     if (b == 0) {
       if (tid == 0) {
         int cur = c->cursor;
@@ -1451,6 +1448,7 @@ window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa,
         ++W;
       }
       if (tid == 0) c->wsize = W;
+      clk.mark(6);
     }
     if (!win_barrier(c, target, &s_bar)) break;
     const int W = *(volatile int32_t*)&c->wsize;
@@ -1475,6 +1473,7 @@ window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa,
         atomicAdd(&g_stage[14], 1ull);
       }
       if (tid == 0 && rc != OGR_OK) atomicExch(&c->error, rc);
+      if (b == 0) clk.mark(5);
     }
     if (!win_barrier(c, target, &s_bar)) break;
     if (*(volatile int32_t*)&c->error) break;
@@ -1499,6 +1498,7 @@ window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa,
     if (!win_barrier(c, target, &s_bar)) break;
     if (*(volatile int32_t*)&c->error) break;
     // 4. commit
+    clk.start();
     if (b < W) clear_team(slot_of(b, solo).ctl);
     int ff = W;
     for (int m = 0; m < W; ++m)
@@ -1567,6 +1567,7 @@ window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa,
       }
       if (tid == 0 && rc != OGR_OK) atomicExch(&c->error, rc);
     }
+    if (b == 0) clk.mark(5);
     if (!win_barrier(c, target, &s_bar)) break;
     if (*(volatile int32_t*)&c->error) break;
     const int fb = *(volatile int32_t*)&c->fb;
