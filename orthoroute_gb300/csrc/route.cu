@@ -32,7 +32,7 @@ namespace {
 using ogr_phase::kThreads;
 using ogr_phase::kWarps;
 constexpr int kSub = 16;                       // lanes per node (ROI BFS)
-constexpr int kGroups = kThreads / kSub;       // nodes in flight per CTA (ROI BFS)
+constexpr int kBfsThreads = 768;               // of the kernels that only extract ROIs (others: their own)
 
 // Accepted and kept for callers (ogr_search_lanes); the search fits its lanes
 // to the lattice's rows, and results never depended on it.
@@ -185,8 +185,8 @@ __host__ __device__ inline BfsSlot bfs_slot_at(char* base, int32_t N, int64_t qc
 __device__ unsigned long long g_stage[16];
 
 struct Shared {
-  int s_cnt[kWarps];
-  int s_off[kWarps];
+  int s_cnt[32];
+  int s_off[32];
   int nq[4];
   int seen_count;
   int met;
@@ -270,12 +270,13 @@ constexpr int kBfsWords = (int)((ogr_phase::kSmemBytes - kBfsQBytes) / 8);     /
 // nodes at once; marks, queues and the compaction never leave the SM.  With
 // the marks as compare-and-swaps in global memory (a third round trip and an
 // atomic per arc) an ROI of 50,000 nodes on 600x400x12 took 1,352 us and its
-// compaction 250; now 600 and 60.
+// compaction 250; now 547 and 55 with 768 threads (512: 600, 1,024: 540, but
+// 14,000-node ROIs then take 180 us instead of 165).
 __device__ bool roi_build_box(Shared& sh, const ogr_graph& g, const ogr_net_args& a, int32_t* const* q, int64_t qcap,
                               int32_t* out, int32_t out_cap, char* smem, StageClock& clk) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = blockDim.x, nw = nt >> 5;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
-  const int32_t src = a.src, dst = a.dst;
+  const int32_t src = a.src, dst = a.dst, plane = nx * ny;
   const int32_t* __restrict__ indptr = g.indptr;
   const int32_t* __restrict__ indices = g.indices;
   const Div by_plane((unsigned)(nx * ny)), by_nx((unsigned)nx);
@@ -303,7 +304,7 @@ __device__ bool roi_build_box(Shared& sh, const ogr_graph& g, const ogr_net_args
     if (reach <= 0) return false;
   }
   const int NW = RW * BH * nz;
-  for (int i = tid; i < NW; i += kThreads) bits[0][i] = bits[1][i] = 0u;
+  for (int i = tid; i < NW; i += nt) bits[0][i] = bits[1][i] = 0u;
   if (tid == 0) {
     sh.nq[0] = sh.nq[2] = 1;
     sq[0] = src;
@@ -335,14 +336,19 @@ __device__ bool roi_build_box(Shared& sh, const ogr_graph& g, const ogr_net_args
       if (tid == 0) sh.nq[nxt] = 0;
       __syncthreads();
       int met = 0;
-      for (int base = warp * 16; base < n; base += kWarps * 16) {
+      for (int base = warp * 16; base < n; base += nw * 16) {
         const int i = base + (lane >> 1);
-        int32_t f = 0, f1 = 0;
+        int32_t u = 0, f = 0, f1 = 0;
         if (i < n) {
-          const int32_t u = i < kBfsQ ? sq[cur * kBfsQ + i] : q[cur][i];
+          u = i < kBfsQ ? sq[cur * kBfsQ + i] : q[cur][i];
           f = indptr[u] + (lane & 1);
           f1 = indptr[u + 1];
         }
+        // (in the shadow of the row bounds' load)
+        int ux, uy, uz;
+        coord(u, ux, uy, uz);
+        const int32_t ur = u - uz * plane;
+        const int ubx = ux - X0, uby = uy - Y0;
         while (__any_sync(0xffffffffu, f < f1)) {
           int32_t v[kBfsArcs];
 #pragma unroll
@@ -354,9 +360,16 @@ __device__ bool roi_build_box(Shared& sh, const ogr_graph& g, const ogr_net_args
           for (int j = 0; j < kBfsArcs; ++j) {
             bool fresh = false;
             if (v[j] >= 0) {
-              int x, y, z;
-              coord(v[j], x, y, z);
-              const int bx = x - X0, by = y - Y0;
+              // the next cell, or another layer of the same one
+              const int32_t d = v[j] - u;
+              int bx = ubx, by = uby, z = (int)by_plane((unsigned)v[j]);
+              const int32_t r = v[j] - z * plane;
+              if (r != ur) {
+                if (d == 1 || d == -1) bx += d;
+                else if (d == nx || d == -nx) by += d > 0 ? 1 : -1;
+                else bx = -1;      // (an arc of no lattice: the caller takes the large form)
+                if ((unsigned)(bx + X0) >= (unsigned)nx || (unsigned)(by + Y0) >= (unsigned)ny) bx = -1;
+              }
               if ((unsigned)bx >= (unsigned)BW || (unsigned)by >= (unsigned)BH) {
                 sh.left = 1;
               } else {
@@ -367,8 +380,8 @@ __device__ bool roi_build_box(Shared& sh, const ogr_graph& g, const ogr_net_args
                     met = 1;
                   } else {
                     fresh = true;
-                    lx0 = min(lx0, x); lx1 = max(lx1, x);
-                    ly0 = min(ly0, y); ly1 = max(ly1, y);
+                    lx0 = min(lx0, bx); lx1 = max(lx1, bx);
+                    ly0 = min(ly0, by); ly1 = max(ly1, by);
                   }
                 }
               }
@@ -407,15 +420,17 @@ __device__ bool roi_build_box(Shared& sh, const ogr_graph& g, const ogr_net_args
   ly0 = __reduce_min_sync(0xffffffffu, ly0);
   ly1 = __reduce_max_sync(0xffffffffu, ly1);
   if (lane == 0) {
-    atomicMin(&sh.bx0, lx0); atomicMax(&sh.bx1, lx1);
-    atomicMin(&sh.by0, ly0); atomicMax(&sh.by1, ly1);
+    if (lx1 >= 0) {
+      atomicMin(&sh.bx0, X0 + lx0); atomicMax(&sh.bx1, X0 + lx1);
+      atomicMin(&sh.by0, Y0 + ly0); atomicMax(&sh.by1, Y0 + ly1);
+    }
   }
   __syncthreads();
   clk.mark(0);
   // Ordered compaction (ascending global id): each warp owns a contiguous run
   // of words; count, scan the counts, then write.  Only positions below
   // out_cap are stored; those of src and dst are recorded.
-  const int per = ((NW + kWarps - 1) / kWarps + 31) & ~31;
+  const int per = ((NW + nw - 1) / nw + 31) & ~31;
   const int w0 = warp * per, w1 = min(NW, w0 + per);
   int cnt = 0;
   for (int i = w0 + lane; i < w1; i += 32) cnt += __popc(bits[0][i] | bits[1][i]);
@@ -424,7 +439,7 @@ __device__ bool roi_build_box(Shared& sh, const ogr_graph& g, const ogr_net_args
   __syncthreads();
   if (tid == 0) {
     int t = 0;
-    for (int i = 0; i < kWarps; ++i) {
+    for (int i = 0; i < nw; ++i) {
       sh.s_off[i] = t;
       t += sh.s_cnt[i];
     }
@@ -467,7 +482,7 @@ __device__ bool roi_build_box(Shared& sh, const ogr_graph& g, const ogr_net_args
 __device__ __noinline__ void roi_build_large(Shared& sh, const ogr_graph& g, const ogr_net_args& a, int32_t* seen, int32_t* const* q,
                           int64_t qcap, int32_t* out, int32_t out_cap, StageClock& clk) {
   const int tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5;
+  const int lane = tid & 31, warp = tid >> 5, nt = blockDim.x, nw = nt >> 5, groups = nt / kSub;
   const int sl = tid & (kSub - 1), grp = tid / kSub;
   const int nx = g.nx, nz = g.nz;
   const int32_t plane = nx * g.ny;
@@ -506,7 +521,7 @@ __device__ __noinline__ void roi_build_large(Shared& sh, const ogr_graph& g, con
       int32_t* qn = q[nxt];
       int local_met = 0, local_new = 0, local_ovf = 0;
       int lx0 = 1 << 30, lx1 = -1, ly0 = 1 << 30, ly1 = -1;
-      for (int i = grp; i < n; i += kGroups) {
+      for (int i = grp; i < n; i += groups) {
         const int32_t u = qc[i];
         const int32_t e1 = indptr[u + 1];
         for (int32_t e = indptr[u] + sl; e < e1; e += kSub) {
@@ -561,7 +576,7 @@ __device__ __noinline__ void roi_build_large(Shared& sh, const ogr_graph& g, con
   const int W = sh.bx1 - sh.bx0 + 1, H = sh.by1 - sh.by0 + 1;
   const int32_t area = W * H;
   const int32_t V = area * nz;
-  const int32_t seg = (((V + kWarps - 1) / kWarps) + 31) & ~31;
+  const int32_t seg = (((V + nw - 1) / nw) + 31) & ~31;
   const int32_t w0 = warp * seg, w1 = min(V, w0 + seg);
   const int bx0 = sh.bx0, by0 = sh.by0;
   auto gid_of = [&](int32_t i) -> int32_t {
@@ -580,14 +595,14 @@ __device__ __noinline__ void roi_build_large(Shared& sh, const ogr_graph& g, con
   if (lane == 0) sh.s_cnt[warp] = cnt;
   __syncthreads();
   if (warp == 0) {
-    const int c = lane < kWarps ? sh.s_cnt[lane] : 0;
+    const int c = lane < nw ? sh.s_cnt[lane] : 0;
     int x = c;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int y = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o) x += y;
     }
-    if (lane < kWarps) sh.s_off[lane] = x - c;
+    if (lane < nw) sh.s_off[lane] = x - c;
     if (lane == 31) sh.R = x;
   }
   __syncthreads();
@@ -612,7 +627,7 @@ __device__ __noinline__ void roi_build_large(Shared& sh, const ogr_graph& g, con
   __syncthreads();
   roi_finish(sh, a, out, out_cap);
   // restore seen[] to zero over the bounding box
-  for (int32_t i = tid; i < V; i += kThreads) seen[gid_of(i)] = 0;
+  for (int32_t i = tid; i < V; i += nt) seen[gid_of(i)] = 0;
   __syncthreads();
   clk.mark(1);
 }
@@ -1030,7 +1045,7 @@ __device__ int apply_path_dev(const ogr_graph& g, const ogr_state& st, const int
 
 // ---- kernels -------------------------------------------------------------------
 // The ROI of a net into w.roi: result[0] = status, result[3] = its size.
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kBfsThreads, 1)
 build_roi_kernel(ogr_graph g, ogr_net_args a, Ws w) {
   extern __shared__ __align__(16) char smem[];
   __shared__ Shared sh;
@@ -1064,7 +1079,7 @@ find_team_kernel(ogr_graph g, ogr_state st, ogr_net_args a, Ws w, const int32_t*
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kBfsThreads, 1)
 roi_kernel(ogr_graph g, ogr_net_args a, Ws w, int32_t* roi_out, int32_t roi_cap) {
   extern __shared__ __align__(16) char smem[];
   __shared__ Shared sh;
@@ -1078,7 +1093,7 @@ roi_kernel(ogr_graph g, ogr_net_args a, Ws w, int32_t* roi_out, int32_t roi_cap)
     if (threadIdx.x == 0 && R > roi_cap) sh.status = OGR_ERR_CAPACITY;
     __syncthreads();
     if (sh.status == OGR_OK)
-      for (int r = threadIdx.x; r < R; r += kThreads) roi_out[r] = r;
+      for (int r = threadIdx.x; r < R; r += blockDim.x) roi_out[r] = r;
   } else {
     roi_build(sh, g, a, w.seen, w.q, w.qcap, roi_out, roi_cap, smem, clk);
     R = sh.R;
@@ -1197,7 +1212,7 @@ paths_commit_kernel(ogr_graph g, ogr_state st, const int32_t* nodes, const int32
 // Extract the (cost-independent) ROIs of every ROI net of the pass, one net
 // per CTA at a time, each CTA with its own BFS slot.  roi_len[n] = -1 when a
 // queue overflowed (the pass then extracts that ROI inline).
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kBfsThreads, 1)
 roi_batch_kernel(ogr_graph g, ogr_net_table t, ogr_pass_args pa, ogr_roi_batch rb) {
   extern __shared__ __align__(16) char smem[];
   __shared__ Shared sh;
@@ -1733,7 +1748,7 @@ int launch_find(const ogr_graph& g, const ogr_state& st, const ogr_net_args& a, 
   OGR_CUDA_TRY(cudaMemsetAsync(&w.ctl->team, 0, sizeof(ogr_phase::Ctl), s));
   if (roi == nullptr && !a.full_graph) {
     OGR_CUDA_TRY(wide_smem((const void*)build_roi_kernel));
-    build_roi_kernel<<<1, kThreads, ogr_phase::kSmemBytes, s>>>(g, a, w);
+    build_roi_kernel<<<1, kBfsThreads, ogr_phase::kSmemBytes, s>>>(g, a, w);
     OGR_LAUNCH_CHECK();
   }
   if (a.full_graph) R = g.num_nodes;
@@ -1919,7 +1934,7 @@ extern "C" int ogr_extract_roi(const ogr_graph* g, const ogr_net_args* net, void
   ws_layout(g->num_nodes, (char*)ws, &w);
   cudaStream_t s = ogr_stream(stream);
   OGR_CUDA_TRY(wide_smem((const void*)roi_kernel));
-  roi_kernel<<<1, kThreads, ogr_phase::kSmemBytes, s>>>(*g, *net, w, roi_out, roi_cap);
+  roi_kernel<<<1, kBfsThreads, ogr_phase::kSmemBytes, s>>>(*g, *net, w, roi_out, roi_cap);
   OGR_LAUNCH_CHECK();
   int64_t res[2];
   OGR_CUDA_TRY(cudaMemcpyAsync(res, w.result, sizeof(res), cudaMemcpyDeviceToHost, s));
@@ -1987,7 +2002,7 @@ extern "C" int ogr_route_pass(const ogr_graph* g, const ogr_state* st, const ogr
     rbv = *rb;
     OGR_CUDA_TRY(cudaMemsetAsync(rbv.next, 0, sizeof(int32_t), s));
     OGR_CUDA_TRY(wide_smem((const void*)roi_batch_kernel));
-    roi_batch_kernel<<<rbv.slots, kThreads, ogr_phase::kSmemBytes, s>>>(*g, *t, *pa, rbv);
+    roi_batch_kernel<<<rbv.slots, kBfsThreads, ogr_phase::kSmemBytes, s>>>(*g, *t, *pa, rbv);
     OGR_LAUNCH_CHECK();
   }
   const bool windows = win != nullptr && win->slots > 0 && batch && rbv.roi_box != nullptr;

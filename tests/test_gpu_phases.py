@@ -140,6 +140,9 @@ def test_roi_forms_match_oracle(row, kind):
     ((260, 250, 16), 400_000, 80, False),    # the box is cut to fit and the search leaves it
     ((64, 64, 4), 900, 80, False),           # truncated, terminals swapped in
     ((90, 70, 6), 50_000, 3, False),         # the waves do not meet
+    ((60, 50, 20), 50_000, 80, False),       # more than 16 layers
+    ((20, 16, 36), 50_000, 80, True),        # more than 32
+    ((1, 90, 6), 50_000, 80, False), ((90, 1, 6), 50_000, 80, False),
 ])
 def test_roi_extraction_matches_oracle(dims, max_nodes, depth, blocked):
     from oracle.roi import extract_roi_bfs
