@@ -116,7 +116,7 @@ __device__ __forceinline__ bool tick_finite(float c) { return tick_exact(c) && _
 __device__ __forceinline__ unsigned long long ticks(float c) {
   const unsigned b = __float_as_uint(c);
   // the shift is at most 28: one wide multiply instead of a 64-bit shift
-  return b < kBitsLow ? 0ull : (unsigned long long)((b & 0x7fffffu) | 0x800000u) * (1u << ((b >> 23) - 120u));
+  return b < kBitsLow ? 0ull : (unsigned long long)((b & 0x7fffffu) | 0x800000u) * (1u << (((b >> 23) - 120u) & 31u));
 }
 
 // The largest tick count that rounds (to nearest even) to the same float32
@@ -437,8 +437,11 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
           load(j);
         }
       }
-      // pull: the candidate alt through the arc, cin from the others
+      // Pull.  In ticks alt is the candidate through a settled neighbour's arc;
+      // through any other arc it is the least that may yet come that way, and
+      // v is final if its key's class ends below all of those.
       u64 alt[K], mx = kNone, hi = 0;
+      unsigned open = 0;           // arcs of the second kind
       u64 gx = kNone, gl = kNone;  // general form: the lane's best candidate, its relaxer
       int32_t gu = 0x7fffffff;
       float cin = kInf, mn = kInf, m32 = kInf;
@@ -447,13 +450,14 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
       if (!kGen) {
 #pragma unroll
         for (int j = 0; j < K; ++j) {
-          alt[j] = kNone;
-          if ((unsigned)(r[j].sp - 2) < (unsigned)phase) {      // settled before this phase
-            if (!(kMulti && (uf[j] & kTgt)) && ci[j] < kInf) alt[j] = r[j].lab + (ticks(ci[j]) + pt);
-          } else if (r[j].sp >= 0 && !(kMulti && (uf[j] & kTgt))) {
-            cin = fminf(cin, ci[j]);
+          const bool in = r[j].sp >= 0 && ci[j] < kInf && !(kMulti && (uf[j] & kTgt));
+          const bool done = in && (unsigned)(r[j].sp - 2) < (unsigned)phase;      // settled before this phase
+          alt[j] = (done ? r[j].lab : T) + (ticks(ci[j]) + pt);
+          if (done) mx = alt[j] < mx ? alt[j] : mx;
+          if (!done) {
+            if (in) open |= 1u << j;
           }
-          mx = alt[j] < mx ? alt[j] : mx;
+          if (!in) alt[j] = kNone;
         }
       } else {
         for (int f = sl; f < deg; f += L) {
@@ -486,15 +490,15 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
           mx = ox < mx ? ox : mx;
         } else {
           m32 = fminf(m32, __shfl_xor_sync(kAll, m32, o));
+          cin = fminf(cin, __shfl_xor_sync(kAll, cin, o));
         }
-        cin = fminf(cin, __shfl_xor_sync(kAll, cin, o));
       }
       bool tied;
       if (!kGen) {
-        hi = round_hi(mx);
+        hi = mx != kNone ? round_hi(mx) : 0ull;
 #pragma unroll
         for (int j = 0; j < K; ++j)
-          if (alt[j] != kNone && alt[j] <= hi && (gx == kNone || r[j].lab < gl || (r[j].lab == gl && u[j] < gu))) {
+          if (!((open >> j) & 1) && alt[j] <= hi && (gx == kNone || r[j].lab < gl || (r[j].lab == gl && u[j] < gu))) {
             gx = alt[j];
             gl = r[j].lab;
             gu = u[j];
@@ -552,7 +556,10 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
       bool final;
       if (!kGen) {
         if (mine && lv > kTickLimit) sm.inexact = 1;
-        final = lv == T || !(cin < kInf) || T + ticks(cin) + pt > hi;
+        bool late = false;         // an open arc's bound within the class (hi may be a seed's)
+#pragma unroll
+        for (int j = 0; j < K; ++j) late |= ((open >> j) & 1) && alt[j] <= hi;
+        final = (__ballot_sync(kAll, late) & gmask) == 0 || lv == T;
       } else {
         final = lv == T || m32 < __double2float_rn((__longlong_as_double((long long)T) + (double)cin) + pd);
       }
@@ -601,9 +608,8 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
           if (expand && r[j].sp >= 0 && (unsigned)(r[j].sp - 2) >= (unsigned)phase) {
             u64 ly = kNone;
             if (!kGen) {
-              // (whoever reached u first checked its penalty)
-              if (!tick_finite(r[j].pen)) sm.inexact = 1;
-              else if (co[j] < kInf) ly = lv + (ticks(co[j]) + ticks(r[j].pen));
+              // (whoever reaches u first checks its penalty)
+              if (co[j] < kInf) ly = lv + (ticks(co[j]) + ticks(r[j].pen));
             } else {
               const double y = (__longlong_as_double((long long)lv) + (double)co[j]) + (double)r[j].pen;
               if (__double2float_rn(y) < kInf) ly = ogr_dbits(y);
@@ -624,6 +630,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
             int4 ne = en;
             if (take) {
               if (push) {
+                if (!kGen && !tick_finite(r[j].pen)) sm.inexact = 1;
                 const int32_t flags = kMulti ? uf[j] : 0;
                 __stcg(&rec[u[j]].sp, 1 | flags);
                 ne = make_int4(u[j], (int)(unsigned)r[j].lab, (int)(unsigned)(r[j].lab >> 32) | flags,
