@@ -970,24 +970,108 @@ __device__ void build_roi(Shared& sh, const ogr_graph& g, const ogr_net_args& a,
 }
 
 // ---- commit / rip-up ---------------------------------------------------------
+constexpr int kViaHops = kMaxViaNodes / 3;     // via hops listed in s_via[kMaxViaNodes]
+
+// Calls f(node) once for every node that the via hops of a path span, from any
+// thread of the block; true if there are more than kMaxViaNodes of them.
+// s_via: kMaxViaNodes words, s_cnt: two words.
+//
+// The hops are sorted out by all threads, and a node that several hops span
+// belongs to the one listed first.  (One thread walking the path with four
+// divisions per hop took 150 us for 450 hops, most of a commit.)
+template <typename F>
+__device__ bool each_via_node(const int32_t* path, int hops, int32_t plane, int32_t* s_via, int* s_cnt, F&& f) {
+  const int tid = threadIdx.x, nt = blockDim.x;
+  if (tid == 0) { s_cnt[0] = 0; s_cnt[1] = 0; }
+  __syncthreads();
+  for (int i = tid; i < hops; i += nt) {
+    const int32_t u = path[i], v = path[i + 1];
+    const int zu = u / plane, zv = v / plane;
+    if (u - zu * plane != v - zv * plane || zu == zv) continue;
+    const int k = atomicAdd(&s_cnt[0], 1);
+    if (k < kViaHops) {
+      s_via[k] = u - zu * plane;
+      s_via[kViaHops + k] = min(zu, zv);
+      s_via[2 * kViaHops + k] = max(zu, zv);
+    }
+  }
+  __syncthreads();
+  const int n = s_cnt[0];
+  if (n <= kViaHops) {
+    for (int k = tid; k < n; k += nt) {
+      const int32_t r = s_via[k];
+      const int lo = s_via[kViaHops + k], hi = s_via[2 * kViaHops + k];
+      for (int z = lo; z <= hi; ++z) {
+        bool dup = false;
+        for (int j = 0; j < k && !dup; ++j)
+          dup = s_via[j] == r && z >= s_via[kViaHops + j] && z <= s_via[2 * kViaHops + j];
+        if (!dup && atomicAdd(&s_cnt[1], 1) < kMaxViaNodes) f(z * plane + r);
+      }
+    }
+    __syncthreads();
+    return s_cnt[1] > kMaxViaNodes;
+  }
+  // more hops than the list holds: one thread collects the nodes
+  __syncthreads();
+  if (tid == 0) {
+    int nv = 0;
+    bool full = false;
+    for (int i = 0; i < hops && !full; ++i) {
+      const int32_t u = path[i], v = path[i + 1];
+      const int zu = u / plane, zv = v / plane;
+      const int32_t r = u - zu * plane;
+      if (r != v - zv * plane || zu == zv) continue;
+      for (int z = min(zu, zv); z <= max(zu, zv); ++z) {
+        const int32_t nd = z * plane + r;
+        bool dup = false;
+        for (int k = 0; k < nv && !dup; ++k) dup = s_via[k] == nd;
+        if (dup) continue;
+        if (nv >= kMaxViaNodes) { full = true; break; }
+        s_via[nv++] = nd;
+      }
+    }
+    s_cnt[0] = nv;
+    s_cnt[1] = full ? 1 : 0;
+  }
+  __syncthreads();
+  const int nv = s_cnt[0];
+  for (int k = tid; k < nv; k += nt) f(s_via[k]);
+  const bool full = s_cnt[1] != 0;
+  __syncthreads();
+  return full;
+}
+
+// The arc u -> v (-1: none).  A row's arcs come four at a time, so a hop waits
+// once or twice for its row, not once per arc.
+__device__ __forceinline__ int32_t arc_to(const ogr_graph& g, int32_t u, int32_t v) {
+  const int32_t e1 = g.indptr[u + 1];
+  for (int32_t e = g.indptr[u]; e < e1; e += 4) {
+    int32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = e + j < e1 ? g.indices[e + j] : -1;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (w[j] == v) return e + j;
+  }
+  return -1;
+}
+
 // commit_path / clear_path (:1096-1135) + refresh_live_present_costs (:1403),
 // _mark/_clear_path_node_use (:4635-4659), barrel ownership of every node a
 // via hop spans (:4934-5034), arcs in _path_to_edges order (:9981-10046).
 // Returns OGR_OK, OGR_ERR_ARG (a hop is not an arc) or OGR_ERR_CAPACITY.
+// s_flags: three words.
 __device__ int apply_path_dev(const ogr_graph& g, const ogr_state& st, const int32_t* path, int32_t len,
                               int32_t net_id, int32_t sign, float pres_fac, int32_t live, int32_t* arcs_out,
                               int32_t* s_via, int* s_flags) {
   const int tid = threadIdx.x, nt = blockDim.x;
-  if (tid == 0) { s_flags[0] = 0; s_flags[1] = 0; }
+  if (tid == 0) s_flags[2] = 0;
   __syncthreads();
   const int hops = len - 1;
   const int32_t plane = g.nx * g.ny;
   for (int i = tid; i < hops; i += nt) {
-    const int32_t u = path[i], v = path[i + 1];
-    int32_t f = -1;
-    for (int32_t e = g.indptr[u]; e < g.indptr[u + 1]; ++e)
-      if (g.indices[e] == v) { f = e; break; }
-    if (f < 0) { s_flags[1] = 1; continue; }
+    const int32_t f = arc_to(g, path[i], path[i + 1]);
+    if (f < 0) { s_flags[2] = 1; continue; }
     const int32_t r = g.rev[f];
     const int j = hops - 1 - i;
     if (arcs_out) { arcs_out[i] = f; arcs_out[hops + j] = r; }
@@ -1012,35 +1096,16 @@ __device__ int apply_path_dev(const ogr_graph& g, const ogr_state& st, const int
     st.path_node_use[n] = sign > 0 ? u + 1 : max(u - 1, 0);
   }
   __syncthreads();
-  if (tid == 0) {
-    int nv = 0;
-    for (int i = 0; i < hops && !s_flags[1]; ++i) {
-      const int32_t u = path[i], v = path[i + 1];
-      const int32_t ru = u % plane, rv = v % plane;
-      const int zu = u / plane, zv = v / plane;
-      if (ru != rv || zu == zv) continue;
-      for (int z = min(zu, zv); z <= max(zu, zv); ++z) {
-        const int32_t nd = z * plane + ru;
-        bool dup = false;
-        for (int k = 0; k < nv; ++k)
-          if (s_via[k] == nd) { dup = true; break; }
-        if (dup) continue;
-        if (nv >= kMaxViaNodes) { s_flags[1] = 2; break; }
-        s_via[nv++] = nd;
-      }
-    }
-    s_flags[0] = nv;
+  if (s_flags[2]) {
+    __syncthreads();
+    return OGR_ERR_ARG;
   }
-  __syncthreads();
-  const int nv = s_flags[0];
-  for (int k = tid; k < nv; k += nt) {
-    const int32_t nd = s_via[k];
+  const bool full = each_via_node(path, hops, plane, s_via, s_flags, [&](int32_t nd) {
     st.owner_count[nd] += sign > 0 ? 1 : -1;
     st.owner_xor[nd] ^= net_id;
-  }
-  const int bad = s_flags[1];
+  });
   __syncthreads();
-  return bad ? (bad == 1 ? OGR_ERR_ARG : OGR_ERR_CAPACITY) : OGR_OK;
+  return full ? OGR_ERR_CAPACITY : OGR_OK;
 }
 
 // ---- kernels -------------------------------------------------------------------
@@ -1128,7 +1193,7 @@ __global__ void __launch_bounds__(kApplyThreads)
 path_apply_kernel(ogr_graph g, ogr_state st, const int32_t* path, int32_t len, int32_t net_id, int32_t sign,
                   float pres_fac, int32_t live, int32_t* arcs_out, int32_t* status) {
   __shared__ int32_t s_via[kMaxViaNodes];
-  __shared__ int s_flags[2];
+  __shared__ int s_flags[3];
   const int rc = apply_path_dev(g, st, path, len, net_id, sign, pres_fac, live, arcs_out, s_via, s_flags);
   if (threadIdx.x == 0) *status = rc;
 }
@@ -1146,7 +1211,7 @@ paths_commit_kernel(ogr_graph g, ogr_state st, const int32_t* nodes, const int32
                     int32_t n_paths, int32_t* arcs, int32_t* store_path, int32_t* store_len,
                     int32_t* store_arcs, const int32_t* store_slot, int32_t slot_cap, int32_t* status) {
   __shared__ int32_t s_via[kMaxViaNodes];
-  __shared__ int s_nv, s_bad;
+  __shared__ int s_cnt[2], s_bad;
   const int tid = threadIdx.x, nt = blockDim.x;
   const int32_t plane = g.nx * g.ny;
   for (int32_t k = blockIdx.x; k < n_paths; k += gridDim.x) {
@@ -1156,13 +1221,10 @@ paths_commit_kernel(ogr_graph g, ogr_state st, const int32_t* nodes, const int32
     int32_t* a_out = arcs + 2 * (int64_t)(o - k);
     int32_t* a_store = (store_arcs != nullptr && len <= slot_cap)
                            ? store_arcs + (int64_t)store_slot[k] * 2 * slot_cap : nullptr;
-    if (tid == 0) { s_nv = 0; s_bad = 0; }
+    if (tid == 0) s_bad = 0;
     __syncthreads();
     for (int i = tid; i < hops; i += nt) {
-      const int32_t u = path[i], v = path[i + 1];
-      int32_t f = -1;
-      for (int32_t e = g.indptr[u]; e < g.indptr[u + 1]; ++e)
-        if (g.indices[e] == v) { f = e; break; }
+      const int32_t f = arc_to(g, path[i], path[i + 1]);
       if (f < 0) { s_bad = 1; continue; }
       const int32_t r = g.rev[f];
       a_out[i] = f;
@@ -1178,32 +1240,13 @@ paths_commit_kernel(ogr_graph g, ogr_state st, const int32_t* nodes, const int32
     if (store_path != nullptr && len <= slot_cap)
       for (int i = tid; i < len; i += nt) store_path[(int64_t)store_slot[k] * slot_cap + i] = path[i];
     __syncthreads();
-    if (tid == 0) {
-      int nv = 0;
-      for (int i = 0; i < hops && !s_bad; ++i) {
-        const int32_t u = path[i], v = path[i + 1];
-        const int32_t ru = u % plane, rv = v % plane;
-        const int zu = u / plane, zv = v / plane;
-        if (ru != rv || zu == zv) continue;
-        for (int z = min(zu, zv); z <= max(zu, zv); ++z) {
-          const int32_t nd = z * plane + ru;
-          bool dup = false;
-          for (int q = 0; q < nv; ++q)
-            if (s_via[q] == nd) { dup = true; break; }
-          if (dup) continue;
-          if (nv >= kMaxViaNodes) { s_bad = 2; break; }
-          s_via[nv++] = nd;
-        }
-      }
-      s_nv = nv;
-      if (store_len != nullptr) store_len[store_slot[k]] = len <= slot_cap ? len : 0;
-      if (len > slot_cap && store_path != nullptr) s_bad = 2;
-    }
-    __syncthreads();
-    for (int q = tid; q < s_nv; q += nt) {
-      atomicAdd(&st.owner_count[s_via[q]], 1);
-      atomicXor(&st.owner_xor[s_via[q]], net_ids[k]);
-    }
+    if (tid == 0 && store_len != nullptr) store_len[store_slot[k]] = len <= slot_cap ? len : 0;
+    const int32_t id = net_ids[k];
+    const bool full = !s_bad && each_via_node(path, hops, plane, s_via, s_cnt, [&](int32_t nd) {
+      atomicAdd(&st.owner_count[nd], 1);
+      atomicXor(&st.owner_xor[nd], id);
+    });
+    if (tid == 0 && (full || (len > slot_cap && store_path != nullptr))) s_bad = 2;
     if (tid == 0 && s_bad) atomicMax(status, s_bad);
     __syncthreads();
   }
@@ -1357,7 +1400,7 @@ window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa,
                    char* ctl_base, Ws w, int32_t look, unsigned long long* discarded) {
   extern __shared__ __align__(16) char smem[];
   __shared__ Shared sh;
-  __shared__ int s_flags[2];
+  __shared__ int s_flags[3];
   __shared__ int s_bar;
   __shared__ int s_box[4];
   __shared__ int s_skip[4 * kMaxSkip];
@@ -1648,7 +1691,7 @@ __global__ void window_ws_init_kernel(char* base, int32_t slots, size_t slot_byt
 __global__ void __launch_bounds__(kThreads, 1)
 pass_ripup_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa, int32_t k, Ws w) {
   __shared__ int32_t s_via[kMaxViaNodes];
-  __shared__ int s_flags[2];
+  __shared__ int s_flags[3];
   if (w.result[0] < 0) return;
   const int32_t n = pa.order[k];
   const int32_t old_len = t.store_len[n];
@@ -1672,7 +1715,7 @@ pass_full_tail_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args 
                       const int32_t* full_res) {
   extern __shared__ __align__(16) char smem[];
   __shared__ Shared sh;
-  __shared__ int s_flags[2];
+  __shared__ int s_flags[3];
   int32_t* s_via = reinterpret_cast<int32_t*>(smem);
   if (w.result[0] < 0) return;
   const int32_t n = pa.order[k];

@@ -160,3 +160,33 @@ def test_roi_extraction_matches_oracle(dims, max_nodes, depth, blocked):
                                   max_nodes=max_nodes)
         net = ops.net_args(0, src, dst, max_depth=depth, halo=2, max_roi_nodes=max_nodes)
         np.testing.assert_array_equal(ops.extract_roi(net), want)
+
+
+@pytest.mark.parametrize("columns", [3, 270, 300])
+def test_commit_of_many_vias_matches_oracle(columns):
+    """Ownership of the nodes that overlapping via hops of one column span: 15, 1350 (listed, sorted out by every
+    thread) and 1500 hops (more than the list of 1365 holds)."""
+    from oracle.tallies import NodeState
+    g, s, ops, ref = make(302, 302, 8)
+    ns = NodeState(g.N, ref.nx, ref.plane)
+    at = 300 // 2
+    row = ref.indices[ref.indptr[ref.plane + at * 303]:ref.indptr[ref.plane + at * 303 + 1]]
+    along_x = ref.plane + at * 303 + 1 in row
+    path = []
+    for c in range(1, columns + 1):
+        r = at * ref.nx + c if along_x else c * ref.nx + at
+        zs = [1, 4, 2, 6, 3, 5]
+        path += [z * ref.plane + r for z in (zs if c % 2 else zs[::-1])]
+    owner = lambda: np.where(s.owner_count.cpu().numpy() == 0, -1,
+                             np.where(s.owner_count.cpu().numpy() == 1, s.owner_xor.cpu().numpy(), -2))
+    ops.apply_path(path, 5, +1, 1.0, live=False)
+    ns.mark_owner(5, path)
+    ns.mark_use(path)
+    np.testing.assert_array_equal(owner(), ns.owner)
+    np.testing.assert_array_equal(s.path_node_use.cpu().numpy(), ns.path_node_use.astype(np.int32))
+    ops.commit_paths([np.asarray(path)], [6])
+    ns.mark_owner(6, path)
+    np.testing.assert_array_equal(owner(), ns.owner)
+    ops.apply_path(path, 5, -1, 1.0, live=False)
+    ns.clear_owner(5, path)
+    np.testing.assert_array_equal(owner(), ns.owner)
