@@ -32,7 +32,8 @@ namespace {
 using ogr_phase::kThreads;
 using ogr_phase::kWarps;
 constexpr int kSub = 16;                       // lanes per node (ROI BFS)
-constexpr int kBfsThreads = 768;               // of the kernels that only extract ROIs (others: their own)
+constexpr int kBfsThreads = 768;               // of the kernel that only extracts ROIs, one per CTA
+constexpr int kClusterThreads = 512;           // of a cluster's CTA that extracts one ROI
 
 // Accepted and kept for callers (ogr_search_lanes); the search fits its lanes
 // to the lattice's rows, and results never depended on it.
@@ -190,7 +191,7 @@ struct Shared {
   int nq[4];
   int seen_count;
   int met;
-  int left;        // the BFS left its box
+  int flags[3];    // of a BFS wave
   int overflow;
   int bx0, bx1, by0, by1;
   int pos_src, pos_dst;
@@ -253,36 +254,92 @@ struct Div {
   }
 };
 
-// Shared memory of a BFS: the four queues' first kBfsQ entries, then two
-// bitmaps of the box around both terminals.
-constexpr int kBfsQ = 4096;
-constexpr int kBfsArcs = 6;                    // arcs of a row that one of a node's two lanes loads at once
-constexpr size_t kBfsQBytes = 4 * kBfsQ * sizeof(int32_t);
-constexpr int kBfsWords = (int)((ogr_phase::kSmemBytes - kBfsQBytes) / 8);     // words per bitmap
+// Shared memory of a BFS: the mail of a cluster's CTAs, two queues (this wave's
+// and the next one's), then the marks of the box around both terminals, two
+// bits a cell (1: seen from src, 2: from dst; both: where the waves met).
+constexpr int kBfsCtas = 8;                    // CTAs of a cluster that extracts one ROI
+struct BfsMail {
+  int4 in[2][kBfsCtas];                        // from each CTA: nodes for this one, new nodes, flags
+  int out[kBfsCtas];                           // nodes found so far for each CTA
+};
+constexpr int kBfsQ = 8192;
+constexpr int kBfsSeg = kBfsQ / kBfsCtas;      // of a queue, one CTA's finds
+constexpr size_t kBfsHead = 512;
+constexpr size_t kBfsBitsAt = kBfsHead + 2 * kBfsQ * sizeof(int32_t);
+constexpr int kBfsWords = (int)((ogr_phase::kSmemBytes - kBfsBitsAt) / 4);
+static_assert(sizeof(BfsMail) <= kBfsHead && 2 * kBfsQ <= 16384, "mail and queues");
+constexpr int kMet = 1, kLeft = 2, kOverflow = 4;
 
-// Bidirectional BFS from src/dst on two bitmaps (bit set: seen by that wave;
-// both: where the waves met) of a box in shared memory; writes the ROI
+// Another CTA's copy of a variable in shared memory.
+__device__ __forceinline__ unsigned peer_addr(const void* p, unsigned rank) {
+  unsigned r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+  return r;
+}
+// *addr |= bit if on; the word before (all ones if not on).
+__device__ __forceinline__ unsigned peer_or(unsigned addr, unsigned bit, bool on) {
+  unsigned old;
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n mov.u32 %0, 0xffffffff;\n"
+      " @p atom.relaxed.cluster.shared::cluster.or.b32 %0, [%1], %2;\n}"
+      : "=r"(old) : "r"(addr), "r"(bit), "r"((unsigned)on) : "memory");
+  return old;
+}
+__device__ __forceinline__ unsigned peer_ld(unsigned addr) {
+  unsigned v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void peer_st(unsigned addr, int v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ void peer_st(unsigned addr, int4 v) {
+  asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+               : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
+}
+// The CTA that keeps a word of the marks, whose queue its cells go to.
+__device__ __forceinline__ unsigned bfs_owner(int wd) { return ((unsigned)wd * 0x9e3779b1u) >> 29; }
+static_assert(kBfsCtas == 8, "three bits of the hash");
+
+// Bidirectional BFS from src/dst on a box in shared memory; writes the ROI
 // (ascending id, truncated with the must-keep swap) into out[0..out_cap) and
 // its size into sh.R.  False: the search left the box (the caller takes
-// roi_build_large).
+// roi_build_large; of a cluster, its first CTA).
 //
-// A wave step is two dependent round trips (row bounds, row) for up to 256
-// nodes at once; marks, queues and the compaction never leave the SM.  With
+// Both terminals' waves go on together.  A cell that both find in one step
+// goes to one queue only: the ROI is what either has seen, the cell's
+// neighbours are found by whichever has it, and the step at which the waves
+// meet is the same (the second of two marks of a cell tells).
+//
+// A step is two dependent round trips (row bounds, row) and the marks, which
+// never leave the SM; the lanes of a node wait for their row together.  With
 // the marks as compare-and-swaps in global memory (a third round trip and an
 // atomic per arc) an ROI of 50,000 nodes on 600x400x12 took 1,352 us and its
-// compaction 250; now 547 and 55 with 768 threads (512: 600, 1,024: 540, but
-// 14,000-node ROIs then take 180 us instead of 165).
+// compaction 250; one terminal's wave after the other 550 and 55.
+//
+// kCluster: by the kBfsCtas CTAs of a cluster.  A word of the marks has an
+// owner, whose copy counts; the others' copies only spare them asking twice.
+// Whoever marks a cell first sends it to its owner's queue, and the counts of
+// what was sent cross with the flags at the end of the step.  The same ROI
+// then takes 237 us and 18 (8 CTAs of 512 threads, 4 lanes a node; 8 lanes:
+// 277; 1,024 threads: 217, but 14,000 nodes 106 instead of 90; one CTA 165).
+// Owners by column, which keeps most marks in their CTA, were no faster.
+template <bool kCluster, int kLanes, int kArcs>
 __device__ bool roi_build_box(Shared& sh, const ogr_graph& g, const ogr_net_args& a, int32_t* const* q, int64_t qcap,
-                              int32_t* out, int32_t out_cap, char* smem, StageClock& clk) {
+                              int32_t* out, int32_t out_cap, char* smem, StageClock& clk, int rank) {
+  constexpr int kNodes = 32 / kLanes;          // a warp's nodes at a time
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = blockDim.x, nw = nt >> 5;
   const int nx = g.nx, ny = g.ny, nz = g.nz;
   const int32_t src = a.src, dst = a.dst, plane = nx * ny;
   const int32_t* __restrict__ indptr = g.indptr;
   const int32_t* __restrict__ indices = g.indices;
   const Div by_plane((unsigned)(nx * ny)), by_nx((unsigned)nx);
-  int32_t* sq = reinterpret_cast<int32_t*>(smem);
-  unsigned* bits[2] = {reinterpret_cast<unsigned*>(smem + kBfsQBytes),
-                       reinterpret_cast<unsigned*>(smem + kBfsQBytes) + kBfsWords};
+  BfsMail& mail = *reinterpret_cast<BfsMail*>(smem);
+  int32_t* sq = reinterpret_cast<int32_t*>(smem + kBfsHead);
+  unsigned* marks = reinterpret_cast<unsigned*>(smem + kBfsBitsAt);
   auto coord = [&](int32_t v, int& x, int& y, int& z) {
     z = (int)by_plane((unsigned)v);
     const unsigned r = (unsigned)v - (unsigned)z * by_plane.d;
@@ -299,179 +356,284 @@ __device__ bool roi_build_box(Shared& sh, const ogr_graph& g, const ogr_net_args
     Y0 = max(0, min(sy, dy) - reach);
     BW = min(nx - 1, max(sx, dx) + reach) - X0 + 1;
     BH = min(ny - 1, max(sy, dy) + reach) - Y0 + 1;
-    RW = (BW + 31) >> 5;
+    RW = (BW + 15) >> 4;
     if ((int64_t)RW * BH * nz <= kBfsWords) break;
     if (reach <= 0) return false;
   }
   const int NW = RW * BH * nz;
-  for (int i = tid; i < NW; i += nt) bits[0][i] = bits[1][i] = 0u;
+  for (int i = tid; i < NW; i += nt) marks[i] = 0u;
+  if (tid < kBfsCtas) {
+    mail.out[tid] = 0;
+    mail.in[0][tid] = make_int4(kCluster && rank == 0 && tid == 0 ? 2 : 0, 0, 0, 0);
+  }
   if (tid == 0) {
-    sh.nq[0] = sh.nq[2] = 1;
     sq[0] = src;
-    sq[2 * kBfsQ] = dst;
+    sq[1] = (int32_t)((unsigned)dst | 0x80000000u);
+    sh.nq[0] = 2;                              // (wave w takes nq[w % 3] entries, sets flags[w % 3])
+    sh.nq[1] = sh.nq[2] = 0;
+    sh.flags[0] = sh.flags[1] = sh.flags[2] = 0;
     sh.overflow = 0;
-    sh.met = 0;
     sh.pos_src = -1;
     sh.pos_dst = -1;
     sh.bx0 = min(sx, dx); sh.bx1 = max(sx, dx);
     sh.by0 = min(sy, dy); sh.by1 = max(sy, dy);
-    sh.left = 0;
   }
   __syncthreads();
   if (tid == 0) {
-    if (src != dst) bits[0][(sz * BH + (sy - Y0)) * RW + ((sx - X0) >> 5)] |= 1u << ((sx - X0) & 31);
-    bits[1][(dz * BH + (dy - Y0)) * RW + ((dx - X0) >> 5)] |= 1u << ((dx - X0) & 31);
+    const int xs = sx - X0, xd = dx - X0;
+    if (src != dst) marks[(sz * BH + (sy - Y0)) * RW + (xs >> 4)] |= 1u << (2 * (xs & 15));
+    marks[(dz * BH + (dy - Y0)) * RW + (xd >> 4)] |= 2u << (2 * (xd & 15));
   }
-  int depth = 0, meet = -1;
+  int depth = 0, meet = -1, par = 0, slot = 0;
   int64_t seen = src != dst ? 2 : 1;
-  int cur_s = 0, cur_d = 2;
+  int64_t total = 2;
   int lx0 = 1 << 30, lx1 = -1, ly0 = 1 << 30, ly1 = -1;
-  __syncthreads();
-  while (depth < a.bfs_max_depth && (sh.nq[cur_s] > 0 || sh.nq[cur_d] > 0)) {
-    for (int wave = 0; wave < 2; ++wave) {
-      const int cur = wave == 0 ? cur_s : cur_d, nxt = cur ^ 1;
-      unsigned* mine = bits[wave];
-      const unsigned* other = bits[wave ^ 1];
-      const int n = (int)min((int64_t)sh.nq[cur], qcap);
-      if (tid == 0) sh.nq[nxt] = 0;
-      __syncthreads();
-      int met = 0;
-      for (int base = warp * 16; base < n; base += nw * 16) {
-        const int i = base + (lane >> 1);
-        int32_t u = 0, f = 0, f1 = 0;
-        if (i < n) {
-          u = i < kBfsQ ? sq[cur * kBfsQ + i] : q[cur][i];
-          f = indptr[u] + (lane & 1);
-          f1 = indptr[u + 1];
+  if constexpr (kCluster) cluster_sync(); else __syncthreads();
+  while (depth < a.bfs_max_depth && total > 0) {
+    const int nslot = slot == 2 ? 0 : slot + 1;
+    int n, before[kBfsCtas];                   // cluster: entries before each CTA's segment
+    if constexpr (kCluster) {
+      n = 0;
+#pragma unroll
+      for (int k = 0; k < kBfsCtas; ++k) {
+        before[k] = n;
+        n += mail.in[par][k].x;
+      }
+    } else {
+      n = (int)total;
+      if (tid == 0) {                          // (both last read two waves ago)
+        sh.nq[nslot == 2 ? 0 : nslot + 1] = 0;
+        sh.flags[nslot] = 0;
+      }
+    }
+    int flags = 0;
+    for (int base = warp * kNodes; base < n; base += nw * kNodes) {
+      const int i = base + lane / kLanes;
+      int32_t u = 0, f = 0, f1 = 0;
+      unsigned mark = 1;
+      if (i < n) {
+        int at = i;
+        if constexpr (kCluster) {
+          int k = 0, b = 0;
+#pragma unroll
+          for (int c = 1; c < kBfsCtas; ++c)
+            if (i >= before[c]) { k = c; b = before[c]; }
+          at = k * kBfsSeg + i - b;
         }
-        // (in the shadow of the row bounds' load)
-        int ux, uy, uz;
-        coord(u, ux, uy, uz);
-        const int32_t ur = u - uz * plane;
-        const int ubx = ux - X0, uby = uy - Y0;
-        while (__any_sync(0xffffffffu, f < f1)) {
-          int32_t v[kBfsArcs];
+        int32_t x;
+        if (kCluster || at < kBfsQ) x = sq[par * kBfsQ + at];
+        else x = at < qcap ? q[par][at] : q[par + 2][at - qcap];
+        mark = 1u + ((unsigned)x >> 31);
+        u = x & 0x7fffffff;
+        f = indptr[u] + lane % kLanes;
+        f1 = indptr[u + 1];
+      }
+      // (in the shadow of the row bounds' load)
+      int ux, uy, uz;
+      coord(u, ux, uy, uz);
+      const int32_t ur = u - uz * plane;
+      const int ubx = ux - X0, uby = uy - Y0;
+      while (__any_sync(0xffffffffu, f < f1)) {
+        int32_t v[kArcs];
+        int wd[kArcs];
+        unsigned old[kArcs];
+        int cx[kArcs], cy[kArcs];
 #pragma unroll
-          for (int j = 0; j < kBfsArcs; ++j) {
-            const int32_t e = f + 2 * j;
-            v[j] = e < f1 && !(g.blocked != nullptr && g.blocked[e]) ? indices[e] : -1;
+        for (int j = 0; j < kArcs; ++j) {
+          const int32_t e = f + kLanes * j;
+          v[j] = e < f1 && !(g.blocked != nullptr && g.blocked[e]) ? indices[e] : -1;
+        }
+#pragma unroll
+        for (int j = 0; j < kArcs; ++j) {
+          // the next cell, or another layer of the same one
+          const int32_t d = v[j] - u;
+          int bx = ubx, by = uby;
+          const int z = (int)by_plane((unsigned)max(v[j], 0));
+          const int32_t r = v[j] - z * plane;
+          if (r != ur) {
+            if (d == 1 || d == -1) bx += d;
+            else if (d == nx || d == -nx) by += d > 0 ? 1 : -1;
+            else bx = -1;          // (an arc of no lattice: the caller takes the large form)
+            if ((unsigned)(bx + X0) >= (unsigned)nx || (unsigned)(by + Y0) >= (unsigned)ny) bx = -1;
           }
+          if (v[j] >= 0 && ((unsigned)bx >= (unsigned)BW || (unsigned)by >= (unsigned)BH)) {
+            flags |= kLeft;
+            v[j] = -1;
+          }
+          cx[j] = bx;
+          cy[j] = by;
+          wd[j] = v[j] >= 0 ? (z * BH + by) * RW + (bx >> 4) : 0;
+          old[j] = v[j] >= 0 ? *(volatile unsigned*)&marks[wd[j]] : 0xffffffffu;
+        }
 #pragma unroll
-          for (int j = 0; j < kBfsArcs; ++j) {
-            bool fresh = false;
-            if (v[j] >= 0) {
-              // the next cell, or another layer of the same one
-              const int32_t d = v[j] - u;
-              int bx = ubx, by = uby, z = (int)by_plane((unsigned)v[j]);
-              const int32_t r = v[j] - z * plane;
-              if (r != ur) {
-                if (d == 1 || d == -1) bx += d;
-                else if (d == nx || d == -nx) by += d > 0 ? 1 : -1;
-                else bx = -1;      // (an arc of no lattice: the caller takes the large form)
-                if ((unsigned)(bx + X0) >= (unsigned)nx || (unsigned)(by + Y0) >= (unsigned)ny) bx = -1;
-              }
-              if ((unsigned)bx >= (unsigned)BW || (unsigned)by >= (unsigned)BH) {
-                sh.left = 1;
-              } else {
-                const int wd = (z * BH + by) * RW + (bx >> 5);
-                const unsigned bit = 1u << (bx & 31);
-                if (!(mine[wd] & bit) && !(atomicOr(&mine[wd], bit) & bit)) {
-                  if (other[wd] & bit) {
-                    met = 1;
-                  } else {
-                    fresh = true;
-                    lx0 = min(lx0, bx); lx1 = max(lx1, bx);
-                    ly0 = min(ly0, by); ly1 = max(ly1, by);
-                  }
-                }
-              }
+        for (int j = 0; j < kArcs; ++j) {
+          const unsigned bit = mark << (2 * (cx[j] & 15));
+          bool on = !(old[j] & bit);
+          if constexpr (kCluster) {
+            const unsigned o = bfs_owner(wd[j]);
+            if (on && o != (unsigned)rank) on = !(atomicOr(&marks[wd[j]], bit) & bit);
+            old[j] = peer_or(peer_addr(&marks[wd[j]], o), bit, on);
+          } else if (on) {
+            old[j] = atomicOr(&marks[wd[j]], bit);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < kArcs; ++j) {
+          const unsigned cell = old[j] >> (2 * (cx[j] & 15)) & 3u;
+          const bool fresh = cell == 0;
+          if (cell == 3u - mark) flags |= kMet;
+          const int32_t x = (int32_t)((unsigned)v[j] | (mark - 1u) << 31);
+          if constexpr (kCluster) {
+            if (fresh) {
+              const unsigned o = bfs_owner(wd[j]);
+              const int p = atomicAdd(&mail.out[o], 1);
+              if (p < kBfsSeg) peer_st(peer_addr(&sq[(par ^ 1) * kBfsQ + rank * kBfsSeg + p], o), x);
+              else flags |= kLeft;             // (more than a queue holds)
+            }
+          } else {
+            if (fresh) {
+              lx0 = min(lx0, cx[j]); lx1 = max(lx1, cx[j]);
+              ly0 = min(ly0, cy[j]); ly1 = max(ly1, cy[j]);
             }
             const unsigned m = __ballot_sync(0xffffffffu, fresh);
             if (m) {
               int p = 0;
-              if (lane == 0) p = atomicAdd(&sh.nq[nxt], __popc(m));
+              if (lane == 0) p = atomicAdd(&sh.nq[nslot], __popc(m));
               p = __shfl_sync(0xffffffffu, p, 0) + __popc(m & ((1u << lane) - 1u));
               if (fresh) {
-                if (p < kBfsQ) sq[nxt * kBfsQ + p] = v[j];
-                else if (p < qcap) q[nxt][p] = v[j];
-                else sh.overflow = 1;
+                if (p < kBfsQ) sq[(par ^ 1) * kBfsQ + p] = x;
+                else if (p < qcap) q[par ^ 1][p] = x;
+                else if (p < 2 * qcap) q[(par ^ 1) + 2][p - qcap] = x;
+                else flags |= kOverflow;
               }
             }
           }
-          f += 2 * kBfsArcs;
         }
+        f += kLanes * kArcs;
       }
-      if (met) sh.met = 1;
-      __syncthreads();
-      seen += sh.nq[nxt];
-      if (wave == 0) cur_s = nxt; else cur_d = nxt;
     }
+    flags = __reduce_or_sync(0xffffffffu, flags);
+    if (lane == 0 && flags) atomicOr(&sh.flags[slot], flags);
+    __syncthreads();
+    if constexpr (kCluster) {
+      if (tid < kBfsCtas) {
+        const int mine = mail.out[tid];
+        const int all = __reduce_add_sync((1u << kBfsCtas) - 1u, mine);
+        mail.out[tid] = 0;
+        peer_st(peer_addr(&mail.in[par ^ 1][rank], tid), make_int4(min(mine, kBfsSeg), all, sh.flags[slot], 0));
+        if (tid == 0) sh.flags[nslot] = 0;
+      }
+      cluster_sync();
+      total = 0;
+      flags = 0;
+      for (int k = 0; k < kBfsCtas; ++k) {
+        const int4 x = mail.in[par ^ 1][k];
+        total += x.y;
+        flags |= x.z;
+      }
+    } else {
+      total = sh.nq[nslot];
+      flags = sh.flags[slot];
+    }
+    par ^= 1;
+    slot = nslot;
+    seen += total;
     ++depth;
-    if (tid == 0) atomicAdd(&g_stage[11], 2ull);
-    if (sh.left) return false;     // uniform: read after the wave's barrier, written before it
-    if (sh.met && meet < 0) meet = depth;
+    if (tid == 0 && rank == 0) atomicAdd(&g_stage[11], 1ull);
+    if (flags & kLeft) return false;           // (the same in every thread, and in every CTA)
+    if ((flags & kMet) && meet < 0) meet = depth;
+    if (flags & kOverflow) { if (tid == 0) sh.overflow = 1; break; }
     if (meet >= 0 && depth >= meet + a.bfs_halo) break;
     if ((double)seen > a.bfs_stop_count) break;
-    if (sh.overflow) break;
-    __syncthreads();               // (the next wave resets what was read here)
   }
-  lx0 = __reduce_min_sync(0xffffffffu, lx0);
-  lx1 = __reduce_max_sync(0xffffffffu, lx1);
-  ly0 = __reduce_min_sync(0xffffffffu, ly0);
-  ly1 = __reduce_max_sync(0xffffffffu, ly1);
-  if (lane == 0) {
-    if (lx1 >= 0) {
+  if constexpr (!kCluster) {
+    lx0 = __reduce_min_sync(0xffffffffu, lx0);
+    lx1 = __reduce_max_sync(0xffffffffu, lx1);
+    ly0 = __reduce_min_sync(0xffffffffu, ly0);
+    ly1 = __reduce_max_sync(0xffffffffu, ly1);
+    if (lane == 0 && lx1 >= 0) {
       atomicMin(&sh.bx0, X0 + lx0); atomicMax(&sh.bx1, X0 + lx1);
       atomicMin(&sh.by0, Y0 + ly0); atomicMax(&sh.by1, Y0 + ly1);
     }
   }
   __syncthreads();
-  clk.mark(0);
-  // Ordered compaction (ascending global id): each warp owns a contiguous run
-  // of words; count, scan the counts, then write.  Only positions below
-  // out_cap are stored; those of src and dst are recorded.
-  const int per = ((NW + nw - 1) / nw + 31) & ~31;
-  const int w0 = warp * per, w1 = min(NW, w0 + per);
+  if (rank == 0) clk.mark(0);
+  // Ordered compaction (ascending global id): each CTA, in it each warp, owns
+  // a contiguous run of words; count, scan the counts, then write.  Only
+  // positions below out_cap are stored; those of src and dst are recorded.
+  const Div by_rw((unsigned)RW), by_bh((unsigned)BH);
+  auto cells = [&](int i) -> unsigned {        // the low bit of each seen cell
+    unsigned w;
+    if constexpr (kCluster) w = peer_ld(peer_addr(&marks[i], bfs_owner(i)));
+    else w = marks[i];
+    return (w | w >> 1) & 0x55555555u;
+  };
+  const int share = kCluster ? ((NW + kBfsCtas - 1) / kBfsCtas + 31) & ~31 : NW;
+  const int c0 = kCluster ? min(NW, rank * share) : 0, c1 = min(NW, c0 + share);
+  const int per = ((c1 - c0 + nw - 1) / nw + 31) & ~31;
+  const int w0 = c0 + warp * per, w1 = min(c1, w0 + per);
   int cnt = 0;
-  for (int i = w0 + lane; i < w1; i += 32) cnt += __popc(bits[0][i] | bits[1][i]);
+#pragma unroll 4
+  for (int i = w0 + lane; i < w1; i += 32) cnt += __popc(cells(i));
   cnt = __reduce_add_sync(0xffffffffu, cnt);
   if (lane == 0) sh.s_cnt[warp] = cnt;
   __syncthreads();
-  if (tid == 0) {
-    int t = 0;
-    for (int i = 0; i < nw; ++i) {
-      sh.s_off[i] = t;
-      t += sh.s_cnt[i];
+  if (tid < 32) {
+    const int c = tid < nw ? sh.s_cnt[tid] : 0;
+    int x = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
     }
-    sh.R = t;
+    sh.s_off[tid] = x - c;
+    x = __shfl_sync(0xffffffffu, x, 31);
+    if (tid == 0) sh.R = x;
+    if constexpr (kCluster)
+      if (tid < kBfsCtas) peer_st(peer_addr(&mail.in[par ^ 1][rank], tid), make_int4(x, 0, 0, 0));
   }
   __syncthreads();
   int off = sh.s_off[warp];
-  const Div by_rw((unsigned)RW), by_bh((unsigned)BH);
+  if constexpr (kCluster) {
+    cluster_sync();
+    int all = 0;
+    for (int k = 0; k < kBfsCtas; ++k) {
+      if (k == rank) off += all;
+      all += mail.in[par ^ 1][k].x;
+    }
+    if (tid == 0) sh.R = all;
+  }
   for (int i0 = w0; i0 < w1; i0 += 32) {
-    const unsigned word = i0 + lane < w1 ? bits[0][i0 + lane] | bits[1][i0 + lane] : 0u;
+    const unsigned word = i0 + lane < w1 ? cells(i0 + lane) : 0u;
     unsigned some = __ballot_sync(0xffffffffu, word != 0u);
+    some = (some | some >> 1) & 0x55555555u;   // two words, 32 cells, at a time
     while (some) {
-      const int k = __ffs(some) - 1;
+      const int k = __ffs(some) - 1 + (lane >> 4);
       some &= some - 1;
-      const unsigned b = __shfl_sync(0xffffffffu, word, k);
-      const unsigned row = by_rw((unsigned)(i0 + k)), z = by_bh(row);
-      const int32_t first = (int32_t)(z * by_plane.d + (unsigned)(Y0 + (int)(row - z * by_bh.d)) * by_nx.d) + X0 +
-                            32 * (int)(i0 + k - row * by_rw.d);
-      if ((b >> lane) & 1u) {
+      const bool in = __shfl_sync(0xffffffffu, word, k) >> (2 * (lane & 15)) & 1u;
+      const unsigned b = __ballot_sync(0xffffffffu, in);
+      if (in) {
+        const unsigned row = by_rw((unsigned)(i0 + k)), z = by_bh(row);
         const int pos = off + __popc(b & ((1u << lane) - 1u));
-        const int32_t gid = first + lane;
+        const int32_t gid = (int32_t)(z * by_plane.d + (unsigned)(Y0 + (int)(row - z * by_bh.d)) * by_nx.d) + X0 +
+                            16 * (int)(i0 + k - row * by_rw.d) + (lane & 15);
         if (pos < out_cap) out[pos] = gid;
-        if (gid == src) sh.pos_src = pos;
-        if (gid == dst) sh.pos_dst = pos;
+        if constexpr (kCluster) {
+          if (gid == src) peer_st(peer_addr(&sh.pos_src, 0), pos);
+          if (gid == dst) peer_st(peer_addr(&sh.pos_dst, 0), pos);
+        } else {
+          if (gid == src) sh.pos_src = pos;
+          if (gid == dst) sh.pos_dst = pos;
+        }
       }
       off += __popc(b);
     }
   }
+  if constexpr (kCluster) cluster_sync();
   __syncthreads();
-  roi_finish(sh, a, out, out_cap);
+  if (rank == 0) roi_finish(sh, a, out, out_cap);
   __syncthreads();
-  clk.mark(1);
+  if (rank == 0) clk.mark(1);
   return true;
 }
 
@@ -634,9 +796,22 @@ __device__ __noinline__ void roi_build_large(Shared& sh, const ogr_graph& g, con
 
 __device__ void roi_build(Shared& sh, const ogr_graph& g, const ogr_net_args& a, int32_t* seen, int32_t* const* q,
                           int64_t qcap, int32_t* out, int32_t out_cap, char* smem, StageClock& clk) {
-  if (roi_build_box(sh, g, a, q, qcap, out, out_cap, smem, clk)) return;
+  if (roi_build_box<false, 2, 6>(sh, g, a, q, qcap, out, out_cap, smem, clk, 0)) return;
   __syncthreads();
   roi_build_large(sh, g, a, seen, q, qcap, out, out_cap, clk);
+}
+
+// The same by a cluster of kBfsCtas CTAs (rank: this one's); the result is in
+// the first one's sh.
+__device__ void roi_build_cluster(Shared& sh, const ogr_graph& g, const ogr_net_args& a, const Ws& w, int32_t* out,
+                                  int32_t out_cap, char* smem, int rank) {
+  StageClock clk;
+  clk.start();
+  if (threadIdx.x == 0) sh.status = OGR_OK;
+  __syncthreads();
+  if (roi_build_box<true, 4, 4>(sh, g, a, w.q, w.qcap, out, out_cap, smem, clk, rank) || rank != 0) return;
+  __syncthreads();
+  roi_build_large(sh, g, a, w.seen, w.q, w.qcap, out, out_cap, clk);
 }
 
 // ---- the search on a given ROI ---------------------------------------------------
@@ -1109,13 +1284,14 @@ __device__ int apply_path_dev(const ogr_graph& g, const ogr_state& st, const int
 }
 
 // ---- kernels -------------------------------------------------------------------
-// The ROI of a net into w.roi: result[0] = status, result[3] = its size.
-__global__ void __launch_bounds__(kBfsThreads, 1)
+// The ROI of a net (not a full-graph one) into w.roi, by one cluster:
+// result[0] = status, result[3] = its size.
+__global__ void __cluster_dims__(kBfsCtas) __launch_bounds__(kClusterThreads, 1)
 build_roi_kernel(ogr_graph g, ogr_net_args a, Ws w) {
   extern __shared__ __align__(16) char smem[];
   __shared__ Shared sh;
-  build_roi(sh, g, a, w, smem);
-  if (threadIdx.x == 0) {
+  roi_build_cluster(sh, g, a, w, w.roi, a.max_roi_nodes, smem, blockIdx.x);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     w.result[0] = sh.status;
     w.result[1] = 0;
     w.result[3] = sh.R;
@@ -1144,28 +1320,25 @@ find_team_kernel(ogr_graph g, ogr_state st, ogr_net_args a, Ws w, const int32_t*
   }
 }
 
-__global__ void __launch_bounds__(kBfsThreads, 1)
+__global__ void __cluster_dims__(kBfsCtas) __launch_bounds__(kClusterThreads, 1)
 roi_kernel(ogr_graph g, ogr_net_args a, Ws w, int32_t* roi_out, int32_t roi_cap) {
   extern __shared__ __align__(16) char smem[];
   __shared__ Shared sh;
-  StageClock clk;
-  clk.start();
-  if (threadIdx.x == 0) sh.status = OGR_OK;
-  __syncthreads();
-  int R = 0;
+  const bool leader = blockIdx.x == 0 && threadIdx.x == 0;
   if (a.full_graph) {
-    R = g.num_nodes;
-    if (threadIdx.x == 0 && R > roi_cap) sh.status = OGR_ERR_CAPACITY;
-    __syncthreads();
-    if (sh.status == OGR_OK)
-      for (int r = threadIdx.x; r < R; r += blockDim.x) roi_out[r] = r;
-  } else {
-    roi_build(sh, g, a, w.seen, w.q, w.qcap, roi_out, roi_cap, smem, clk);
-    R = sh.R;
+    const int32_t R = g.num_nodes;
+    if (R <= roi_cap)
+      for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < R; r += gridDim.x * blockDim.x) roi_out[r] = r;
+    if (leader) {
+      w.result[0] = R > roi_cap ? OGR_ERR_CAPACITY : OGR_OK;
+      w.result[1] = R;
+    }
+    return;
   }
-  if (threadIdx.x == 0) {
+  roi_build_cluster(sh, g, a, w, roi_out, roi_cap, smem, blockIdx.x);
+  if (leader) {
     w.result[0] = sh.status;
-    w.result[1] = R;
+    w.result[1] = sh.R;
   }
 }
 
@@ -1791,7 +1964,7 @@ int launch_find(const ogr_graph& g, const ogr_state& st, const ogr_net_args& a, 
   OGR_CUDA_TRY(cudaMemsetAsync(&w.ctl->team, 0, sizeof(ogr_phase::Ctl), s));
   if (roi == nullptr && !a.full_graph) {
     OGR_CUDA_TRY(wide_smem((const void*)build_roi_kernel));
-    build_roi_kernel<<<1, kBfsThreads, ogr_phase::kSmemBytes, s>>>(g, a, w);
+    build_roi_kernel<<<kBfsCtas, kClusterThreads, ogr_phase::kSmemBytes, s>>>(g, a, w);
     OGR_LAUNCH_CHECK();
   }
   if (a.full_graph) R = g.num_nodes;
@@ -1977,7 +2150,7 @@ extern "C" int ogr_extract_roi(const ogr_graph* g, const ogr_net_args* net, void
   ws_layout(g->num_nodes, (char*)ws, &w);
   cudaStream_t s = ogr_stream(stream);
   OGR_CUDA_TRY(wide_smem((const void*)roi_kernel));
-  roi_kernel<<<1, kBfsThreads, ogr_phase::kSmemBytes, s>>>(*g, *net, w, roi_out, roi_cap);
+  roi_kernel<<<kBfsCtas, kClusterThreads, ogr_phase::kSmemBytes, s>>>(*g, *net, w, roi_out, roi_cap);
   OGR_LAUNCH_CHECK();
   int64_t res[2];
   OGR_CUDA_TRY(cudaMemcpyAsync(res, w.result, sizeof(res), cudaMemcpyDeviceToHost, s));
