@@ -254,21 +254,21 @@ __device__ __forceinline__ void arrive(const Problem& pr, Head& sm, int k, unsig
   asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(&s->a), "l"(add) : "memory");
 }
 
-// Thread 0: wait for barrier k; sm.a / sm.t get its word.  The wait is
-// bounded: sm.ok = 0 once any CTA of the team gave up.
-__device__ __forceinline__ void await(const Problem& pr, Head& sm, int k) {
-  if (pr.nranks == 1) return;
+// Thread 0: wait for barrier k and take its word.  The wait is bounded:
+// sm.ok = 0 once any CTA of the team gave up.
+__device__ __forceinline__ void await(const Problem& pr, Head& sm, int k, unsigned long long& a,
+                                      unsigned long long& t) {
+  if (pr.nranks == 1) {
+    a = sm.a;
+    t = sm.t;
+    return;
+  }
   const Slot* s = &pr.ctl->slot[k & 3];
   const unsigned want = (unsigned)pr.nranks;
   unsigned it = 0;
   while (true) {
-    unsigned long long a, t;
     ld_slot(s, a, t);
-    if ((unsigned)(a & kArriveMask) >= want) {
-      sm.a = a;
-      sm.t = t;
-      return;
-    }
+    if ((unsigned)(a & kArriveMask) >= want) return;
     ++it;
     if (it > pr.spin || ((it & 63) == 0 && *(const volatile int32_t*)&pr.ctl->err)) {
       atomicExch(&pr.ctl->err, 1);
@@ -277,6 +277,14 @@ __device__ __forceinline__ void await(const Problem& pr, Head& sm, int k) {
     }
     if (it > 256) __nanosleep(32);
   }
+}
+
+// The same, the word left in sm.a / sm.t.
+__device__ __forceinline__ void await(const Problem& pr, Head& sm, int k) {
+  unsigned long long a = 0, t = 0;
+  await(pr, sm, k, a, t);
+  sm.a = a;
+  sm.t = t;
 }
 
 // The phases of one search.  Before the call: rec of every node holds
@@ -309,9 +317,12 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
   bool dst_done = false;
   u64 ld = 0;
   int head = 0;
-  auto plan = [&](int phase, int b3, int nf, int nk) {
-    // the barrier's word is in sm.a / sm.t
-    const u64 word = sm.a, T = ~sm.t;
+  const unsigned team = (unsigned)pr.nranks, per_team = team > 1 ? (unsigned)((1ull << 32) / team) : 0;
+  const float share = 1.0f / (float)team;
+  auto plan = [&](int phase, int b3, int nf, int nk, u64 word, u64 tbits) {
+    // (word, tbits: the barrier's.  The whole team waits for this; with the
+    // word taken through shared memory and three divisions it was 540 clocks.)
+    const u64 T = ~tbits;
     const unsigned total = (unsigned)(word >> 32);
     int verdict = kGo;
     if (!kMulti && !dst_done && (word & kDst)) {
@@ -333,7 +344,11 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
     unsigned nov = (unsigned)(word >> 11) & kOutMask;
     if (nov) {
       if (nov >= kMostOut) nov = (unsigned)__ldcg(&pr.ctl->nov[b3]);
-      if (nov > (unsigned)pr.rank) n += (int)((nov - pr.rank + pr.nranks - 1) / (unsigned)pr.nranks);
+      if (nov > (unsigned)pr.rank) {
+        // ceil((nov - rank) / team); the high product is the floor or one less
+        const unsigned x = nov - (unsigned)pr.rank + team - 1, d = team > 1 ? __umulhi(x, per_team) : x;
+        n += (int)(x - d * team >= team ? d + 1 : d);
+      }
     }
     // A CTA with more entries than its share sends all of a phase's new ones
     // away.  A phase that takes surplus in is longer for everyone, so only
@@ -342,7 +357,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
     // us a phase at 600x400x12 / 307x199x8 / 1000x800x32: 8.7 / 4.4 / 16.8;
     // dealing every phase 9.5 / 4.8 / 17.4, every fourth 8.9 / 4.6 / 16.5,
     // every eighth 9.4 / 5.5 / 20.
-    const float avg = __fdividef((float)total, (float)pr.nranks);
+    const float avg = (float)total * share;
     const bool deal = (phase & 1) != 0;
     const bool over = pr.nranks > 1 && n > max(deal ? kGroups / 4 : kGroups, (int)fminf((deal ? 1.25f : 2.0f) * avg, 1e6f));
     head += nf;
@@ -360,7 +375,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
     sm.nov_out = 0;
     sm.dst_hit = 0;
     sm.inexact = 0;
-    plan(0, 0, 0, 0);
+    plan(0, 0, 0, 0, sm.a, sm.t);
   }
   __syncthreads();
   const long long c_start = clock64();
@@ -709,10 +724,11 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
     if (tid == 0) {
       const long long c0 = clock64();
       sm.ok = 1;
-      await(pr, sm, k0 + phase + 1);
+      u64 a = 0, t = 0;
+      await(pr, sm, k0 + phase + 1, a, t);
       out.wait += clock64() - c0;
       if (sm.ok)
-        plan(phase + 1, bn, nf, nk);
+        plan(phase + 1, bn, nf, nk, a, t);
       else
         sm.plan.verdict = kTimedOut;
       sm.push[q ^ 1] = 0;
