@@ -737,12 +737,14 @@ class PathFinderRouter:
         P = len(arrays)
         key = _sorted_unique(np.concatenate(arrays) * P +
                              np.repeat(np.arange(P, dtype=np.int64), [a.size for a in arrays]))
-        cnt = np.bincount(key // P, minlength=self.N)
-        hit = np.flatnonzero(cnt)
+        # the runs of the sorted nodes, not a count over the lattice's nodes (2.7M: 4 ms a call)
+        node = key // P
+        first = np.flatnonzero(np.concatenate(([True], node[1:] != node[:-1])))
+        hit, cnt = node[first], np.diff(np.append(first, node.size))
         if sign > 0:
-            self.node_use[hit] += cnt[hit].astype(self.node_use.dtype)
+            self.node_use[hit] += cnt.astype(self.node_use.dtype)
         else:
-            self.node_use[hit] = np.maximum(self.node_use[hit].astype(np.int64) - cnt[hit], 0).astype(self.node_use.dtype)
+            self.node_use[hit] = np.maximum(self.node_use[hit].astype(np.int64) - cnt, 0).astype(self.node_use.dtype)
 
     def _mark_nodes(self, name, path, sign, array=None):
         """path_node_use of one net's path (``_mark_path_node_use`` :4635);
@@ -1531,9 +1533,9 @@ class PathFinderRouter:
         arrs = [self._net_paths.array(n) for n in names]
         ids = [self._net_id(n) for n in names]
         slots = [self._task_index[n] for n in names] if self.store is not None else None
-        for n, a, edges in zip(names, arrs, self.ops.commit_paths(arrs, ids, self.store, slots)):
-            self._mark_nodes(n, None, +1, a)
+        for n, edges in zip(names, self.ops.commit_paths(arrs, ids, self.store, slots)):
             self._update_tracking(n, edges)
+        self._mark_many(arrs, +1)
         self._add_trivial_use()
         self._rebuild_via_usage()
 
