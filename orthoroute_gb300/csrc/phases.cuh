@@ -195,7 +195,7 @@ struct Head {
   unsigned long long ld;           // label of dst, once settled
   unsigned long long wmin[kWarps];
   unsigned push[2];                // entries carried (bits 20-31) and places asked for (0-19) in a phase
-  int tail;                        // free ring: end
+  unsigned tail;                   // free ring: end
   int inexact, nov_out, dst_hit, ok;
   int res[3];
 };
@@ -593,31 +593,29 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
           if (loc && unclaimed) bd.ent[slot].z = en.z & 0x7fffffff;
         }
       }
-      // entries that leave free their place
-      const unsigned gone = __ballot_sync(kAll, loc && !carry && sl == 0);
-      if (gone) {
-        int t = 0;
-        if (lane == 0) t = atomicAdd(&sm.tail, __popc(gone));
-        t = __shfl_sync(kAll, t, 0);
-        if ((gone >> lane) & 1) bd.freel[(unsigned)(t + __popc(gone & below)) % (unsigned)kS] = (uint16_t)slot;
-      }
       // Offer the labels of the open neighbours, mark and push the unreached
       // ones.  Carried entries keep their place; new ones (and carried surplus
-      // entries) take a free one, or go to the surplus list.
+      // entries) take a free one, or go to the surplus list; entries that
+      // leave free theirs.  One turn for all arcs of a lane: its places are
+      // counted out once, by two lanes side by side.
       const bool expand = settle && !vt;
-      bool self = carry && sl == 0;
+      bool self = carry && sl == 0, leaves = loc && !carry && sl == 0;
       int f = sl;
-#pragma unroll
-      for (int j = 0; j < K; ++j) {
-        do {                       // the general form goes round once per arc
-          if (kGen) {
-            r[0].sp = -1;
-            if (expand && f < deg) {
-              fetch(0, f);
-              load(0);
-            }
+      do {                         // the general form goes round once per arc
+        if (kGen) {
+          r[0].sp = -1;
+          if (expand && f < deg) {
+            fetch(0, f);
+            load(0);
           }
-          bool push = false;
+        }
+        bool push[K];
+        unsigned mt[K];
+        int nt = 0;
+        const bool keep = self && loc;
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+          push[j] = false;
           // open: not settled before this phase (whether it settles in this
           // one must not matter: T is the same whatever the timing)
           if (expand && r[j].sp >= 0 && (unsigned)(r[j].sp - 2) >= (unsigned)phase) {
@@ -630,21 +628,30 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
               if (__double2float_rn(y) < kInf) ly = ogr_dbits(y);
             }
             tmin = ly < tmin ? ly : tmin;
-            push = ly != kNone && r[j].sp == 0;
+            push[j] = ly != kNone && r[j].sp == 0;
           }
-          const bool keep = self && loc, take = push || (self && !loc);
-          self = false;
-          const unsigned mt = __ballot_sync(kAll, take), mk = __ballot_sync(kAll, keep);
-          if (mt | mk) {
-            unsigned p = 0;
-            if (lane == 0) p = atomicAdd(&sm.push[q], (unsigned)__popc(mt) + ((unsigned)__popc(mk) << 20));
-            p = __shfl_sync(kAll, p, 0);
-            if (keep) bd.carr[q ^ 1][(p >> 20) + __popc(mk & below)] = (uint16_t)slot;
-            const int at = (int)(p & 0xfffffu) + __popc(mt & below);
+          mt[j] = __ballot_sync(kAll, push[j] || (j == 0 && self && !loc));
+          nt += __popc(mt[j]);
+        }
+        const unsigned mk = __ballot_sync(kAll, keep), mg = __ballot_sync(kAll, leaves);
+        if (nt | mk | mg) {
+          unsigned p = 0;
+          if (lane < 2)
+            p = atomicAdd(lane == 0 ? &sm.push[q] : &sm.tail,
+                          lane == 0 ? (unsigned)nt + ((unsigned)__popc(mk) << 20) : (unsigned)__popc(mg));
+          const unsigned t = __shfl_sync(kAll, p, 1);
+          p = __shfl_sync(kAll, p, 0);
+          if (leaves) bd.freel[(t + __popc(mg & below)) % (unsigned)kS] = (uint16_t)slot;
+          if (keep) bd.carr[q ^ 1][(p >> 20) + __popc(mk & below)] = (uint16_t)slot;
+          int at0 = (int)(p & 0xfffffu);
+#pragma unroll
+          for (int j = 0; j < K; ++j) {
+            const int at = at0 + __popc(mt[j] & below);
+            at0 += __popc(mt[j]);
             bool surplus = false;
             int4 ne = en;
-            if (take) {
-              if (push) {
+            if ((mt[j] >> lane) & 1) {
+              if (push[j]) {
                 if (!kGen && !tick_finite(r[j].pen)) sm.inexact = 1;
                 const int32_t flags = kMulti ? uf[j] : 0;
                 __stcg(&rec[u[j]].sp, 1 | flags);
@@ -655,27 +662,30 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
                 const int s = bd.freel[(unsigned)(hd + at) % (unsigned)kS];
                 bd.fresh[q ^ 1][at] = (uint16_t)s;
                 int4 e = ne;
-                if (push) e.z |= 0x80000000;
+                if (push[j]) e.z |= 0x80000000;
                 bd.ent[s] = e;
               } else {
                 // on the surplus list every node stands once: claimed here
-                surplus = !push || atomicExch(&pr.claim[u[j]], pr.sid) != pr.sid;
+                surplus = !push[j] || atomicExch(&pr.claim[u[j]], pr.sid) != pr.sid;
               }
             }
-            const unsigned ms = __ballot_sync(kAll, surplus);
-            if (ms) {
-              int b = 0;
-              if (lane == 0) {
-                b = atomicAdd(&pr.ctl->nov[bn], __popc(ms));
-                atomicAdd(&sm.nov_out, __popc(ms));
+            if (av - at0 < 0) {    // (some of this turn's places are beyond those free)
+              const unsigned ms = __ballot_sync(kAll, surplus);
+              if (ms) {
+                int b = 0;
+                if (lane == 0) {
+                  b = atomicAdd(&pr.ctl->nov[bn], __popc(ms));
+                  atomicAdd(&sm.nov_out, __popc(ms));
+                }
+                b = __shfl_sync(kAll, b, 0);
+                if (surplus) __stcg((q ? pr.ov[0] : pr.ov[1]) + b + __popc(ms & below), ne);
               }
-              b = __shfl_sync(kAll, b, 0);
-              if (surplus) __stcg((q ? pr.ov[0] : pr.ov[1]) + b + __popc(ms & below), ne);
             }
           }
-          f += L;
-        } while (kGen && __any_sync(kAll, expand && f < deg));
-      }
+        }
+        self = leaves = false;
+        f += L;
+      } while (kGen && __any_sync(kAll, expand && f < deg));
     }
     tmin = warp_min_u64(tmin);
     if (lane == 0) sm.wmin[warp] = tmin;
