@@ -44,8 +44,8 @@
 //   are exact wherever the doubles are: costs and penalties of 2^-7 or more
 //   (or 0) are multiples of 2^-30, and below 2^22 their double sums do not
 //   round.  A search that meets any other value is redone in doubles.
-// * A CTA with more entries than its share sends a phase's new entries to a
-//   list in global memory that the next phase deals over the team (see plan()).
+// * A CTA with more entries than its share sends new ones to a list in global
+//   memory that the next phase deals over the team (see plan()).
 #pragma once
 #include "common.cuh"
 
@@ -319,7 +319,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
   int head = 0;
   const unsigned team = (unsigned)pr.nranks, per_team = team > 1 ? (unsigned)((1ull << 32) / team) : 0;
   const float share = 1.0f / (float)team;
-  auto plan = [&](int phase, int b3, int nf, int nk, u64 word, u64 tbits) {
+  auto plan = [&](int phase, int b3, int nf, int nk, float carried, u64 word, u64 tbits) {
     // (word, tbits: the barrier's.  The whole team waits for this; with the
     // word taken through shared memory and three divisions it was 540 clocks.)
     const u64 T = ~tbits;
@@ -350,16 +350,26 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
         n += (int)(x - d * team >= team ? d + 1 : d);
       }
     }
-    // A CTA with more entries than its share sends all of a phase's new ones
-    // away.  A phase that takes surplus in is longer for everyone, so only
-    // every other one deals the small excesses (a quarter above the average);
-    // in between it takes twice the average (and more than one round).
-    // us a phase at 600x400x12 / 307x199x8 / 1000x800x32: 8.7 / 4.4 / 16.8;
-    // dealing every phase 9.5 / 4.8 / 17.4, every fourth 8.9 / 4.6 / 16.5,
-    // every eighth 9.4 / 5.5 / 20.
-    const float avg = (float)total * share;
+    // The places given to new entries: the most entries that the CTA should
+    // have in the next phase, less those it will carry (the same share of its n
+    // as of the last phase's).  Entries beyond them are dealt over the team.
+    // A round of kGroups entries costs the same whether full or not (600x400x12:
+    // 5,500 clocks one, 10,000 two, 14,800 three), and the last CTA's rounds are
+    // the phase: the average is rounded up to whole rounds.  A phase that takes
+    // surplus in is longer for everyone, so only every other one evens out
+    // finer than that; of a thin frontier all new entries go, to spread it.
+    // us a phase at 600x400x12 / 307x199x8 / 1000x800x32, ROIs of 14,000 nodes:
+    // 7.6 / 3.9 / 16.3, 3.57.  Evened out every phase 7.8 / 4.3 / 16.9, 3.9; all
+    // of a phase's new entries sent away by CTAs a quarter above the average
+    // 8.3 / 4.0 / 18.3, 3.6; limits a fifth higher 7.8 / 4.0 / 17.3, 3.6.
     const bool deal = (phase & 1) != 0;
-    const bool over = pr.nranks > 1 && n > max(deal ? kGroups / 4 : kGroups, (int)fminf((deal ? 1.25f : 2.0f) * avg, 1e6f));
+    const float avg = (float)total * share;
+    float room = 1e6f;
+    if (team > 1) {
+      const float unit = (float)(deal ? kGroups / 8 : kGroups);
+      room = unit * ceilf(avg / unit) - (float)n * carried;
+      if (deal && avg < (float)(kGroups / 8)) room = n > kGroups / 4 ? 0.0f : 1e6f;
+    }
     head += nf;
     sm.plan.T = T;
     sm.plan.verdict = verdict;
@@ -367,7 +377,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
     sm.plan.ncarr = nk;
     sm.plan.n = n;
     sm.plan.head = head;
-    sm.plan.avail = over ? 0 : sm.tail - head;
+    sm.plan.avail = min(sm.tail - head, (unsigned)fmaxf(room, 0.0f));
   };
   if (tid == 0) {
     sm.push[0] = sm.push[1] = 0;
@@ -375,7 +385,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
     sm.nov_out = 0;
     sm.dst_hit = 0;
     sm.inexact = 0;
-    plan(0, 0, 0, 0, sm.a, sm.t);
+    plan(0, 0, 0, 0, 0.0f, sm.a, sm.t);
   }
   __syncthreads();
   const long long c_start = clock64();
@@ -735,10 +745,11 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
       const long long c0 = clock64();
       sm.ok = 1;
       u64 a = 0, t = 0;
+      const float carried = n > 0 ? __fdividef((float)nk, (float)n) : 0.5f;
       await(pr, sm, k0 + phase + 1, a, t);
       out.wait += clock64() - c0;
       if (sm.ok)
-        plan(phase + 1, bn, nf, nk, a, t);
+        plan(phase + 1, bn, nf, nk, carried, a, t);
       else
         sm.plan.verdict = kTimedOut;
       sm.push[q ^ 1] = 0;
