@@ -1482,7 +1482,6 @@ struct WinSlots {
   int32_t* solo;                   // 1: ROI extracted inline (the batched one overflowed)
   int32_t* st;                     // status of the b-th search
   int32_t* len;                    // path length of the b-th search
-  int32_t* box;                    // [4] footprint box
   unsigned long long* stats;       // [4] the b-th search's statistics, added on acceptance
   int32_t* inorder;                // 1: no pending net precedes the b-th net
 };
@@ -1490,9 +1489,9 @@ struct WinSlots {
 __host__ __device__ inline size_t win_ctl_layout(int32_t slots, char* base, WinCtl** c, WinSlots* s) {
   size_t off = round256(sizeof(WinCtl));
   const size_t k = (size_t)slots;
-  char* p[7];
-  const size_t sz[7] = {4 * k, 4 * k, 4 * k, 4 * k, 16 * k, 32 * k, 4 * k};
-  for (int i = 0; i < 7; ++i) {
+  char* p[6];
+  const size_t sz[6] = {4 * k, 4 * k, 4 * k, 4 * k, 32 * k, 4 * k};
+  for (int i = 0; i < 6; ++i) {
     p[i] = base ? base + off : nullptr;
     off += round256(sz[i]);
   }
@@ -1502,9 +1501,8 @@ __host__ __device__ inline size_t win_ctl_layout(int32_t slots, char* base, WinC
     s->solo = (int32_t*)p[1];
     s->st = (int32_t*)p[2];
     s->len = (int32_t*)p[3];
-    s->box = (int32_t*)p[4];
-    s->stats = (unsigned long long*)p[5];
-    s->inorder = (int32_t*)p[6];
+    s->stats = (unsigned long long*)p[4];
+    s->inorder = (int32_t*)p[5];
   }
   return off;
 }
@@ -1537,8 +1535,9 @@ __device__ bool win_barrier(WinCtl* c, unsigned long long& target, int* s_flag) 
   return *s_flag != 0;
 }
 
-__device__ __forceinline__ bool boxes_meet(const int* a, const int* b) {
-  return !(a[1] < b[0] || b[1] < a[0] || a[3] < b[2] || b[3] < a[2]);
+// Of boxes {x0, x1, y0, y1}.
+__device__ __forceinline__ bool boxes_meet(int4 a, int4 b) {
+  return !(a.y < b.x || b.y < a.x || a.w < b.z || b.w < a.z);
 }
 
 // Copies a path found into scratch to the net's store slot and commits it.
@@ -1575,8 +1574,8 @@ window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa,
   __shared__ Shared sh;
   __shared__ int s_flags[3];
   __shared__ int s_bar;
-  __shared__ int s_box[4];
-  __shared__ int s_skip[4 * kMaxSkip];
+  __shared__ int4 s_box[kWarps], s_grown[kWarps], s_skip[kMaxSkip];
+  __shared__ int2 s_cand[kWarps];
   __shared__ int s_win[4];
   int32_t* s_via = reinterpret_cast<int32_t*>(smem);     // (no search is on while paths are applied)
   const int b = blockIdx.x, tid = threadIdx.x, G = gridDim.x;
@@ -1611,72 +1610,103 @@ window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa,
     StageClock clk;
     clk.start();
     if (b == 0) {
-      if (tid == 0) {
+      // A warp looks up each candidate's footprint, kWarps candidates at a
+      // time, and the first warp decides on them in order.  (One candidate
+      // after the other, by all threads, took 13 us a window at 100x100x6.)
+      const int lane = tid & 31, warp = tid >> 5;
+      int4* members = reinterpret_cast<int4*>(smem);
+      if (warp == 0) {
         int cur = c->cursor;
-        while (cur < pa.count && pa.net_status[cur] != -1) ++cur;
-        c->cursor = cur;
-        c->fb = 0;
-        s_win[0] = cur;
+        while (true) {
+          const bool open = cur + lane >= pa.count || __ldcg(&pa.net_status[cur + lane]) == -1;
+          const unsigned m = __ballot_sync(0xffffffffu, open);
+          cur += m ? __ffs(m) - 1 : 32;
+          if (m) break;
+        }
+        cur = min(cur, pa.count);
+        if (lane == 0) {
+          c->cursor = cur;
+          c->fb = 0;
+          s_win[0] = cur;
+          s_win[1] = 0;
+        }
       }
       __syncthreads();
-      const int k0 = s_win[0];
+      const int k0 = s_win[0], kend = min(pa.count, k0 + 4 * wmax);
       int W = 0, nskip = 0;
-      for (int k = k0; k < pa.count && W < wmax && k - k0 < 4 * wmax; ++k) {
-        if (*(volatile int32_t*)&pa.net_status[k] != -1) continue;   // done out of order earlier
-        const int32_t n = pa.order[k];
-        const int32_t R = use_batch ? rb.roi_len[n] : -1;
-        if (R <= 0) {
-          if (W == 0 && nskip == 0) {
-            if (tid == 0) { ws.k[0] = k; ws.solo[0] = 1; ws.inorder[0] = 1; }
-            W = 1;
-          }
-          break;
-        }
-        if (nslots == 0) {                   // one net at a time: no footprints to compare
-          if (tid == 0) { ws.k[0] = k; ws.solo[0] = 0; ws.inorder[0] = 1; }
-          W = 1;
-          break;
-        }
-        if (tid == 0) {
-          for (int q = 0; q < 4; ++q) s_box[q] = rb.roi_box[4 * n + q];
-        }
-        __syncthreads();
-        const int32_t ol = t.store_len[n];
-        const int32_t* op = t.store_path + (int64_t)n * t.slot_cap;
-        for (int i = tid; i < ol; i += kThreads) {
-          const int32_t r = op[i] % plane;
-          const int x = r % g.nx, y = r / g.nx;
-          atomicMin(&s_box[0], x); atomicMax(&s_box[1], x);
-          atomicMin(&s_box[2], y); atomicMax(&s_box[3], y);
-        }
-        __syncthreads();
-        bool clash = false;
-        for (int m = 0; m < W && !clash; ++m) clash = boxes_meet(s_box, ws.box + 4 * m);
-        for (int q = 0; q < nskip && !clash; ++q) clash = boxes_meet(s_box, s_skip + 4 * q);
-        if (clash) {
-          if (nskip >= look) break;   // no look-ahead left: the window ends here
-          if (tid == 0) {
+      for (int kb = k0; kb < kend && W < wmax && s_win[1] == 0; kb += kWarps) {
+        const int k = kb + warp;
+        int32_t n = -1, R = 0;
+        int4 box = make_int4(0, 0, 0, 0), grown = box;
+        if (k < kend && __ldcg(&pa.net_status[k]) == -1) {      // (else done out of order earlier)
+          n = pa.order[k];
+          R = use_batch ? rb.roi_len[n] : -1;
+          if (R > 0 && nslots > 0) {
+            int x0 = rb.roi_box[4 * n], x1 = rb.roi_box[4 * n + 1], y0 = rb.roi_box[4 * n + 2], y1 = rb.roi_box[4 * n + 3];
+            const int32_t ol = t.store_len[n];
+            const int32_t* op = t.store_path + (int64_t)n * t.slot_cap;
+            for (int i = lane; i < ol; i += 32) {
+              const int32_t r = op[i] % plane;
+              const int x = r % g.nx, y = r / g.nx;
+              x0 = min(x0, x); x1 = max(x1, x);
+              y0 = min(y0, y); y1 = max(y1, y);
+            }
+            box.x = __reduce_min_sync(0xffffffffu, x0); box.y = __reduce_max_sync(0xffffffffu, x1);
+            box.z = __reduce_min_sync(0xffffffffu, y0); box.w = __reduce_max_sync(0xffffffffu, y1);
             const int32_t sr = t.net_src[n] % plane, dr = t.net_dst[n] % plane;
             const int sx = sr % g.nx, sy = sr / g.nx, dx = dr % g.nx, dy = dr / g.nx;
             const int m = t.net_depth[2 * n + 1] + t.net_halo[2 * n + 1];
-            int* q = s_skip + 4 * nskip;
-            q[0] = min(s_box[0], min(sx, dx) - m);
-            q[1] = max(s_box[1], max(sx, dx) + m);
-            q[2] = min(s_box[2], min(sy, dy) - m);
-            q[3] = max(s_box[3], max(sy, dy) + m);
+            grown = make_int4(min(box.x, min(sx, dx) - m), max(box.y, max(sx, dx) + m),
+                              min(box.z, min(sy, dy) - m), max(box.w, max(sy, dy) + m));
           }
-          __syncthreads();
-          ++nskip;
-          continue;
         }
-        if (tid == 0) {
-          ws.k[W] = k;
-          ws.solo[W] = 0;
-          ws.inorder[W] = nskip == 0 ? 1 : 0;
-          for (int q = 0; q < 4; ++q) ws.box[4 * W + q] = s_box[q];
+        if (lane == 0) {
+          s_cand[warp] = make_int2(n, R);
+          s_box[warp] = box;
+          s_grown[warp] = grown;
         }
         __syncthreads();
-        ++W;
+        if (warp == 0) {
+          bool end = false;
+          for (int j = 0; j < kWarps && kb + j < kend && W < wmax && !end; ++j) {
+            const int2 cand = s_cand[j];
+            if (cand.x < 0) continue;
+            if (cand.y <= 0 || nslots == 0) {
+              // without a ROI from the batch, or one net at a time: alone
+              if (W == 0 && nskip == 0) {
+                if (lane == 0) { ws.k[0] = kb + j; ws.solo[0] = cand.y <= 0 ? 1 : 0; ws.inorder[0] = 1; }
+                W = 1;
+              }
+              end = true;
+              break;
+            }
+            const int4 bx = s_box[j];
+            bool meet = lane < nskip && boxes_meet(bx, s_skip[lane]);
+            for (int m = lane; m < W; m += 32) meet = meet || boxes_meet(bx, members[m]);
+            if (__any_sync(0xffffffffu, meet)) {
+              if (nskip >= look) { end = true; break; }   // no look-ahead left: the window ends here
+              if (lane == 0) s_skip[nskip] = s_grown[j];
+              ++nskip;
+            } else {
+              if (lane == 0) {
+                ws.k[W] = kb + j;
+                ws.solo[W] = 0;
+                ws.inorder[W] = nskip == 0 ? 1 : 0;
+                members[W] = bx;
+              }
+              ++W;
+            }
+            __syncwarp();
+          }
+          if (lane == 0) {
+            s_win[1] = end ? 1 : 0;
+            s_win[2] = W;
+            s_win[3] = nskip;
+          }
+        }
+        __syncthreads();
+        W = s_win[2];
+        nskip = s_win[3];
       }
       if (tid == 0) c->wsize = W;
       clk.mark(6);
