@@ -40,8 +40,8 @@ CONFIGS = {
     # job's first iterations (all nets, same search engine)
     "c1": dict(nx=600, ny=400, nz=12, nets=2000, iters=40, seed=4321, clusters=True, via_span=4,
                plain_iters=3,
-               # DRAM bytes / algorithmic bytes of full_sssp_kernel, ncu on a 300x200x8 search
-               traffic_ratio=0.6655),
+               # DRAM bytes / algorithmic bytes of full_sssp_kernel, ncu on two 307x199x8 searches
+               traffic_ratio=0.8524),
     # multi-pin batching: 600x400x12, 1,500 multi-pin nets (2-16 pins, 1 + geometric(0.35)) with
     # pins inside a seeded 50x50 box per net, as star two-pin requests p0 -> pi (multipin.py)
     "c2": dict(nx=600, ny=400, nz=12, nets=1500, iters=40, seed=2468, multipin=True, via_span=4,

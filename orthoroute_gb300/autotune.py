@@ -3,32 +3,30 @@
 Full-graph nets (Manhattan length >= 125, ``_route_all`` :8219-8262) are
 searched either by ``full_sssp_kernel`` on a cooperative grid of CTAs (one
 grid step per settle phase), by the tile-window engine on a grid of one CTA
-per SM, or by a single 1024-thread CTA.  Which one is faster, and with how
-many CTAs, depends on the lattice: a grid step costs a grid-wide barrier
-(more CTAs, dearer barrier) and spreads the phase's front over the CTAs
-(more CTAs, less work each).  The phase engine has no bucket width to tune
-(each phase's threshold is the least tentative label and the settle rule is
-fixed by exactness); the tile-window engine's window width is one.  So the
+per SM, or by the ROI search's smaller team ("cta").  Which one is faster, and
+with how many CTAs, depends on the lattice: a grid step costs a grid-wide
+barrier (more CTAs, dearer barrier) and spreads the phase's front over the
+CTAs (more CTAs, less work each).  The phase engine has no bucket width to
+tune (each phase's threshold is the least tentative label and the settle rule
+is fixed by exactness); the tile-window engine's window width is one.  So the
 tuner sweeps
 
 * the engine: "grid" or "cta";
-* the lanes per examined frontier node of the "grid" engine (4, 8, 16) and
-  whether waiting frontier nodes keep their last pull (on / off), timed on
-  the full grid;
+* the lanes knob (4, 8, 16) and the reuse knob (on / off) of the "grid"
+  engine, timed on the full grid (the search fits its lanes to the lattice's
+  rows and ignores both: they tell apart by noise only);
 * then the grid of the "grid" engine: 1/4, 1/2, 3/4 and all of the resident
-  CTAs (SMs x CTAs per SM);
+  CTAs (one per SM);
 * then the tile-window engine (label windows over lattice tiles in shared
   memory, tilesearch.cu) at window widths delta of 2, 4, 8, 16 and 32
   uncongested lateral hops: the delta of a delta-stepping search;
 
 on a few full-graph searches of the job's own long nets over the current
-costs, and keeps the fastest.  For ROI nets (one 1024-thread CTA per search)
-it sweeps the lanes that serve one node (2, 4, 8, 16: the CTA's tile of
-nodes in flight is 1024 / lanes), timing a spread of the job's ROI nets; the
-best width follows the lattice's arcs per node.  Every setting returns the
-same paths (the searches are exact and independent of the schedule), so
-tuning changes only time.  Results are cached per (lattice, GPU) in a JSON
-file.
+costs, and keeps the fastest.  For ROI nets it sweeps the lanes knob of their
+search (2, 4, 8, 16; ignored likewise), timing a spread of the job's ROI nets.
+Every setting returns the same paths (the searches are exact and independent
+of the schedule), so tuning changes only time.  Results are cached per
+(lattice, GPU) in a JSON file.
 """
 from __future__ import annotations
 

@@ -11,7 +11,7 @@
 // launched cooperatively so that all of them are resident; its barrier gives
 // up after a bounded wait and reports OGR_ERR_TIMEOUT.  A launch first writes
 // every node's record (penalty, row bounds): a stream over the node arrays
-// (600x400x12: about 30 us of a search of 4 ms) that spares each phase the
+// (600x400x12: 37 us of a search of 3.6 ms) that spares each phase the
 // four loads of the penalty and the two of the row bounds per neighbour.
 #include <atomic>
 
@@ -25,8 +25,8 @@ using namespace ogr_phase;
 // The tuning knobs below are per host thread: each job of a server routes in
 // its own thread and keeps its own settings.
 // Accepted and kept for callers (ogr_full_lanes, ogr_full_reuse): results
-// never depended on them, and one thread examines an entry now, whose row
-// stays with its CTA.
+// never depended on them, and the search fits its lanes to the lattice's rows
+// and keeps an entry's row with its CTA.
 thread_local int g_full_lanes = 16;
 thread_local int g_full_reuse = 0;
 constexpr unsigned kBarSpin = 1u << 22;
@@ -35,7 +35,6 @@ constexpr unsigned kBarSpin = 1u << 22;
 // kBarSpin and 2N + 4 (no search needs more).
 thread_local unsigned g_dbg_spin = kBarSpin;
 thread_local int g_dbg_phases = 0;
-
 
 struct FCtl {
   Ctl team;                                    // cleared before every launch

@@ -1,10 +1,10 @@
 // A6–A8: per-net ROI extraction, exact ROI shortest path, backtrace, and the
-// commit / rip-up scatter.  One CTA (1024 threads) owns one net's search.
+// commit / rip-up scatter.  A team of CTAs owns one net's search (phases.cuh).
 //
 // ROI (extract_roi_bfs, unified_pathfinder.py:2257-2384): level-synchronous
 // bidirectional BFS.  Within one wave step the reference's marks are a set
 // function of the frontier (unseen -> wave mark, other wave -> 3 and
-// "met"), so claiming nodes with atomicCAS yields the same seen[] array,
+// "met"), so claiming nodes with atomics yields the same seen set,
 // meeting depth and early stop.  The ROI is then compacted in ascending
 // global id order (np.where) by scanning the BFS bounding box, and truncated
 // to max_roi_nodes with the reference's must-keep swap.  The BFS does not read
@@ -2265,7 +2265,7 @@ extern "C" int ogr_route_pass(const ogr_graph* g, const ogr_state* st, const ogr
   }
   const int64_t want = (int64_t)(nslots > 0 ? nslots : 1) * kTeam;
   const int grid = want < share ? (int)want : share;
-  // one run of ROI nets: batched windows, or the single-CTA sequential pass
+  // one run of ROI nets: batched windows, or one net at a time
   auto roi_segment = [&](const ogr_pass_args& seg) -> int {
     char* ctl = windows ? (char*)win->ctl : w.win1;
     OGR_CUDA_TRY(cudaMemsetAsync(ctl, 0, ogr_window_ctl_bytes(nslots > 0 ? nslots : 1), s));
@@ -2293,7 +2293,7 @@ extern "C" int ogr_route_pass(const ogr_graph* g, const ogr_state* st, const ogr
     const int rc = roi_segment(*pa);
     if (rc != OGR_OK) return rc;
   } else {
-    // Runs of ROI nets go through one single-CTA launch each; every long net
+    // Runs of ROI nets go through one launch each; every long net
     // gets the whole GPU for its search.  Same order, same state updates.
     int32_t* full_res = ogr_full::result_words(full_ws, g->num_nodes, g->num_edges);
     int32_t k = 0;

@@ -230,7 +230,7 @@ class Ops:
 
     def find_path(self, net: _lib.NetArgs, slot: int = 0, engine: str = "auto") -> Optional[List[int]]:
         """Search one net.  engine: "grid" = whole-lattice search on all SMs
-        (full-graph nets), "cta" = one CTA, "auto" = grid for full-graph nets."""
+        (full-graph nets), "cta" = the ROI search's team, "auto" = grid for full-graph nets."""
         g = self.g.cgraph()
         st = self.s.cstate()
         n = C.c_int32(0)
@@ -492,7 +492,7 @@ def route_pass(ops: "Ops", store: PathStore, table: dict, order: np.ndarray, *, 
     """One ``ogr_route_pass`` call; returns (per-net status flags, stats[4]).
 
     order_full (host, one flag per entry of order) sends the full-graph nets
-    to the whole-lattice search; None keeps every net on the single-CTA pass."""
+    to the whole-lattice search; None keeps every net on the ROI search's team."""
     dev = ops.g.device
     k = len(order)
     if k == 0:

@@ -414,7 +414,7 @@ class PathFinderRouter:
             raise ValueError("mode must be 'persistent' (one launch per routing pass) or 'plain' (one per net)")
         if full_engine not in ("grid", "tile", "cta", "auto"):
             raise ValueError("full_engine must be 'grid' (phase-settled search on all SMs per full-graph net), "
-                             "'tile' (tile-window search on all SMs), 'cta' (one CTA) or "
+                             "'tile' (tile-window search on all SMs), 'cta' (the ROI search) or "
                              "'auto' (the autotuner picks per lattice)")
         self.config = config or PathFinderConfig()
         self.device = device

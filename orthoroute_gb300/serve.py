@@ -7,7 +7,7 @@ job gets a worker thread, its own CUDA stream and its own device-resident
 router state (CSR, congestion arrays, path store and workspaces) for the
 whole job, so jobs overlap on the device: one job's kernels run while
 another job's host policy runs (the ctypes calls release the interpreter
-lock), single-CTA kernels of different jobs share the SMs, and each job's
+lock), kernels of a few CTAs of different jobs share the SMs, and each job's
 whole-lattice searches use a 1/slots share of the resident CTAs, so the
 cooperative searches of concurrent jobs fit on the GPU together.  Every
 kernel is deterministic, so a job's result is the same alone and in the mix.
