@@ -197,7 +197,6 @@ struct Shared {
   int pos_src, pos_dst;
   int R;
   int status;
-  int len;
 };
 
 struct StageClock {
