@@ -26,6 +26,7 @@
 #include "common.cuh"
 #include "fullgraph.cuh"
 #include "phases.cuh"
+#include "roibox.h"
 
 namespace {
 
@@ -348,18 +349,9 @@ __device__ bool roi_build_box(Shared& sh, const ogr_graph& g, const ogr_net_args
   int sx, sy, sz, dx, dy, dz;
   coord(src, sx, sy, sz);
   coord(dst, dx, dy, dz);
-  // the deepest search whose box fits (an arc leads at most one cell aside)
-  int reach = a.bfs_max_depth, X0, Y0, BW, BH, RW;
-  for (;; --reach) {
-    X0 = max(0, min(sx, dx) - reach);
-    Y0 = max(0, min(sy, dy) - reach);
-    BW = min(nx - 1, max(sx, dx) + reach) - X0 + 1;
-    BH = min(ny - 1, max(sy, dy) + reach) - Y0 + 1;
-    RW = (BW + 15) >> 4;
-    if ((int64_t)RW * BH * nz <= kBfsWords) break;
-    if (reach <= 0) return false;
-  }
-  const int NW = RW * BH * nz;
+  const ogr_box::Box box = ogr_box::fit(nx, ny, nz, sx, sy, dx, dy, a.bfs_max_depth, kBfsWords);
+  if (box.words == 0) return false;
+  const int X0 = box.x0, Y0 = box.y0, BW = box.w, BH = box.h, RW = box.row, NW = box.words;
   for (int i = tid; i < NW; i += nt) marks[i] = 0u;
   if (tid < kBfsCtas) {
     mail.out[tid] = 0;
