@@ -405,7 +405,8 @@ typedef struct {
  * cooperative launch; they then commit in order.  A net whose ROI search
  * fails ends its window: the later nets' rip-ups are undone and it takes its
  * fallback in order.  The results are those of the sequential pass.
- * ws holds `slots` search slots of slot_bytes (ogr_window_workspace_*),
+ * ws holds `slots` search slots of slot_bytes (ogr_window_workspace_*, sized
+ * for the largest max_roi_nodes of the passes that use them),
  * scratch holds slots x slot_cap path nodes, ctl is device scratch of
  * ogr_window_ctl_bytes(slots) bytes.  discarded (device int64[3], may be
  * NULL) accumulates {searches, arcs scanned, nodes popped} of the window

@@ -1875,6 +1875,17 @@ __global__ void window_ws_init_kernel(char* base, int32_t slots, size_t slot_byt
     ws_slot_layout(N, rmax, base + (size_t)sidx * slot_bytes, &t);
     const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = i0; i < N; i += step) t.g2r[i] = -1;
+  }
+}
+
+// Claims and stamps of the window slots, cleared for every pass: they lie
+// where the pass's own ROI limit puts them, over whatever a pass of another
+// limit left there.  Only the node map, first in a slot, outlives a pass.
+__global__ void window_claims_kernel(char* base, int32_t slots, size_t slot_bytes, int32_t N, int32_t rmax) {
+  const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+  for (int32_t sidx = blockIdx.y; sidx < slots; sidx += gridDim.y) {
+    Ws t;
+    ws_slot_layout(N, rmax, base + (size_t)sidx * slot_bytes, &t);
     for (int64_t i = i0; i < rmax; i += step) t.claim[i] = 0;
     for (int64_t i = i0; i < (int64_t)(sizeof(SlotCtl) / 4); i += step) reinterpret_cast<int32_t*>(t.ctl)[i] = 0;
   }
@@ -2253,6 +2264,8 @@ extern "C" int ogr_route_pass(const ogr_graph* g, const ogr_state* st, const ogr
         win->slot_bytes < ogr_window_workspace_bytes(g->num_nodes, pa->max_roi_nodes, 1))
       return OGR_ERR_ARG;
     nslots = win->slots < share ? win->slots : share;
+    window_claims_kernel<<<dim3(8, nslots), 256, 0, s>>>((char*)win->ws, nslots, win->slot_bytes, g->num_nodes, need_cap);
+    OGR_LAUNCH_CHECK();
   }
   const int64_t want = (int64_t)(nslots > 0 ? nslots : 1) * kTeam;
   const int grid = want < share ? (int)want : share;

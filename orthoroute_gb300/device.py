@@ -528,7 +528,7 @@ def route_pass(ops: "Ops", store: PathStore, table: dict, order: np.ndarray, *, 
     ops._ev1.synchronize()
     ops.counters["search_ms"] += ops._ev0.elapsed_time(ops._ev1)
     ops.counters["search_launches"] += 1
-    n_launch = 1 if rb is not None else 0
+    n_launch = int(rb is not None) + int(win is not None)
     if full_flags is None:
         n_launch += 1
     else:
