@@ -223,6 +223,8 @@ typedef struct {
   const int32_t* indices;
   const int32_t* rev;
   const uint8_t* blocked;      /* NULL: none */
+  int32_t max_row;             /* arcs of the longest row, 0: not told.  Chooses the
+                                  form of the search; results do not depend on it */
 } ogr_graph;
 
 typedef struct {
@@ -568,7 +570,8 @@ int ogr_full_profile(int64_t* out8, int32_t reset);
  * team, rip-up and commit, window formation (both of a pass's first CTA),
  * statistics and backtrace, cleanup; then searches, settle
  * phases, BFS waves, ROI nodes, entries examined, ROIs taken from the batched
- * extraction).  Synchronous. */
+ * extraction, searches that left the form of their kernel for one of longer
+ * rows or for doubles).  Synchronous. */
 int ogr_search_profile(int64_t* out16, int32_t reset);
 
 /* Allocation-free variant of ogr_find_path.  It has no counterpart in the

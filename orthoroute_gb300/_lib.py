@@ -61,7 +61,7 @@ class CostArgs(C.Structure):
 
 class Graph(C.Structure):
     _fields_ = [("nx", I32), ("ny", I32), ("nz", I32), ("num_nodes", I32), ("num_edges", I64),
-                ("indptr", P), ("indices", P), ("rev", P), ("blocked", P)]
+                ("indptr", P), ("indices", P), ("rev", P), ("blocked", P), ("max_row", I32)]
 
 
 class State(C.Structure):

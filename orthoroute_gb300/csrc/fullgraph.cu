@@ -441,12 +441,16 @@ int size_grid(int dev) {
 
 namespace ogr_full {
 
-// As many arcs as a row of the lattice's inner layers has.  The outermost
-// layer has few arcs or none, so the average over the others comes near the
-// longest row (600x400x12, spans up to 4: 8.0, longest 10; 300x200x8: 7.7,
-// longest 8; 1000x800x32: 3.9, longest 4).  A lattice whose rows are longer
-// all the same is still searched right (run_search).
+// The least form that holds the lattice's longest row, where the caller tells
+// it.  Else by the average over the inner layers, which is below the longest
+// row: a search that meets a longer one takes the 32-arc form out of line, 16
+// entries at a time instead of 64 (two whole-lattice searches each, told
+// against not told: 600x400x10 with spans up to 4, average 7.5 and longest 10,
+// 7.50 ms against 9.65; 600x400x8 with spans up to 3 and wrong-way arcs, 7.7
+// and 10, 6.74 against 8.62; 600x400x12 with sites on a checkerboard, 6.8 and
+// 12, 6.88 against 8.06).
 int row_for(const ogr_graph& g) {
+  if (g.max_row > 0) return g.max_row <= 4 ? 4 : g.max_row <= 8 ? 8 : g.max_row <= 16 ? 16 : 32;
   const double n = (double)(g.num_nodes > 0 ? g.num_nodes : 1), z = (double)(g.nz > 1 ? g.nz : 2);
   const double inner = (double)g.num_edges / n * z / (z - 1.0);
   return inner <= 3.95 ? 4 : inner <= 7.75 ? 8 : inner <= 16.0 ? 16 : 32;

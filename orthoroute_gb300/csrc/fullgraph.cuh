@@ -34,7 +34,7 @@ struct Job {
 
 size_t workspace_bytes(int32_t num_nodes, int64_t num_edges);
 
-// The row length (4, 8, 16 or 32 arcs) whose form of the search fits lattice g.
+// The row length (4, 8, 16 or 32 arcs) whose form of the search is to be launched for lattice g.
 int row_for(const ogr_graph& g);
 
 // CTAs that this host thread's cooperative searches take on the current device

@@ -788,7 +788,10 @@ constexpr int kMaxRow = 32;
 
 // The search with L lanes of K arcs per entry if the rows (of at most max_deg
 // arcs) allow it, else in the form that takes them; labels in ticks, or (only
-// and always in the general form) in doubles.
+// and always in the general form) in doubles.  A kernel holds one form inline
+// and is launched by the lattice's longest row (ogr_full::row_for): with all
+// four in it, chosen by max_deg, registers spilled and every search was 5 to
+// 16 % slower; with the larger ones out of line still 2 to 11 %.
 template <int L, int K, bool kMulti, bool kRoi>
 __device__ __forceinline__ Outcome run_search(const Problem& pr, char* smem, int k0, int max_deg, bool in_ticks) {
   if (in_ticks && max_deg <= L * K) {

@@ -183,7 +183,8 @@ __host__ __device__ inline BfsSlot bfs_slot_at(char* base, int32_t N, int64_t qc
 // [5] rip-up and commit, [6] window formation (CTA 0 of a pass), [7] statistics
 // + backtrace, [8] cleanup, [9] searches, [10] phases, [11] BFS
 // waves run, [12] ROI nodes, [13] entries examined, [14] ROIs taken from the
-// batched extraction.
+// batched extraction, [15] searches that left the form of their kernel (longer
+// rows, or values redone in doubles).
 __device__ unsigned long long g_stage[16];
 
 struct Shared {
@@ -923,6 +924,7 @@ __device__ __noinline__ void roi_search(const RoiJob* jp, char* smem, int* statu
     const int max_deg = sm.res[2];
     const int ready = sm.ok;
     if (max_deg > kMaxRow) fix = false;
+    if (leader && (attempt == 0) == (max_deg > L * K)) atomicAdd(&g_stage[15], 1ull);
     int32_t rs = -1, rd = -1;
     if (!kMulti && ready) {
       rs = __ldcg(&w.g2r[a.src]);

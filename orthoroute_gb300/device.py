@@ -48,6 +48,7 @@ class DeviceGraph:
         _lib.check(self.lib.ogr_csr_num_edges(C.byref(desc), C.byref(E)), "ogr_csr_num_edges")
         self.E = int(E.value)
         self.N = lattice.num_nodes
+        self.max_row = lattice.max_row()
         dev = self.device
         self.indptr = torch.empty(self.N + 1, dtype=torch.int32, device=dev)
         self.indices = torch.empty(self.E, dtype=torch.int32, device=dev)
@@ -68,7 +69,7 @@ class DeviceGraph:
     def cgraph(self) -> _lib.Graph:
         L = self.lattice
         return _lib.Graph(L.nx, L.ny, L.nz, self.N, self.E, _p(self.indptr), _p(self.indices), _p(self.rev),
-                          _p(self.blocked))
+                          _p(self.blocked), self.max_row)
 
 
 class DeviceState:

@@ -100,6 +100,20 @@ class Lattice:
             return self.via_cost * self.adjacent_via_step_scale
         return self.via_cost * (1.0 + 0.15 * (abs(b - a) - 1))
 
+    def max_row(self) -> int:
+        """Arcs of the longest row: a layer's via partners and, on lateral
+        layers, its lateral neighbours (via sites at the edge alone, on a
+        board a few cells wide, may have fewer)."""
+        partners = [0] * self.nz
+        for a, b in self.via_pairs():
+            partners[a] += 1
+            partners[b] += 1
+        side = {"h": min(2, self.nx - 1), "v": min(2, self.ny - 1)}
+        lateral = [0] * self.nz
+        for z in self.lateral_layers():
+            lateral[z] = sum(side[a] for a in self.allowed_axes(z))
+        return max(p + t for p, t in zip(partners, lateral))
+
     # -- device descriptor ----------------------------------------------------
     def descriptor(self):
         """Return (ogr_lattice_desc, keep-alive arrays)."""
