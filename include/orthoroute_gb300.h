@@ -545,9 +545,9 @@ int ogr_search_lanes(int32_t lanes, int32_t* current);
  * counterpart. */
 int ogr_window_lookahead(int32_t nets, int32_t* current);
 
-/* Limits for tests of failure handling in the phase-settled whole-lattice
- * search: barrier_spin = n > 0 lets a CTA poll the grid barrier n - 1 times
- * before it gives up (the search then returns OGR_ERR_TIMEOUT), 0 restores
+/* Limits for tests of failure handling in the phase-settled searches,
+ * whole-lattice and ROI: barrier_spin = n > 0 lets a CTA poll the barrier of
+ * its search's team n - 1 times before it gives up (the search then returns OGR_ERR_TIMEOUT), 0 restores
  * the default bound; max_phases > 0 caps the settle phases (OGR_ERR_ITER_CAP
  * when a search needs more), 0 restores the default (2N + 4, never reached);
  * -1 leaves a setting.  *cur_spin / *cur_phases (host, may be NULL) receive

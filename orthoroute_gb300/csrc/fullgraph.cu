@@ -30,9 +30,9 @@ using namespace ogr_phase;
 thread_local int g_full_lanes = 16;
 thread_local int g_full_reuse = 0;
 constexpr unsigned kBarSpin = 1u << 22;
-// Limits for tests of failure handling (ogr_debug_limits): the grid
-// barrier's spin bound and a cap on settle phases; the defaults are
-// kBarSpin and 2N + 4 (no search needs more).
+// Limits for tests of failure handling (ogr_debug_limits): the spin bound of a
+// search team's barrier and a cap on settle phases, of whole-lattice and ROI
+// searches alike; the defaults are kBarSpin and 2N + 4 (no search needs more).
 thread_local unsigned g_dbg_spin = kBarSpin;
 thread_local int g_dbg_phases = 0;
 
@@ -165,8 +165,10 @@ full_sssp_kernel(ogr_graph g, ogr_state st, ogr_full::Job job, FWs w) {
   pr.ctl = &ctl->team;
   pr.rank = blockIdx.x;
   pr.nranks = gridDim.x;
-  pr.spin = w.bar_spin;
-  pr.max_phase = w.max_phases > 0 ? min(w.max_phases, 2 * N + 4) : 2 * N + 4;
+  if (tid == 0) {
+    sm.spin = w.bar_spin;
+    sm.max_phase = w.max_phases > 0 ? min(w.max_phases, 2 * N + 4) : 2 * N + 4;
+  }
   // With statistics requested the search goes on after dst is settled until
   // every node with a label <= L(dst) is settled (T > L(dst)): the IN bound
   // can settle dst before cheaper nodes, which the heap pops earlier.
@@ -461,6 +463,9 @@ int grid_blocks() {
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
   return size_grid(dev) == OGR_OK ? g_grid_blocks[dev] : 0;
 }
+
+unsigned wait_limit() { return g_dbg_spin; }
+int phase_limit() { return g_dbg_phases; }
 
 size_t workspace_bytes(int32_t num_nodes, int64_t num_edges) {
   return fws_layout(num_nodes, num_edges, nullptr, nullptr);

@@ -41,6 +41,11 @@ int row_for(const ogr_graph& g);
 // (ogr_full_grid), 0 on an error.
 int grid_blocks();
 
+// Bounds of this host thread's searches (ogr_debug_limits): polls of a wait, and
+// settle phases (0: what the nodes allow).
+unsigned wait_limit();
+int phase_limit();
+
 // Device int32[4] the search writes: status, path length, phases, 0.
 int32_t* result_words(void* ws, int32_t num_nodes, int64_t num_edges);
 

@@ -165,8 +165,6 @@ struct Problem {
   const double* mseed;             // multi-source: cost of each node marked kSeed
   Ctl* ctl;
   int rank, nranks;                // this CTA and the CTAs of the team
-  unsigned spin;                   // bound of a wait
-  int max_phase;
   bool want_stats;
 };
 
@@ -198,6 +196,10 @@ struct Head {
   unsigned tail;                   // free ring: end
   int inexact, nov_out, dst_hit, ok;
   int res[3];
+  // bounds of the search: polls of a wait, settle phases (thread 0 sets and
+  // reads them; in registers of all threads they were spilled)
+  unsigned spin;
+  int max_phase;
 };
 
 template <int A>
@@ -270,7 +272,7 @@ __device__ __forceinline__ void await(const Problem& pr, Head& sm, int k, unsign
     ld_slot(s, a, t);
     if ((unsigned)(a & kArriveMask) >= want) return;
     ++it;
-    if (it > pr.spin || ((it & 63) == 0 && *(const volatile int32_t*)&pr.ctl->err)) {
+    if (it > sm.spin || ((it & 63) == 0 && *(const volatile int32_t*)&pr.ctl->err)) {
       atomicExch(&pr.ctl->err, 1);
       sm.ok = 0;
       return;
@@ -336,7 +338,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
         verdict = dst_done || kMulti ? kFound : kEmpty;
       else if (dst_done && T > ld)
         verdict = kFound;
-      else if (phase > pr.max_phase)
+      else if (phase > sm.max_phase)
         verdict = kCapped;
     }
     if (!kGen && phase > 0 && T == 0) verdict = kInexactSeen;

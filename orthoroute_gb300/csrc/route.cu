@@ -75,6 +75,8 @@ struct Ws {
   char* win1;                // control block of a pass without windows
   int64_t* result;           // [0] status, [1] path length, [2] fallbacks used, [3] ROI size
   int64_t qcap;
+  unsigned spin;             // bounds of a search: polls of a wait, settle phases (0: what R allows)
+  int32_t max_phases;
 };
 
 // Seeds and targets of a multi-source multi-sink search
@@ -124,6 +126,8 @@ __host__ inline size_t ws_layout(int32_t N, char* base, Ws* w) {
   t.win1 = take(kWin1Bytes);
   t.result = (int64_t*)take(64);
   t.qcap = (int64_t)n;
+  t.spin = ogr_full::wait_limit();
+  t.max_phases = ogr_full::phase_limit();
   if (w) *w = t;
   return off;
 }
@@ -833,8 +837,9 @@ struct RoiJob {
 };
 
 // One team's search.  Every CTA of the team calls it with the slot's team
-// words zero; *status_out / *len_out are the result in the team's first CTA
-// (in the others the status lacks what the backtrace finds).
+// words zero; *status_out / *len_out are the result in the first thread of the
+// team (elsewhere the status may lack what the backtrace finds, or a wait that
+// another CTA gave up).
 template <int L, int K, bool kMulti>
 __device__ __noinline__ void roi_search(const RoiJob* jp, char* smem, int* status_out, int* len_out) {
   using namespace ogr_phase;
@@ -879,8 +884,10 @@ __device__ __noinline__ void roi_search(const RoiJob* jp, char* smem, int* statu
   pr.ctl = &w.ctl->team;
   pr.rank = job.rank;
   pr.nranks = job.nranks;
-  pr.spin = 1u << 22;
-  pr.max_phase = 2 * R + 4;
+  if (tid == 0) {
+    sm.spin = w.spin;
+    sm.max_phase = w.max_phases > 0 ? min(w.max_phases, 2 * R + 4) : 2 * R + 4;
+  }
   // With statistics requested the search goes on after dst is settled until
   // every node with a label <= L(dst) is settled (T > L(dst)): the IN bound
   // can settle dst before cheaper nodes, which the heap pops earlier.
@@ -1106,7 +1113,11 @@ __device__ __noinline__ void roi_search(const RoiJob* jp, char* smem, int* statu
     __syncthreads();
   }
   for (int r = first; r < R; r += step) w.g2r[roi[r]] = -1;
-  if (leader) w.ctl->sid = pr.sid;
+  if (leader) {
+    w.ctl->sid = pr.sid;
+    // (a CTA that gave up on the last wait left its part of the statistics out)
+    if (*(const volatile int32_t*)&w.ctl->team.err) status = OGR_ERR_TIMEOUT;
+  }
   __syncthreads();
   mark(8);
   *status_out = status;
@@ -1584,10 +1595,17 @@ window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa,
   auto slot_of = [&](int m, bool solo) {
     Ws x = w;
     if (nslots > 0 && !solo) ws_slot_layout(g.num_nodes, rmax, slot_base + (size_t)m * slot_bytes, &x);
+    x.spin = w.spin;
+    x.max_phases = w.max_phases;
     return x;
   };
   auto path_of = [&](int m, int32_t n) {
     return nslots > 0 ? scratch + (int64_t)m * t.slot_cap : t.store_path + (int64_t)n * t.slot_cap;
+  };
+  // On an error before the commits every member of the window is without its
+  // old path: so says the store.
+  auto ripped_up = [&](int members) {
+    if (b < members && tid == 0) t.store_len[pa.order[ws.k[b]]] = 0;
   };
   if (b < wmax) clear_team(slot_of(b, false).ctl);
   if (b == 0) clear_team(w.ctl);
@@ -1730,7 +1748,10 @@ window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa,
       if (b == 0) clk.mark(5);
     }
     if (!win_barrier(c, target, &s_bar)) break;
-    if (*(volatile int32_t*)&c->error) break;
+    if (*(volatile int32_t*)&c->error) {
+      ripped_up(W);
+      break;
+    }
     // 3. search, one team of CTAs per member, paths into scratch
     const int T = min(kTeam, G / W), mem = b / T, rank = b - mem * T;
     if (mem < W) {
@@ -1750,7 +1771,10 @@ window_pass_kernel(ogr_graph g, ogr_state st, ogr_net_table t, ogr_pass_args pa,
       }
     }
     if (!win_barrier(c, target, &s_bar)) break;
-    if (*(volatile int32_t*)&c->error) break;
+    if (*(volatile int32_t*)&c->error) {
+      ripped_up(W);
+      break;
+    }
     // 4. commit
     clk.start();
     if (b < W) clear_team(slot_of(b, solo).ctl);
