@@ -485,13 +485,15 @@ int ogr_find_path_full_multi(const ogr_graph* g, const ogr_state* st, const ogr_
                              void* workspace, size_t workspace_bytes, int32_t* path_out, int32_t path_cap,
                              int32_t* path_len_out, int64_t* stats, void* stream);
 
-/* Grid of the whole-lattice search on the current device (a tuning knob;
- * results do not depend on it): ctas > 0 sets the number of cooperative CTAs,
- * 0 only reads.  *limit (host, may be NULL) receives the maximum, one per SM
- * (a CTA's shared memory holds its part of the frontier); up to twice that
- * may be asked for and runs as the maximum.  *current (may be NULL) receives
- * the grid in use.  The setting is per device and per host thread.  Chosen by
- * the autotuner (orthoroute_gb300/autotune.py); no reference counterpart. */
+/* Share of the SMs that this host thread's searches take on the current device
+ * (a tuning knob; results do not depend on it): ctas > 0 sets the number of
+ * cooperative CTAs of a whole-lattice search and the most that an ROI search
+ * or a pass of ROI nets takes, 0 only reads.  *limit (host, may be NULL)
+ * receives the maximum, one per SM (a CTA's shared memory holds its part of
+ * the frontier); up to twice that may be asked for and runs as the maximum.
+ * *current (may be NULL) receives the grid in use.  The setting is per device
+ * and per host thread.  Chosen by the autotuner
+ * (orthoroute_gb300/autotune.py); no reference counterpart. */
 int ogr_full_grid(int32_t ctas, int32_t* current, int32_t* limit);
 
 /* Lanes per examined frontier node of the whole-lattice search (4, 8 or 16;

@@ -197,7 +197,7 @@ def inject_fault(name: str, rc: int):
 
 
 def debug_limits(barrier_spin: int = -1, max_phases: int = -1):
-    """Set (>= 0) or read (-1) the whole-lattice search's failure-test limits
+    """Set (>= 0) or read (-1) the failure-test limits of whole-lattice and ROI searches
     (ogr_debug_limits): (barrier spin, phase cap), 0 = default."""
     a, b = C.c_int32(0), C.c_int32(0)
     check(load().ogr_debug_limits(int(barrier_spin), int(max_phases), C.byref(a), C.byref(b)), "ogr_debug_limits")

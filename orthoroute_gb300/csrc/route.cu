@@ -2032,9 +2032,13 @@ int launch_find(const ogr_graph& g, const ogr_state& st, const ogr_net_args& a, 
   Ws wv = w;
   MultiSeeds mv = ms ? *ms : MultiSeeds{};
   void* args[] = {&gv, &sv, &av, &wv, &roi, &R, &roi_pen, &mv, &path_out, &path_cap, &stats};
+  // a team within this host thread's share of the SMs (ogr_full_grid): a
+  // cooperative launch wider than that waits for other jobs' searches to end
+  const int share = ogr_full::grid_blocks();
+  if (share < 1) return OGR_ERR_CUDA;
   const void* f = nullptr;
   OGR_WITH_ROW(ROW, g, f = ms ? (const void*)find_team_kernel<ROW, true> : (const void*)find_team_kernel<ROW, false>);
-  return launch_team(f, kTeam, args, s);
+  return launch_team(f, share < kTeam ? share : kTeam, args, s);
 }
 
 }  // namespace
