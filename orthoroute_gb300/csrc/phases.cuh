@@ -75,6 +75,7 @@ struct __align__(16) Slot {
 constexpr unsigned long long kArrive = 1ull, kDst = 1ull << 10, kOut = 1ull << 11, kCount = 1ull << 32;
 constexpr unsigned long long kArriveMask = 0x3ffull;
 constexpr unsigned kOutMask = 0x1fffff, kMostOut = 2047;
+constexpr int kMostEntries = 1 << 14;        // (with rows of up to 32 arcs they ask for fewer than 2^20 places)
 constexpr int kMaxTeam = 1023;      // CTAs of a team
 constexpr int kStInexact = 100;    // Outcome::status: redo in doubles
 
@@ -192,7 +193,9 @@ struct Head {
   unsigned long long a, t;         // the barrier's word, as thread 0 read it
   unsigned long long ld;           // label of dst, once settled
   unsigned long long wmin[kWarps];
-  unsigned push[2];                // entries carried (bits 20-31) and places asked for (0-19) in a phase
+  // entries carried (bits 0-11) and places asked for (12-31: the count may run
+  // over where none are given, with kMostEntries or more) in a phase
+  unsigned push[2];
   unsigned tail;                   // free ring: end
   int inexact, nov_out, dst_hit, ok;
   int res[3];
@@ -379,7 +382,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
     sm.plan.ncarr = nk;
     sm.plan.n = n;
     sm.plan.head = head;
-    sm.plan.avail = min(sm.tail - head, (unsigned)fmaxf(room, 0.0f));
+    sm.plan.avail = n < kMostEntries ? min(sm.tail - head, (unsigned)fmaxf(room, 0.0f)) : 0;
   };
   if (tid == 0) {
     sm.push[0] = sm.push[1] = 0;
@@ -650,12 +653,14 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
           unsigned p = 0;
           if (lane < 2)
             p = atomicAdd(lane == 0 ? &sm.push[q] : &sm.tail,
-                          lane == 0 ? (unsigned)nt + ((unsigned)__popc(mk) << 20) : (unsigned)__popc(mg));
+                          lane == 0 ? ((unsigned)nt << 12) + (unsigned)__popc(mk) : (unsigned)__popc(mg));
+          // (a row of the general form has any length)
+          if (kGen && lane == 0 && p >= (1u << 31)) atomicSub(&sm.push[q], (unsigned)nt << 12);
           const unsigned t = __shfl_sync(kAll, p, 1);
           p = __shfl_sync(kAll, p, 0);
           if (leaves) bd.freel[(t + __popc(mg & below)) % (unsigned)kS] = (uint16_t)slot;
-          if (keep) bd.carr[q ^ 1][(p >> 20) + __popc(mk & below)] = (uint16_t)slot;
-          int at0 = (int)(p & 0xfffffu);
+          if (keep) bd.carr[q ^ 1][(p & 0xfffu) + __popc(mk & below)] = (uint16_t)slot;
+          int at0 = (int)(p >> 12);
 #pragma unroll
           for (int j = 0; j < K; ++j) {
             const int at = at0 + __popc(mt[j] & below);
@@ -704,7 +709,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
     __syncthreads();
     // the phase's writes are done: hand in, fetch the new entries' rows, wait
     const unsigned pushed = sm.push[q];
-    const int nf = min((int)(pushed & 0xfffffu), av), nk = (int)(pushed >> 20);
+    const int nf = min((int)(pushed >> 12), av), nk = (int)(pushed & 0xfffu);
     if (warp == 0) {
       u64 t = warp_min_u64(lane < kWarps ? sm.wmin[lane] : kNone);
       if (lane == 0) {
