@@ -70,6 +70,7 @@ struct Ws {
   ogr_phase::Rec* rec;
   int32_t* par;
   int32_t* claim;
+  int32_t nclaim;            // nodes that claim[] has words for
   int4* ov[2];
   SlotCtl* ctl;
   char* win1;                // control block of a pass without windows
@@ -118,6 +119,7 @@ __host__ inline size_t ws_layout(int32_t N, char* base, Ws* w) {
   t.roi = (int32_t*)take(4 * n);
   t.par = (int32_t*)take(4 * n);
   t.claim = (int32_t*)take(4 * n);
+  t.nclaim = N;
   t.rec = (ogr_phase::Rec*)take(16 * n);
   t.ov[0] = (int4*)take(16 * n);
   t.ov[1] = (int4*)take(16 * n);
@@ -149,6 +151,7 @@ __host__ __device__ inline size_t ws_slot_layout(int32_t N, int32_t Rmax, char* 
     t.rec = (ogr_phase::Rec*)p[1];
     t.par = (int32_t*)p[2];
     t.claim = (int32_t*)p[3];
+    t.nclaim = Rmax;
     t.ov[0] = (int4*)p[4];
     t.ov[1] = (int4*)p[5];
     t.ctl = (SlotCtl*)p[6];
@@ -865,7 +868,11 @@ __device__ __noinline__ void roi_search(const RoiJob* jp, char* smem, int* statu
   const int32_t* roi = full ? roi_w : job.roi;
   int32_t sid = __ldcg(&w.ctl->sid) + 1;
   const bool wrap = sid < 1 || sid == 0x7fffffff;
-  if (wrap) sid = 1;
+  if (wrap) {
+    // the stamps begin again: of all nodes, not of this ROI's alone
+    sid = 1;
+    for (int r = first; r < w.nclaim; r += step) w.claim[r] = 0;
+  }
   Problem pr{};
   pr.R = R;
   pr.indptr = g.indptr;
@@ -902,7 +909,6 @@ __device__ __noinline__ void roi_search(const RoiJob* jp, char* smem, int* statu
       const int32_t gid = full ? r : roi[r];
       if (full) roi_w[r] = r;
       w.g2r[gid] = r;
-      if (wrap && attempt == 0) w.claim[r] = 0;
       const int32_t f0 = g.indptr[gid], f1 = g.indptr[gid + 1];
       md = max(md, f1 - f0);
       const float pen = job.roi_pen ? job.roi_pen[r] : ogr_node_penalty(st, a, gid);
