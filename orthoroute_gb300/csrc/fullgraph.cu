@@ -189,6 +189,21 @@ full_sssp_kernel(ogr_graph g, ogr_state st, ogr_full::Job job, FWs w) {
     }
     md = __reduce_max_sync(0xffffffffu, md);
     if ((tid & 31) == 0) sm.wmin[tid >> 5] = (unsigned long long)md;
+    // Thread 0: the first frontier (the leader's nf0 entries, their least label
+    // t0) at barrier k0 + 1.
+    auto enter = [&](int nf0, unsigned long long t0) {
+      if (leader) {
+        ctl->team.nov[0] = nf0;
+        ctl->team.nov[1] = 0;
+        ctl->team.nov[2] = 0;
+        if (attempt == 0) t_init = gtimer();
+      }
+      if (sm.ok) {
+        arrive(pr, sm, k0 + 1, kArrive + kOut * (unsigned long long)(nf0 < (int)kMostOut ? nf0 : (int)kMostOut) + kCount * (unsigned long long)nf0, t0);
+        await(pr, sm, k0 + 1);
+      }
+      if (leader && attempt == 0) t_loop = gtimer();
+    };
     __syncthreads();
     if (tid == 0) {
       unsigned long long t0 = kNone;
@@ -202,60 +217,75 @@ full_sssp_kernel(ogr_graph g, ogr_state st, ogr_full::Job job, FWs w) {
       arrive(pr, sm, k0, kArrive, ~(unsigned long long)md);
       await(pr, sm, k0);
       sm.res[2] = (int)sm.t;
-      const bool in_ticks = fix && (int)sm.t <= kMaxRow;
       if (leader && attempt) clear_slot(pr, k0 + 3);
       if (leader && !kMulti) {
         w.claim[src] = pr.sid;
         w.ov[0][0] = make_int4(src, indptr[src], indptr[src + 1] - indptr[src], __float_as_int(0.0f));
         nf0 = 1;
         t0 = 0ull;
-      } else if (leader) {
-        // mark the targets, then put every seed in the first frontier with
-        // its label seed cost + penalty (of a redone search they are marked)
-        int bad = 0;
-        for (int i = 0; i < job.n_targets && !bad; ++i) {
+      }
+      if (kMulti) {
+        sm.res[0] = 0;             // first entries
+        sm.res[1] = 0;             // a bad or repeated seed or target
+        sm.wmin[0] = kNone;        // their least label
+      } else {
+        enter(nf0, t0);
+      }
+    }
+    if constexpr (kMulti) {
+      // CTA 0 marks the targets, then puts every seed in the first frontier
+      // with its label seed cost + penalty (of a redone search they are marked)
+      __syncthreads();
+      const bool mine = blockIdx.x == 0 && sm.ok;
+      const bool in_ticks = fix && sm.res[2] <= kMaxRow;
+      if (mine) {
+        for (int i = tid; i < job.n_targets; i += kThreads) {
           const int32_t t = job.targets[i];
           const double tc = job.target_cost[i];
-          if (t < 0 || t >= N || tc != tc) { bad = 1; break; }
-          unsigned long long* p = reinterpret_cast<unsigned long long*>(&w.mtgt[t]);
-          if (attempt == 0 && *p != kNoTerm) { bad = 1; break; }   // repeated target
-          *p = (unsigned long long)__double_as_longlong(tc);
+          if (t < 0 || t >= N || tc != tc) {
+            sm.res[1] = 1;
+            continue;
+          }
+          const unsigned long long was = atomicExch(reinterpret_cast<unsigned long long*>(&w.mtgt[t]),
+                                                    (unsigned long long)__double_as_longlong(tc));
+          if (attempt == 0 && was != kNoTerm) sm.res[1] = 1;
           w.rec[t].sp = kTgt;
         }
-        for (int i = 0; i < job.n_seeds && !bad; ++i) {
+      }
+      __syncthreads();
+      if (mine) {
+        for (int i = tid; i < job.n_seeds; i += kThreads) {
           const int32_t s0 = job.seeds[i];
           const double sc = job.seed_cost[i];
-          if (s0 < 0 || s0 >= N || !(sc >= 0.0)) { bad = 1; break; }
-          unsigned long long* p = reinterpret_cast<unsigned long long*>(&w.mseed[s0]);
-          if (attempt == 0 && *p != kNoTerm) { bad = 1; break; }   // repeated seed
-          *p = (unsigned long long)__double_as_longlong(sc);
-          const float pen = ogr_node_penalty(st, a, s0);
+          if (s0 < 0 || s0 >= N || !(sc >= 0.0)) {
+            sm.res[1] = 1;
+            continue;
+          }
+          const unsigned long long was = atomicExch(reinterpret_cast<unsigned long long*>(&w.mseed[s0]),
+                                                    (unsigned long long)__double_as_longlong(sc));
+          if (attempt == 0 && was != kNoTerm) {
+            sm.res[1] = 1;
+            continue;
+          }
+          const float pen = __ldcg(&w.rec[s0].pen);
           w.claim[s0] = pr.sid;
-          const int32_t flags = kSeed | (w.rec[s0].sp & kTgt);
+          const int32_t f0 = indptr[s0], flags = kSeed | (__ldcg(&w.rec[s0].sp) & kTgt);
           w.rec[s0].sp = 1 | flags;
-          w.ov[0][nf0++] = make_int4(s0, indptr[s0], (indptr[s0 + 1] - indptr[s0]) | flags, __float_as_int(pen));
+          w.ov[0][atomicAdd(&sm.res[0], 1)] = make_int4(s0, f0, (indptr[s0 + 1] - f0) | flags, __float_as_int(pen));
           unsigned long long lb = ogr_dbits(sc + (double)pen);
           if (in_ticks) {
             lb = 0ull;
             if (seed_ticks(sc, &lb) && tick_finite(pen)) lb += ticks(pen);
           }
-          t0 = lb < t0 ? lb : t0;
+          atomicMin(&sm.wmin[0], lb);
         }
-        if (bad) nf0 = 0;
-        ctl->merr = bad;
       }
-      if (leader) {
-        ctl->team.nov[0] = nf0;
-        ctl->team.nov[1] = 0;
-        ctl->team.nov[2] = 0;
-        if (attempt == 0) t_init = gtimer();
+      __syncthreads();
+      if (tid == 0) {
+        if (leader) ctl->merr = sm.res[1];
+        enter(leader && !sm.res[1] ? sm.res[0] : 0, leader ? sm.wmin[0] : kNone);
+        if (sm.ok && __ldcg(&ctl->merr)) sm.ok = 2;
       }
-      if (sm.ok) {
-        arrive(pr, sm, k0 + 1, kArrive + kOut * (unsigned long long)(nf0 < (int)kMostOut ? nf0 : (int)kMostOut) + kCount * (unsigned long long)nf0, t0);
-        await(pr, sm, k0 + 1);
-      }
-      if (kMulti && sm.ok && __ldcg(&ctl->merr)) sm.ok = 2;
-      if (leader && attempt == 0) t_loop = gtimer();
     }
     __syncthreads();
     const int ok = sm.ok, max_deg = sm.res[2];
