@@ -134,7 +134,7 @@ full_sssp_kernel(ogr_graph g, ogr_state st, ogr_full::Job job, FWs w) {
   unsigned long long t_start = 0, t_init = 0, t_loop = 0;
   if (leader) t_start = gtimer();
   const int32_t* __restrict__ indptr = g.indptr;
-  // claim stamps count the searches (two for one that is redone in doubles);
+  // claim stamps count the searches (two for one that goes over to doubles);
   // when the count runs out they are cleared
   int32_t sid = __ldcg(&ctl->sid) + 1;
   const bool wrap = sid < 1 || sid == 0x7fffffff;
@@ -168,6 +168,7 @@ full_sssp_kernel(ogr_graph g, ogr_state st, ogr_full::Job job, FWs w) {
   if (tid == 0) {
     sm.spin = w.bar_spin;
     sm.max_phase = w.max_phases > 0 ? min(w.max_phases, 2 * N + 4) : 2 * N + 4;
+    sm.first = 0;
   }
   // With statistics requested the search goes on after dst is settled until
   // every node with a label <= L(dst) is settled (T > L(dst)): the IN bound
@@ -175,134 +176,139 @@ full_sssp_kernel(ogr_graph g, ogr_state st, ogr_full::Job job, FWs w) {
   pr.want_stats = job.stats != nullptr;
   Outcome o{};
   bool fix = true;
-  int k0 = 0;                  // barriers used so far
-  for (int attempt = 0; attempt < 2; ++attempt) {
-    pr.sid = sid + attempt;
-    // every node's record
-    int md = 0;
+  pr.sid = sid;
+  // every node's record
+  int md = 0;
 #pragma unroll 4
-    for (int64_t i = gtid; i < N; i += gthreads) {
-      const int32_t f0 = indptr[i], f1 = indptr[i + 1];
-      md = max(md, f1 - f0);
-      const float pen = ogr_node_penalty(st, a, (int32_t)i);
-      __stcg(reinterpret_cast<int4*>(&w.rec[i]), make_int4(f0, f1 - f0, 0, __float_as_int(pen)));
+  for (int64_t i = gtid; i < N; i += gthreads) {
+    const int32_t f0 = indptr[i], f1 = indptr[i + 1];
+    md = max(md, f1 - f0);
+    const float pen = ogr_node_penalty(st, a, (int32_t)i);
+    __stcg(reinterpret_cast<int4*>(&w.rec[i]), make_int4(f0, f1 - f0, 0, __float_as_int(pen)));
+  }
+  md = __reduce_max_sync(0xffffffffu, md);
+  if ((tid & 31) == 0) sm.wmin[tid >> 5] = (unsigned long long)md;
+  // Thread 0: the first frontier (the leader's nf0 entries, their least label
+  // t0) at the second barrier.
+  auto enter = [&](int nf0, unsigned long long t0) {
+    if (leader) {
+      ctl->team.nov[0] = nf0;
+      ctl->team.nov[1] = 0;
+      ctl->team.nov[2] = 0;
+      t_init = gtimer();
     }
-    md = __reduce_max_sync(0xffffffffu, md);
-    if ((tid & 31) == 0) sm.wmin[tid >> 5] = (unsigned long long)md;
-    // Thread 0: the first frontier (the leader's nf0 entries, their least label
-    // t0) at barrier k0 + 1.
-    auto enter = [&](int nf0, unsigned long long t0) {
-      if (leader) {
-        ctl->team.nov[0] = nf0;
-        ctl->team.nov[1] = 0;
-        ctl->team.nov[2] = 0;
-        if (attempt == 0) t_init = gtimer();
+    if (sm.ok) {
+      arrive(pr, sm, 1, kArrive + kOut * (unsigned long long)(nf0 < (int)kMostOut ? nf0 : (int)kMostOut) + kCount * (unsigned long long)nf0, t0);
+      await(pr, sm, 1);
+    }
+    if (leader) t_loop = gtimer();
+  };
+  __syncthreads();
+  if (tid == 0) {
+    unsigned long long t0 = kNone;
+    int nf0 = 0;
+    sm.ok = 1;
+    // The records are written and the longest row is known (it travels in
+    // the word's maximum).  Several seeds may settle in one phase, each the
+    // other's neighbour, so only now are their records marked reached.
+    for (int i = 1; i < kWarps; ++i) md = max(md, (int)sm.wmin[i]);
+    arrive(pr, sm, 0, kArrive, ~(unsigned long long)md);
+    await(pr, sm, 0);
+    sm.res[2] = (int)sm.t;
+    if (leader && !kMulti) {
+      w.claim[src] = pr.sid;
+      w.ov[0][0] = make_int4(src, indptr[src], indptr[src + 1] - indptr[src], __float_as_int(0.0f));
+      nf0 = 1;
+      t0 = 0ull;
+    }
+    if (kMulti) {
+      sm.res[0] = 0;             // first entries
+      sm.res[1] = 0;             // a bad or repeated seed or target
+      sm.wmin[0] = kNone;        // their least label
+    } else {
+      enter(nf0, t0);
+    }
+  }
+  if constexpr (kMulti) {
+    // CTA 0 marks the targets, then puts every seed in the first frontier
+    // with its label seed cost + penalty
+    __syncthreads();
+    const bool mine = blockIdx.x == 0 && sm.ok;
+    const bool in_ticks = sm.res[2] <= kMaxRow;
+    if (mine) {
+      for (int i = tid; i < job.n_targets; i += kThreads) {
+        const int32_t t = job.targets[i];
+        const double tc = job.target_cost[i];
+        if (t < 0 || t >= N || tc != tc) {
+          sm.res[1] = 1;
+          continue;
+        }
+        const unsigned long long was = atomicExch(reinterpret_cast<unsigned long long*>(&w.mtgt[t]),
+                                                  (unsigned long long)__double_as_longlong(tc));
+        if (was != kNoTerm) sm.res[1] = 1;
+        w.rec[t].sp = kTgt;
       }
-      if (sm.ok) {
-        arrive(pr, sm, k0 + 1, kArrive + kOut * (unsigned long long)(nf0 < (int)kMostOut ? nf0 : (int)kMostOut) + kCount * (unsigned long long)nf0, t0);
-        await(pr, sm, k0 + 1);
+    }
+    __syncthreads();
+    if (mine) {
+      for (int i = tid; i < job.n_seeds; i += kThreads) {
+        const int32_t s0 = job.seeds[i];
+        const double sc = job.seed_cost[i];
+        if (s0 < 0 || s0 >= N || !(sc >= 0.0)) {
+          sm.res[1] = 1;
+          continue;
+        }
+        const unsigned long long was = atomicExch(reinterpret_cast<unsigned long long*>(&w.mseed[s0]),
+                                                  (unsigned long long)__double_as_longlong(sc));
+        if (was != kNoTerm) {
+          sm.res[1] = 1;
+          continue;
+        }
+        const float pen = __ldcg(&w.rec[s0].pen);
+        w.claim[s0] = pr.sid;
+        const int32_t f0 = indptr[s0], flags = kSeed | (__ldcg(&w.rec[s0].sp) & kTgt);
+        w.rec[s0].sp = 1 | flags;
+        w.ov[0][atomicAdd(&sm.res[0], 1)] = make_int4(s0, f0, (indptr[s0 + 1] - f0) | flags, __float_as_int(pen));
+        unsigned long long lb = ogr_dbits(sc + (double)pen);
+        if (in_ticks) {
+          lb = 0ull;
+          if (seed_ticks(sc, &lb) && tick_finite(pen)) lb += ticks(pen);
+        }
+        atomicMin(&sm.wmin[0], lb);
       }
-      if (leader && attempt == 0) t_loop = gtimer();
-    };
+    }
     __syncthreads();
     if (tid == 0) {
-      unsigned long long t0 = kNone;
-      int nf0 = 0;
-      sm.ok = 1;
-      // The records are written and the longest row is known (it travels in
-      // the word's maximum).  Several seeds may settle in one phase, each the
-      // other's neighbour, so only now are their records marked reached.
-      for (int i = 1; i < kWarps; ++i) md = max(md, (int)sm.wmin[i]);
-      if (leader && attempt) clear_slot(pr, k0 + 2);   // the last two barriers' words are used ones
-      arrive(pr, sm, k0, kArrive, ~(unsigned long long)md);
-      await(pr, sm, k0);
-      sm.res[2] = (int)sm.t;
-      if (leader && attempt) clear_slot(pr, k0 + 3);
-      if (leader && !kMulti) {
-        w.claim[src] = pr.sid;
-        w.ov[0][0] = make_int4(src, indptr[src], indptr[src + 1] - indptr[src], __float_as_int(0.0f));
-        nf0 = 1;
-        t0 = 0ull;
-      }
-      if (kMulti) {
-        sm.res[0] = 0;             // first entries
-        sm.res[1] = 0;             // a bad or repeated seed or target
-        sm.wmin[0] = kNone;        // their least label
+      if (leader) ctl->merr = sm.res[1];
+      enter(leader && !sm.res[1] ? sm.res[0] : 0, leader ? sm.wmin[0] : kNone);
+      if (sm.ok && __ldcg(&ctl->merr)) sm.ok = 2;
+    }
+  }
+  __syncthreads();
+  const int ok = sm.ok, max_deg = sm.res[2];
+  __syncthreads();
+  int k0 = 2;                  // barriers used so far
+  if (max_deg > kMaxRow) fix = false;
+  if (ok != 1) {
+    o.status = ok == 0 ? OGR_ERR_TIMEOUT : OGR_ERR_ARG;
+  } else {
+    // (as a loop of two turns: with the second one plainly behind the first the
+    // search in ticks is 1 to 2 % slower, by how the compiler places it)
+    for (int attempt = 0; attempt < 2; ++attempt) {
+      if (attempt == 0) {
+        o = run_search<L, K, kMulti, false>(pr, smem_raw, 1, max_deg, fix);
+        k0 = 1 + o.phases;
+        if (o.status != kStInexact) break;
       } else {
-        enter(nf0, t0);
+        const Problem p = pr;
+        Outcome io = o;
+        int k = k0;
+        go_over<kMulti, false>(&p, smem_raw, &k, gtid, gthreads, &io);
+        o = io;
+        k0 = k;
+        fix = false;
       }
     }
-    if constexpr (kMulti) {
-      // CTA 0 marks the targets, then puts every seed in the first frontier
-      // with its label seed cost + penalty (of a redone search they are marked)
-      __syncthreads();
-      const bool mine = blockIdx.x == 0 && sm.ok;
-      const bool in_ticks = fix && sm.res[2] <= kMaxRow;
-      if (mine) {
-        for (int i = tid; i < job.n_targets; i += kThreads) {
-          const int32_t t = job.targets[i];
-          const double tc = job.target_cost[i];
-          if (t < 0 || t >= N || tc != tc) {
-            sm.res[1] = 1;
-            continue;
-          }
-          const unsigned long long was = atomicExch(reinterpret_cast<unsigned long long*>(&w.mtgt[t]),
-                                                    (unsigned long long)__double_as_longlong(tc));
-          if (attempt == 0 && was != kNoTerm) sm.res[1] = 1;
-          w.rec[t].sp = kTgt;
-        }
-      }
-      __syncthreads();
-      if (mine) {
-        for (int i = tid; i < job.n_seeds; i += kThreads) {
-          const int32_t s0 = job.seeds[i];
-          const double sc = job.seed_cost[i];
-          if (s0 < 0 || s0 >= N || !(sc >= 0.0)) {
-            sm.res[1] = 1;
-            continue;
-          }
-          const unsigned long long was = atomicExch(reinterpret_cast<unsigned long long*>(&w.mseed[s0]),
-                                                    (unsigned long long)__double_as_longlong(sc));
-          if (attempt == 0 && was != kNoTerm) {
-            sm.res[1] = 1;
-            continue;
-          }
-          const float pen = __ldcg(&w.rec[s0].pen);
-          w.claim[s0] = pr.sid;
-          const int32_t f0 = indptr[s0], flags = kSeed | (__ldcg(&w.rec[s0].sp) & kTgt);
-          w.rec[s0].sp = 1 | flags;
-          w.ov[0][atomicAdd(&sm.res[0], 1)] = make_int4(s0, f0, (indptr[s0 + 1] - f0) | flags, __float_as_int(pen));
-          unsigned long long lb = ogr_dbits(sc + (double)pen);
-          if (in_ticks) {
-            lb = 0ull;
-            if (seed_ticks(sc, &lb) && tick_finite(pen)) lb += ticks(pen);
-          }
-          atomicMin(&sm.wmin[0], lb);
-        }
-      }
-      __syncthreads();
-      if (tid == 0) {
-        if (leader) ctl->merr = sm.res[1];
-        enter(leader && !sm.res[1] ? sm.res[0] : 0, leader ? sm.wmin[0] : kNone);
-        if (sm.ok && __ldcg(&ctl->merr)) sm.ok = 2;
-      }
-    }
-    __syncthreads();
-    const int ok = sm.ok, max_deg = sm.res[2];
-    __syncthreads();
-    ++k0;
-    if (max_deg > kMaxRow) fix = false;
-    if (ok != 1) {
-      o.status = ok == 0 ? OGR_ERR_TIMEOUT : OGR_ERR_ARG;
-      o.phases = 0;
-      k0 += 1;
-      break;
-    }
-    o = run_search<L, K, kMulti, false>(pr, smem_raw, k0, max_deg, fix);
-    k0 += o.phases;
-    if (o.status != kStInexact) break;
-    fix = false;
-    __syncthreads();
   }
   unsigned long long t_done = 0;
   if (leader) t_done = gtimer();
@@ -415,7 +421,7 @@ full_sssp_kernel(ogr_graph g, ogr_state st, ogr_full::Job job, FWs w) {
   ctl->res[0] = status;
   ctl->res[1] = len;
   ctl->res[2] = o.phases;
-  ctl->sid = pr.sid;
+  ctl->sid = fix || max_deg > kMaxRow ? sid : sid + 1;      // (one that went over to doubles took two)
   const unsigned long long t_end = gtimer();
   const unsigned long long clocks = (unsigned long long)(o.clocks > 0 ? o.clocks : 1);
   const unsigned long long wait = (unsigned long long)((double)(t_done - t_loop) * ((double)o.wait / (double)clocks));

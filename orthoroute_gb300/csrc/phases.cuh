@@ -43,7 +43,8 @@
 //   fell from 13.9 to 9.3 us a phase, 1000x800x32 from 46 to 28).  Ticks
 //   are exact wherever the doubles are: costs and penalties of 2^-7 or more
 //   (or 0) are multiples of 2^-30, and below 2^22 their double sums do not
-//   round.  A search that meets any other value is redone in doubles.
+//   round.  A search that meets any other value goes on in doubles from the
+//   phase in which it did (go_over).
 // * A CTA with more entries than its share sends new ones to a list in global
 //   memory that the next phase deals over the team (see plan()).
 #pragma once
@@ -77,13 +78,15 @@ constexpr unsigned long long kArriveMask = 0x3ffull;
 constexpr unsigned kOutMask = 0x1fffff, kMostOut = 2047;
 constexpr int kMostEntries = 1 << 14;        // (with rows of up to 32 arcs they ask for fewer than 2^20 places)
 constexpr int kMaxTeam = 1023;      // CTAs of a team
-constexpr int kStInexact = 100;    // Outcome::status: redo in doubles
+constexpr int kStInexact = 100;    // Outcome::status: to go on in doubles (go_over)
+constexpr int kFirstOver = 6;      // first phase of a search that does (a multiple of 2 and of 3)
 
 // Control words of a team in global memory, zero before a search.
 struct Ctl {
   alignas(128) Slot slot[4];
   alignas(128) int32_t err;        // a CTA gave up waiting
   alignas(128) int32_t nov[3];     // surplus entries by phase mod 3
+  int32_t kept;                    // frontier of a search that goes over to doubles
 };
 
 constexpr int32_t kTgt = 1 << 30, kSeed = 1 << 29, kSpMask = kSeed - 1;
@@ -174,7 +177,7 @@ struct Outcome {
   int status;                      // OGR_OK with found, OGR_NO_PATH, or an error
   bool found;                      // single source: dst settled; multi-source: frontier exhausted
   bool exhausted;                  // the frontier ran out before dst
-  int phases;
+  int phases;                      // (kStInexact: the last two are the phase to be taken back, and the look at its end)
   unsigned long long ld;           // label of dst (as in Rec)
   unsigned long long examined;     // entries this CTA examined
   long long wait, clocks;          // clocks thread 0 spent waiting, and in all
@@ -203,6 +206,7 @@ struct Head {
   // reads them; in registers of all threads they were spilled)
   unsigned spin;
   int max_phase;
+  int first;                       // general form: the first phase, 0 or kFirstOver
 };
 
 template <int A>
@@ -376,7 +380,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
       if (deal && avg < (float)(kGroups / 8)) room = n > kGroups / 4 ? 0.0f : 1e6f;
     }
     head += nf;
-    sm.plan.T = T;
+    if (kGen || verdict != kInexactSeen) sm.plan.T = T;     // (else that of the phase to be taken back)
     sm.plan.verdict = verdict;
     sm.plan.nloc = nf + nk;
     sm.plan.ncarr = nk;
@@ -390,11 +394,11 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
     sm.nov_out = 0;
     sm.dst_hit = 0;
     sm.inexact = 0;
-    plan(0, 0, 0, 0, 0.0f, sm.a, sm.t);
+    plan(kGen ? sm.first : 0, 0, 0, 0, 0.0f, sm.a, sm.t);
   }
   __syncthreads();
   const long long c_start = clock64();
-  int phase = 0, b3 = 0;           // b3 = phase mod 3
+  int phase = kGen ? sm.first : 0, b3 = 0;           // b3 = phase mod 3
   int verdict;
   while ((verdict = sm.plan.verdict) == kGo) {
     const u64 T = sm.plan.T;
@@ -775,7 +779,7 @@ __device__ __forceinline__ Outcome run_phases(const Problem& pr, Head& sm, Body<
   out.found = verdict == kFound || verdict == kFoundEarly;
   out.exhausted = verdict == kEmpty;
   // a search that stops on dst did no work in its last phase
-  out.phases = verdict == kFoundEarly || verdict == kTimedOut ? phase : phase + 1;
+  out.phases = (verdict == kFoundEarly || verdict == kTimedOut ? phase : phase + 1) - (kGen ? sm.first : 0);
   out.clocks = clock64() - c_start;
   out.ld = sm.ld;
   return out;
@@ -787,7 +791,7 @@ __device__ __noinline__ void run_rare(const Problem* ppr, char* smem, int k0, Ou
   const Problem pr = *ppr;
   Head& sm = *reinterpret_cast<Head*>(smem);
   Body<L * K>& bd = *reinterpret_cast<Body<L * K>*>(smem + kHeadBytes);
-  *out = run_phases<L, K, kGen, kMulti, kRoi>(pr, sm, bd, k0);
+  *out = run_phases<L, K, kGen, kMulti, kRoi>(pr, sm, bd, kGen ? k0 - sm.first : k0);
 }
 
 // The longest row that is searched in ticks.
@@ -813,6 +817,95 @@ __device__ __forceinline__ Outcome run_search(const Problem& pr, char* smem, int
   else
     run_rare<32, 1, false, kMulti, kRoi>(&p, smem, k0, &o);
   return o;
+}
+
+// A search that met a value ticks cannot hold (out: its outcome, k0: barriers
+// it has used) goes on in doubles from the start of phase p, in which it did:
+// what settled before stays settled, its label converted (exact, being below
+// 2^52 ticks).  The frontier at p is entered in surplus list 0: what p settled,
+// the seeds, and every reached node with a neighbour settled before p that
+// relaxes it.  A node that only p reached is unreached again, for its neighbour
+// may not settle in doubles.  (Other CTAs convert at the same time; the test of
+// a neighbour says the same before and after.)  This CTA's nodes are first,
+// first + step, ....  Uses claim stamp sid + 1; *k0 is brought up to date.
+//
+// Out of line, and called once, so that the search in ticks keeps its
+// registers.  Two long searches of 600x400x12 whose labels pass 2^22 late took
+// 16.6 ms begun anew in doubles, and 9.9 this way.
+template <bool kMulti, bool kRoi>
+__device__ __noinline__ void go_over(const Problem* ppr, char* smem, int* k0, int64_t first, int64_t step, Outcome* out) {
+  Problem pr = *ppr;
+  Head& sm = *reinterpret_cast<Head*>(smem);
+  const int tid = threadIdx.x;
+  const bool leader = pr.rank == 0 && tid == 0;
+  const int p = out->phases - 2, b = *k0;
+  const unsigned long long T = sm.plan.T;
+  pr.sid += 1;
+  for (int64_t i = first; i < pr.R; i += step) {
+    const Rec x = ld_rec(&pr.rec[i]);
+    const int32_t s = kMulti ? x.sp & kSpMask : x.sp, flags = kMulti ? x.sp & ~kSpMask : 0;
+    if (s == 0) continue;
+    if (s >= 2 && s - 2 < p) {
+      st_rec(&pr.rec[i], ogr_dbits(label_value<true>(x.lab)), 2 | flags, x.pen);
+      continue;
+    }
+    const int32_t g = kRoi ? pr.roi[i] : (int32_t)i, f0 = pr.indptr[g], f1 = pr.indptr[g + 1];
+    bool in = s >= 2 || (flags & kSeed);
+    for (int32_t e = f0; e < f1 && !in; ++e) {
+      const int32_t u = kRoi ? pr.g2r[pr.indices[e]] : pr.indices[e];
+      if (u < 0) continue;
+      const int32_t sp = __ldcg(&pr.rec[u].sp), su = kMulti ? sp & kSpMask : sp;
+      in = su >= 2 && su - 2 < p && !(kMulti && (sp & kTgt)) &&
+           (pr.rcost ? pr.rcost[e] : pr.cost[pr.rev[e]]) < __int_as_float(0x7f800000);
+    }
+    __stcg(reinterpret_cast<int4*>(&pr.rec[i]), make_int4(f0, f1 - f0, (in ? 1 : 0) | flags, __float_as_int(x.pen)));
+    if (in) {
+      pr.claim[i] = pr.sid;
+      __stcg(&pr.ov[0][atomicAdd(&pr.ctl->kept, 1)], make_int4((int)i, f0, (f1 - f0) | flags, __float_as_int(x.pen)));
+    }
+  }
+  __syncthreads();
+  if (tid == 0) {
+    sm.ok = 1;
+    sm.first = kFirstOver;
+    sm.max_phase = max(sm.max_phase - p, 0) + kFirstOver;
+    if (leader) clear_slot(pr, b + 2);       // the last two barriers' words are used ones
+    arrive(pr, sm, b, kArrive, kNone);
+    await(pr, sm, b);
+    unsigned long long a = kArrive, t = kNone;
+    if (leader) {
+      clear_slot(pr, b + 3);
+      const int n = __ldcg(&pr.ctl->kept);
+      pr.ctl->nov[0] = n;
+      pr.ctl->nov[1] = 0;
+      pr.ctl->nov[2] = 0;
+      if (!kMulti && __ldcg(&pr.rec[pr.dst].sp) >= 2) a += kDst;
+      a += kOut * (unsigned long long)(n < (int)kMostOut ? n : (int)kMostOut) + kCount * (unsigned long long)n;
+      // T of phase p bounds its labels; above 2^53 their two sums may have rounded
+      t = ogr_dbits((double)(T > kTickLimit ? (T - 16) & ~15ull : T) * (1.0 / 1073741824.0));
+    }
+    if (sm.ok) {
+      arrive(pr, sm, b + 1, a, t);
+      await(pr, sm, b + 1);
+    }
+  }
+  __syncthreads();
+  const int ok = sm.ok;
+  __syncthreads();
+  if (!ok) {
+    out->status = OGR_ERR_TIMEOUT;
+    out->found = out->exhausted = false;
+    *k0 = b + 2;
+    return;
+  }
+  const unsigned long long examined = out->examined;
+  const long long wait = out->wait, clocks = out->clocks;
+  run_rare<16, 1, true, kMulti, kRoi>(&pr, smem, b + 1, out);
+  *k0 = b + 1 + out->phases;
+  out->phases += p;
+  out->examined += examined;
+  out->wait += wait;
+  out->clocks += clocks;
 }
 
 // Statistics of a finished search, added by this CTA for the nodes first,

@@ -191,7 +191,7 @@ __host__ __device__ inline BfsSlot bfs_slot_at(char* base, int32_t N, int64_t qc
 // + backtrace, [8] cleanup, [9] searches, [10] phases, [11] BFS
 // waves run, [12] ROI nodes, [13] entries examined, [14] ROIs taken from the
 // batched extraction, [15] searches that left the form of their kernel (longer
-// rows, or values redone in doubles).
+// rows, or values that ticks cannot hold).
 __device__ unsigned long long g_stage[16];
 
 struct Shared {
@@ -894,6 +894,7 @@ __device__ __noinline__ void roi_search(const RoiJob* jp, char* smem, int* statu
   if (tid == 0) {
     sm.spin = w.spin;
     sm.max_phase = w.max_phases > 0 ? min(w.max_phases, 2 * R + 4) : 2 * R + 4;
+    sm.first = 0;
   }
   // With statistics requested the search goes on after dst is settled until
   // every node with a label <= L(dst) is settled (T > L(dst)): the IN bound
@@ -901,139 +902,140 @@ __device__ __noinline__ void roi_search(const RoiJob* jp, char* smem, int* statu
   pr.want_stats = job.stats != nullptr;
   Outcome o{};
   bool fix = true;
-  int k0 = 0;
-  for (int attempt = 0; attempt < 2; ++attempt) {
-    pr.sid = sid + attempt;
-    int md = 0;
-    for (int r = first; r < R; r += step) {
-      const int32_t gid = full ? r : roi[r];
-      if (full) roi_w[r] = r;
-      w.g2r[gid] = r;
-      const int32_t f0 = g.indptr[gid], f1 = g.indptr[gid + 1];
-      md = max(md, f1 - f0);
-      const float pen = job.roi_pen ? job.roi_pen[r] : ogr_node_penalty(st, a, gid);
-      __stcg(reinterpret_cast<int4*>(&w.rec[r]), make_int4(f0, f1 - f0, 0, __float_as_int(pen)));
-      if (kMulti) {
-        job.ms->init[r] = __longlong_as_double((long long)kNoTerm);
-        job.ms->tcost[r] = __longlong_as_double((long long)kNoTerm);
-      }
+  pr.sid = sid;
+  int md = 0;
+  for (int r = first; r < R; r += step) {
+    const int32_t gid = full ? r : roi[r];
+    if (full) roi_w[r] = r;
+    w.g2r[gid] = r;
+    const int32_t f0 = g.indptr[gid], f1 = g.indptr[gid + 1];
+    md = max(md, f1 - f0);
+    const float pen = job.roi_pen ? job.roi_pen[r] : ogr_node_penalty(st, a, gid);
+    __stcg(reinterpret_cast<int4*>(&w.rec[r]), make_int4(f0, f1 - f0, 0, __float_as_int(pen)));
+    if (kMulti) {
+      job.ms->init[r] = __longlong_as_double((long long)kNoTerm);
+      job.ms->tcost[r] = __longlong_as_double((long long)kNoTerm);
     }
-    md = __reduce_max_sync(0xffffffffu, md);
-    if ((tid & 31) == 0) sm.wmin[tid >> 5] = (unsigned long long)md;
-    __syncthreads();
-    if (tid == 0) {
-      sm.ok = 1;
-      for (int i = 1; i < kWarps; ++i) md = max(md, (int)sm.wmin[i]);
-      if (leader && attempt) clear_slot(pr, k0 + 2);   // the last two barriers' words are used ones
-      arrive(pr, sm, k0, kArrive, ~(unsigned long long)md);
-      await(pr, sm, k0);
-      sm.res[2] = (int)sm.t;
-      if (leader && attempt) clear_slot(pr, k0 + 3);
-      sm.res[0] = 0;               // first entries
-      sm.res[1] = 0;               // bad seeds or targets
-      sm.wmin[0] = kNone;          // their least label
-    }
-    __syncthreads();
-    const int max_deg = sm.res[2];
-    const int ready = sm.ok;
-    if (max_deg > kMaxRow) fix = false;
-    if (leader && (attempt == 0) == (max_deg > L * K)) atomicAdd(&g_stage[15], 1ull);
-    int32_t rs = -1, rd = -1;
-    if (!kMulti && ready) {
-      rs = __ldcg(&w.g2r[a.src]);
-      rd = __ldcg(&w.g2r[a.dst]);
-    }
-    const bool none = !kMulti && (rs < 0 || rd < 0 || rs == rd);
-    pr.src = rs;
-    pr.dst = rd;
-    auto enter = [&](int32_t r, int at, int32_t flags) {
-      const int32_t gid = roi[r], f0 = g.indptr[gid];
-      w.claim[r] = pr.sid;
-      w.ov[0][at] = make_int4(r, f0, (g.indptr[gid + 1] - f0) | flags, __float_as_int(__ldcg(&w.rec[r].pen)));
-    };
-    if (ready && job.rank == 0) {
-      if constexpr (kMulti) {
-        // Seeds and targets outside the ROI are dropped (as the reference
-        // does); a repeated seed or target id is an argument error.
-        const MultiSeeds& ms = *job.ms;
-        for (int i = tid; i < ms.ntargets; i += kThreads) {
-          const int32_t gid = ms.targets[i];
-          const int32_t r = gid < 0 || gid >= g.num_nodes ? -2 : w.g2r[gid];
-          if (r < 0) {
-            if (r == -2) sm.res[1] = 1;
-            continue;
-          }
-          const double c = ms.target_cost[i];
-          const unsigned long long was = atomicExch(reinterpret_cast<unsigned long long*>(&ms.tcost[r]),
-                                                    (unsigned long long)__double_as_longlong(c));
-          if (was != kNoTerm) sm.res[1] = 1;
-          // (a target cost that is not a number marks no target)
-          if (c == c) w.rec[r].sp = kTgt;
+  }
+  md = __reduce_max_sync(0xffffffffu, md);
+  if ((tid & 31) == 0) sm.wmin[tid >> 5] = (unsigned long long)md;
+  __syncthreads();
+  if (tid == 0) {
+    sm.ok = 1;
+    for (int i = 1; i < kWarps; ++i) md = max(md, (int)sm.wmin[i]);
+    arrive(pr, sm, 0, kArrive, ~(unsigned long long)md);
+    await(pr, sm, 0);
+    sm.res[2] = (int)sm.t;
+    sm.res[0] = 0;               // first entries
+    sm.res[1] = 0;               // bad seeds or targets
+    sm.wmin[0] = kNone;          // their least label
+  }
+  __syncthreads();
+  const int max_deg = sm.res[2];
+  const int ready = sm.ok;
+  if (max_deg > kMaxRow) fix = false;
+  if (leader && max_deg > L * K) atomicAdd(&g_stage[15], 1ull);
+  int32_t rs = -1, rd = -1;
+  if (!kMulti && ready) {
+    rs = __ldcg(&w.g2r[a.src]);
+    rd = __ldcg(&w.g2r[a.dst]);
+  }
+  const bool none = !kMulti && (rs < 0 || rd < 0 || rs == rd);
+  pr.src = rs;
+  pr.dst = rd;
+  auto enter = [&](int32_t r, int at, int32_t flags) {
+    const int32_t gid = roi[r], f0 = g.indptr[gid];
+    w.claim[r] = pr.sid;
+    w.ov[0][at] = make_int4(r, f0, (g.indptr[gid + 1] - f0) | flags, __float_as_int(__ldcg(&w.rec[r].pen)));
+  };
+  if (ready && job.rank == 0) {
+    if constexpr (kMulti) {
+      // Seeds and targets outside the ROI are dropped (as the reference
+      // does); a repeated seed or target id is an argument error.
+      const MultiSeeds& ms = *job.ms;
+      for (int i = tid; i < ms.ntargets; i += kThreads) {
+        const int32_t gid = ms.targets[i];
+        const int32_t r = gid < 0 || gid >= g.num_nodes ? -2 : w.g2r[gid];
+        if (r < 0) {
+          if (r == -2) sm.res[1] = 1;
+          continue;
         }
-        __syncthreads();
-        for (int i = tid; i < ms.nseeds; i += kThreads) {
-          const int32_t gid = ms.seeds[i];
-          const int32_t r = gid < 0 || gid >= g.num_nodes ? -2 : w.g2r[gid];
-          if (r < 0) {
-            if (r == -2) sm.res[1] = 1;
-            continue;
-          }
-          const double c = ms.seed_cost[i];
-          const unsigned long long was = atomicExch(reinterpret_cast<unsigned long long*>(&ms.init[r]),
-                                                    (unsigned long long)__double_as_longlong(c));
-          if (was != kNoTerm) {
-            sm.res[1] = 1;
-            continue;
-          }
-          if (!(c < __longlong_as_double(0x7ff0000000000000ll))) continue;      // not a start
-          const float pen = __ldcg(&w.rec[r].pen);
-          unsigned long long lb = ogr_dbits(c + (double)pen);
-          if (fix) {
-            lb = 0ull;
-            if (seed_ticks(c, &lb) && tick_finite(pen)) lb += ticks(pen);
-          }
-          const int32_t flags = kSeed | (__ldcg(&w.rec[r].sp) & kTgt);
-          enter(r, atomicAdd(&sm.res[0], 1), flags);
-          w.rec[r].sp = 1 | flags;
-          atomicMin(&sm.wmin[0], lb);
+        const double c = ms.target_cost[i];
+        const unsigned long long was = atomicExch(reinterpret_cast<unsigned long long*>(&ms.tcost[r]),
+                                                  (unsigned long long)__double_as_longlong(c));
+        if (was != kNoTerm) sm.res[1] = 1;
+        // (a target cost that is not a number marks no target)
+        if (c == c) w.rec[r].sp = kTgt;
+      }
+      __syncthreads();
+      for (int i = tid; i < ms.nseeds; i += kThreads) {
+        const int32_t gid = ms.seeds[i];
+        const int32_t r = gid < 0 || gid >= g.num_nodes ? -2 : w.g2r[gid];
+        if (r < 0) {
+          if (r == -2) sm.res[1] = 1;
+          continue;
         }
-      } else if (tid == 0 && !none) {
-        enter(rs, 0, 0);
-        w.ov[0][0].w = 0;          // src's penalty does not count
-        sm.res[0] = 1;
-        sm.wmin[0] = 0ull;
+        const double c = ms.seed_cost[i];
+        const unsigned long long was = atomicExch(reinterpret_cast<unsigned long long*>(&ms.init[r]),
+                                                  (unsigned long long)__double_as_longlong(c));
+        if (was != kNoTerm) {
+          sm.res[1] = 1;
+          continue;
+        }
+        if (!(c < __longlong_as_double(0x7ff0000000000000ll))) continue;      // not a start
+        const float pen = __ldcg(&w.rec[r].pen);
+        unsigned long long lb = ogr_dbits(c + (double)pen);
+        if (fix) {
+          lb = 0ull;
+          if (seed_ticks(c, &lb) && tick_finite(pen)) lb += ticks(pen);
+        }
+        const int32_t flags = kSeed | (__ldcg(&w.rec[r].sp) & kTgt);
+        enter(r, atomicAdd(&sm.res[0], 1), flags);
+        w.rec[r].sp = 1 | flags;
+        atomicMin(&sm.wmin[0], lb);
       }
+    } else if (tid == 0 && !none) {
+      enter(rs, 0, 0);
+      w.ov[0][0].w = 0;          // src's penalty does not count
+      sm.res[0] = 1;
+      sm.wmin[0] = 0ull;
     }
-    __syncthreads();
-    if (tid == 0 && ready) {
-      unsigned long long nf0 = 0, tl = kNone;
-      if (job.rank == 0) {
-        nf0 = sm.res[1] ? 0 : (unsigned)sm.res[0];
-        tl = sm.wmin[0];
-        w.ctl->merr = sm.res[1];
-        w.ctl->team.nov[0] = (int)nf0;
-        w.ctl->team.nov[1] = 0;
-        w.ctl->team.nov[2] = 0;
-      }
-      arrive(pr, sm, k0 + 1, kArrive + kOut * (nf0 < kMostOut ? nf0 : kMostOut) + kCount * nf0, tl);
-      await(pr, sm, k0 + 1);
-      if (kMulti && sm.ok && __ldcg(&w.ctl->merr)) sm.ok = 2;
+  }
+  __syncthreads();
+  if (tid == 0 && ready) {
+    unsigned long long nf0 = 0, tl = kNone;
+    if (job.rank == 0) {
+      nf0 = sm.res[1] ? 0 : (unsigned)sm.res[0];
+      tl = sm.wmin[0];
+      w.ctl->merr = sm.res[1];
+      w.ctl->team.nov[0] = (int)nf0;
+      w.ctl->team.nov[1] = 0;
+      w.ctl->team.nov[2] = 0;
     }
-    __syncthreads();
-    const int ok = sm.ok;
-    __syncthreads();
-    if (attempt == 0) mark(2);
-    ++k0;
-    if (ok != 1 || none) {
-      o.status = ok == 0 ? OGR_ERR_TIMEOUT : ok == 2 ? OGR_ERR_ARG : OGR_NO_PATH;
-      ++k0;
-      break;
+    arrive(pr, sm, 1, kArrive + kOut * (nf0 < kMostOut ? nf0 : kMostOut) + kCount * nf0, tl);
+    await(pr, sm, 1);
+    if (kMulti && sm.ok && __ldcg(&w.ctl->merr)) sm.ok = 2;
+  }
+  __syncthreads();
+  const int ok = sm.ok;
+  __syncthreads();
+  mark(2);
+  int k0 = 2;                  // barriers used so far
+  if (ok != 1 || none) {
+    o.status = ok == 0 ? OGR_ERR_TIMEOUT : ok == 2 ? OGR_ERR_ARG : OGR_NO_PATH;
+  } else {
+    o = run_search<L, K, kMulti, true>(pr, smem, 1, max_deg, fix);
+    k0 = 1 + o.phases;
+    if (o.status == kStInexact) {
+      if (leader && max_deg <= L * K) atomicAdd(&g_stage[15], 1ull);
+      const Problem p = pr;
+      Outcome io = o;
+      int k = k0;
+      go_over<kMulti, true>(&p, smem, &k, first, step, &io);
+      o = io;
+      k0 = k;
+      fix = false;
     }
-    o = run_search<L, K, kMulti, true>(pr, smem, k0, max_deg, fix);
-    k0 += o.phases;
-    if (o.status != kStInexact) break;
-    fix = false;
-    __syncthreads();
   }
   mark(3);
   if (leader) {
@@ -1120,7 +1122,7 @@ __device__ __noinline__ void roi_search(const RoiJob* jp, char* smem, int* statu
   }
   for (int r = first; r < R; r += step) w.g2r[roi[r]] = -1;
   if (leader) {
-    w.ctl->sid = pr.sid;
+    w.ctl->sid = fix || max_deg > kMaxRow ? sid : sid + 1;      // (one that went over to doubles took two)
     // (a CTA that gave up on the last wait left its part of the statistics out)
     if (*(const volatile int32_t*)&w.ctl->team.err) status = OGR_ERR_TIMEOUT;
   }
