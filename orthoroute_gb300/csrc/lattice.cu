@@ -32,6 +32,7 @@ struct LatDev {
   const int* pz;
   const float* pcost;
   const int* psite;
+  bool plain;          // every list ascends, each layer once, without its own
 };
 
 __device__ __forceinline__ bool site_ok(int mode, int x, int y) {
@@ -65,25 +66,6 @@ struct Axes {
   }
 };
 
-// Via partners of (x, y, z) below layer `upto`, in row order.
-__device__ __forceinline__ int partners_below(const LatDev& L, int x, int y, int z, int upto) {
-  int k = 0;
-  for (int p = L.h.pptr[z]; p < L.h.pptr[z + 1] && L.pz[p] < upto; ++p) k += site_ok(L.psite[p], x, y) ? 1 : 0;
-  return k;
-}
-
-// Place of partner `want` among the via partners of (x, y, z) below or at it;
-// -1 if (x, y, z) has no arc to that layer.
-__device__ __forceinline__ int partner_place(const LatDev& L, int x, int y, int z, int want) {
-  int k = 0;
-  for (int p = L.h.pptr[z]; p < L.h.pptr[z + 1] && L.pz[p] <= want; ++p) {
-    const bool ok = site_ok(L.psite[p], x, y);
-    if (L.pz[p] == want) return ok ? k : -1;
-    k += ok ? 1 : 0;
-  }
-  return -1;
-}
-
 // Lateral arcs of (x, y) on a layer with axes ax: all of them, or those that
 // come before the one to side (0: y-1, 1: x-1, 2: x+1, 3: y+1).
 __device__ __forceinline__ int laterals_before(const LatDev& L, const Axes& ax, int x, int y, int side) {
@@ -95,9 +77,46 @@ __device__ __forceinline__ int laterals_before(const LatDev& L, const Axes& ax, 
   return k;
 }
 
+// The row of (x, y, z): the via partners listed before the first that is not
+// below z, the laterals, the partners above z.  (A list that does not ascend,
+// repeats a layer or names z itself is read by the same rule everywhere; of a
+// plain one the rule asks for less: 222 us a build of 600x400x12 against 245.)
+__device__ __forceinline__ int partners_below(const LatDev& L, int x, int y, int z) {
+  int k = 0;
+  for (int p = L.h.pptr[z]; p < L.h.pptr[z + 1] && L.pz[p] < z; ++p) k += site_ok(L.psite[p], x, y) ? 1 : 0;
+  return k;
+}
+
 __device__ __forceinline__ int degree(const LatDev& L, int x, int y, int z) {
-  const Axes ax(L.h, z);
-  return partners_below(L, x, y, z, kMaxLayers) + laterals_before(L, ax, x, y, 4);
+  int k = laterals_before(L, Axes(L.h, z), x, y, 4);
+  bool below = true;
+  for (int p = L.h.pptr[z]; p < L.h.pptr[z + 1]; ++p) {
+    const int zz = L.pz[p];
+    below = below && zz < z;
+    if (L.plain || below || zz > z) k += site_ok(L.psite[p], x, y) ? 1 : 0;
+  }
+  return k;
+}
+
+// Place in the row of (x, y, z) of its first arc to layer `want`; -1: none.
+__device__ __forceinline__ int partner_place(const LatDev& L, int x, int y, int z, int want) {
+  int k = want > z ? laterals_before(L, Axes(L.h, z), x, y, 4) : 0;
+  bool below = true;
+  for (int p = L.h.pptr[z]; p < L.h.pptr[z + 1]; ++p) {
+    const int zz = L.pz[p];
+    const bool ok = site_ok(L.psite[p], x, y);
+    if (L.plain) {
+      if (zz >= want) return ok && zz == want ? k : -1;
+      k += ok ? 1 : 0;
+      continue;
+    }
+    below = below && zz < z;
+    if ((below || zz > z) && ok) {
+      if (zz == want) return k;
+      ++k;
+    }
+  }
+  return -1;
 }
 
 // Row starts: degrees and their sums within tiles of kScanTile nodes, the sum
@@ -214,14 +233,12 @@ __global__ void __launch_bounds__(kFillThreads) fill_kernel(LatDev L, int tile_n
         s_kind[k] = (unsigned char)via;
         ++k;
       };
-      // the arc back from a via partner zz: after its partners below z, and
-      // its laterals if zz < z (they come between)
       auto via = [&](int p, int zz) {
         const int32_t v = zz * plane + r;
         int32_t back = -1;
         if (rev) {
           back = partner_place(L, x, y, zz, z);
-          if (back >= 0) back += indptr[v] + (zz < z ? laterals_before(L, Axes(L.h, zz), x, y, 4) : 0);
+          if (back >= 0) back += indptr[v];
         }
         put(v, L.pcost[p], 1, back);
       };
@@ -233,7 +250,7 @@ __global__ void __launch_bounds__(kFillThreads) fill_kernel(LatDev L, int tile_n
       }
       // laterals: the arc back stands on the neighbour's other side
       auto lateral = [&](int dx, int dy, int32_t v, float c, int side) {
-        put(v, c, 0, rev ? indptr[v] + partners_below(L, x + dx, y + dy, z, z) +
+        put(v, c, 0, rev ? indptr[v] + partners_below(L, x + dx, y + dy, z) +
                                laterals_before(L, ax, x + dx, y + dy, side)
                          : -1);
       };
@@ -272,6 +289,10 @@ int load_desc(const ogr_lattice_desc* d, int* dev_tab, cudaStream_t s, LatDev* o
   for (int z = 0; z <= d->nz; ++z) h.pptr[z] = d->partner_ptr[z];
   const int np = d->partner_ptr[d->nz];
   if (np > kMaxPartners || np < 0) return OGR_ERR_ARG;
+  L.plain = true;
+  for (int z = 0; z < d->nz; ++z)
+    for (int p = h.pptr[z]; p < h.pptr[z + 1]; ++p)
+      L.plain = L.plain && d->partner_z[p] != z && (p == h.pptr[z] || d->partner_z[p] > d->partner_z[p - 1]);
   L.pz = dev_tab;
   L.pcost = nullptr;
   L.psite = nullptr;
@@ -354,12 +375,15 @@ extern "C" int ogr_csr_build(const ogr_lattice_desc* d, int32_t* indptr, int32_t
   scan_add<<<ogr_blocks(N + 1, 256), 256, 0, s>>>(indptr, N, tile_sums, total);
   OGR_LAUNCH_CHECK();
   // A tile's rows have to fit in shared memory: 17 bytes per arc, the layers'
-  // longest row times the tile's nodes (a multiple of 32), at most 48 KB.
+  // longest row times the tile's nodes, at most 48 KB (rows of up to 67 arcs,
+  // each layer's partners once: 36,448 bytes at 32 nodes); one row may take more.
   int row = 1;
   for (int z = 0; z < d->nz; ++z) row = std::max(row, d->partner_ptr[z + 1] - d->partner_ptr[z] + 4);
   int tile_nodes = kFillThreads;
-  while (tile_nodes > 32 && tile_nodes * row * 17 > 48 * 1024) tile_nodes -= 32;
-  const int cap = tile_nodes * row;          // rows of up to 67 arcs: 36,448 bytes at 32 nodes
+  while (tile_nodes > 1 && tile_nodes * row * 17 > 48 * 1024) tile_nodes -= tile_nodes > 32 ? 32 : (tile_nodes + 1) / 2;
+  const int cap = tile_nodes * row;
+  if (cap * 17 > 48 * 1024)
+    OGR_CUDA_TRY(cudaFuncSetAttribute((const void*)fill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, cap * 17));
   const int plane = d->nx * d->ny;
   const dim3 grid((unsigned)std::min((plane + tile_nodes - 1) / tile_nodes, 65535), (unsigned)d->nz);
   fill_kernel<<<grid, kFillThreads, (size_t)cap * 17, s>>>(L, tile_nodes, indptr, indices, base_costs, edge_layer,
