@@ -218,10 +218,11 @@ __global__ void __launch_bounds__(kFillThreads) fill_kernel(LatDev L, int tile_n
   const Axes ax(L.h, z);
   const Div by_nx((unsigned)nx);
   const int p0 = L.h.pptr[z], p1 = L.h.pptr[z + 1];
-  for (int32_t r0 = blockIdx.x * tile_nodes; r0 < plane; r0 += gridDim.x * tile_nodes) {
-    const int32_t r1 = min(plane, r0 + tile_nodes);
+  for (int64_t t0 = (int64_t)blockIdx.x * tile_nodes; t0 < plane; t0 += (int64_t)gridDim.x * tile_nodes) {
+    const int32_t r0 = (int32_t)t0, r1 = (int32_t)min((int64_t)plane, t0 + tile_nodes);
     const int32_t e0 = indptr[z * plane + r0], e1 = indptr[z * plane + r1];
-    for (int32_t r = r0 + threadIdx.x; r < r1; r += kFillThreads) {
+    for (int32_t i = threadIdx.x; i < r1 - r0; i += kFillThreads) {
+      const int32_t r = r0 + i;
       const int y = (int)by_nx((unsigned)r), x = r - y * nx;
       const int32_t n = z * plane + r;
       int k = indptr[n] - e0;
@@ -384,8 +385,8 @@ extern "C" int ogr_csr_build(const ogr_lattice_desc* d, int32_t* indptr, int32_t
   const int cap = tile_nodes * row;
   if (cap * 17 > 48 * 1024)
     OGR_CUDA_TRY(cudaFuncSetAttribute((const void*)fill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, cap * 17));
-  const int plane = d->nx * d->ny;
-  const dim3 grid((unsigned)std::min((plane + tile_nodes - 1) / tile_nodes, 65535), (unsigned)d->nz);
+  const int64_t plane = (int64_t)d->nx * d->ny;
+  const dim3 grid((unsigned)std::min<int64_t>((plane + tile_nodes - 1) / tile_nodes, 65535), (unsigned)d->nz);
   fill_kernel<<<grid, kFillThreads, (size_t)cap * 17, s>>>(L, tile_nodes, indptr, indices, base_costs, edge_layer,
                                                           edge_kind, edge_src, rev, cap);
   OGR_LAUNCH_CHECK();

@@ -42,7 +42,7 @@ def rows(nx, ny, nz, axis, partners, ww):
     return out
 
 
-def build(nx, ny, nz, axis, partners, ww):
+def build(nx, ny, nz, axis, partners, ww, device=False):
     from orthoroute_gb300 import _lib
     flat = [p for z in range(nz) for p in partners[z]]
     a = dict(axis=np.asarray(axis, np.uint8), ptr=np.cumsum([0] + [len(partners[z]) for z in range(nz)]).astype(np.int32),
@@ -61,7 +61,11 @@ def build(nx, ny, nz, axis, partners, ww):
     rc = lib.ogr_csr_build(C.byref(d), *(v.data_ptr() for v in out), ws.data_ptr(), nb,
                            torch.cuda.current_stream().cuda_stream)
     _lib.check(rc, "ogr_csr_build")
-    return [v.cpu().numpy() for v in out]
+    return out if device else [v.cpu().numpy() for v in out]
+
+
+def build_device(*a):
+    return build(*a, device=True)[0]
 
 
 F = lambda v: float(np.float32(v))
@@ -99,3 +103,11 @@ def test_csr_of_partner_lists(name, dims, ww):
     np.testing.assert_array_equal(lay[:n], [a[0] // (nx * ny) for a in flat])
     back = [next((int(ptr[v]) + j for j, b in enumerate(want[v]) if b[0] == u), -1) for u, v, _, _ in flat]
     np.testing.assert_array_equal(rev[:n], back)
+
+
+def test_a_layer_of_nearly_2_to_the_31_cells():
+    """Steps from tile to tile and from row to row pass 2^31 behind the last ones: one layer without arcs (8.6 GB of row
+    starts, all 0)."""
+    indptr = build_device(46_340, 46_341, 1, [0], [[]], -1.0)
+    assert indptr.numel() == 46_340 * 46_341 + 1
+    assert int(indptr.min()) == 0 and int(indptr.max()) == 0
