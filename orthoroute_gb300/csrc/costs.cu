@@ -21,7 +21,9 @@ __device__ __forceinline__ float arc_bias(const float* layer_bias, unsigned char
 // nearest even like __int2float_rn.  The rounded value is a whole number below
 // 2^32, so its float remainder is the integer one (fmodf held the cost update
 // at 99 us for 21 M arcs, above its memory time of 69).
+// Arcs from 2^31 on take the conversion of 64-bit numbers and fmodf.
 __device__ __forceinline__ float jitter(int64_t e) {
+  if (e > 0x7fffffff) return __fmul_rn(fmodf(__ll2float_rn(e), 9973.0f), 1e-6f);
   const unsigned fe = __float2uint_rz(__int2float_rn((int)e));
   return __fmul_rn((float)(fe % 9973u), 1e-6f);
 }
