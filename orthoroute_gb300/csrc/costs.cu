@@ -195,8 +195,8 @@ __device__ __forceinline__ unsigned long long ema_units(float eo, unsigned* bad)
   const int ex = (int)(b >> 23) - 127;
   const unsigned m = (b & 0x7fffffu) | 0x800000u;      // eo * 2^23 = m * 2^ex
   if (ex >= 0) {
-    if (ex > 39) *bad = 1;
-    return ex > 39 ? ~0ull : (unsigned long long)m << ex;
+    if (ex > 40) *bad = 1;                             // (m has 24 bits)
+    return ex > 40 ? ~0ull : (unsigned long long)m << ex;
   }
   if (ex < -23 || (m & ((1u << -ex) - 1u))) *bad = 1;
   return ex < -23 ? 0ull : m >> -ex;
