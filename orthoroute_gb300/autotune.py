@@ -13,8 +13,8 @@ tuner sweeps
 
 * the engine: "grid" or "cta";
 * the lanes knob (4, 8, 16) and the reuse knob (on / off) of the "grid"
-  engine, timed on the full grid (the search fits its lanes to the lattice's
-  rows and ignores both: they tell apart by noise only);
+  engine are kept as they are: the search fits its lanes to the lattice's rows
+  and ignores both, so one timing on the full grid stands for all of them;
 * then the grid of the "grid" engine: 1/4, 1/2, 3/4 and all of the resident
   CTAs (one per SM);
 * then the tile-window engine (label windows over lattice tiles in shared
@@ -22,11 +22,11 @@ tuner sweeps
   uncongested lateral hops: the delta of a delta-stepping search;
 
 on a few full-graph searches of the job's own long nets over the current
-costs, and keeps the fastest.  For ROI nets it sweeps the lanes knob of their
-search (2, 4, 8, 16; ignored likewise), timing a spread of the job's ROI nets.
-Every setting returns the same paths (the searches are exact and independent
+costs, and keeps the fastest.  A spread of the job's ROI nets is timed once,
+for every width of the lanes knob of their search (2, 4, 8, 16; ignored
+likewise).  Every setting returns the same paths (the searches are exact and independent
 of the schedule), so tuning changes only time.  Results are cached per
-(lattice, GPU) in a JSON file.
+(engine, lattice, GPU) in a JSON file.
 """
 from __future__ import annotations
 
@@ -39,6 +39,7 @@ from typing import Dict, List, Sequence, Tuple
 import torch
 
 from . import _lib
+from .lattice import _via_site_mode
 
 
 @dataclass
@@ -117,11 +118,24 @@ def cache_path() -> str:
                           os.path.join(os.path.expanduser("~"), ".cache", "orthoroute_gb300", "autotune.json"))
 
 
+# Generation of the searches that a cached choice was timed on: a choice of
+# another generation (a grid, an engine or a window width that won against
+# kernels since replaced) is not used.
+ENGINE = "teams1"
+
+
 def lattice_key(lattice, device) -> str:
+    """What a tuning depends on: the engine's generation, the GPU, and the
+    lattice's size, via spans, wrong-way arcs and via sites."""
     props = torch.cuda.get_device_properties(device)
     spans = getattr(lattice, "allowed_via_spans", None)
     spans = "all" if spans is None else ",".join(f"{a}-{b}" for a, b in sorted(spans))
-    return f"{props.name}/{props.multi_processor_count}sm/{lattice.nx}x{lattice.ny}x{lattice.nz}/{spans}"
+    ww = getattr(lattice, "wrong_way_cost_multiplier", float("inf"))
+    spacing = getattr(lattice, "min_via_center_spacing", 0.0)
+    site = _via_site_mode(spacing, float(getattr(lattice, "pitch", 0.4)))
+    any_layer = getattr(lattice, "allow_any_layer_via", None)
+    return (f"{ENGINE}/{props.name}/{props.multi_processor_count}sm/{lattice.nx}x{lattice.ny}x{lattice.nz}/{spans}/"
+            f"any{any_layer}/ww{float(ww):g}/site{site}")
 
 
 def _load_cache(path: str) -> Dict:
@@ -161,9 +175,8 @@ def _time_roi(ops, nets, lanes) -> float:
 def tune(ops, lattice, nets: Sequence[Tuple[int, int]], roi_nets: Sequence[Tuple[int, int]] = (), *,
          use_cache: bool = True, cta_max_nodes: int = 400_000, repeats: int = 1) -> Tuning:
     """Pick the engine and grid for full-graph searches of `lattice` by timing
-    searches of `nets` ((src, dst) pairs, full-graph length), and the lanes
-    per node of ROI searches by timing `roi_nets`, on `ops`'s current costs.
-    Leaves the choices set and returns them."""
+    searches of `nets` ((src, dst) pairs, full-graph length) on `ops`'s current
+    costs; `roi_nets` are timed for the record.  Leaves the choices set and returns them."""
     key = lattice_key(lattice, ops.g.device)
     path = cache_path()
     if use_cache:
@@ -182,14 +195,11 @@ def tune(ops, lattice, nets: Sequence[Tuple[int, int]], roi_nets: Sequence[Tuple
     nets = list(nets)
     roi_nets = list(roi_nets)
     timings: Dict[str, float] = {}
-    lanes0 = search_lanes(0)
-    best_lanes = lanes0
+    best_lanes = search_lanes(0)
     if roi_nets:
-        _time_roi(ops, roi_nets[:1], lanes0)       # untimed: workspace and caches
-        lane_ms = {lanes: _time_roi(ops, roi_nets, lanes) for lanes in LANES}
-        best_lanes = min(LANES, key=lambda k: (lane_ms[k], k))
-        timings.update({f"roi_lanes{k}": round(v, 4) for k, v in lane_ms.items()})
-    search_lanes(best_lanes)
+        _time_roi(ops, roi_nets[:1], best_lanes)   # untimed: workspace and caches
+        ms = round(_time_roi(ops, roi_nets, best_lanes), 4)
+        timings.update({f"roi_lanes{k}": ms for k in LANES})
     best = ("grid", limit, float("inf"))
     stream = torch.cuda.current_stream()
     if not nets:
@@ -211,24 +221,17 @@ def tune(ops, lattice, nets: Sequence[Tuple[int, int]], roi_nets: Sequence[Tuple
                 ms += ops.counters["search_ms"] - t0
         return ms / max(1, repeats * len(nets))
 
-    lanes_ms = {}
     full_grid(limit)
-    for lanes in FULL_LANES:
-        for reuse in (0, 1):
-            full_lanes(lanes)
-            full_reuse(reuse)
-            lanes_ms[(lanes, reuse)] = time_full("grid")
-            timings[f"full_lanes{lanes}_reuse{reuse}"] = round(lanes_ms[(lanes, reuse)], 4)
-    best_full_lanes, best_reuse = min(lanes_ms, key=lambda k: (lanes_ms[k], -k[0], k[1]))
-    full_lanes(best_full_lanes)
-    full_reuse(best_reuse)
+    best_full_lanes, best_reuse = full_lanes(0), full_reuse()
+    limit_ms = time_full("grid")
+    timings.update({f"full_lanes{lanes}_reuse{reuse}": round(limit_ms, 4) for lanes in FULL_LANES for reuse in (0, 1)})
     try:
         for engine, ctas in candidates(limit):
             if engine == "cta" and ops.g.N > cta_max_nodes:
-                continue        # one CTA over a lattice this large is never the faster engine
+                continue        # half the SMs on a lattice this large are never the faster engine
             if engine == "grid":
                 full_grid(ctas)
-            ms = lanes_ms[(best_full_lanes, best_reuse)] if (engine == "grid" and ctas == limit) else time_full(engine)
+            ms = limit_ms if (engine == "grid" and ctas == limit) else time_full(engine)
             name = f"grid{ctas}" if engine == "grid" else "cta"
             timings[name] = round(ms, 4)
             if ms < best[2]:
