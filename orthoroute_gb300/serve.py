@@ -59,17 +59,22 @@ class JobResult:
 
 def job_footprint(nx: int, ny: int, nz: int, num_edges: int, num_nets: int, window_slots: int = 32,
                   max_roi_nodes: int = 50_000, slot_cap: int = 8192, bfs_slots: int = 64) -> int:
-    """HBM bytes of one job's device state (the allocations of a router):
-    CSR, congestion arrays, search workspaces, path store, ROI pool."""
+    """HBM bytes of one job's device state (the allocations of a router): CSR,
+    congestion arrays, search workspaces (as the library sizes them), path
+    store, ROI pool."""
+    from . import _lib
+    lib = _lib.load()
     N, E = nx * ny * nz, int(num_edges)
     R = min(max_roi_nodes, N)
     csr = 4 * (N + 1) + E * (4 + 4 + 1 + 1 + 4 + 4)
     state = E * 4 * 7 + N * 4 * 4 + 4 * nz
-    roi_ws = 72 * N + 2 * 4 * min(N, 65536) * 32 + 4 * min(N, 65536)
-    full_ws = 44 * N + 4 * E
+    roi_ws = int(lib.ogr_route_workspace_bytes(N)) + 4 * N            # and the path buffer
+    full_ws = int(lib.ogr_full_workspace_bytes(N, E))
     qcap = min(N, max(4 * max_roi_nodes, 1 << 18))
-    bfs = min(bfs_slots, max(1, num_nets)) * (4 * N + 4 * 4 * qcap)
-    window = window_slots * (4 * N + 48 * R + 8 * min(R, 65536) * 32 + slot_cap * 4)
+    bfs = int(lib.ogr_bfs_workspace_bytes(N, qcap, min(bfs_slots, max(1, num_nets))))
+    window = 0
+    if window_slots > 0:
+        window = int(lib.ogr_window_workspace_bytes(N, max_roi_nodes, window_slots)) + window_slots * slot_cap * 4
     store = num_nets * (slot_cap * 12 + R * 4 + 24)
     return int(csr + state + roi_ws + full_ws + bfs + window + store + (64 << 20))
 
