@@ -305,6 +305,19 @@ __device__ __forceinline__ void peer_st(unsigned addr, int4 v) {
   asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
                : "memory");
 }
+__device__ __forceinline__ int peer_add(unsigned addr, int v) {
+  int old;
+  asm volatile("atom.relaxed.cluster.shared::cluster.add.s32 %0, [%1], %2;" : "=r"(old) : "r"(addr), "r"(v) : "memory");
+  return old;
+}
+__device__ __forceinline__ void peer_min(unsigned addr, int v) {
+  int old;
+  asm volatile("atom.relaxed.cluster.shared::cluster.min.s32 %0, [%1], %2;" : "=r"(old) : "r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ void peer_max(unsigned addr, int v) {
+  int old;
+  asm volatile("atom.relaxed.cluster.shared::cluster.max.s32 %0, [%1], %2;" : "=r"(old) : "r"(addr), "r"(v) : "memory");
+}
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
 }
@@ -315,7 +328,7 @@ static_assert(kBfsCtas == 8, "three bits of the hash");
 // Bidirectional BFS from src/dst on a box in shared memory; writes the ROI
 // (ascending id, truncated with the must-keep swap) into out[0..out_cap) and
 // its size into sh.R.  False: the search left the box (the caller takes
-// roi_build_large; of a cluster, its first CTA).
+// roi_build_large).
 //
 // Both terminals' waves go on together.  A cell that both find in one step
 // goes to one queue only: the ROI is what either has seen, the cell's
@@ -640,17 +653,45 @@ __device__ bool roi_build_box(Shared& sh, const ogr_graph& g, const ogr_net_args
 // entry, restored to zero on exit) with queues of qcap entries; writes the ROI (ascending id,
 // truncated with the must-keep swap) into out[0..out_cap) and its size into
 // sh.R.  sh.status = OGR_ERR_CAPACITY when a queue overflowed.
+//
+// kCluster: by the kBfsCtas CTAs of a cluster, the counts and flags in the
+// first one's sh (400x300x20, two ROIs of 200,000 nodes: 4.3 ms; by the
+// first CTA alone 19.3; by one of 1,024 threads, before there was a box to try
+// first, 9.5).
+template <bool kCluster>
 __device__ __noinline__ void roi_build_large(Shared& sh, const ogr_graph& g, const ogr_net_args& a, int32_t* seen, int32_t* const* q,
-                          int64_t qcap, int32_t* out, int32_t out_cap, StageClock& clk) {
+                          int64_t qcap, int32_t* out, int32_t out_cap, char* smem, StageClock& clk, int rank) {
   const int tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5, nt = blockDim.x, nw = nt >> 5, groups = nt / kSub;
-  const int sl = tid & (kSub - 1), grp = tid / kSub;
+  const int lane = tid & 31, warp = tid >> 5, nt = blockDim.x, nw = nt >> 5;
+  const int ctas = kCluster ? kBfsCtas : 1;
+  const int sl = tid & (kSub - 1), grp = (rank * nt + tid) / kSub, groups = ctas * nt / kSub;
   const int nx = g.nx, nz = g.nz;
   const int32_t plane = nx * g.ny;
   const int32_t src = a.src, dst = a.dst;
   const int32_t* __restrict__ indptr = g.indptr;
   const int32_t* __restrict__ indices = g.indices;
-  if (tid == 0) {
+  auto sync_all = [&]() {
+    if constexpr (kCluster) cluster_sync();
+    else __syncthreads();
+  };
+  // a word of the first CTA's sh
+  auto get = [&](int& x) -> int {
+    if constexpr (kCluster) return (int)peer_ld(peer_addr(&x, 0));
+    else return x;
+  };
+  auto add = [&](int& x, int v) -> int {
+    if constexpr (kCluster) return peer_add(peer_addr(&x, 0), v);
+    else return atomicAdd(&x, v);
+  };
+  auto lower = [&](int& x, int v) {
+    if constexpr (kCluster) peer_min(peer_addr(&x, 0), v);
+    else atomicMin(&x, v);
+  };
+  auto raise = [&](int& x, int v) {
+    if constexpr (kCluster) peer_max(peer_addr(&x, 0), v);
+    else atomicMax(&x, v);
+  };
+  if (tid == 0 && rank == 0) {
     seen[src] = 1;
     seen[dst] = 2;
     q[0][0] = src;
@@ -667,30 +708,35 @@ __device__ __noinline__ void roi_build_large(Shared& sh, const ogr_graph& g, con
     sh.pos_src = -1;
     sh.pos_dst = -1;
   }
-  __syncthreads();
+  sync_all();
   int depth = 0, meet = -1;
   int cur_s = 0, cur_d = 2;
-  while (depth < a.bfs_max_depth && (sh.nq[cur_s] > 0 || sh.nq[cur_d] > 0)) {
+  while (depth < a.bfs_max_depth && (get(sh.nq[cur_s]) > 0 || get(sh.nq[cur_d]) > 0)) {
     for (int wave = 0; wave < 2; ++wave) {
       const int cur = wave == 0 ? cur_s : cur_d;
       const int nxt = cur ^ 1;
       const int32_t mark = wave == 0 ? 1 : 2;
-      if (tid == 0) sh.nq[nxt] = 0;
-      __syncthreads();
-      const int n = (int)min((int64_t)sh.nq[cur], qcap);
+      if (tid == 0 && rank == 0) sh.nq[nxt] = 0;
+      sync_all();
+      const int n = (int)min((int64_t)get(sh.nq[cur]), qcap);
       const int32_t* qc = q[cur];
       int32_t* qn = q[nxt];
       int local_met = 0, local_new = 0, local_ovf = 0;
       int lx0 = 1 << 30, lx1 = -1, ly0 = 1 << 30, ly1 = -1;
       for (int i = grp; i < n; i += groups) {
-        const int32_t u = qc[i];
+        const int32_t u = __ldcg(&qc[i]);
         const int32_t e1 = indptr[u + 1];
         for (int32_t e = indptr[u] + sl; e < e1; e += kSub) {
           if (g.blocked != nullptr && g.blocked[e]) continue;
           const int32_t v = indices[e];
           const int32_t old = atomicCAS(&seen[v], 0, mark);
           if (old == 0) {
-            const int pos = atomicAdd(&sh.nq[nxt], 1);
+            // (one count for the lanes that are here together)
+            const unsigned here = __activemask();
+            const int first = __ffs(here) - 1;
+            int pos = 0;
+            if (lane == first) pos = add(sh.nq[nxt], __popc(here));
+            pos = __shfl_sync(here, pos, first) + __popc(here & ((1u << lane) - 1u));
             if (pos < qcap) qn[pos] = v; else local_ovf = 1;
             ++local_new;
             const int32_t r = v % plane;
@@ -703,6 +749,7 @@ __device__ __noinline__ void roi_build_large(Shared& sh, const ogr_graph& g, con
           }
         }
       }
+      __syncwarp();
       local_new = __reduce_add_sync(0xffffffffu, local_new);
       local_met = __reduce_or_sync(0xffffffffu, local_met);
       local_ovf = __reduce_or_sync(0xffffffffu, local_ovf);
@@ -711,35 +758,37 @@ __device__ __noinline__ void roi_build_large(Shared& sh, const ogr_graph& g, con
       ly0 = __reduce_min_sync(0xffffffffu, ly0);
       ly1 = __reduce_max_sync(0xffffffffu, ly1);
       if (lane == 0) {
-        if (local_met) sh.met = 1;
-        if (local_ovf) sh.overflow = 1;
+        if (local_met) raise(sh.met, 1);
+        if (local_ovf) raise(sh.overflow, 1);
         if (local_new) {
-          atomicAdd(&sh.seen_count, local_new);
-          atomicMin(&sh.bx0, lx0); atomicMax(&sh.bx1, lx1);
-          atomicMin(&sh.by0, ly0); atomicMax(&sh.by1, ly1);
+          add(sh.seen_count, local_new);
+          lower(sh.bx0, lx0); raise(sh.bx1, lx1);
+          lower(sh.by0, ly0); raise(sh.by1, ly1);
         }
       }
-      __syncthreads();
+      sync_all();
       if (wave == 0) cur_s = nxt; else cur_d = nxt;
     }
     ++depth;
-    if (tid == 0) atomicAdd(&g_stage[11], 2ull);
-    if (sh.met && meet < 0) meet = depth;
+    if (tid == 0 && rank == 0) atomicAdd(&g_stage[11], 2ull);
+    if (get(sh.met) && meet < 0) meet = depth;
     if (meet >= 0 && depth >= meet + a.bfs_halo) break;
-    if ((double)sh.seen_count > a.bfs_stop_count) break;
-    if (sh.overflow) break;
+    if ((double)get(sh.seen_count) > a.bfs_stop_count) break;
+    if (get(sh.overflow)) break;
   }
-  __syncthreads();
-  clk.mark(0);
-  // Ordered compaction over the bounding box (ascending global id): each warp
-  // owns a contiguous segment; count, scan the counts, then write.  Only
+  sync_all();
+  if (rank == 0) clk.mark(0);
+  // Ordered compaction over the bounding box (ascending global id): each CTA,
+  // in it each warp, owns a contiguous segment; count, scan the counts, then write.  Only
   // positions below out_cap are stored; those of src and dst are recorded.
-  const int W = sh.bx1 - sh.bx0 + 1, H = sh.by1 - sh.by0 + 1;
+  const int bx0 = get(sh.bx0), by0 = get(sh.by0);
+  const int W = get(sh.bx1) - bx0 + 1, H = get(sh.by1) - by0 + 1;
   const int32_t area = W * H;
   const int32_t V = area * nz;
-  const int32_t seg = (((V + nw - 1) / nw) + 31) & ~31;
-  const int32_t w0 = warp * seg, w1 = min(V, w0 + seg);
-  const int bx0 = sh.bx0, by0 = sh.by0;
+  const int32_t share = kCluster ? ((V + ctas - 1) / ctas + 31) & ~31 : V;
+  const int32_t c0 = kCluster ? min((int64_t)V, (int64_t)rank * share) : 0, c1 = min((int64_t)V, (int64_t)c0 + share);
+  const int32_t seg = (((c1 - c0 + nw - 1) / nw) + 31) & ~31;
+  const int32_t w0 = c0 + min((int64_t)(c1 - c0), (int64_t)warp * seg), w1 = min((int64_t)c1, (int64_t)w0 + seg);
   auto gid_of = [&](int32_t i) -> int32_t {
     const int z = i / area;
     const int32_t rem = i - z * area;
@@ -750,7 +799,7 @@ __device__ __noinline__ void roi_build_large(Shared& sh, const ogr_graph& g, con
   int cnt = 0;
   for (int32_t b = w0; b < w1; b += 32) {
     const int32_t i = b + lane;
-    const bool f = i < w1 && seen[gid_of(i)] != 0;
+    const bool f = i < w1 && __ldcg(&seen[gid_of(i)]) != 0;
     cnt += __popc(__ballot_sync(0xffffffffu, f));
   }
   if (lane == 0) sh.s_cnt[warp] = cnt;
@@ -764,40 +813,59 @@ __device__ __noinline__ void roi_build_large(Shared& sh, const ogr_graph& g, con
       if (lane >= o) x += y;
     }
     if (lane < nw) sh.s_off[lane] = x - c;
+    x = __shfl_sync(0xffffffffu, x, 31);
     if (lane == 31) sh.R = x;
+    if constexpr (kCluster) {
+      BfsMail& mail = *reinterpret_cast<BfsMail*>(smem);
+      if (lane < kBfsCtas) peer_st(peer_addr(&mail.in[0][rank], lane), make_int4(x, 0, 0, 0));
+    }
   }
-  __syncthreads();
+  sync_all();
   int off = sh.s_off[warp];
+  if constexpr (kCluster) {
+    const BfsMail& mail = *reinterpret_cast<const BfsMail*>(smem);
+    int all = 0;
+    for (int k = 0; k < kBfsCtas; ++k) {
+      if (k == rank) off += all;
+      all += mail.in[0][k].x;
+    }
+    if (tid == 0) sh.R = all;
+  }
   for (int32_t b = w0; b < w1; b += 32) {
     const int32_t i = b + lane;
     int32_t gid = 0;
     bool f = false;
     if (i < w1) {
       gid = gid_of(i);
-      f = seen[gid] != 0;
+      f = __ldcg(&seen[gid]) != 0;
     }
     const unsigned m = __ballot_sync(0xffffffffu, f);
     if (f) {
       const int pos = off + __popc(m & ((1u << lane) - 1));
       if (pos < out_cap) out[pos] = gid;
-      if (gid == src) sh.pos_src = pos;
-      if (gid == dst) sh.pos_dst = pos;
+      if constexpr (kCluster) {
+        if (gid == src) peer_st(peer_addr(&sh.pos_src, 0), pos);
+        if (gid == dst) peer_st(peer_addr(&sh.pos_dst, 0), pos);
+      } else {
+        if (gid == src) sh.pos_src = pos;
+        if (gid == dst) sh.pos_dst = pos;
+      }
     }
     off += __popc(m);
   }
-  __syncthreads();
-  roi_finish(sh, a, out, out_cap);
+  sync_all();
+  if (rank == 0) roi_finish(sh, a, out, out_cap);
   // restore seen[] to zero over the bounding box
-  for (int32_t i = tid; i < V; i += nt) seen[gid_of(i)] = 0;
+  for (int32_t i = c0 + tid; i < c1; i += nt) seen[gid_of(i)] = 0;
   __syncthreads();
-  clk.mark(1);
+  if (rank == 0) clk.mark(1);
 }
 
 __device__ void roi_build(Shared& sh, const ogr_graph& g, const ogr_net_args& a, int32_t* seen, int32_t* const* q,
                           int64_t qcap, int32_t* out, int32_t out_cap, char* smem, StageClock& clk) {
   if (roi_build_box<false, 2, 6>(sh, g, a, q, qcap, out, out_cap, smem, clk, 0)) return;
   __syncthreads();
-  roi_build_large(sh, g, a, seen, q, qcap, out, out_cap, clk);
+  roi_build_large<false>(sh, g, a, seen, q, qcap, out, out_cap, smem, clk, 0);
 }
 
 // The same by a cluster of kBfsCtas CTAs (rank: this one's); the result is in
@@ -808,9 +876,9 @@ __device__ void roi_build_cluster(Shared& sh, const ogr_graph& g, const ogr_net_
   clk.start();
   if (threadIdx.x == 0) sh.status = OGR_OK;
   __syncthreads();
-  if (roi_build_box<true, 4, 4>(sh, g, a, w.q, w.qcap, out, out_cap, smem, clk, rank) || rank != 0) return;
+  if (roi_build_box<true, 4, 4>(sh, g, a, w.q, w.qcap, out, out_cap, smem, clk, rank)) return;
   __syncthreads();
-  roi_build_large(sh, g, a, w.seen, w.q, w.qcap, out, out_cap, clk);
+  roi_build_large<true>(sh, g, a, w.seen, w.q, w.qcap, out, out_cap, smem, clk, rank);
 }
 
 // ---- the search on a given ROI ---------------------------------------------------
