@@ -51,6 +51,7 @@ constexpr int kMaxSkip = 16;                   // nets a window may skip over (l
 // ROI of 50,000 nodes on 600x400x12: 8.7 us with 8 CTAs, 6.5 with 16, 5.3
 // with 32, 4.5 with 76 and with 152; ROIs of 14,000 nodes: 4.4, 3.9, 3.8, 3.7.
 constexpr int kTeam = 76;
+constexpr int kLoneNodes = 512;                // below it one CTA
 
 // Control words of one search slot, kept between searches (sid) or zero at
 // the start of each (team).
@@ -570,18 +571,32 @@ __device__ bool roi_build_box(Shared& sh, const ogr_graph& g, const ogr_net_args
   }
   __syncthreads();
   if (rank == 0) clk.mark(0);
-  // Ordered compaction (ascending global id): each CTA, in it each warp, owns
-  // a contiguous run of words; count, scan the counts, then write.  Only
-  // positions below out_cap are stored; those of src and dst are recorded.
-  const Div by_rw((unsigned)RW), by_bh((unsigned)BH);
+  // Ordered compaction (ascending global id) of the words within `depth` cells
+  // of the terminals' rectangle (beyond it nothing is marked): each CTA, in it
+  // each warp, owns a contiguous run of them; count, scan the counts, then write.
+  // Only positions below out_cap are stored; those of src and dst are recorded.
+  const int cy0 = max(0, min(sy, dy) - Y0 - depth), cy1 = min(BH - 1, max(sy, dy) - Y0 + depth);
+  const int cx0 = max(0, min(sx, dx) - X0 - depth) >> 4, cx1 = min(BW - 1, max(sx, dx) - X0 + depth) >> 4;
+  const Div by_rw((unsigned)(cx1 - cx0 + 1)), by_bh((unsigned)(cy1 - cy0 + 1));
+  const int words = (int)(by_rw.d * by_bh.d) * nz;
+  // layer, row and column of the box of the i-th of these words
+  auto place = [&](int i, int& z, int& y, int& c) {
+    const unsigned row = by_rw((unsigned)i), zz = by_bh(row);
+    z = (int)zz;
+    y = cy0 + (int)(row - zz * by_bh.d);
+    c = cx0 + (int)((unsigned)i - row * by_rw.d);
+  };
   auto cells = [&](int i) -> unsigned {        // the low bit of each seen cell
+    int z, y, c;
+    place(i, z, y, c);
+    const int at = (z * BH + y) * RW + c;
     unsigned w;
-    if constexpr (kCluster) w = peer_ld(peer_addr(&marks[i], bfs_owner(i)));
-    else w = marks[i];
+    if constexpr (kCluster) w = peer_ld(peer_addr(&marks[at], bfs_owner(at)));
+    else w = marks[at];
     return (w | w >> 1) & 0x55555555u;
   };
-  const int share = kCluster ? ((NW + kBfsCtas - 1) / kBfsCtas + 31) & ~31 : NW;
-  const int c0 = kCluster ? min(NW, rank * share) : 0, c1 = min(NW, c0 + share);
+  const int share = kCluster ? ((words + kBfsCtas - 1) / kBfsCtas + 31) & ~31 : words;
+  const int c0 = kCluster ? min(words, rank * share) : 0, c1 = min(words, c0 + share);
   const int per = ((c1 - c0 + nw - 1) / nw + 31) & ~31;
   const int w0 = c0 + warp * per, w1 = min(c1, w0 + per);
   int cnt = 0;
@@ -625,10 +640,10 @@ __device__ bool roi_build_box(Shared& sh, const ogr_graph& g, const ogr_net_args
       const bool in = __shfl_sync(0xffffffffu, word, k) >> (2 * (lane & 15)) & 1u;
       const unsigned b = __ballot_sync(0xffffffffu, in);
       if (in) {
-        const unsigned row = by_rw((unsigned)(i0 + k)), z = by_bh(row);
+        int z, y, c;
+        place(i0 + k, z, y, c);
         const int pos = off + __popc(b & ((1u << lane) - 1u));
-        const int32_t gid = (int32_t)(z * by_plane.d + (unsigned)(Y0 + (int)(row - z * by_bh.d)) * by_nx.d) + X0 +
-                            16 * (int)(i0 + k - row * by_rw.d) + (lane & 15);
+        const int32_t gid = z * plane + (Y0 + y) * nx + X0 + 16 * c + (lane & 15);
         if (pos < out_cap) out[pos] = gid;
         if constexpr (kCluster) {
           if (gid == src) peer_st(peer_addr(&sh.pos_src, 0), pos);
@@ -1390,8 +1405,14 @@ find_team_kernel(ogr_graph g, ogr_state st, ogr_net_args a, Ws w, const int32_t*
     roi = w.roi;
     R = (int32_t)w.result[3];
   }
+  // A ROI of a few hundred nodes is searched by the first CTA alone, which has
+  // no barrier to wait at: given ROIs of 98, 210 and 362 nodes of 100x100x6 take
+  // 46, 58 and 63 us instead of 52, 60 and 72; of 567 and 1,071 a team takes 77
+  // and 96, one CTA 83 and 109.
+  const int team = R < kLoneNodes ? 1 : (int)gridDim.x;
+  if ((int)blockIdx.x >= team) return;
   const RoiJob job{&g,       &st,      &a,    &w, roi, R, roi_pen, &ms, path_out, path_cap,
-                   reinterpret_cast<unsigned long long*>(stats), (int)blockIdx.x, (int)gridDim.x};
+                   reinterpret_cast<unsigned long long*>(stats), (int)blockIdx.x, team};
   int status, len;
   roi_search_row<ROW, kMulti>(job, smem, &status, &len);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
