@@ -422,7 +422,7 @@ def run_ours(args, cfg, rank, world):
                                      "lattice, scaled by the algorithmic bytes)" if cfg.get("traffic_ratio")
                                      else None,
                      "kernel": "search launches of the routing pass (full_sssp_kernel on all SMs for "
-                               "full-graph nets, route_pass_kernel / roi_batch_kernel for ROI nets)",
+                               "full-graph nets, window_pass_kernel / roi_batch_kernel for ROI nets)",
                      "peak_kind": pk_kind,
                      "algorithmic_bytes": "24 B per arc scanned + 20 B per node popped by the sequential search"},
         "e2e": {"value": round(float(np.median(e2e_t)), 6), "unit": "s/job",

@@ -21,6 +21,17 @@ static inline int ogr_blocks(int64_t n, int threads, int cap = 152 * 16) {
   return (int)b;
 }
 
+// Division by a fixed d > 0 of any v < 2^32: the high product with
+// floor(2^32 / d) is the quotient or one less.
+struct OgrDiv {
+  unsigned d, m;
+  __device__ explicit OgrDiv(unsigned dd) : d(dd), m(dd > 1 ? (unsigned)((1ull << 32) / dd) : 0xffffffffu) {}
+  __device__ unsigned operator()(unsigned v) const {
+    const unsigned q = __umulhi(v, m);
+    return v - q * d >= d ? q + 1 : q;
+  }
+};
+
 // Non-negative doubles order like their bit patterns as unsigned integers.
 __device__ __forceinline__ unsigned long long ogr_dbits(double d) {
   return (unsigned long long)__double_as_longlong(d);

@@ -41,17 +41,6 @@ __device__ __forceinline__ bool site_ok(int mode, int x, int y) {
   return (x % mode) == 0 && (y % mode) == 0;
 }
 
-// Division by a fixed d > 0 of any v < 2^32 (the high product with
-// floor(2^32 / d) is the quotient or one less).
-struct Div {
-  unsigned d, m;
-  __device__ explicit Div(unsigned dd) : d(dd), m(dd > 1 ? (unsigned)((1ull << 32) / dd) : 0xffffffffu) {}
-  __device__ unsigned operator()(unsigned v) const {
-    const unsigned q = __umulhi(v, m);
-    return v - q * d >= d ? q + 1 : q;
-  }
-};
-
 // Whether layer z has arcs along x / along y, and their costs.
 struct Axes {
   bool h, v;
@@ -153,7 +142,7 @@ __device__ __forceinline__ int block_scan(int v, int* s_warp, int* total) {
 
 __global__ void __launch_bounds__(kScanThreads) scan_tiles(LatDev L, int64_t N, int32_t* out, int32_t* tile_sums) {
   __shared__ int s_warp[32];
-  const Div by_plane((unsigned)(L.h.nx * L.h.ny)), by_nx((unsigned)L.h.nx);
+  const OgrDiv by_plane((unsigned)(L.h.nx * L.h.ny)), by_nx((unsigned)L.h.nx);
   const int64_t i0 = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanPer;
   int d[kScanPer], sum = 0;
 #pragma unroll
@@ -216,7 +205,7 @@ __global__ void __launch_bounds__(kFillThreads) fill_kernel(LatDev L, int tile_n
   const int nx = L.h.nx, ny = L.h.ny, z = blockIdx.y;
   const int32_t plane = nx * ny;
   const Axes ax(L.h, z);
-  const Div by_nx((unsigned)nx);
+  const OgrDiv by_nx((unsigned)nx);
   const int p0 = L.h.pptr[z], p1 = L.h.pptr[z + 1];
   for (int64_t t0 = (int64_t)blockIdx.x * tile_nodes; t0 < plane; t0 += (int64_t)gridDim.x * tile_nodes) {
     const int32_t r0 = (int32_t)t0, r1 = (int32_t)min((int64_t)plane, t0 + tile_nodes);

@@ -252,17 +252,6 @@ __device__ void roi_finish(Shared& sh, const ogr_net_args& a, int32_t* out, int3
   atomicAdd(&g_stage[12], (unsigned long long)R);
 }
 
-// Division by a fixed d > 0 of any v < 2^32: the high product with
-// floor(2^32 / d) is the quotient or one less.
-struct Div {
-  unsigned d, m;
-  __device__ explicit Div(unsigned dd) : d(dd), m(dd > 1 ? (unsigned)((1ull << 32) / dd) : 0xffffffffu) {}
-  __device__ unsigned operator()(unsigned v) const {
-    const unsigned q = __umulhi(v, m);
-    return v - q * d >= d ? q + 1 : q;
-  }
-};
-
 // Shared memory of a BFS: the mail of a cluster's CTAs, two queues (this wave's
 // and the next one's), then the marks of the box around both terminals, two
 // bits a cell (1: seen from src, 2: from dst; both: where the waves met).
@@ -358,7 +347,7 @@ __device__ bool roi_build_box(Shared& sh, const ogr_graph& g, const ogr_net_args
   const int32_t src = a.src, dst = a.dst, plane = nx * ny;
   const int32_t* __restrict__ indptr = g.indptr;
   const int32_t* __restrict__ indices = g.indices;
-  const Div by_plane((unsigned)(nx * ny)), by_nx((unsigned)nx);
+  const OgrDiv by_plane((unsigned)(nx * ny)), by_nx((unsigned)nx);
   BfsMail& mail = *reinterpret_cast<BfsMail*>(smem);
   int32_t* sq = reinterpret_cast<int32_t*>(smem + kBfsHead);
   unsigned* marks = reinterpret_cast<unsigned*>(smem + kBfsBitsAt);
@@ -577,7 +566,7 @@ __device__ bool roi_build_box(Shared& sh, const ogr_graph& g, const ogr_net_args
   // Only positions below out_cap are stored; those of src and dst are recorded.
   const int cy0 = max(0, min(sy, dy) - Y0 - depth), cy1 = min(BH - 1, max(sy, dy) - Y0 + depth);
   const int cx0 = max(0, min(sx, dx) - X0 - depth) >> 4, cx1 = min(BW - 1, max(sx, dx) - X0 + depth) >> 4;
-  const Div by_rw((unsigned)(cx1 - cx0 + 1)), by_bh((unsigned)(cy1 - cy0 + 1));
+  const OgrDiv by_rw((unsigned)(cx1 - cx0 + 1)), by_bh((unsigned)(cy1 - cy0 + 1));
   const int words = (int)(by_rw.d * by_bh.d) * nz;
   // layer, row and column of the box of the i-th of these words
   auto place = [&](int i, int& z, int& y, int& c) {
