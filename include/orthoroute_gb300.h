@@ -224,7 +224,9 @@ typedef struct {
   const int32_t* rev;
   const uint8_t* blocked;      /* NULL: none */
   int32_t max_row;             /* arcs of the longest row, 0: not told.  Chooses the
-                                  form of the search; results do not depend on it */
+                                  form of the search; results do not depend on it.
+                                  (Newer than the fields above: callers are to be
+                                  compiled against this header) */
 } ogr_graph;
 
 typedef struct {
